@@ -69,6 +69,17 @@ FitParams make_fit_params(const mars_params& p) {
     fp.a_min = af;
     fp.two_a = 2.0f * af;
     fp.a_half = 0.5f * af;
+    int exponent = 0;
+    fp.inv_max_alfa = std::frexp(p.max_alfa, &exponent) == 0.5 && std::abs(exponent) < 1000
+                          ? 1.0 / p.max_alfa
+                          : 0.0;
+    const double top = std::max(a, p.max_alfa - a);
+    float lo = (float)top, hi = (float)top;
+    if ((double)lo > top) lo = std::nextafter(lo, 0.0f);
+    if ((double)hi < top) hi = std::nextafter(hi, INFINITY);
+    fp.a_max = hi;
+    fp.max_half = 0.5f * lo;
+    fp.min_over_max = std::nextafter(fp.a_min / hi, 0.0f);
     fp.eta_per_n = 1e-6 * (1.0 + p.max_alfa) * (1.0 + p.max_alfa);
     return fp;
 }
@@ -340,166 +351,221 @@ bool make_digit_maps(mars_ctx* ctx, const uint8_t* d_digits, uint32_t w, uint32_
 }
 
 // A tensor-core level set up for its correlation: buffers taken from a Scratch, tensor
-// maps, split count, and the coarse pre-pass of block size 8.
+// maps and split count.
 struct TcLevel {
     mars::LevelGeom g{};
     size_t n = 0;
-    bool digits = false;
+    mars::tc::Path path = mars::tc::kFold;
     int msplit = 1;
     mars::RangeStats rs{};
     mars::DomainStats ds{};
-    uint8_t* d_phases = nullptr;
+    uint8_t* d_a = nullptr;  // phase or digit planes, or the unit form's A operand
     uint8_t* d_b = nullptr;
     mars::tc::SeedOut* d_seed = nullptr;
     mars::tc::TcMaps maps{};
+    mars::tc::UnitSource unit{};
+    uint32_t *d_domains = nullptr, *d_ranges = nullptr, *d_bins = nullptr;  // unit form
+    float2* d_contrasts = nullptr;
     mars::Partial* partials = nullptr;
     unsigned long long* gch = nullptr;
     int* tickets = nullptr;  // all-levels launch only
     int32_t* dtmp = nullptr;  // the separable domain statistics' scratch (all-levels launch)
-    int* coarse_tickets = nullptr;  // all-levels launch: the in-kernel coarse pre-pass
-    int* ready = nullptr;
     int tail_tiles = 0, tail_msplit = 0;  // all-levels launch: the finer-split tail
-    bool coarse = false;
-    mars::LevelGeom g1{};
-    mars::DomainStats ds1{};
-    uint8_t* d_ph1 = nullptr;
-    mars::tc::TcMaps maps1{};
-    int ms1 = 1;
-    mars::Partial* part1 = nullptr;
 };
 
 // The separable domain statistics take scratch up to this many words (256 MiB); larger
 // levels use the direct kernel.
 constexpr size_t kDomainTmpWords = 64ull << 20;
 
-// Whether a level takes the split-digit operand (block sizes 16..64 unless pinned off).
-bool tc_digits(const mars_ctx* ctx, const mars::LevelGeom& g) {
-    return mars::tc::digits_supported(g.size, g.shift) && !ctx->tma_16_boxes && !ctx->fold_only;
+// The unit form's A operand holds every domain window (32 or 128 bytes a position at sizes 4 and
+// 8), up to this many bytes a level: planes to about 11,500 pixels a side at size 8, stride 2.
+// Beyond it the fold reads the windows from copies of the plane.
+constexpr size_t kUnitBytes = 4ull << 30;
+// Its work items cost 25,000 cycles to set up, preview and drain, the fold's about 6,000, and its
+// operands eight more launches: levels of fewer tiles (128 domains x 32 ranges) than this keep
+// the fold.  (One level from host memory, 384 x 256 at size 8, 8,400 tiles: 358 us on the fold,
+// 449 in the unit form; 512 x 512 at size 8, 62,000 tiles: 845 and 660 us.)  MARS_UNIT_TILES
+// overrides it (0: the unit form wherever it applies).
+constexpr size_t kUnitTiles = 16384;
+size_t unit_tiles() {
+    const char* e = std::getenv("MARS_UNIT_TILES");
+    return e && *e ? (size_t)std::strtoull(e, nullptr, 10) : kUnitTiles;
 }
 
-// Coarse pre-pass at block size 8: the same search over every 4th domain position of each
-// axis, whose champions seed the full sweep (tighter thresholds from the first tile: exact
-// fits of the 512x512 level 1.09 M -> 0.23 M, 0.98 -> 0.86 ms).  At size 4 its cost
-// outweighs the survivors it saves, and at 16..64 it is neutral or slower.
-constexpr int kCoarseRatio = 4;
-constexpr size_t kCoarseAllLevels = 65536;
+// Which form serves a level of n ranges: unit vectors at sizes 4 and 8 (512 x 512, stride 2: the
+// whole step 3.70 -> 2.35 ms; 1024 x 1024: 49.8 -> 27.3), the contracted plane's digits above, the
+// fold for small levels and where the others are pinned off (mars_ctx_set_search_path 3, 4).
+mars::tc::Path tc_path(const mars_ctx* ctx, const mars::LevelGeom& g, size_t n) {
+    if (ctx->tma_16_boxes || ctx->fold_only) return mars::tc::kFold;
+    if (mars::tc::unit_supported(g.size, g.shift) && mars::tc::unit_a_bytes(g) <= kUnitBytes) {
+        const size_t tiles = (size_t)mars::tc::domain_tiles(g, mars::tc::kUnit) * ((n + 31) / 32);
+        if (tiles >= unit_tiles()) return mars::tc::kUnit;
+    }
+    return mars::tc::digits_supported(g.size, g.shift) ? mars::tc::kDigits : mars::tc::kFold;
+}
 
-// Buffers and tensor maps of a level (g, rs and ds already set).  msplit 0 picks the
-// per-level launch's split count; tickets adds the all-levels launch's per-tile counters;
-// coarse_ok allows the coarse pre-pass.  The all-levels launch keeps it for large levels
-// only (kCoarseAllLevels ranges and up): the pre-pass sits on the path before the one
-// launch, where at 512 x 512 it costs 0.16 ms, more than the 0.12 ms of correlation it
-// saves; on large planes it is a small part of the step and cuts the level's exact fits.
-// A level whose digit views the driver rejects takes the fold path (L.digits false).
+// Buffers and tensor maps of a level (g, rs and ds already set) in form `path`.  msplit 0 picks
+// the per-level launch's split count; tickets adds the all-levels launch's per-tile counters.
+// A level whose digit views the driver rejects takes the fold path (L.path kFold).
 int tc_level_setup(mars_ctx* ctx, Scratch& sc, uint32_t w, uint32_t h, size_t n, int msplit,
-                   bool tickets, bool coarse_ok, TcLevel& L) {
+                   bool tickets, mars::tc::Path path, TcLevel& L) {
     const mars::LevelGeom& g = L.g;
     L.n = n;
-    L.digits = tc_digits(ctx, g);
-    if (L.digits) {
-        MARS_CUDA(sc.get(&L.d_phases, mars::tc::digit_plane_bytes((int)w, (int)h, g.shift)));
-        L.digits = make_digit_maps(ctx, L.d_phases, w, h, (uint32_t)g.shift, &L.maps);
+    L.path = path;
+    if (L.path == mars::tc::kUnit) {
+        MARS_CUDA(sc.get(&L.d_a, mars::tc::unit_a_bytes(g)));
+        MARS_CUDA(sc.get(&L.d_domains, (size_t)g.nrow_d * g.ncol_d));
+        MARS_CUDA(sc.get(&L.d_ranges, n));
+        MARS_CUDA(sc.get(&L.d_bins, 2 * mars::tc::unit_bins_words()));
+        MARS_CUDA(sc.get(&L.d_contrasts, (size_t)mars::tc::domain_tiles(g, L.path)));
+    } else if (L.path == mars::tc::kDigits) {
+        MARS_CUDA(sc.get(&L.d_a, mars::tc::digit_plane_bytes((int)w, (int)h, g.shift)));
+        if (!make_digit_maps(ctx, L.d_a, w, h, (uint32_t)g.shift, &L.maps)) L.path = mars::tc::kFold;
     }
-    if (!L.digits) {
-        MARS_CUDA(sc.get(&L.d_phases, mars::tc::phase_bytes((int)w, (int)h, g.shift)));
-        if (int e = make_maps(ctx, L.d_phases, w, h, (uint32_t)g.shift, &L.maps)) return e;
+    if (L.path == mars::tc::kFold) {
+        MARS_CUDA(sc.get(&L.d_a, mars::tc::phase_bytes((int)w, (int)h, g.shift)));
+        if (int e = make_maps(ctx, L.d_a, w, h, (uint32_t)g.shift, &L.maps)) return e;
     }
-    MARS_CUDA(sc.get(&L.d_b, mars::tc::b_bytes(g.size, (int)n, L.digits)));
+    MARS_CUDA(sc.get(&L.d_b, mars::tc::b_bytes(g.size, (int)n, L.path)));
     MARS_CUDA(sc.get(&L.d_seed, n));
-    L.msplit = msplit > 0 ? msplit : mars::tc::msplit_for(g, (int)n, ctx->num_sms, L.digits);
+    L.msplit = msplit > 0 ? msplit : mars::tc::msplit_for(g, (int)n, ctx->num_sms, L.path);
     MARS_CUDA(sc.get(&L.partials, (size_t)L.msplit * n));
     // The M-splits' shared champion records (rms bits, index, t1_x4).
     MARS_CUDA(sc.get(&L.gch, 2 * n));
     if (tickets) {
-        const int rt = mars::tc::ranges_per_tile(L.digits);
+        const int rt = mars::tc::ranges_per_tile(L.path);
         MARS_CUDA(sc.get(&L.tickets, (n + rt - 1) / rt));
-    }
-    L.coarse = false;
-    if (coarse_ok && !L.digits && g.size == 8 && g.shift * kCoarseRatio <= 16 && n >= 256) {
-        L.g1 = level_geom(w, h, (uint32_t)g.size, (uint32_t)(g.shift * kCoarseRatio));
-        if (L.g1.nrow_d > 0 && L.g1.ncol_d > 0) {
-            L.coarse = true;
-            const size_t ndom1 = (size_t)L.g1.nrow_d * L.g1.ncol_d;
-            MARS_CUDA(sc.get(&L.ds1.s1x4, ndom1));
-            MARS_CUDA(sc.get(&L.ds1.s2x16, ndom1));
-            MARS_CUDA(sc.get(&L.ds1.detf, ndom1));
-            MARS_CUDA(sc.get(&L.ds1.sdetf, ndom1));
-            MARS_CUDA(sc.get(&L.d_ph1, mars::tc::phase_bytes((int)w, (int)h, L.g1.shift)));
-            if (int e = make_maps(ctx, L.d_ph1, w, h, (uint32_t)L.g1.shift, &L.maps1)) return e;
-            L.ms1 = mars::tc::msplit_for(L.g1, (int)n, ctx->num_sms, false);
-            MARS_CUDA(sc.get(&L.part1, (size_t)L.ms1 * n));
-        }
     }
     return MARS_OK;
 }
 
-// Everything of a level before its correlation, on stream st: phase (or digit phase)
-// copies, the B operand, seed champions, the coarse pre-pass (its statistics and planes
-// only when the all-levels launch runs it: L.ready set), the shared champion records and
-// tickets.
-// st_planes (all-levels launch only): a second stream for the phase planes and the B
-// operand, which do not depend on the statistics the seeds need.
-int tc_level_prep(mars_ctx* ctx, const TcLevel& L, const uint8_t* d_plane, const int32_t* d_D,
+// Everything of a level before its correlation: the statistics, the A operand (planes or unit
+// vectors), the B operand, seed champions, the shared champion records and tickets.  Range-side
+// work and the seeds run on stream st, domain-side work on sp (the same stream, or a second one:
+// `stats_done` then orders the seeds after the domain statistics).
+int tc_level_prep(mars_ctx* ctx, TcLevel& L, const uint8_t* d_plane, const int32_t* d_D,
                   const uint8_t* d_dplane, uint32_t w, uint32_t h, const mars::FitParams& fp,
-                  const uint32_t* d_rows, const uint32_t* d_cols, cudaStream_t st,
-                  cudaStream_t st_planes = nullptr) {
+                  const uint32_t* d_rows, const uint32_t* d_cols, cudaStream_t st, cudaStream_t sp,
+                  cudaEvent_t stats_done) {
     const mars::LevelGeom& g = L.g;
     const int n = (int)L.n;
-    const cudaStream_t sp = st_planes ? st_planes : st;
-    if (L.digits)
-        MARS_CUDA(mars::tc::launch_digit_planes(d_D, (int)w, (int)h, g.shift, L.d_phases, sp));
-    else
-        MARS_CUDA(mars::tc::launch_phase_planes(d_dplane, (int)w, (int)h, g.shift, L.d_phases, sp));
-    MARS_CUDA(mars::tc::launch_build_b(g.size, d_plane, (int)w, (int)h, d_rows, d_cols, n, L.d_b,
-                                       L.digits, sp));
-    MARS_CUDA(mars::tc::launch_seed(d_D, g, d_plane, (int)w, d_rows, d_cols, n, L.rs, L.ds, fp,
-                                    L.d_seed, st));
-    ctx->launches += 3;
-    if (L.coarse) {
-        MARS_CUDA(mars::launch_domain_stats(d_D, L.g1, L.ds1, st));
-        MARS_CUDA(mars::tc::launch_phase_planes(d_dplane, (int)w, (int)h, L.g1.shift, L.d_ph1, sp));
-        ctx->launches += 2;
-        if (L.ready) {
-            const int rt = mars::tc::ranges_per_tile(false);
-            const size_t nt = (L.n + rt - 1) / rt;
-            MARS_CUDA(cudaMemsetAsync(L.ready, 0, nt * sizeof(int), st));
-            MARS_CUDA(cudaMemsetAsync(L.coarse_tickets, 0, nt * sizeof(int), st));
-        } else {
-            MARS_CUDA(mars::tc::launch_corr(L.maps1, L.d_b, L.g1, n, L.rs, L.ds1, fp, L.d_seed,
-                                            L.part1, nullptr, L.ms1, false, ctx->d_err,
-                                            ctx->d_counter, st));
-            MARS_CUDA(mars::tc::launch_seed_merge(L.part1, L.ms1, n, L.g1.ncol_d, g.ncol_d,
-                                                  kCoarseRatio, L.d_seed, st));
-            ctx->launches += 2;
-        }
+    MARS_CUDA(mars::launch_domain_stats(d_D, g, L.ds, sp, L.dtmp));
+    if (sp != st) MARS_CUDA(cudaEventRecord(stats_done, sp));
+    MARS_CUDA(mars::launch_range_stats(d_plane, (int)w, (int)h, d_rows, d_cols, n, g.size, fp, L.rs,
+                                       st));
+    if (L.path == mars::tc::kUnit) {
+        L.unit = mars::tc::UnitSource{L.d_a, L.d_domains, L.d_ranges, L.d_contrasts,
+                                      d_D,   d_plane,     d_rows,     d_cols};
+        MARS_CUDA(mars::tc::launch_unit_a(d_D, g, L.ds, L.d_bins, L.d_domains, L.d_contrasts, L.d_a,
+                                          sp));
+        MARS_CUDA(mars::tc::launch_unit_b(g.size, d_plane, (int)w, (int)h, d_rows, d_cols, n, L.rs,
+                                          L.d_bins + mars::tc::unit_bins_words(), L.d_ranges, L.d_b,
+                                          st));
+        ctx->launches += 5;
+    } else {
+        const bool digits = L.path == mars::tc::kDigits;
+        if (digits)
+            MARS_CUDA(mars::tc::launch_digit_planes(d_D, (int)w, (int)h, g.shift, L.d_a, sp));
+        else
+            MARS_CUDA(mars::tc::launch_phase_planes(d_dplane, (int)w, (int)h, g.shift, L.d_a, sp));
+        MARS_CUDA(mars::tc::launch_build_b(g.size, d_plane, (int)w, (int)h, d_rows, d_cols, n,
+                                           L.d_b, digits, sp));
     }
     MARS_CUDA(cudaMemsetAsync(L.gch, 0xFF, 2 * L.n * sizeof(unsigned long long), st));
     if (L.tickets) {
-        const int rt = mars::tc::ranges_per_tile(L.digits);
+        const int rt = mars::tc::ranges_per_tile(L.path);
         MARS_CUDA(cudaMemsetAsync(L.tickets, 0, (L.n + rt - 1) / rt * sizeof(int), st));
     }
+    if (sp != st) MARS_CUDA(cudaStreamWaitEvent(st, stats_done, 0));
+    MARS_CUDA(mars::tc::launch_seed(d_D, g, d_plane, (int)w, d_rows, d_cols, n, L.rs, L.ds, fp,
+                                    L.d_seed, st));
+    ctx->launches += 5;
     return MARS_OK;
 }
 
+// A level as jobs of the all-levels launch: its range tiles, the last of them with finer splits.
+void add_level_jobs(const TcLevel& L, const mars::FitParams& fp, mars::CandidateOut* out,
+                    std::vector<mars::tc::LevelJob>* jobs) {
+    mars::tc::LevelJob J;
+    J.maps = L.maps;
+    J.bglob = L.d_b;
+    J.g = L.g;
+    J.nranges = (int)L.n;
+    J.rs = L.rs;
+    J.ds = L.ds;
+    J.fp = fp;
+    J.seeds = L.d_seed;
+    J.partials = L.partials;
+    J.gch = L.gch;
+    J.tickets = L.tickets;
+    J.out = out;
+    const int rt = mars::tc::ranges_per_tile(L.path);
+    const int ntiles = (int)((L.n + rt - 1) / rt);
+    J.path = L.path;
+    J.unit = L.unit;
+    J.tile_begin = 0;
+    J.tile_count = ntiles - L.tail_tiles;
+    J.msplit = L.msplit;
+    jobs->push_back(J);
+    if (L.tail_tiles > 0) {
+        J.tile_begin = ntiles - L.tail_tiles;
+        J.tile_count = L.tail_tiles;
+        J.msplit = L.tail_msplit;
+        jobs->push_back(J);
+    }
+}
+
 // The tcgen05 path for one level: set-up, the correlation + exact-bound kernel, and the
-// final champion per block.
+// final champion per block.  The unit form has one kernel, the persistent one of
+// launch_corr_all, which takes the level as its only work.
 int run_level_tc(mars_ctx* ctx, Scratch& sc, const uint8_t* d_plane, const int32_t* d_D,
                  uint32_t w, uint32_t h, const mars::LevelGeom& g, const mars::FitParams& fp,
                  const uint32_t* d_rows, const uint32_t* d_cols, size_t n, mars::RangeStats rs,
-                 mars::DomainStats ds, mars::CandidateOut* d_out, const uint8_t* d_dplane) {
+                 mars::DomainStats ds, int32_t* dtmp, mars::CandidateOut* d_out,
+                 const uint8_t* d_dplane) {
     const cudaStream_t st = ctx->stream;
     TcLevel L;
     L.g = g;
     L.rs = rs;
     L.ds = ds;
-    if (int e = tc_level_setup(ctx, sc, w, h, n, 0, false, true, L)) return e;
-    if (int e = tc_level_prep(ctx, L, d_plane, d_D, d_dplane, w, h, fp, d_rows, d_cols, st))
+    L.dtmp = dtmp;
+    const mars::tc::Path path = tc_path(ctx, g, n);
+    int ms = 0, tail_tiles = 0, tail_ms = 0;
+    if (path == mars::tc::kUnit) {
+        const int nr = (int)n;
+        mars::tc::all_levels_splits(&g, &nr, &path, 1, ctx->num_sms, &ms, &tail_tiles, &tail_ms);
+    }
+    if (int e = tc_level_setup(ctx, sc, w, h, n, std::max(ms, tail_ms), path == mars::tc::kUnit,
+                               path, L))
         return e;
+    if (int e = tc_level_prep(ctx, L, d_plane, d_D, d_dplane, w, h, fp, d_rows, d_cols, st, st,
+                              nullptr))
+        return e;
+    if (L.path == mars::tc::kUnit) {
+        L.msplit = ms;
+        L.tail_tiles = tail_tiles;
+        L.tail_msplit = tail_ms;
+        std::vector<mars::tc::LevelJob> jobs;
+        add_level_jobs(L, fp, d_out, &jobs);
+        int* d_work = nullptr;
+        MARS_CUDA(sc.get(&d_work, 2));
+        MARS_CUDA(cudaMemsetAsync(d_work, 0, 2 * sizeof(int), st));
+        MARS_CUDA(mars::tc::launch_corr_all(jobs.data(), (int)jobs.size(), d_work, ctx->d_err,
+                                            ctx->d_counter, ctx->num_sms, st, st));
+        ctx->launches += 1;
+        return MARS_OK;
+    }
     MARS_CUDA(mars::tc::launch_corr(L.maps, L.d_b, g, (int)n, rs, ds, fp, L.d_seed, L.partials,
-                                    L.gch, L.msplit, L.digits, ctx->d_err, ctx->d_counter, st));
+                                    L.gch, L.msplit, L.path == mars::tc::kDigits, ctx->d_err,
+                                    ctx->d_counter, st));
     MARS_CUDA(mars::tc::launch_finish(L.partials, L.msplit, (int)n, g, rs, ds, fp, d_out, st));
     ctx->launches += 2;
     return MARS_OK;
+}
+
+// Whether a ranked level takes the split-digit operand (block sizes 16..64 unless pinned off).
+bool topk_digits(const mars_ctx* ctx, const mars::LevelGeom& g) {
+    return mars::tc::digits_supported(g.size, g.shift) && !ctx->tma_16_boxes && !ctx->fold_only;
 }
 
 // The ranked search (k = 2..kMaxTopK) of one level on the tcgen05 path: phase (or digit)
@@ -513,7 +579,7 @@ int run_level_tc_topk(mars_ctx* ctx, Scratch& sc, const uint8_t* d_plane, const 
     const cudaStream_t st = ctx->stream;
     uint8_t* d_phases = nullptr;
     mars::tc::TcMaps maps{};
-    bool digits = tc_digits(ctx, g);
+    bool digits = topk_digits(ctx, g);
     if (digits) {
         MARS_CUDA(sc.get(&d_phases, mars::tc::digit_plane_bytes((int)w, (int)h, g.shift)));
         digits = make_digit_maps(ctx, d_phases, w, h, (uint32_t)g.shift, &maps);
@@ -527,9 +593,10 @@ int run_level_tc_topk(mars_ctx* ctx, Scratch& sc, const uint8_t* d_plane, const 
     uint8_t* d_b = nullptr;
     mars::tc::SeedOut* d_seed = nullptr;
     mars::Partial* partials = nullptr;
-    const int msplit = std::min(mars::tc::msplit_for(g, (int)n, ctx->num_sms, digits),
+    const mars::tc::Path path = digits ? mars::tc::kDigits : mars::tc::kFold;
+    const int msplit = std::min(mars::tc::msplit_for(g, (int)n, ctx->num_sms, path),
                                 mars::kMaxTopKSplits);
-    MARS_CUDA(sc.get(&d_b, mars::tc::b_bytes(g.size, (int)n, digits)));
+    MARS_CUDA(sc.get(&d_b, mars::tc::b_bytes(g.size, (int)n, path)));
     MARS_CUDA(sc.get(&d_seed, n * k));
     MARS_CUDA(sc.get(&partials, (size_t)msplit * n * k));
     if (digits)
@@ -581,14 +648,17 @@ int run_level(mars_ctx* ctx, Scratch& sc, const uint8_t* d_plane, const int32_t*
     MARS_CUDA(sc.get(&ds.s2x16, ndom));
     MARS_CUDA(sc.get(&ds.detf, ndom));
     MARS_CUDA(sc.get(&ds.sdetf, ndom));
-    MARS_CUDA(mars::launch_range_stats(d_plane, (int)w, (int)h, d_rows, d_cols, (int)n,
-                                       (int)size, fp, rs, st));
     int32_t* dtmp = nullptr;
     const size_t dwords = mars::domain_stats_tmp_words(g);
     if (dwords > 0 && dwords <= kDomainTmpWords) MARS_CUDA(sc.get(&dtmp, dwords));
+    if (k == 1 && use_tc(ctx, size, shift))
+        return run_level_tc(ctx, sc, d_plane, d_D, w, h, g, fp, d_rows, d_cols, n, rs, ds, dtmp,
+                            d_out, d_dplane ? d_dplane : d_plane);
+    MARS_CUDA(mars::launch_range_stats(d_plane, (int)w, (int)h, d_rows, d_cols, (int)n,
+                                       (int)size, fp, rs, st));
     MARS_CUDA(mars::launch_domain_stats(d_D, g, ds, st, dtmp));
     ctx->launches += 2;
-    if (k > 1 && use_tc(ctx, size, shift) && mars::tc::topk_supported(g.size, tc_digits(ctx, g)))
+    if (k > 1 && use_tc(ctx, size, shift) && mars::tc::topk_supported(g.size, topk_digits(ctx, g)))
         return run_level_tc_topk(ctx, sc, d_plane, d_D, w, h, g, fp, d_rows, d_cols, n, rs, ds,
                                  d_out, k, d_dplane ? d_dplane : d_plane);
     if (k > 1) {
@@ -601,9 +671,6 @@ int run_level(mars_ctx* ctx, Scratch& sc, const uint8_t* d_plane, const int32_t*
         ctx->launches += 2;
         return MARS_OK;
     }
-    if (use_tc(ctx, size, shift))
-        return run_level_tc(ctx, sc, d_plane, d_D, w, h, g, fp, d_rows, d_cols, n, rs, ds, d_out,
-                            d_dplane ? d_dplane : d_plane);
     const int nsplit = mars::search_simt_splits(g, (int)n, ctx->num_sms);
     mars::Partial* partials;
     MARS_CUDA(sc.get(&partials, (size_t)nsplit * n));
@@ -735,11 +802,11 @@ bool all_levels_eligible(const mars_ctx* ctx, uint32_t w, uint32_t h, const std:
         if (j.rows.empty() || !use_tc(ctx, j.size, j.shift)) continue;
         const mars::LevelGeom g = level_geom(w, h, j.size, j.shift);
         if (g.nrow_d <= 0 || g.ncol_d <= 0) continue;
-        if (!mars::tc::all_levels_supported(g.size, tc_digits(ctx, g))) return false;
+        if (!mars::tc::all_levels_supported(g.size, tc_path(ctx, g, j.rows.size()))) return false;
         ++levels;
     }
-    // A level may add a tail job, and the block-size-8 level a coarse pre-pass job.
-    return levels > 0 && levels + 2 <= mars::tc::kMaxLevelJobs;
+    // One level adds a tail job.
+    return levels > 0 && levels + 1 <= mars::tc::kMaxLevelJobs;
 }
 
 // run_jobs for the exhaustive single-candidate search with the correlation of every
@@ -789,7 +856,7 @@ int run_jobs_all_levels(mars_ctx* ctx, Scratch& sc, const uint8_t* d_plane, uint
                 TcLevel L;
                 L.g = g;
                 L.n = j.rows.size();
-                L.digits = tc_digits(ctx, g);
+                L.path = tc_path(ctx, g, L.n);
                 lv.push_back(L);
                 lv_off.push_back(off);
             }
@@ -799,13 +866,13 @@ int run_jobs_all_levels(mars_ctx* ctx, Scratch& sc, const uint8_t* d_plane, uint
     const int nl = (int)lv.size();
     std::vector<mars::LevelGeom> gs(nl);
     std::vector<int> ns(nl), ms(nl), tail_t(nl), tail_ms(nl);
-    std::unique_ptr<bool[]> dg(new bool[std::max(1, nl)]);
+    std::vector<mars::tc::Path> pt(nl);
     for (int l = 0; l < nl; ++l) {
         gs[l] = lv[l].g;
         ns[l] = (int)lv[l].n;
-        dg[l] = lv[l].digits;
+        pt[l] = lv[l].path;
     }
-    mars::tc::all_levels_splits(gs.data(), ns.data(), dg.get(), nl, ctx->num_sms, ms.data(),
+    mars::tc::all_levels_splits(gs.data(), ns.data(), pt.data(), nl, ctx->num_sms, ms.data(),
                                 tail_t.data(), tail_ms.data());
     for (int l = 0; l < nl; ++l) {
         TcLevel& L = lv[l];
@@ -822,26 +889,19 @@ int run_jobs_all_levels(mars_ctx* ctx, Scratch& sc, const uint8_t* d_plane, uint
         MARS_CUDA(sc.get(&L.ds.sdetf, ndom));
         const size_t dwords = mars::domain_stats_tmp_words(L.g);
         if (dwords > 0 && dwords <= kDomainTmpWords) MARS_CUDA(sc.get(&L.dtmp, dwords));
-        const bool wanted = L.digits;
-        if (int e = tc_level_setup(ctx, sc, w, h, n, std::max(ms[l], tail_ms[l]), true,
-                                   n >= kCoarseAllLevels, L))
+        if (int e = tc_level_setup(ctx, sc, w, h, n, std::max(ms[l], tail_ms[l]), true, pt[l], L))
             return e;
-        if (L.digits != wanted)  // the driver rejected the digit views: no fold kernel here
+        if (L.path != pt[l])  // the driver rejected the digit views: no fold kernel here
             return fail(MARS_ECUDA, "the split-digit tensor maps were rejected");
         L.msplit = ms[l];
         L.tail_tiles = tail_t[l];
         L.tail_msplit = tail_ms[l];
-        if (L.coarse) {
-            // The coarse pre-pass runs inside the launch, ahead of this level's items.
-            const int rt = mars::tc::ranges_per_tile(false);
-            MARS_CUDA(sc.get(&L.ready, (n + rt - 1) / rt));
-            MARS_CUDA(sc.get(&L.coarse_tickets, (n + rt - 1) / rt));
-        }
     }
     int* d_work = nullptr;
-    MARS_CUDA(sc.get(&d_work, 1));
-    // Every branch is forked: a level's statistics and seeds run on branch b, its planes and
-    // B operand on branch b + kBranches / 2.
+    MARS_CUDA(sc.get(&d_work, 2));
+    MARS_CUDA(cudaMemsetAsync(d_work, 0, 2 * sizeof(int), main));
+    // Every branch is forked: a level's range side and seeds run on branch b, its domain side on
+    // branch b + kBranches / 2.
     MARS_CUDA(cudaEventRecord(ctx->fork_ev, main));
     const int nb = mars_ctx::kBranches;
     constexpr int kHalf = mars_ctx::kBranches / 2;
@@ -857,17 +917,8 @@ int run_jobs_all_levels(mars_ctx* ctx, Scratch& sc, const uint8_t* d_plane, uint
         const int l = level_of[i];
         if (l >= 0) {
             TcLevel& L = lv[l];
-            const mars::LevelGeom& g = L.g;
-            if (cudaError_t ce = mars::launch_range_stats(d_plane, (int)w, (int)h, rows, cols,
-                                                          (int)L.n, g.size, fp, L.rs, bs)) {
-                err = fail(MARS_ECUDA, cudaGetErrorString(ce));
-            } else if (cudaError_t ce2 = mars::launch_domain_stats(d_D, g, L.ds, bs, L.dtmp)) {
-                err = fail(MARS_ECUDA, cudaGetErrorString(ce2));
-            } else {
-                ctx->launches += 2;
-                err = tc_level_prep(ctx, L, d_plane, d_D, d_plane, w, h, fp, rows, cols, bs,
-                                    ctx->branch[b + kHalf]);
-            }
+            err = tc_level_prep(ctx, L, d_plane, d_D, d_plane, w, h, fp, rows, cols, bs,
+                                ctx->branch[b + kHalf], ctx->join_ev[b + kHalf]);
         } else {
             ctx->stream = bs;
             {
@@ -886,56 +937,7 @@ int run_jobs_all_levels(mars_ctx* ctx, Scratch& sc, const uint8_t* d_plane, uint
     }
     if (err) return err;
     std::vector<mars::tc::LevelJob> lj;
-    for (int l = 0; l < nl; ++l) {
-        const TcLevel& L = lv[l];
-        mars::tc::LevelJob J;
-        J.maps = L.maps;
-        J.bglob = L.d_b;
-        J.g = L.g;
-        J.nranges = (int)L.n;
-        J.rs = L.rs;
-        J.ds = L.ds;
-        J.fp = fp;
-        J.seeds = L.d_seed;
-        J.partials = L.partials;
-        J.gch = L.gch;
-        J.tickets = L.tickets;
-        J.out = d_out + lv_off[l];
-        const int rt = mars::tc::ranges_per_tile(L.digits);
-        const int ntiles = (int)((L.n + rt - 1) / rt);
-        J.digits = L.digits ? 1 : 0;
-        J.tile_begin = 0;
-        J.tile_count = ntiles - L.tail_tiles;
-        J.msplit = L.msplit;
-        if (L.coarse) {
-            // The pre-pass job: the same B operand and ranges, the coarse grid's planes and
-            // statistics; its last split of each tile merges the tile's seeds.
-            mars::tc::LevelJob C = J;
-            C.maps = L.maps1;
-            C.g = L.g1;
-            C.ds = L.ds1;
-            C.partials = L.part1;
-            C.gch = nullptr;
-            C.tickets = L.coarse_tickets;
-            C.out = nullptr;
-            C.tile_begin = 0;
-            C.tile_count = ntiles;
-            C.msplit = L.ms1;
-            C.merge_seeds = L.d_seed;
-            C.merge_ratio = kCoarseRatio;
-            C.fine_ncol = L.g.ncol_d;
-            C.ready = L.ready;
-            lj.push_back(C);
-            J.wait_ready = L.ready;
-        }
-        lj.push_back(J);
-        if (L.tail_tiles > 0) {
-            J.tile_begin = ntiles - L.tail_tiles;
-            J.tile_count = L.tail_tiles;
-            J.msplit = L.tail_msplit;
-            lj.push_back(J);
-        }
-    }
+    for (int l = 0; l < nl; ++l) add_level_jobs(lv[l], fp, d_out + lv_off[l], &lj);
     // Optional timing events around the launch: event-record nodes inside a capture (the
     // external flag is for captures only), plain records otherwise.
     unsigned rec_flags = cudaEventRecordDefault;
@@ -945,10 +947,16 @@ int run_jobs_all_levels(mars_ctx* ctx, Scratch& sc, const uint8_t* d_plane, uint
         if (cs == cudaStreamCaptureStatusActive) rec_flags = cudaEventRecordExternal;
         MARS_CUDA(cudaEventRecordWithFlags(timing[0], main, rec_flags));
     }
-    MARS_CUDA(mars::tc::launch_corr_all(lj.data(), (int)lj.size(), d_work, ctx->d_err,
-                                        ctx->d_counter, ctx->num_sms, main));
+    MARS_CUDA(cudaEventRecord(ctx->fork_ev, main));
+    MARS_CUDA(cudaStreamWaitEvent(ctx->branch[0], ctx->fork_ev, 0));
+    const cudaError_t le =
+        mars::tc::launch_corr_all(lj.data(), (int)lj.size(), d_work, ctx->d_err, ctx->d_counter,
+                                  ctx->num_sms, main, ctx->branch[0]);
+    MARS_CUDA(cudaEventRecord(ctx->join_ev[0], ctx->branch[0]));
+    MARS_CUDA(cudaStreamWaitEvent(main, ctx->join_ev[0], 0));
+    MARS_CUDA(le);
     if (timing) MARS_CUDA(cudaEventRecordWithFlags(timing[1], main, rec_flags));
-    ctx->launches += 1;
+    ctx->launches += 2;
     return MARS_OK;
 }
 

@@ -40,7 +40,11 @@ struct FitParams {
     float a_min;       // smallest nonzero alfa2, max_alfa / 2^bits_alfa, rounded down
     float a_half;      // a_min / 2 (exact)
     float two_a;       // 2 * a_min (exact)
+    float a_max;         // largest alfa2, max_alfa (1 - 2^-bits_alfa), rounded up
+    float max_half;      // a_max / 2, rounded down
+    float min_over_max;  // a_min / a_max, rounded down
     double eta_per_n;  // 1e-6 * (1 + max_alfa)^2
+    double inv_max_alfa;  // 1 / max_alfa when that is a power of two (exact), else 0
 };
 
 struct FitResult {
@@ -56,11 +60,16 @@ __device__ __forceinline__ uint32_t quantise_exact(double x, uint32_t max) {
     return (uint32_t)y;
 }
 
-// fit_f64 with the reference's operation order (encode.rs:247-289).
+// fit_f64 with the reference's operation order (encode.rs:247-289).  The divisions by powers of
+// two -- s0 (a block's pixel count, a power of four), 2^bits_alfa and, where it is one,
+// max_alfa -- are multiplications by the exact reciprocal, the same doubles: three of the
+// seven dependent f64 divisions, some 300 cycles each, that make a fit's latency.
 __device__ __forceinline__ FitResult fit_exact(int64_t s0i, int64_t s1_x4, int64_t s2_x16,
                                                int64_t t0i, int64_t t1_x4, int64_t t2i,
                                                const FitParams& fp) {
     const double s0 = (double)s0i;
+    // 2^-k from 2^k: the exponent field mirrored about 1023.
+    const double inv_s0 = __longlong_as_double(0x7FE0000000000000ll - __double_as_longlong(s0));
     const double s1 = __dmul_rn((double)s1_x4, 0.25);     // == / 4.0 (exact scaling)
     const double s2 = __dmul_rn((double)s2_x16, 0.0625);  // == / 16.0
     const double t0 = (double)t0i;
@@ -73,12 +82,16 @@ __device__ __forceinline__ FitResult fit_exact(int64_t s0i, int64_t s1_x4, int64
     if (alfa < 0.0) alfa = 0.0;
 
     const double qscale = (double)(1u << fp.bits_alfa);
+    const double inv_qscale =
+        __longlong_as_double(0x7FE0000000000000ll - __double_as_longlong(qscale));
     const uint32_t max_qalfa = (1u << fp.bits_alfa) - 1u;
     FitResult r;
-    r.qalfa = quantise_exact(__dmul_rn(__ddiv_rn(alfa, fp.max_alfa), qscale), max_qalfa);
-    const double alfa2 = __dmul_rn(__ddiv_rn((double)r.qalfa, qscale), fp.max_alfa);
+    const double rel = fp.inv_max_alfa != 0.0 ? __dmul_rn(alfa, fp.inv_max_alfa)
+                                              : __ddiv_rn(alfa, fp.max_alfa);
+    r.qalfa = quantise_exact(__dmul_rn(rel, qscale), max_qalfa);
+    const double alfa2 = __dmul_rn(__dmul_rn((double)r.qalfa, inv_qscale), fp.max_alfa);
 
-    double beta = __ddiv_rn(__dsub_rn(t0, __dmul_rn(alfa2, s1)), s0);
+    double beta = __dmul_rn(__dsub_rn(t0, __dmul_rn(alfa2, s1)), inv_s0);
     if (alfa2 > 0.0) beta = __dadd_rn(beta, __dmul_rn(alfa2, 255.0));
     const uint32_t max_qbeta = (1u << fp.bits_beta) - 1u;
     const double span = __dmul_rn(__dadd_rn(1.0, fabs(alfa2)), 255.0);
@@ -94,7 +107,7 @@ __device__ __forceinline__ FitResult fit_exact(int64_t s0i, int64_t s1_x4, int64
     x = __dadd_rn(x, __dmul_rn(__dmul_rn(__dmul_rn(2.0, alfa2), beta2), s1));
     x = __dadd_rn(x, __dmul_rn(__dmul_rn(s0, beta2), beta2));
     r.sum = x;
-    double q = __ddiv_rn(x, s0);
+    double q = __dmul_rn(x, inv_s0);
     if (!(q >= 0.0)) q = 0.0;
     r.rms = __dsqrt_rn(q);
     return r;

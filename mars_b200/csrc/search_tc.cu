@@ -41,6 +41,7 @@
 // ranked search keeping each range's best k; and corr_tc_all_kernel, every tensor-core
 // level of a plane in one persistent launch over (level, range tile, split) work items.
 #include <cuda.h>
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -509,57 +510,8 @@ __device__ __forceinline__ SeedOut load_seed(const SeedOut* p) {
                    __ldcg(reinterpret_cast<const double*>(p) + 1), it.x, (int32_t)it.y};
 }
 
-__device__ __forceinline__ int ld_acquire_gpu(const int* p) {
-    int v;
-    asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
-__device__ __forceinline__ void st_release_gpu(int* p, int v) {
-    asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
-// The coarse pre-pass's champion of range r (the best of its M-splits over every
-// `ratio`-th domain position of each axis) as a seed on the full grid: its domain index is
-// mapped to the fine grid, and it replaces the seed when it is better by (rms, index).
-// Any real candidate is a valid seed; a better one prunes more from the first tile.
-__device__ __forceinline__ void seed_merge_range(const Partial* partials, int nsplit, int nranges,
-                                                 int r, int coarse_ncol, int fine_ncol,
-                                                 int ratio, SeedOut* seeds) {
-    const SeedOut s = load_seed(seeds + r);
-    if (s.idx == UINT32_MAX) return;  // no range block here
-    // The pre-pass started from this seed, whose index is on the fine grid.  A split's
-    // champion only ever changes to a strictly better (rms, index) pair, so a partial equal
-    // to the seed's pair is the seed itself; every other one is a coarse-grid candidate.
-    bool have = false;
-    double best_rms = 0.0, best_sum = 0.0;
-    uint32_t best_idx = UINT32_MAX;
-    int32_t best_t1 = 0;
-    for (int t = 0; t < nsplit; ++t) {
-        const Partial* p = partials + (size_t)t * nranges + r;
-        const double rms = __ldcg(reinterpret_cast<const double*>(p));
-        const double sum = __ldcg(reinterpret_cast<const double*>(p) + 1);
-        const uint2 it = __ldcg(reinterpret_cast<const uint2*>(p) + 2);
-        if (it.x == UINT32_MAX || (rms == s.rms && it.x == s.idx)) continue;
-        if (!have || rms < best_rms || (rms == best_rms && it.x < best_idx)) {
-            best_rms = rms;
-            best_sum = sum;
-            best_idx = it.x;
-            best_t1 = (int32_t)it.y;
-        }
-        have = true;
-    }
-    if (!have) return;
-    const uint32_t dom1 = best_idx >> 3;
-    const uint32_t a1 = dom1 / (uint32_t)coarse_ncol, b1 = dom1 % (uint32_t)coarse_ncol;
-    const uint32_t idx =
-        ((a1 * (uint32_t)ratio) * (uint32_t)fine_ncol + b1 * (uint32_t)ratio) * 8u + (best_idx & 7u);
-    if (best_rms < s.rms || (best_rms == s.rms && idx < s.idx))
-        seeds[r] = SeedOut{best_rms, best_sum, idx, best_t1};
-}
-
-// What one work item reads and writes: a level's B operand, statistics, seeds, its split
-// of the domain tiles and the outputs of its range tile.
+// What one work item reads and writes: a level's operands, statistics, seeds, its split of
+// the domain tiles and the outputs of its range tile.
 struct ItemArgs {
     const uint8_t* bglob;
     LevelGeom g;
@@ -574,13 +526,7 @@ struct ItemArgs {
     int* tickets;             // per range tile: splits done (all-levels launch), or null
     CandidateOut* out;        // the level's candidates when tickets is set
     int k;                    // candidates kept per range (> 1: the ranked kernel)
-    // The all-levels launch's coarse pre-pass job: the last split of a range tile merges
-    // the tile's champions into merge_seeds (the fine level's seeds) and sets ready[tile];
-    // the fine level's items wait for wait_ready[tile] before reading their seeds.
-    SeedOut* merge_seeds;
-    int merge_ratio, fine_ncol;
-    int* ready;
-    const int* wait_ready;
+    UnitSource unit;          // the unit form's A operand and the exact integers behind it
 };
 
 // Per-thread pipeline state of the roles (each role thread keeps its own copy).  It carries
@@ -620,7 +566,7 @@ __device__ __forceinline__ uint32_t cta_setup(Smem& sm) {
         for (int q = 0; q < kGroups; ++q) sm.qcount[q] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    for (int i = threadIdx.x; i < kM * kN / 32; i += kThreads) sm.evaluated[i] = 0u;
+    for (int i = threadIdx.x; i < kM * kN / 32; i += blockDim.x) sm.evaluated[i] = 0u;
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                          smem_u32(&sm.tmem_base)),
@@ -644,14 +590,44 @@ __device__ __forceinline__ void cta_teardown(Smem& sm, uint32_t tmem, unsigned l
     }
 }
 
+// The end of a single-winner item: this split's partial champions and, with tickets, the final
+// candidates of a range tile whose last split this is (the threadfence-reduction pattern:
+// partials, fence, ticket; the last CTA fences again and reads every split's partials around
+// L1).
+// r: this thread's range (thread t < 32 holds champion t), or nranges and above for none.
+template <class Sm>
+__device__ __forceinline__ void finish_item(const ItemArgs& a, Sm& sm, int ntile, int split, int r) {
+    const bool mine = r < a.nranges;
+    if (mine) {
+        const Champ& C = sm.ch[threadIdx.x];
+        Partial p;
+        p.rms = C.rms;
+        p.sum = C.sum;
+        p.idx = C.idx;
+        p.t1x4 = C.t1x4;
+        p.qalfa = 0;
+        p.qbeta = 0;
+        p.pad = 0;
+        a.partials[(size_t)split * a.nranges + r] = p;
+    }
+    if (!a.tickets) return;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) sm.last = atomicAdd(&a.tickets[ntile], 1) == a.msplit - 1;
+    __syncthreads();
+    if (sm.last) {
+        __threadfence();
+        if (mine)
+            finish_range(a.partials, a.msplit, a.nranges, r, a.g, a.rs, a.ds, a.fp, a.out);
+    }
+}
+
 // One work item: range tile `ntile` of a level against domain tiles [split * m_per_cta,
 // ...) -- the champions seeded, the loads / MMAs / exact-bound epilogue over those domain
 // tiles, the tile's partial champions written.  With tickets set, the last split of the
-// range tile to finish also writes the tile's final candidates, or, for a coarse pre-pass
-// job, merges them into the fine level's seeds and sets the tile's ready flag; with
-// wait_ready set the item first waits for that flag.  TOPK: the ranked search, a k-list
-// per range in *tk.  Every thread of the CTA calls this together; it begins and ends with a
-// CTA barrier.
+// range tile to finish also writes the tile's final candidates.  TOPK: the ranked search, a
+// k-list per range in *tk.  Every thread of the CTA calls this together; it begins and
+// ends with a CTA barrier.
 template <int S, bool DIG, bool TOPK = false>
 __device__ __forceinline__ void process_item(const TcMaps& maps, const ItemArgs& a, int ntile,
                                              int split, Smem& sm, unsigned char* stages,
@@ -689,22 +665,6 @@ __device__ __forceinline__ void process_item(const TcMaps& maps, const ItemArgs&
     const int tiles_per_row = (g.ncol_d + kM - 1) / kM;
     const uint8_t* btile = a.bglob + (size_t)ntile * KST * kStageB;
 
-    if (a.wait_ready) {
-        // The coarse pre-pass items of this range tile were claimed before any item of this
-        // level, by CTAs that are running them: the wait ends (bounded all the same).
-        if (threadIdx.x == 0) {
-            const long long t0 = clock64();
-            while (ld_acquire_gpu(a.wait_ready + ntile) == 0) {
-                if (clock64() - t0 > kWaitCycles) {
-                    sm.abort_flag = 1;
-                    atomicOr(err, 32);
-                    break;
-                }
-                __nanosleep(256);
-            }
-        }
-        __syncthreads();
-    }
     if (threadIdx.x < RT) {
         Champ& C = sm.ch[threadIdx.x];
         const int r = ntile * RT + threadIdx.x;
@@ -766,6 +726,7 @@ __device__ __forceinline__ void process_item(const TcMaps& maps, const ItemArgs&
             publish_threshold(sm, threadIdx.x, fp, N);
         }
     }
+    fence_proxy_async();
     __syncthreads();
     volatile int* abort_flag = &sm.abort_flag;
 
@@ -1108,43 +1069,9 @@ __device__ __forceinline__ void process_item(const TcMaps& maps, const ItemArgs&
                 a.partials[((size_t)split * nranges + r) * a.k + j] = p;
             }
         }
-    } else if (threadIdx.x < RT) {
-        const Champ& C = sm.ch[threadIdx.x];
-        const int r = ntile * RT + threadIdx.x;
-        if (r < nranges) {
-            Partial p;
-            p.rms = C.rms;
-            p.sum = C.sum;
-            p.idx = C.idx;
-            p.t1x4 = C.t1x4;
-            p.qalfa = 0;
-            p.qbeta = 0;
-            p.pad = 0;
-            a.partials[(size_t)split * nranges + r] = p;
-        }
-    }
-    if (a.tickets) {
-        // The last of the range tile's splits to get here finishes its ranges (the
-        // threadfence-reduction pattern: partials, fence, ticket; the last CTA fences
-        // again and reads every split's partials around L1).
-        __threadfence();
-        __syncthreads();
-        if (threadIdx.x == 0) sm.last = atomicAdd(&a.tickets[ntile], 1) == a.msplit - 1;
-        __syncthreads();
-        if (sm.last) {
-            __threadfence();
-            const int r = ntile * RT + threadIdx.x;
-            if (a.merge_seeds) {
-                if (threadIdx.x < RT && r < nranges)
-                    seed_merge_range(a.partials, a.msplit, nranges, r, g.ncol_d, a.fine_ncol,
-                                     a.merge_ratio, a.merge_seeds);
-                __threadfence();
-                __syncthreads();
-                if (threadIdx.x == 0) st_release_gpu(a.ready + ntile, 1);
-            } else if (threadIdx.x < RT && r < nranges) {
-                finish_range(a.partials, a.msplit, nranges, r, g, a.rs, ds, fp, a.out);
-            }
-        }
+    } else {
+        finish_item(a, sm, ntile, split,
+                    (int)threadIdx.x < RT ? ntile * RT + (int)threadIdx.x : nranges);
     }
 }
 
@@ -1175,6 +1102,22 @@ __global__ void __launch_bounds__(kThreads, 1)
     cta_teardown(sm, tmem, exact, exact_counter);
 }
 
+// isometry::map (crates/mars-codec/src/isometry.rs:7-19) as a flat range index i*S + j.
+__device__ __forceinline__ int iso_src_rt(int k, int u, int v, int S) {
+    switch (k) {
+        case 0: return u * S + v;
+        case 1: return (S - 1 - v) * S + u;
+        case 2: return v * S + (S - 1 - u);
+        case 3: return (S - 1 - u) * S + (S - 1 - v);
+        case 4: return u * S + (S - 1 - v);
+        case 5: return (S - 1 - u) * S + v;
+        case 6: return v * S + u;
+        default: return (S - 1 - v) * S + (S - 1 - u);
+    }
+}
+
+#include "search_unit.cuh"
+
 // All tensor-core levels of a plane in one persistent launch: one CTA per SM takes work
 // items -- (level job, range tile, domain-tile split) -- from a global counter until none
 // are left.  TMEM, the mbarriers and the epilogue's queues are set up once per CTA; the
@@ -1184,7 +1127,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 struct AllLevels {
     TcMaps maps[kMaxLevelJobs];
     ItemArgs args[kMaxLevelJobs];
-    int kind[kMaxLevelJobs];  // 0: S=4 fold, 1: S=8 fold, 2/3/4: S=16/32/64 digits
+    int kind[kMaxLevelJobs];  // 0/1: S=4/8 fold, 2/3/4: S=16/32/64 digits
     int tile_begin[kMaxLevelJobs];
     int tile_count[kMaxLevelJobs];
     int item_begin[kMaxLevelJobs + 1];
@@ -1361,20 +1304,6 @@ __global__ void phase_planes_kernel(const uint8_t* __restrict__ plane, int w, in
         }
         *reinterpret_cast<uint4*>(out + ((size_t)p * h + y) * wp + x) =
             make_uint4(wd[0], wd[1], wd[2], wd[3]);
-    }
-}
-
-// isometry::map (crates/mars-codec/src/isometry.rs:7-19) as a flat range index i*S + j.
-__device__ __forceinline__ int iso_src_rt(int k, int u, int v, int S) {
-    switch (k) {
-        case 0: return u * S + v;
-        case 1: return (S - 1 - v) * S + u;
-        case 2: return v * S + (S - 1 - u);
-        case 3: return (S - 1 - u) * S + (S - 1 - v);
-        case 4: return u * S + (S - 1 - v);
-        case 5: return (S - 1 - u) * S + v;
-        case 6: return v * S + u;
-        default: return (S - 1 - v) * S + (S - 1 - u);
     }
 }
 
@@ -1631,16 +1560,6 @@ __global__ void __launch_bounds__(256) seed_small_kernel(
     if (lane == bl) out[r] = SeedOut{best, best_sum, best_idx, best_t1};
 }
 
-// The coarse pre-pass's seeds merged into the full grid's (seed_merge_range), one thread
-// per range.
-__global__ void seed_merge_kernel(const Partial* __restrict__ partials, int nsplit, int nranges,
-                                  int coarse_ncol, int fine_ncol, int ratio,
-                                  SeedOut* __restrict__ seeds) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r < nranges)
-        seed_merge_range(partials, nsplit, nranges, r, coarse_ncol, fine_ncol, ratio, seeds);
-}
-
 // Final champion over the M-splits of each range (finish_range).
 __global__ void finish_kernel(const Partial* __restrict__ partials, int nsplit, int nranges,
                               LevelGeom g, RangeStats rs, DomainStats ds, FitParams fp,
@@ -1681,8 +1600,46 @@ cudaError_t launch_t(const TcMaps& maps, const uint8_t* bglob, const LevelGeom& 
     dim3 grid(ntiles, msplit);
     const ItemArgs a{bglob, g,        nranges,  rs,       ds,      fp,     seeds,
                      m_tiles, m_per_cta, msplit, partials, gch, nullptr, nullptr, k,
-                     nullptr, 0, 0, nullptr, nullptr};
+                     UnitSource{}};
     kern<<<grid, kThreads, smem, st>>>(maps, a, err, counter);
+    return cudaGetLastError();
+}
+
+template <int S>
+constexpr size_t unit_smem_bytes() {
+    return 1024 + kUnitHead + UCfg<S>::kBytes;
+}
+static_assert(unit_smem_bytes<4>() <= 232448 && unit_smem_bytes<8>() <= 232448,
+              "shared memory per CTA (227 KB)");
+
+template <int S>
+cudaError_t build_unit_a_t(const int32_t* D, const LevelGeom& g, DomainStats ds,
+                           const uint32_t* domains, uint8_t* out, cudaStream_t st) {
+    const long long total = (long long)domain_tiles(g, kUnit) * kM * UCfg<S>::KG;
+    unit_a_kernel<S><<<(unsigned)((total + 255) / 256), 256, 0, st>>>(
+        D, g, ds, domains, total, reinterpret_cast<uint4*>(out));
+    return cudaGetLastError();
+}
+
+template <bool RANGES>
+cudaError_t launch_order_t(DomainStats ds, RangeStats rs, int n, uint32_t* bins, uint32_t* order,
+                           cudaStream_t st) {
+    cudaError_t e = cudaMemsetAsync(bins, 0, 2 * kBins * sizeof(uint32_t), st);
+    if (e != cudaSuccess) return e;
+    const unsigned blocks = (unsigned)((n + kOrderItems - 1) / kOrderItems);
+    order_count_kernel<RANGES><<<blocks, 1024, 0, st>>>(ds, rs, n, bins);
+    order_scatter_kernel<RANGES><<<blocks, 1024, 0, st>>>(ds, rs, n, bins, order);
+    return cudaGetLastError();
+}
+
+template <int S>
+cudaError_t build_unit_b_t(const uint8_t* plane, int w, int h, const uint32_t* rows,
+                           const uint32_t* cols, int nranges, RangeStats rs,
+                           const uint32_t* ranges, uint8_t* out, cudaStream_t st) {
+    const long long ntiles = (nranges + kRangesPerTile - 1) / kRangesPerTile;
+    const long long total = ntiles * kN * UCfg<S>::KG;
+    unit_b_kernel<S><<<(unsigned)((total + 255) / 256), 256, 0, st>>>(
+        plane, w, h, rows, cols, nranges, rs, ranges, total, reinterpret_cast<uint4*>(out));
     return cudaGetLastError();
 }
 
@@ -1710,14 +1667,56 @@ bool digits_supported(int size, int shift) {
            (shift == 2 || shift == 4 || shift == 8 || shift == 16);
 }
 
-int ranges_per_tile(bool digits) { return digits ? 16 : 32; }
+int ranges_per_tile(Path path) { return path == kDigits ? 16 : 32; }
 
-size_t b_bytes(int size, int nranges, bool digits) {
-    // K-groups of 16 bytes per B row: fold J * 2S with J = max(1, S / 8); digits S * S / 16.
-    const int KG = digits ? size * size / 16 : (size >= 8 ? size / 8 : 1) * 2 * size;
-    const int rt = ranges_per_tile(digits);
+bool unit_supported(int size, int shift) {
+    return (size == 4 || size == 8) && (shift == 2 || shift == 4 || shift == 8 || shift == 16);
+}
+
+int domain_tiles(const LevelGeom& g, Path path) {
+    if (path == kUnit) return (int)(((long long)g.nrow_d * g.ncol_d + kM - 1) / kM);
+    return g.nrow_d * ((g.ncol_d + kM - 1) / kM);
+}
+
+size_t unit_a_bytes(const LevelGeom& g) {
+    return (size_t)domain_tiles(g, kUnit) * kM * g.size * g.size * 2;
+}
+
+size_t b_bytes(int size, int nranges, Path path) {
+    const int rt = ranges_per_tile(path);
     const size_t ntiles = (size_t)(nranges + rt - 1) / rt;
+    if (path == kUnit) return ntiles * (size_t)(rt * 8) * size * size * 2;
+    // K-groups of 16 bytes per B row: fold J * 2S with J = max(1, S / 8); digits S * S / 16.
+    const int KG = path == kDigits ? size * size / 16 : (size >= 8 ? size / 8 : 1) * 2 * size;
     return ntiles * (size_t)(rt * 8) * (size_t)KG * 16;
+}
+
+size_t unit_bins_words() { return 2 * kBins; }
+
+cudaError_t launch_unit_a(const int32_t* D, const LevelGeom& g, DomainStats ds, uint32_t* bins,
+                          uint32_t* domains, float2* contrasts, uint8_t* out, cudaStream_t st) {
+    const int ndom = g.nrow_d * g.ncol_d, tiles = domain_tiles(g, kUnit);
+    cudaError_t e = launch_order_t<false>(ds, RangeStats{}, ndom, bins, domains, st);
+    if (e != cudaSuccess) return e;
+    tile_contrast_kernel<<<(tiles + 7) / 8, 256, 0, st>>>(ds, domains, ndom, tiles, contrasts);
+    switch (g.size) {
+        case 4: return build_unit_a_t<4>(D, g, ds, domains, out, st);
+        case 8: return build_unit_a_t<8>(D, g, ds, domains, out, st);
+        default: return cudaErrorInvalidValue;
+    }
+}
+
+cudaError_t launch_unit_b(int size, const uint8_t* plane, int w, int h, const uint32_t* rows,
+                          const uint32_t* cols, int nranges, RangeStats rs, uint32_t* bins,
+                          uint32_t* ranges, uint8_t* out, cudaStream_t st) {
+    if (nranges == 0) return cudaSuccess;
+    cudaError_t e = launch_order_t<true>(DomainStats{}, rs, nranges, bins, ranges, st);
+    if (e != cudaSuccess) return e;
+    switch (size) {
+        case 4: return build_unit_b_t<4>(plane, w, h, rows, cols, nranges, rs, ranges, out, st);
+        case 8: return build_unit_b_t<8>(plane, w, h, rows, cols, nranges, rs, ranges, out, st);
+        default: return cudaErrorInvalidValue;
+    }
 }
 
 int phase_count(int shift) { return 16 / shift; }
@@ -1802,11 +1801,10 @@ cudaError_t launch_seed(const int32_t* D, const LevelGeom& g, const uint8_t* pla
 // CTA sweeping ceil(m_tiles / msplit) domain tiles after a fixed set-up (B load, range
 // records, pipeline fill) worth about kSetupTiles tiles.  Pick the split with the fewest
 // tile-times over all waves.
-int msplit_for(const LevelGeom& g, int nranges, int num_sms, bool digits) {
+int msplit_for(const LevelGeom& g, int nranges, int num_sms, Path path) {
     constexpr long long kSetupTiles = 4;
-    const int tiles_per_row = (g.ncol_d + kM - 1) / kM;
-    const int m_tiles = g.nrow_d * tiles_per_row;
-    const int rt = ranges_per_tile(digits);
+    const int m_tiles = domain_tiles(g, path);
+    const int rt = ranges_per_tile(path);
     const int ntiles = (nranges + rt - 1) / rt;
     int best = 1;
     long long best_cost = -1;
@@ -1848,21 +1846,23 @@ cudaError_t launch_corr(const TcMaps& maps, const uint8_t* bglob, const LevelGeo
 #undef MARS_CORR
 }
 
-bool all_levels_supported(int size, bool digits) {
-    return digits ? (size == 16 || size == 32 || size == 64) : (size == 4 || size == 8);
+bool all_levels_supported(int size, Path path) {
+    return path == kDigits ? size == 16 || size == 32 || size == 64 : size == 4 || size == 8;
 }
 
 namespace {
-int all_levels_kind(int size, bool digits) {
-    if (!digits) return size == 4 ? 0 : 1;
+int all_levels_kind(int size) {
+    if (size <= 8) return size == 4 ? 0 : 1;
     return size == 16 ? 2 : (size == 32 ? 3 : 4);
 }
 
 // Device time of one domain tile of one range tile, by kind (per-level CUDA-event times of a
-// 512 x 512 plane on one B200 / tiles: S = 4 fold 1.48 us, S = 8 fold 1.93, S = 16 digits
-// 2.09, S = 32 digits 8.0; S = 64 digits four times S = 32, K being four times larger).
-double all_levels_tile_us(int size, bool digits) {
-    if (!digits) return size == 4 ? 1.48 : 1.93;
+// 512 x 512 plane on one B200 / tiles: S = 4 fold 1.48 us, S = 8 fold 1.93, S = 16 digits 2.09,
+// S = 32 digits 8.0; S = 64 digits four times S = 32, K being four times larger; the unit
+// form's from its cycles a tile).
+double all_levels_tile_us(int size, Path path) {
+    if (path == kUnit) return size == 4 ? 0.6 : 0.7;
+    if (path == kFold) return size == 4 ? 1.48 : 1.93;
     return size == 16 ? 2.09 : (size == 32 ? 8.0 : 32.0);
 }
 constexpr double kItemSetupTiles = 4.0;  // B load, champions, pipeline fill: ~4 tiles
@@ -1871,27 +1871,38 @@ constexpr int kItemsPerSm = 8;           // work items per SM the splits aim at
 // split-major items keep the CTAs running together inside one band of domain rows (one
 // split), which L2 then holds for all of them.
 constexpr double kMaxItemUs = 1500.0;
+// A unit item's set-up, preview and drain take 25,000 cycles, some 20 tiles: items of fewer than
+// kUnitItemTiles tiles only where the level would leave SMs idle, and none under kUnitLeastTiles.
+constexpr int kUnitItemTiles = 96;
+constexpr int kUnitLeastTiles = 16;
+
+int unit_split_cap(int m_tiles, int ntiles, int num_sms) {
+    const int fill = std::min(num_sms / std::max(1, ntiles), m_tiles / kUnitLeastTiles);
+    return std::max(1, std::max(m_tiles / kUnitItemTiles, fill));
+}
 }  // namespace
 
-void all_levels_splits(const LevelGeom* g, const int* nranges, const bool* digits, int n,
+void all_levels_splits(const LevelGeom* g, const int* nranges, const Path* path, int n,
                        int num_sms, int* msplit, int* tail_tiles, int* tail_msplit) {
     double total = 0.0;
     for (int i = 0; i < n; ++i) {
-        const int tiles_per_row = (g[i].ncol_d + kM - 1) / kM;
-        const double m_tiles = (double)g[i].nrow_d * tiles_per_row;
-        const int rt = ranges_per_tile(digits[i]);
+        const double m_tiles = (double)domain_tiles(g[i], path[i]);
+        const int rt = ranges_per_tile(path[i]);
         const double ntiles = (double)((nranges[i] + rt - 1) / rt);
-        total += ntiles * m_tiles * all_levels_tile_us(g[i].size, digits[i]);
+        total += ntiles * m_tiles * all_levels_tile_us(g[i].size, path[i]);
     }
     const double target = std::min(kMaxItemUs, total / ((double)num_sms * kItemsPerSm));
     int last = -1;
     double last_cost = 0.0;
     for (int i = 0; i < n; ++i) {
-        const int tiles_per_row = (g[i].ncol_d + kM - 1) / kM;
-        const int m_tiles = g[i].nrow_d * tiles_per_row;
-        const double tile_us = all_levels_tile_us(g[i].size, digits[i]);
+        const int m_tiles = domain_tiles(g[i], path[i]);
+        const double tile_us = all_levels_tile_us(g[i].size, path[i]);
         const int ms = (int)((m_tiles * tile_us + target - 1e-9) / target);
-        msplit[i] = std::max(1, std::min(ms, m_tiles));
+        const int rt = ranges_per_tile(path[i]);
+        const int cap = path[i] == kUnit
+                            ? unit_split_cap(m_tiles, (nranges[i] + rt - 1) / rt, num_sms)
+                            : m_tiles;
+        msplit[i] = std::max(1, std::min(ms, cap));
         tail_tiles[i] = 0;
         tail_msplit[i] = msplit[i];
         const double cost = ((m_tiles + msplit[i] - 1) / msplit[i] + kItemSetupTiles) * tile_us;
@@ -1902,76 +1913,113 @@ void all_levels_splits(const LevelGeom* g, const int* nranges, const bool* digit
     }
     if (last < 0) return;
     // The tail: items a quarter as long, about two per SM.
-    const int tiles_per_row = (g[last].ncol_d + kM - 1) / kM;
-    const int m_tiles = g[last].nrow_d * tiles_per_row;
-    const int rt = ranges_per_tile(digits[last]);
+    const int m_tiles = domain_tiles(g[last], path[last]);
+    const int rt = ranges_per_tile(path[last]);
     const int ntiles = (nranges[last] + rt - 1) / rt;
-    const int fine = std::min(m_tiles, 4 * msplit[last]);
+    const int fine = std::min(
+        path[last] == kUnit ? unit_split_cap(m_tiles, ntiles, num_sms) : m_tiles, 4 * msplit[last]);
     if (fine > msplit[last] && ntiles >= 2) {
         tail_msplit[last] = fine;
         tail_tiles[last] = std::min(ntiles / 2, (2 * num_sms + fine - 1) / fine);
     }
 }
 
-cudaError_t launch_corr_all(const LevelJob* jobs, int njobs, int* work, int* err,
-                            unsigned long long* counter, int num_sms, cudaStream_t st) {
-    if (njobs <= 0) return cudaSuccess;
-    if (njobs > kMaxLevelJobs) return cudaErrorInvalidValue;
-    // Largest items first.
-    int order[kMaxLevelJobs];
-    double cost[kMaxLevelJobs];
-    for (int i = 0; i < njobs; ++i) {
-        const LevelJob& J = jobs[i];
-        if (!all_levels_supported(J.g.size, J.digits != 0) || J.msplit < 1) return cudaErrorInvalidValue;
-        const int tiles_per_row = (J.g.ncol_d + kM - 1) / kM;
-        const int m_tiles = J.g.nrow_d * tiles_per_row;
-        const int m_per = (m_tiles + J.msplit - 1) / J.msplit;
-        cost[i] = (m_per + kItemSetupTiles) * all_levels_tile_us(J.g.size, J.digits != 0);
-        if (J.merge_seeds) cost[i] = 1e30;  // coarse pre-pass jobs first: others wait on them
-        order[i] = i;
-    }
-    std::sort(order, order + njobs, [&](int x, int y) { return cost[x] > cost[y]; });
-    std::unique_ptr<AllLevels> hold(new AllLevels());  // the kernel parameter, ~10 KB
-    AllLevels& L = *hold;
-    L.njobs = njobs;
-    L.item_begin[0] = 0;
-    for (int k = 0; k < njobs; ++k) {
-        const LevelJob& J = jobs[order[k]];
-        const int tiles_per_row = (J.g.ncol_d + kM - 1) / kM;
-        const int m_tiles = J.g.nrow_d * tiles_per_row;
-        L.maps[k] = J.maps;
-        L.args[k] = ItemArgs{J.bglob,  J.g,      J.nranges,
-                             J.rs,     J.ds,     J.fp,
-                             J.seeds,  m_tiles,  (m_tiles + J.msplit - 1) / J.msplit,
-                             J.msplit, J.partials, J.gch,
-                             J.tickets, J.out, 1,
-                             J.merge_seeds, J.merge_ratio, J.fine_ncol,
-                             J.ready, J.wait_ready};
-        L.kind[k] = all_levels_kind(J.g.size, J.digits != 0);
-        L.tile_begin[k] = J.tile_begin;
-        L.tile_count[k] = J.tile_count;
-        L.item_begin[k + 1] = L.item_begin[k] + J.tile_count * J.msplit;
-    }
-    const int nitems = L.item_begin[njobs];
-    if (nitems == 0) return cudaSuccess;
-    size_t smem = 0;
-    for (int k = 0; k < njobs; ++k) {
-        constexpr size_t sz[5] = {smem_bytes<4, false>(), smem_bytes<8, false>(),
-                                  smem_bytes<16, true>(), smem_bytes<32, true>(),
-                                  smem_bytes<64, true>()};
-        smem = std::max(smem, sz[L.kind[k]]);
-    }
-    cudaError_t e = cudaFuncSetAttribute(corr_tc_all_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    e = cudaMemsetAsync(work, 0, sizeof(int), st);
-    if (e != cudaSuccess) return e;
-    const int grid = std::min(nitems, num_sms);
-    corr_tc_all_kernel<<<grid, kThreads, smem, st>>>(L, work, err, counter);
-    return cudaGetLastError();
+namespace {
+ItemArgs item_args(const LevelJob& J) {
+    const int m_tiles = domain_tiles(J.g, J.path);
+    return ItemArgs{J.bglob,  J.g,      J.nranges,
+                    J.rs,     J.ds,     J.fp,
+                    J.seeds,  m_tiles,  (m_tiles + J.msplit - 1) / J.msplit,
+                    J.msplit, J.partials, J.gch,
+                    J.tickets, J.out,   1, J.unit};
 }
 
-bool topk_supported(int size, bool digits) { return all_levels_supported(size, digits); }
+// The jobs of one form, largest items first.
+int ordered_jobs(const LevelJob* jobs, int njobs, bool unit, int* order) {
+    double cost[kMaxLevelJobs];
+    int n = 0;
+    for (int i = 0; i < njobs; ++i) {
+        const LevelJob& J = jobs[i];
+        if ((J.path == kUnit) != unit) continue;
+        const int m_tiles = domain_tiles(J.g, J.path);
+        const int m_per = (m_tiles + J.msplit - 1) / J.msplit;
+        cost[i] = (m_per + kItemSetupTiles) * all_levels_tile_us(J.g.size, J.path);
+        order[n++] = i;
+    }
+    std::sort(order, order + n, [&](int x, int y) { return cost[x] > cost[y]; });
+    return n;
+}
+}  // namespace
+
+// Two launches, the integer levels' on st_int and the unit levels' on st: each CTA fills an SM,
+// so the second launch's start on the SMs that the first one's leave.
+cudaError_t launch_corr_all(const LevelJob* jobs, int njobs, int* work, int* err,
+                            unsigned long long* counter, int num_sms, cudaStream_t st,
+                            cudaStream_t st_int) {
+    if (njobs <= 0) return cudaSuccess;
+    if (njobs > kMaxLevelJobs) return cudaErrorInvalidValue;
+    for (int i = 0; i < njobs; ++i)
+        if (!all_levels_supported(jobs[i].g.size, jobs[i].path) || jobs[i].msplit < 1)
+            return cudaErrorInvalidValue;
+    int order[kMaxLevelJobs];
+    if (const int n = ordered_jobs(jobs, njobs, false, order)) {
+        std::unique_ptr<AllLevels> hold(new AllLevels());  // the kernel parameter, ~10 KB
+        AllLevels& L = *hold;
+        L.njobs = n;
+        L.item_begin[0] = 0;
+        size_t smem = 0;
+        for (int k = 0; k < n; ++k) {
+            const LevelJob& J = jobs[order[k]];
+            L.maps[k] = J.maps;
+            L.args[k] = item_args(J);
+            L.kind[k] = all_levels_kind(J.g.size);
+            L.tile_begin[k] = J.tile_begin;
+            L.tile_count[k] = J.tile_count;
+            L.item_begin[k + 1] = L.item_begin[k] + J.tile_count * J.msplit;
+            constexpr size_t sz[5] = {smem_bytes<4, false>(), smem_bytes<8, false>(),
+                                      smem_bytes<16, true>(), smem_bytes<32, true>(),
+                                      smem_bytes<64, true>()};
+            smem = std::max(smem, sz[L.kind[k]]);
+        }
+        if (const int nitems = L.item_begin[n]) {
+            cudaError_t e = cudaFuncSetAttribute(
+                corr_tc_all_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            if (e != cudaSuccess) return e;
+            corr_tc_all_kernel<<<std::min(nitems, num_sms), kThreads, smem, st_int>>>(
+                L, work, err, counter);
+            if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        }
+    }
+    if (const int n = ordered_jobs(jobs, njobs, true, order)) {
+        std::unique_ptr<UnitLevels> hold(new UnitLevels());
+        UnitLevels& L = *hold;
+        L.njobs = n;
+        L.item_begin[0] = 0;
+        size_t smem = 0;
+        for (int k = 0; k < n; ++k) {
+            const LevelJob& J = jobs[order[k]];
+            L.args[k] = item_args(J);
+            L.size[k] = J.g.size;
+            L.tile_begin[k] = J.tile_begin;
+            L.tile_count[k] = J.tile_count;
+            L.item_begin[k + 1] = L.item_begin[k] + J.tile_count * J.msplit;
+            smem = std::max(smem, J.g.size == 4 ? unit_smem_bytes<4>() : unit_smem_bytes<8>());
+        }
+        if (const int nitems = L.item_begin[n]) {
+            cudaError_t e = cudaFuncSetAttribute(
+                corr_unit_all_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            if (e != cudaSuccess) return e;
+            corr_unit_all_kernel<<<std::min(nitems, num_sms), kUnitThreads, smem, st>>>(
+                L, work + 1, err, counter);
+            if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        }
+    }
+    return cudaSuccess;
+}
+
+bool topk_supported(int size, bool digits) {
+    return digits ? (size == 16 || size == 32 || size == 64) : (size == 4 || size == 8);
+}
 
 cudaError_t launch_corr_topk(const TcMaps& maps, const uint8_t* bglob, const LevelGeom& g,
                              int nranges, RangeStats rs, DomainStats ds, const FitParams& fp,
@@ -2016,14 +2064,6 @@ cudaError_t launch_seed_topk(const int32_t* D, const LevelGeom& g, const uint8_t
         default: return cudaErrorInvalidValue;
     }
 #undef MARS_SEED_TOPK
-    return cudaGetLastError();
-}
-
-cudaError_t launch_seed_merge(const Partial* partials, int nsplit, int nranges, int coarse_ncol,
-                              int fine_ncol, int ratio, SeedOut* seeds, cudaStream_t st) {
-    if (nranges == 0) return cudaSuccess;
-    seed_merge_kernel<<<(nranges + 127) / 128, 128, 0, st>>>(partials, nsplit, nranges,
-                                                             coarse_ncol, fine_ncol, ratio, seeds);
     return cudaGetLastError();
 }
 

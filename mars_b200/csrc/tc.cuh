@@ -26,6 +26,23 @@ struct alignas(64) TcMaps {
     int32_t use_all;
 };
 
+// The forms of a level's correlation: integer with the 2x2 box folded into K (any size),
+// integer over the contracted plane's two digits (16..64), and unit vectors in f16 (4 and 8;
+// search_unit.cuh).
+enum Path : int { kFold = 0, kDigits = 1, kUnit = 2 };
+
+// What the unit form reads beside the B operand: the A operand, the domains and ranges in its and
+// B's row order (by contrast), each domain tile's smallest and largest contrast; and the
+// contracted plane, the range plane and the range origins its survivors are evaluated from.
+struct UnitSource {
+    const uint8_t* aglob = nullptr;
+    const uint32_t *domains = nullptr, *ranges = nullptr;
+    const float2* contrasts = nullptr;
+    const int32_t* D = nullptr;
+    const uint8_t* plane = nullptr;
+    const uint32_t *rows = nullptr, *cols = nullptr;
+};
+
 struct SeedOut {
     double rms, sum;
     uint32_t idx;
@@ -51,15 +68,8 @@ struct LevelJob {
     int* tickets;
     CandidateOut* out;
     int tile_begin, tile_count, msplit;
-    int digits;
-    // A coarse pre-pass job (merge_seeds set) runs before every other job: the last split
-    // of each range tile merges its champions into merge_seeds (the fine level's seeds, fine
-    // grid fine_ncol, coarse stride merge_ratio times the fine one) and sets ready[tile]
-    // (zero before the launch); the fine level's jobs pass the same array as wait_ready.
-    SeedOut* merge_seeds = nullptr;
-    int merge_ratio = 0, fine_ncol = 0;
-    int* ready = nullptr;
-    const int* wait_ready = nullptr;
+    Path path;
+    UnitSource unit;  // path kUnit
 };
 constexpr int kMaxLevelJobs = 8;
 
@@ -73,17 +83,23 @@ size_t phase_bytes(int w, int h, int shift);
 // of row_pitch(w / 2) bytes (plus slack).
 int digit_phase_count(int shift);
 size_t digit_plane_bytes(int w, int h, int shift);
-size_t b_bytes(int size, int nranges, bool digits);
-int msplit_for(const LevelGeom& g, int nranges, int num_sms, bool digits);
-// Whether the all-levels kernel holds a level: block sizes 4 and 8 on the fold path, 16, 32
-// and 64 on the split-digit path.
-bool all_levels_supported(int size, bool digits);
-int ranges_per_tile(bool digits);
+// Levels the unit form serves (block sizes 4 and 8), and its A operand's bytes.
+bool unit_supported(int size, int shift);
+size_t unit_a_bytes(const LevelGeom& g);
+// Domain tiles of a level: 128 positions of one domain row each, or, in the unit form, any 128
+// consecutive ones.
+int domain_tiles(const LevelGeom& g, Path path);
+size_t b_bytes(int size, int nranges, Path path);
+int msplit_for(const LevelGeom& g, int nranges, int num_sms, Path path);
+// Whether the all-levels launches hold a level: block sizes 4 and 8 in the unit form or the fold,
+// 16, 32 and 64 on the split-digit path.
+bool all_levels_supported(int size, Path path);
+int ranges_per_tile(Path path);
 // Split counts of the levels of one all-levels launch, from a per-kind cost model, so that
 // the work items are of similar duration and several per SM.  The level with the cheapest
 // items (they run last) also gets a tail: its last tail_tiles[i] range tiles at
 // tail_msplit[i] splits, finer items to even out the end of the launch (0 tiles: none).
-void all_levels_splits(const LevelGeom* g, const int* nranges, const bool* digits, int n,
+void all_levels_splits(const LevelGeom* g, const int* nranges, const Path* path, int n,
                        int num_sms, int* msplit, int* tail_tiles, int* tail_msplit);
 
 cudaError_t launch_phase_planes(const uint8_t* plane, int w, int h, int shift, uint8_t* out,
@@ -100,10 +116,19 @@ cudaError_t launch_corr(const TcMaps& maps, const uint8_t* bglob, const LevelGeo
                         RangeStats rs, DomainStats ds, const FitParams& fp, const SeedOut* seeds,
                         Partial* partials, unsigned long long* gch, int msplit, bool digits,
                         int* err, unsigned long long* counter, cudaStream_t st);
-// The persistent launch over jobs[0..njobs) (njobs <= kMaxLevelJobs); `work` is a device
-// counter it zeroes first.
+// The unit form of a level: its operands and orders (the statistics come first; bins:
+// unit_bins_words() words of scratch for each call).  launch_corr_all correlates it.
+size_t unit_bins_words();
+cudaError_t launch_unit_a(const int32_t* D, const LevelGeom& g, DomainStats ds, uint32_t* bins,
+                          uint32_t* domains, float2* contrasts, uint8_t* out, cudaStream_t st);
+cudaError_t launch_unit_b(int size, const uint8_t* plane, int w, int h, const uint32_t* rows,
+                          const uint32_t* cols, int nranges, RangeStats rs, uint32_t* bins,
+                          uint32_t* ranges, uint8_t* out, cudaStream_t st);
+// The persistent launches over jobs[0..njobs) (njobs <= kMaxLevelJobs): the unit levels' on st,
+// the others' on st_int.  `work` is two device counters, zero before both.
 cudaError_t launch_corr_all(const LevelJob* jobs, int njobs, int* work, int* err,
-                            unsigned long long* counter, int num_sms, cudaStream_t st);
+                            unsigned long long* counter, int num_sms, cudaStream_t st,
+                            cudaStream_t st_int);
 // The ranked search (k = 2..kMaxTopK candidates per range) on the tcgen05 path, for the
 // kinds the all-levels kernel holds: seeds (n x k, the best k distinct of the 72 seed
 // candidates), then the correlation, whose partials are msplit x n x k sorted lists
@@ -118,8 +143,6 @@ cudaError_t launch_corr_topk(const TcMaps& maps, const uint8_t* bglob, const Lev
                              const SeedOut* seeds, int k, Partial* partials,
                              unsigned long long* gch, int msplit, bool digits, int* err,
                              unsigned long long* counter, cudaStream_t st);
-cudaError_t launch_seed_merge(const Partial* partials, int nsplit, int nranges, int coarse_ncol,
-                              int fine_ncol, int ratio, SeedOut* seeds, cudaStream_t st);
 cudaError_t launch_finish(const Partial* partials, int nsplit, int nranges, const LevelGeom& g,
                           RangeStats rs, DomainStats ds, const FitParams& fp, CandidateOut* out,
                           cudaStream_t st);

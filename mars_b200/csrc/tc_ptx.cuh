@@ -36,6 +36,12 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
+// One thread's arrival on behalf of `count` threads.
+__device__ __forceinline__ void mbar_arrive_n(uint64_t* bar, uint32_t count) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(count)
+                 : "memory");
+}
+
 // One bounded poll of an mbarrier phase.  The suspend-time hint lets the hardware park
 // the waiting thread until the phase completes (or ~20 us pass) instead of spinning, so
 // waiting warps leave the issue slots to the epilogue warps sharing their scheduler.
@@ -54,6 +60,9 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 // Bounded wait: false when the deadline passed or another warp already gave up.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
                                           int* err_global, int code) {
+    // The clock is read only when the first poll fails: reading it costs a waiting pipeline
+    // about 100 cycles a tile.
+    if (mbar_try_wait(bar, parity)) return true;
     const long long t0 = clock64();
     while (!mbar_try_wait(bar, parity)) {
         if (*abort_flag) return false;
@@ -121,10 +130,33 @@ __device__ __forceinline__ void mma_i8(uint32_t tmem_d, uint64_t adesc, uint64_t
         : "memory");
 }
 
+// Instruction descriptor, kind::f16: D = f32, A and B = f16, both K-major, M = 128, N = NT.
+template <int NT>
+__host__ __device__ constexpr uint32_t idesc_f16() {
+    return (1u << 4) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(kM >> 4) << 24);
+}
+
+template <int NT>
+__device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
+                                        uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+        "l"(adesc), "l"(bdesc), "r"(idesc_f16<NT>()), "r"(accumulate)
+        : "memory");
+}
+
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                      smem_u32(bar))
                  : "memory");
+}
+
+// Orders this thread's earlier shared-memory writes before asynchronous copies into the same
+// bytes (an item's stages may lie where an earlier item kept plain data).
+__device__ __forceinline__ void fence_proxy_async() {
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
 __device__ __forceinline__ void tmem_fence_before() {
