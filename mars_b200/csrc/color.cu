@@ -8,8 +8,11 @@
 //     neighbour inverse;
 //   mse (metrics.rs:29-48): the exact integer sum of squared differences (u64), divided by
 //     the pixel count on the host.
-// All are elementwise or small-stencil byte work, so each is bound by HBM; pixels are
-// processed four to a thread where the planes are word-aligned.
+// All are elementwise or small-stencil byte work, so each should be bound by HBM: a thread takes
+// 16 bytes of a plane (8 where two rows make one) whatever the alignment allows, and the
+// conversions stay off the f64 pipe.  A 3840 x 2160 frame through all of them (convert, halve and
+// restore two planes, convert back, error) took 148 us on one B200 with a byte or an f64 value
+// at a time, and takes 95 us, the host's wait for the error included.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -47,62 +50,210 @@ __device__ __forceinline__ void rgb_pixel(uint32_t y8, uint32_t cb8, uint32_t cr
     *b = round_u8(__dadd_rn(y, __dmul_rn(1.772, cb)));
 }
 
-// Three input planes -> three output planes, pixel by pixel; `inverse` picks the direction.
+// The conversions of four pixels in f32, and in f64 only where f32 cannot decide the rounding.
+// The f32 value is off by less than 2^-13 (three roundings below 512 and the coefficients'), so
+// a value further than 2^-12 from a half rounds as the f64 one does; the others, the exact
+// halves among them (299 r + 587 g + 114 b = 500 mod 1000, one colour in a thousand), take the
+// f64 form.  Adding 1.5 * 2^23 rounds to an integer in the low mantissa bits, so no conversion
+// instruction (a quarter-rate pipe or slower) is left.  The f64 form of every pixel took
+// 25.6 us (ycbcr) and 24.3 us (back) for 3840 x 2160, 2.0 TB/s of the planes' bytes.
+constexpr float kRoundMagic = 12582912.0f;
+constexpr float kNearHalf = 0.5f - 1.0f / 4096.0f;
+
+__device__ __forceinline__ float byte_f32(uint32_t word, int k) {
+    return __uint_as_float(__byte_perm(word, 0x4B000000u, 0x7440 | k)) - 8388608.0f;
+}
+
+// v rounded, in the low bits of the returned word; off: the largest distance rounded so far.
+__device__ __forceinline__ uint32_t round_bits(float v, float& off) {
+    v = fminf(fmaxf(v, 0.0f), 255.0f);
+    const float t = v + kRoundMagic;
+    off = fmaxf(off, fabsf(v - (t - kRoundMagic)));
+    return __float_as_uint(t);
+}
+
 template <bool inverse>
-__global__ void convert_kernel(const uint8_t* __restrict__ p0, const uint8_t* __restrict__ p1,
-                               const uint8_t* __restrict__ p2, size_t n,
-                               uint8_t* __restrict__ q0, uint8_t* __restrict__ q1,
-                               uint8_t* __restrict__ q2, bool words) {
-    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t i = 4 * t;
-    if (i >= n) return;
-    if (words && i + 4 <= n) {
-        const uint32_t a = *reinterpret_cast<const uint32_t*>(p0 + i);
-        const uint32_t b = *reinterpret_cast<const uint32_t*>(p1 + i);
-        const uint32_t c = *reinterpret_cast<const uint32_t*>(p2 + i);
-        uint32_t o0 = 0, o1 = 0, o2 = 0;
+__device__ __forceinline__ void convert4(uint32_t a, uint32_t b, uint32_t c, uint32_t& o0,
+                                         uint32_t& o1, uint32_t& o2) {
+    uint32_t x[4], y[4], z[4], redo = 0u;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            uint32_t x, y, z;
-            const uint32_t s = 8 * k;
-            if (inverse) rgb_pixel((a >> s) & 255u, (b >> s) & 255u, (c >> s) & 255u, &x, &y, &z);
-            else ycc_pixel((a >> s) & 255u, (b >> s) & 255u, (c >> s) & 255u, &x, &y, &z);
-            o0 |= x << s;
-            o1 |= y << s;
-            o2 |= z << s;
+    for (int k = 0; k < 4; ++k) {
+        const float p = byte_f32(a, k);
+        float q = byte_f32(b, k), r = byte_f32(c, k), off = 0.0f;
+        if (inverse) {
+            q -= 128.0f;
+            r -= 128.0f;
+            x[k] = round_bits(fmaf(1.402f, r, p), off);
+            y[k] = round_bits(fmaf(-0.714136f, r, fmaf(-0.344136f, q, p)), off);
+            z[k] = round_bits(fmaf(1.772f, q, p), off);
+        } else {
+            x[k] = round_bits(fmaf(0.114f, r, fmaf(0.587f, q, 0.299f * p)), off);
+            y[k] = round_bits(fmaf(0.5f, r, fmaf(-0.331264f, q, fmaf(-0.168736f, p, 128.0f))), off);
+            z[k] = round_bits(fmaf(-0.081312f, r, fmaf(-0.418688f, q, fmaf(0.5f, p, 128.0f))), off);
         }
-        *reinterpret_cast<uint32_t*>(q0 + i) = o0;
-        *reinterpret_cast<uint32_t*>(q1 + i) = o1;
-        *reinterpret_cast<uint32_t*>(q2 + i) = o2;
+        redo |= off > kNearHalf ? 1u << k : 0u;
+    }
+    auto pack = [](const uint32_t (&v)[4]) {
+        return __byte_perm(__byte_perm(v[0], v[1], 0x0040), __byte_perm(v[2], v[3], 0x0040), 0x5410);
+    };
+    o0 = pack(x);
+    o1 = pack(y);
+    o2 = pack(z);
+    while (redo) {
+        const uint32_t s = 8u * (uint32_t)(__ffs(redo) - 1);
+        redo &= redo - 1u;
+        uint32_t u, v, w;
+        if (inverse) rgb_pixel((a >> s) & 255u, (b >> s) & 255u, (c >> s) & 255u, &u, &v, &w);
+        else ycc_pixel((a >> s) & 255u, (b >> s) & 255u, (c >> s) & 255u, &u, &v, &w);
+        const uint32_t keep = ~(255u << s);
+        o0 = (o0 & keep) | u << s;
+        o1 = (o1 & keep) | v << s;
+        o2 = (o2 & keep) | w << s;
+    }
+}
+
+// Three input planes -> three output planes; `inverse` picks the direction.  T: uint4 where all
+// six planes start on 16 bytes, uint32_t on 4, uint8_t otherwise: a thread takes kPerThread
+// pixels, the last ones byte by byte.
+template <bool inverse, class T>
+__global__ void __launch_bounds__(256)
+    convert_kernel(const uint8_t* __restrict__ p0, const uint8_t* __restrict__ p1,
+                   const uint8_t* __restrict__ p2, size_t n, uint8_t* __restrict__ q0,
+                   uint8_t* __restrict__ q1, uint8_t* __restrict__ q2) {
+    constexpr int P = sizeof(T) < 4 ? 4 : (int)sizeof(T);
+    const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * P;
+    if (i >= n) return;
+    if (sizeof(T) >= 4 && i + P <= n) {
+        constexpr int W = P / 4;
+        union Words {
+            T all;
+            uint32_t w[W];
+        } a, b, c, x, y, z;
+        a.all = *reinterpret_cast<const T*>(p0 + i);
+        b.all = *reinterpret_cast<const T*>(p1 + i);
+        c.all = *reinterpret_cast<const T*>(p2 + i);
+#pragma unroll
+        for (int k = 0; k < W; ++k)
+            convert4<inverse>(a.w[k], b.w[k], c.w[k], x.w[k], y.w[k], z.w[k]);
+        *reinterpret_cast<T*>(q0 + i) = x.all;
+        *reinterpret_cast<T*>(q1 + i) = y.all;
+        *reinterpret_cast<T*>(q2 + i) = z.all;
         return;
     }
-    for (size_t k = i; k < n && k < i + 4; ++k) {
+    for (size_t k = i; k < n && k < i + P; ++k) {
         uint32_t x, y, z;
-        if (inverse) rgb_pixel(p0[k], p1[k], p2[k], &x, &y, &z);
-        else ycc_pixel(p0[k], p1[k], p2[k], &x, &y, &z);
+        convert4<inverse>(p0[k], p1[k], p2[k], x, y, z);
         q0[k] = (uint8_t)x;
         q1[k] = (uint8_t)y;
         q2[k] = (uint8_t)z;
     }
 }
 
-__global__ void downsample_box_kernel(const uint8_t* __restrict__ src, int w, int h,
-                                      uint8_t* __restrict__ dst, int ow, int oh) {
-    const int ox = blockIdx.x * blockDim.x + threadIdx.x, oy = blockIdx.y;
-    if (ox >= ow || oy >= oh) return;
-    const int x0 = 2 * ox, y0 = 2 * oy;
-    const int x1 = min(x0 + 1, w - 1), y1 = min(y0 + 1, h - 1);
-    const uint32_t sum = (uint32_t)src[(size_t)y0 * w + x0] + src[(size_t)y0 * w + x1] +
-                         src[(size_t)y1 * w + x0] + src[(size_t)y1 * w + x1];
-    dst[(size_t)oy * ow + ox] = (uint8_t)((sum + 2) / 4);
+// Eight bytes from address p, not necessarily aligned, of which the caller's plane holds
+// `inside` (at least 8) from p on: two aligned loads where they stay in the plane.
+__device__ __forceinline__ uint64_t unaligned8(const uint8_t* p, size_t inside) {
+    const unsigned s = (unsigned)(reinterpret_cast<uintptr_t>(p) & 7);
+    const uint64_t* q = reinterpret_cast<const uint64_t*>(p - s);
+    if (s == 0) return __ldg(q);
+    if (inside >= 16) {
+        // The first word's leading bytes lie before p, in the same 8-byte word as p's.
+        return (__ldg(q) >> (8 * s)) | (__ldg(q + 1) << (64 - 8 * s));
+    }
+    uint64_t v = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v |= (uint64_t)__ldg(p + k) << (8 * k);
+    return v;
 }
 
-__global__ void upsample_nearest_kernel(const uint8_t* __restrict__ src, int sw, int sh,
-                                        uint8_t* __restrict__ dst, int w, int h) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
-    if (x >= w || y >= h) return;
-    const int sy = min(y / 2, sh - 1), sx = min(x / 2, sw - 1);
-    dst[(size_t)y * w + x] = src[(size_t)sy * sw + sx];
+// Both resamplings walk the output as one run of bytes in aligned chunks of K, so that a chunk
+// is one store at any width; a chunk inside one row and away from the replicated border comes
+// from word loads, any other byte by byte.
+struct Chunk {
+    uint32_t x, y;
+    size_t begin, end;  // of the output's bytes
+};
+
+template <int K>
+__device__ __forceinline__ bool output_chunk(const uint8_t* dst, size_t n, uint32_t w, Chunk* c) {
+    const size_t lead = reinterpret_cast<uintptr_t>(dst) & (K - 1);
+    const size_t at = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * K;
+    if (at >= n + lead) return false;
+    c->begin = at < lead ? 0 : at - lead;
+    c->end = min(at + K - lead, n);
+    c->y = (uint32_t)c->begin / w;  // sides are at most 65535: 32 bits hold any position
+    c->x = (uint32_t)c->begin - c->y * w;
+    return true;
+}
+
+// 9.2 us a 3840 x 2160 plane with a byte a thread.
+__global__ void __launch_bounds__(256)
+    downsample_box_kernel(const uint8_t* __restrict__ src, int w, int h, uint8_t* __restrict__ dst,
+                          int ow, int oh) {
+    Chunk c;
+    if (!output_chunk<8>(dst, (size_t)ow * oh, (uint32_t)ow, &c)) return;
+    const size_t total = (size_t)w * h;
+    if (c.end - c.begin == 8 && c.x + 8 <= (uint32_t)(w / 2)) {
+        const size_t top = (size_t)(2 * c.y) * w + 2 * c.x;
+        const size_t low = (int)(2 * c.y + 1) < h ? top + w : top;
+        uint32_t out[2];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const uint64_t a = unaligned8(src + top + 8 * k, total - top - 8 * k);
+            const uint64_t b = unaligned8(src + low + 8 * k, total - low - 8 * k);
+            // Byte pairs' sums in 16-bit lanes, two rows, rounded.
+            constexpr uint64_t kEven = 0x00FF00FF00FF00FFull;
+            const uint64_t s = (a & kEven) + (a >> 8 & kEven) + (b & kEven) + (b >> 8 & kEven) +
+                               0x0002000200020002ull;
+            const uint64_t m = s >> 2;
+            out[k] = __byte_perm((uint32_t)m, (uint32_t)(m >> 32), 0x6420);
+        }
+        *reinterpret_cast<uint2*>(dst + c.begin) = make_uint2(out[0], out[1]);
+        return;
+    }
+    for (size_t i = c.begin; i < c.end; ++i) {
+        const int x0 = 2 * (int)c.x, y0 = 2 * (int)c.y;
+        const int x1 = min(x0 + 1, w - 1), y1 = min(y0 + 1, h - 1);
+        const uint32_t sum = (uint32_t)src[(size_t)y0 * w + x0] + src[(size_t)y0 * w + x1] +
+                             src[(size_t)y1 * w + x0] + src[(size_t)y1 * w + x1];
+        dst[i] = (uint8_t)((sum + 2) / 4);
+        if (++c.x == (uint32_t)ow) {
+            c.x = 0;
+            ++c.y;
+        }
+    }
+}
+
+// 22.3 us for a 3840 x 2160 output with a byte a thread.
+__global__ void __launch_bounds__(256)
+    upsample_nearest_kernel(const uint8_t* __restrict__ src, int sw, int sh,
+                            uint8_t* __restrict__ dst, int w, int h) {
+    Chunk c;
+    if (!output_chunk<16>(dst, (size_t)w * h, (uint32_t)w, &c)) return;
+    const size_t total = (size_t)sw * sh;
+    const uint32_t sx = c.x / 2;
+    if (c.end - c.begin == 16 && c.x + 16 <= (uint32_t)w && sx + 8 + (c.x & 1u) <= (uint32_t)sw) {
+        const size_t at = (size_t)min((int)(c.y / 2), sh - 1) * sw + sx;
+        const uint64_t v = unaligned8(src + at, total - at);
+        const uint32_t lo = (uint32_t)v, hi = (uint32_t)(v >> 32);
+        uint32_t o[4] = {__byte_perm(lo, 0, 0x1100), __byte_perm(lo, 0, 0x3322),
+                         __byte_perm(hi, 0, 0x1100), __byte_perm(hi, 0, 0x3322)};
+        if (c.x & 1u) {  // starts with the second copy of its first sample
+            const uint32_t last = __ldg(src + at + 8);
+            o[0] = __funnelshift_r(o[0], o[1], 8);
+            o[1] = __funnelshift_r(o[1], o[2], 8);
+            o[2] = __funnelshift_r(o[2], o[3], 8);
+            o[3] = __funnelshift_r(o[3], last, 8);
+        }
+        *reinterpret_cast<uint4*>(dst + c.begin) = make_uint4(o[0], o[1], o[2], o[3]);
+        return;
+    }
+    for (size_t i = c.begin; i < c.end; ++i) {
+        dst[i] = src[(size_t)min((int)(c.y / 2), sh - 1) * sw + min((int)(c.x / 2), sw - 1)];
+        if (++c.x == (uint32_t)w) {
+            c.x = 0;
+            ++c.y;
+        }
+    }
 }
 
 // Sum of squared differences: per-thread partial sums over 16-byte chunks, a warp and block
@@ -121,12 +272,10 @@ __global__ void sse_kernel(const uint8_t* __restrict__ a, const uint8_t* __restr
             const uint32_t xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};
             uint32_t s = 0;  // 16 squares of at most 65025: fits 32 bits
 #pragma unroll
-            for (int k = 0; k < 4; ++k)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const int d = (int)((xs[k] >> (8 * j)) & 255u) - (int)((ys[k] >> (8 * j)) & 255u);
-                    s += (uint32_t)(d * d);
-                }
+            for (int k = 0; k < 4; ++k) {
+                const uint32_t d = __vabsdiffu4(xs[k], ys[k]);
+                s = __dp4a(d, d, s);
+            }
             acc += s;
         }
         for (size_t i = nv * 16 + tid; i < n; i += stride) {
@@ -152,17 +301,25 @@ __global__ void sse_kernel(const uint8_t* __restrict__ a, const uint8_t* __restr
 
 }  // namespace
 
+// Blocks of 256 threads for the chunks of n output bytes (output_chunk).
+static unsigned chunk_blocks(const uint8_t* dst, size_t n, size_t k) {
+    const size_t chunks = (n + (reinterpret_cast<uintptr_t>(dst) & (k - 1)) + k - 1) / k;
+    return (unsigned)((chunks + 255) / 256);
+}
+
 cudaError_t launch_ycbcr(const uint8_t* r, const uint8_t* g, const uint8_t* b, size_t n,
                          uint8_t* y, uint8_t* cb, uint8_t* cr, bool inverse, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
-    const bool words = ((reinterpret_cast<uintptr_t>(r) | reinterpret_cast<uintptr_t>(g) |
+    const uintptr_t at = reinterpret_cast<uintptr_t>(r) | reinterpret_cast<uintptr_t>(g) |
                          reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(y) |
-                         reinterpret_cast<uintptr_t>(cb) | reinterpret_cast<uintptr_t>(cr)) &
-                        3) == 0;
-    const size_t threads = (n + 3) / 4;
-    const unsigned blocks = (unsigned)((threads + 255) / 256);
-    if (inverse) convert_kernel<true><<<blocks, 256, 0, st>>>(r, g, b, n, y, cb, cr, words);
-    else convert_kernel<false><<<blocks, 256, 0, st>>>(r, g, b, n, y, cb, cr, words);
+                         reinterpret_cast<uintptr_t>(cb) | reinterpret_cast<uintptr_t>(cr);
+    auto launch = [&](auto kernel, size_t per_thread) {
+        const size_t threads = (n + per_thread - 1) / per_thread;
+        kernel<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(r, g, b, n, y, cb, cr);
+    };
+    if (at % 16 == 0) inverse ? launch(convert_kernel<true, uint4>, 16) : launch(convert_kernel<false, uint4>, 16);
+    else if (at % 4 == 0) inverse ? launch(convert_kernel<true, uint32_t>, 4) : launch(convert_kernel<false, uint32_t>, 4);
+    else inverse ? launch(convert_kernel<true, uint8_t>, 4) : launch(convert_kernel<false, uint8_t>, 4);
     return cudaGetLastError();
 }
 
@@ -170,14 +327,14 @@ cudaError_t launch_downsample_box(const uint8_t* src, int w, int h, uint8_t* dst
                                   cudaStream_t st) {
     const int ow = (w + 1) / 2, oh = (h + 1) / 2;
     if (ow == 0 || oh == 0) return cudaSuccess;
-    downsample_box_kernel<<<dim3((ow + 255) / 256, oh), 256, 0, st>>>(src, w, h, dst, ow, oh);
+    downsample_box_kernel<<<chunk_blocks(dst, (size_t)ow * oh, 8), 256, 0, st>>>(src, w, h, dst, ow, oh);
     return cudaGetLastError();
 }
 
 cudaError_t launch_upsample_nearest(const uint8_t* src, int sw, int sh, uint8_t* dst, int w,
                                     int h, cudaStream_t st) {
     if (w == 0 || h == 0) return cudaSuccess;
-    upsample_nearest_kernel<<<dim3((w + 255) / 256, h), 256, 0, st>>>(src, sw, sh, dst, w, h);
+    upsample_nearest_kernel<<<chunk_blocks(dst, (size_t)w * h, 16), 256, 0, st>>>(src, sw, sh, dst, w, h);
     return cudaGetLastError();
 }
 

@@ -52,6 +52,62 @@ def test_downsample_and_upsample(ctx, shape):
     assert np.array_equal(ctx.upsample_nearest(d, w, h), orc.upsample_nearest(d, w, h))
 
 
+def test_every_colour(ctx):
+    # All 2^24: every value that lies near a half, the exact halves among them.
+    v = np.arange(1 << 24, dtype=np.uint32)
+    r, g, b = ((v >> s & 255).astype(np.uint8).reshape(4096, 4096) for s in (0, 8, 16))
+    for x, y in zip(ctx.ycbcr(r, g, b), orc.ycbcr(r, g, b)):
+        assert np.array_equal(x, y)
+    for x, y in zip(ctx.rgb_from_ycbcr(r, g, b), orc.rgb_from_ycbcr(r, g, b)):
+        assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("offset", [0, 1, 4, 8, 13])
+@pytest.mark.parametrize("shape", [(2, 15), (3, 16), (5, 33), (8, 64), (7, 130)])
+def test_planes_at_any_address(ctx, shape, offset):
+    # Word loads and stores at every alignment; a byte on either side of each output stays.
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(shape[1] + offset)
+    h, w = shape
+    hw, hh = (w + 1) // 2, (h + 1) // 2
+    host = [rng.integers(0, 256, (h, w), dtype=np.uint8) for _ in range(3)]
+
+    def place(a):
+        buf = torch.full((a.size + 32,), 77, dtype=torch.uint8, device="cuda:0")
+        buf[offset: offset + a.size] = torch.from_numpy(a.ravel()).cuda()
+        return buf
+
+    def out(n):
+        return torch.full((n + 32,), 77, dtype=torch.uint8, device="cuda:0")
+
+    def taken(buf, shape):
+        n = shape[0] * shape[1]
+        got = buf.cpu().numpy()
+        assert (got[:offset] == 77).all() and (got[offset + n:] == 77).all()
+        return got[offset: offset + n].reshape(shape)
+
+    L = mb.lib()
+    src = [place(a) for a in host]
+    dst, down, up = [out(h * w) for _ in range(3)], out(hh * hw), out(h * w)
+    torch.cuda.synchronize()
+    mb.check(L.mars_ycbcr_device(ctx.handle, *(t.data_ptr() + offset for t in src), h * w,
+                                 *(t.data_ptr() + offset for t in dst)))
+    mb.check(L.mars_downsample_box_device(ctx.handle, src[0].data_ptr() + offset, w, h,
+                                          down.data_ptr() + offset))
+    mb.check(L.mars_upsample_nearest_device(ctx.handle, down.data_ptr() + offset, hw, hh,
+                                            up.data_ptr() + offset, w, h))
+    mse = mb.C.c_double()
+    mb.check(L.mars_mse_device(ctx.handle, src[0].data_ptr() + offset, up.data_ptr() + offset,
+                               h * w, mb.C.byref(mse)))
+    for x, y in zip(dst, orc.ycbcr(*host)):
+        assert np.array_equal(taken(x, shape), y)
+    want = orc.downsample_box(host[0])
+    assert np.array_equal(taken(down, (hh, hw)), want)
+    want = orc.upsample_nearest(want, w, h)
+    assert np.array_equal(taken(up, shape), want)
+    assert mse.value == orc.mse(host[0], want)
+
+
 @pytest.mark.parametrize("n", [1, 15, 16, 17, 4096, 1 << 20, (1 << 20) + 3])
 def test_mse(ctx, n):
     rng = np.random.default_rng(n)
