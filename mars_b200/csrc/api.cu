@@ -2523,6 +2523,7 @@ struct mars_decode_plan {
     uint32_t* d_inv = nullptr;
     uint4* d_cellbuf = nullptr;
     uint32_t njobs = 0;
+    bool wide_jobs = false;
 };
 
 namespace {
@@ -2581,7 +2582,20 @@ int mars_decode(mars_ctx* ctx, const mars_header* hdr, const mars_leaf* leaves, 
                                              ctx->stream));
         ctx->launches += 1;
     }
-    MARS_CUDA(cudaMemsetAsync(a, 128, px, ctx->stream));
+    uint32_t* d_sync = nullptr;
+    MARS_CUDA(sc.get(&d_sync, 2));
+    MARS_CUDA(cudaMemsetAsync(d_sync, 0, 2 * sizeof(uint32_t), ctx->stream));
+    bool resident = false;
+    MARS_CUDA(mars::launch_decode_resident(a, b, (int)w, (int)h, lg, d_owner, d_maps, d_rvals,
+                                           iterations, d_sync, nullptr, 0, nullptr, ctx->d_err,
+                                           ctx->num_sms, ctx->stream, &resident));
+    if (resident) {
+        ctx->launches += 1;
+        if (iterations & 1) std::swap(a, b);
+        iterations = 0;
+    } else {
+        MARS_CUDA(cudaMemsetAsync(a, 128, px, ctx->stream));
+    }
     for (uint32_t it = 0; it < iterations; ++it) {
         MARS_CUDA(mars::launch_decode_step(a, b, (int)w, (int)h, lg, d_owner, d_maps, d_rvals,
                                            ctx->stream));
@@ -2639,13 +2653,13 @@ int mars_decode_plan_create(mars_ctx* ctx, const mars_header* hdr, const mars_le
         ctx->launches += 1;
     }
     p->consts = consts;
-    uint32_t *d_key = nullptr, *d_rows = nullptr, *d_cursor = nullptr;
+    uint32_t *d_key = nullptr, *d_rows = nullptr, *d_cursor = nullptr, counts[2] = {0, 0};
     if (e == cudaSuccess && n && want_sorted_decode(p->w, p->h) &&
         mars::decode_sorted_eligible((int)p->w, (int)p->h, lg, !rvals.empty())) {
         const size_t cells = mars::decode_sorted_cells((int)p->w, (int)p->h);
         e = cudaMalloc(&d_key, cells * 4);
         if (e == cudaSuccess) e = cudaMalloc(&d_rows, (size_t)p->h * 4);
-        if (e == cudaSuccess) e = cudaMalloc(&d_cursor, ((size_t)p->h + 1) * 4);
+        if (e == cudaSuccess) e = cudaMalloc(&d_cursor, ((size_t)p->h + 2) * 4);
         if (e == cudaSuccess) e = cudaMalloc(&p->d_jobs, cells * sizeof(uint4));
         if (e == cudaSuccess) e = cudaMalloc(&p->d_inv, cells * 4);
         if (e == cudaSuccess) e = cudaMalloc(&p->d_cellbuf, cells * sizeof(uint4));
@@ -2654,10 +2668,12 @@ int mars_decode_plan_create(mars_ctx* ctx, const mars_header* hdr, const mars_le
                                                  d_leaves, d_key, d_rows, d_cursor, p->d_jobs,
                                                  p->d_inv, ctx->stream);
         if (e == cudaSuccess)
-            e = cudaMemcpyAsync(&p->njobs, d_cursor + p->h, 4, cudaMemcpyDeviceToHost, ctx->stream);
+            e = cudaMemcpyAsync(counts, d_cursor + p->h, 8, cudaMemcpyDeviceToHost, ctx->stream);
         ctx->launches += 3;
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    p->njobs = counts[0];
+    p->wide_jobs = counts[1] != 0;
     cudaFree(d_leaves);
     cudaFree(d_roff);
     cudaFree(d_key);
@@ -2690,8 +2706,8 @@ int mars_decode_plan_run(mars_decode_plan* p, uint32_t iterations, uint8_t* d_ou
     for (uint32_t it = 0; it < iterations; ++it) {
         if (p->d_jobs) {
             MARS_CUDA(mars::launch_decode_sorted_step(a, b, (int)p->w, (int)p->h, p->lg, p->d_owner,
-                                                      p->d_maps, p->d_jobs, p->njobs, p->d_inv,
-                                                      p->consts, p->d_cellbuf, ctx->stream));
+                                                      p->d_maps, p->d_jobs, p->njobs, p->wide_jobs,
+                                                      p->d_inv, p->consts, p->d_cellbuf, ctx->stream));
             ctx->launches += 2;
         } else {
             MARS_CUDA(mars::launch_decode_step(a, b, (int)p->w, (int)p->h, p->lg, p->d_owner,
@@ -2714,14 +2730,24 @@ int mars_decode_plan_run_until_stable(mars_decode_plan* p, uint8_t threshold,
     MARS_CUDA(cudaSetDevice(ctx->device));
     const size_t px = (size_t)p->w * p->h;
     Scratch sc(ctx->stream);
-    int* d_state = nullptr;  // [0] done, [1] used, [2 + i] step i's max delta
-    MARS_CUDA(sc.get(&d_state, 2 + (size_t)iters));
-    MARS_CUDA(cudaMemsetAsync(d_state, 0, (2 + (size_t)iters) * sizeof(int), ctx->stream));
+    // [0] done, [1] used, [2 + i] step i's max delta, then the one launch's two words
+    int* d_state = nullptr;
+    MARS_CUDA(sc.get(&d_state, 4 + (size_t)iters));
+    MARS_CUDA(cudaMemsetAsync(d_state, 0, (4 + (size_t)iters) * sizeof(int), ctx->stream));
     // Step i reads buf[i % 2] and writes buf[(i + 1) % 2]; the decode that stopped after
     // `used` steps ends in buf[used % 2].
     uint8_t* buf[2] = {d_out, p->d_tmp};
-    MARS_CUDA(cudaMemsetAsync(buf[0], 128, px, ctx->stream));
-    for (uint32_t it = 0; it < iters; ++it) {
+    bool resident = false;
+    MARS_CUDA(mars::launch_decode_resident(buf[0], buf[1], (int)p->w, (int)p->h, p->lg, p->d_owner,
+                                           p->d_maps, p->d_rvals, iters,
+                                           (uint32_t*)(d_state + 2 + iters), d_state + 2,
+                                           (int)threshold, d_state, ctx->d_err, ctx->num_sms,
+                                           ctx->stream, &resident));
+    if (resident)
+        ctx->launches += 1;
+    else
+        MARS_CUDA(cudaMemsetAsync(buf[0], 128, px, ctx->stream));
+    for (uint32_t it = 0; !resident && it < iters; ++it) {
         MARS_CUDA(mars::launch_decode_step_stable(buf[it & 1], buf[(it + 1) & 1], (int)p->w,
                                                   (int)p->h, p->lg, p->d_owner, p->d_maps,
                                                   p->d_rvals, d_state, d_state + 2 + it,

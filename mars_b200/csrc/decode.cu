@@ -130,6 +130,33 @@ __global__ void decode_expand_kernel(const DecodeLeaf* __restrict__ leaves,
     } else {
         kind = kLeafDomain;
     }
+    // The integer form.  Where alfa / 4 is A / 64 (A up to 32: contrasts in sixteenths up to 2,
+    // as streams have them), 0.5 + sum * A / 64 is exact and the pixel is the f64 sum of that and
+    // beta, truncated: floor((32 + sum * A + floor(64 beta)) / 64) in integers, unless the f64
+    // sum rounds up to the next integer, for which the fraction of 64 beta must be nearly 1
+    // (sums stay below 2^11, so within 2^-36; the limit of 2^-20 is generous).  An affine pixel's
+    // gradients are sixty-fourths, its half rounds up (below zero everything clamps), and its two
+    // roundings are below 2^-23 sixty-fourths for |64 value| < 2^29.
+    m.n0 = m.n1 = m.n2 = m.unused = 0;
+    const double b64 = 64.0 * (kind == kLeafAffine ? m.a : m.b), low = floor(b64);
+    const bool whole = b64 - low < 1.0 - 0x1p-20;
+    if (kind == kLeafDomain) {
+        const double times = 64.0 * m.a, base = low + 32.0;
+        if (whole && times == floor(times) && times >= 0.0 && times <= 32.0 && base >= -32768.0 &&
+            base + 1020.0 * times <= 32767.0) {
+            m.n0 = (int)(((uint32_t)(int)base & 0xFFFFu) * 0x10001u);
+            m.n1 = (int)times;
+            flags |= kLeafInteger;
+        }
+    } else if (kind == kLeafAffine) {
+        const double reach = (fabs(m.gx) + fabs(m.gy)) * 64.0 * L.size + fabs(b64);
+        if (whole && reach < 0x1p29) {
+            m.n0 = (int)low + 32;
+            m.n1 = (int)leaves[k].z;
+            m.n2 = (int)leaves[k].w;
+            flags |= kLeafInteger;
+        }
+    }
     m.info = (uint32_t)L.size | (kind << 12) | ((uint32_t)L.iso << 14) | flags | (cbyte << 24);
     maps[k] = m;
 }
@@ -140,9 +167,14 @@ __device__ __forceinline__ double domain_value(int sum, const DecodeMap& m) {
     return __dadd_rn(__dadd_rn(0.5, __dmul_rn((double)sum, m.a)), m.b);
 }
 
+__device__ __forceinline__ uint32_t sixty_fourths(int n) {
+    return (uint32_t)min(max(n >> 6, 0), 255);
+}
+
 // Mode 1: round(b0 + gx*u + gy*v) with (u, v) = (i, j) (ifs.rs:416-431); f64::round and
 // CUDA's round() both round half away from zero.
 __device__ __forceinline__ uint32_t affine_pixel(const DecodeMap& m, int i, int j) {
+    if (m.info & kLeafInteger) return sixty_fourths(m.n0 + m.n1 * i + m.n2 * j);
     return clamp_u8(round(__dadd_rn(__dadd_rn(m.a, __dmul_rn(m.gx, (double)i)),
                                     __dmul_rn(m.gy, (double)j))));
 }
@@ -194,9 +226,13 @@ __global__ void decode_pixel_kernel(const uint8_t* __restrict__ src, uint8_t* __
                 const size_t p = ((size_t)(m.dom & 0xFFFFu) + 2 * u) * w + (m.dom >> 16) + 2 * v;
                 sum = (int)src[p] + (int)src[p + w] + (int)src[p + 1] + (int)src[p + w + 1];
             }
-            double value = domain_value(sum, m);
-            if (kind == kLeafResidual) value = __dadd_rn(value, resid[m.roff + u * S + v]);
-            out = to_u8(value);
+            if (m.info & kLeafInteger) {
+                out = sixty_fourths((int)(int16_t)m.n0 + m.n1 * sum);
+            } else {
+                double value = domain_value(sum, m);
+                if (kind == kLeafResidual) value = __dadd_rn(value, resid[m.roff + u * S + v]);
+                out = to_u8(value);
+            }
         }
     }
     dst[(size_t)y * w + x] = (uint8_t)out;
@@ -206,24 +242,189 @@ __global__ void decode_pixel_kernel(const uint8_t* __restrict__ src, uint8_t* __
     }
 }
 
-// Eight bytes of the plane from byte offset `off` (off + 8 <= total), through aligned
-// 8-byte loads where they stay inside the plane.
-__device__ __forceinline__ uint64_t load8(const uint8_t* __restrict__ src, size_t off,
-                                          size_t total) {
-    const size_t a = off & ~(size_t)7;
-    const unsigned s = (unsigned)(off & 7);
-    const uint64_t* p = reinterpret_cast<const uint64_t*>(src + a);
-    if (s == 0) return __ldg(p);
-    if (a + 16 <= total) return (__ldg(p) >> (8 * s)) | (__ldg(p + 1) << (64 - 8 * s));
-    uint64_t v = 0;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) v |= (uint64_t)__ldg(src + off + k) << (8 * k);
+// Loads of a plane, made where they stand.  FRESH: other SMs write the plane during the launch,
+// so L1 is passed by (and no load may move across a barrier).
+template <bool FRESH>
+__device__ __forceinline__ uint4 plane16(const uint8_t* p) {
+    if (!FRESH) return __ldg(reinterpret_cast<const uint4*>(p));
+    uint4 v;
+    asm volatile("ld.global.cg.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "l"(p)
+                 : "memory");
+    return v;
+}
+// Eight bytes where `take`, else 0, without a branch.
+template <bool FRESH>
+__device__ __forceinline__ uint64_t plane8_if(const uint8_t* p, bool take) {
+    uint64_t v;
+    if (FRESH)
+        asm volatile("{.reg .pred q; setp.ne.u32 q, %2, 0; mov.u64 %0, 0;"
+                     " @q ld.global.cg.u64 %0, [%1];}"
+                     : "=l"(v)
+                     : "l"(p), "r"((uint32_t)take)
+                     : "memory");
+    else
+        asm volatile("{.reg .pred q; setp.ne.u32 q, %2, 0; mov.u64 %0, 0;"
+                     " @q ld.global.nc.u64 %0, [%1];}"
+                     : "=l"(v)
+                     : "l"(p), "r"((uint32_t)take));
+    return v;
+}
+template <bool FRESH>
+__device__ __forceinline__ uint32_t plane1(const uint8_t* p) {
+    if (!FRESH) return __ldg(p);
+    uint32_t v;
+    asm volatile("ld.global.cg.u8 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
 
 // Byte-pair sums of a 4-byte word in two 16-bit lanes: [b0 + b1, b2 + b3].
 __device__ __forceinline__ uint32_t pair_sums(uint32_t x) {
     return (x & 0x00FF00FFu) + ((x >> 8) & 0x00FF00FFu);
+}
+
+// The 2x2 sums of the 8x8 byte window at `off` of the plane src[0 .. total), in 16-bit lanes.
+// A row's 8 bytes come from the aligned 16 around their start, and the next 8 where they reach
+// past those (3 in 8, columns being even).  All rows' loads are in flight together: there is one
+// branch, for the windows so close to an end of the plane that an aligned load might leave it.
+// (With a branch and two 8-byte loads a row the rows waited for one another: with the f64 values
+// as well, ten steps of 512 x 512 took 85 us, 47 now, of 4096 x 4096 417, 314 now.)
+template <bool FRESH>
+__device__ __forceinline__ void window_sums(const uint8_t* src, size_t off, int w, size_t total,
+                                            uint32_t (&sums)[4][2]) {
+    if (off >= 15 && off + 7 * (size_t)w + 24 <= total) {
+        const uint8_t* p = src + off;
+        uint4 x[8];
+        uint64_t t[8];
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            const uint8_t* q = p + (size_t)r * w;
+            const unsigned s = (unsigned)(reinterpret_cast<uintptr_t>(q) & 15);
+            x[r] = plane16<FRESH>(q - s);
+            t[r] = plane8_if<FRESH>(q - s + 16, s > 8);
+        }
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            const unsigned s = (unsigned)(reinterpret_cast<uintptr_t>(p + (size_t)r * w) & 15);
+            // The 24 bytes x | t from byte s on, in 32-bit funnel shifts.
+            const bool up = s & 8, mid = s & 4;
+            const uint32_t w0 = up ? x[r].z : x[r].x, w1 = up ? x[r].w : x[r].y;
+            const uint32_t w2 = up ? (uint32_t)t[r] : x[r].z;
+            const uint32_t w3 = up ? (uint32_t)(t[r] >> 32) : x[r].w;
+            const uint32_t a = mid ? w1 : w0, b = mid ? w2 : w1, c = mid ? w3 : w2;
+            const unsigned at = 8 * (s & 3);
+            const uint32_t lo = pair_sums(__funnelshift_r(a, b, at));
+            const uint32_t hi = pair_sums(__funnelshift_r(b, c, at));
+            uint32_t(&to)[2] = sums[r / 2];
+            to[0] = r & 1 ? to[0] + lo : lo;
+            to[1] = r & 1 ? to[1] + hi : hi;
+        }
+        return;
+    }
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+        uint64_t row = 0;
+#pragma unroll 1
+        for (int k = 0; k < 8; ++k)
+            row |= (uint64_t)plane1<FRESH>(src + off + (size_t)r * w + k) << (8 * k);
+        uint32_t(&to)[2] = sums[r / 2];
+        to[0] = (r & 1 ? to[0] : 0u) + pair_sums((uint32_t)row);
+        to[1] = (r & 1 ? to[1] : 0u) + pair_sums((uint32_t)(row >> 32));
+    }
+}
+
+// Four values of the integer form, two to a word: the lanes' products stay below 2^15.
+__device__ __forceinline__ uint32_t integer_values(const uint32_t (&sums)[2], uint32_t times,
+                                                   uint32_t base) {
+    const uint32_t a = __viaddmin_s16x2_relu(sums[0] * times, base, 0x3FFF3FFFu) >> 6;
+    const uint32_t b = __viaddmin_s16x2_relu(sums[1] * times, base, 0x3FFF3FFFu) >> 6;
+    return __byte_perm(a, b, 0x6420);
+}
+
+// Values in sample order (byte q of word p is sample (umin + p, vmin + q)) to output order:
+// sample (p, q) is output pixel (a, b) with a = p (or 3 - p when u counts down) and b = q (or
+// 3 - q when v counts down), transposed for isometries 1, 2, 6, 7.
+__device__ __forceinline__ void to_output_order(int k, uint32_t (&rw)[4]) {
+    const bool tr = (0xC6u >> k) & 1u, uneg = (0xACu >> k) & 1u, vneg = (0x9Au >> k) & 1u;
+    if (vneg) {
+#pragma unroll
+        for (int p = 0; p < 4; ++p) rw[p] = __byte_perm(rw[p], 0, 0x0123);
+    }
+    if (uneg) {
+        const uint32_t t0 = rw[0], t1 = rw[1];
+        rw[0] = rw[3];
+        rw[1] = rw[2];
+        rw[2] = t1;
+        rw[3] = t0;
+    }
+    if (tr) transpose4x4(rw[0], rw[1], rw[2], rw[3]);
+}
+
+// The first sample (umin, vmin) of a domain cell's 4x4, (x0, y0) the cell.
+__device__ __forceinline__ void cell_sample(const DecodeMap& m, int x0, int y0, int* umin,
+                                            int* vmin) {
+    const IsoInv t = iso_inverse((int)((m.info >> 14) & 7u), (int)(m.info & 0xFFFu) - 1);
+    const int i0 = y0 - (int)(m.rc & 0xFFFFu), j0 = x0 - (int)(m.rc >> 16);
+    *umin = t.cu + t.ai * i0 + t.aj * j0 - 3 * ((t.ai < 0) | (t.aj < 0));
+    *vmin = t.cv + t.bi * i0 + t.bj * j0 - 3 * ((t.bi < 0) | (t.bj < 0));
+}
+
+// The four output rows of a cell whose leaf reads no domain, from a loaded map.
+__device__ __forceinline__ void still_rows(const DecodeMap& m, int x0, int y0, uint32_t (&rw)[4]) {
+    if (((m.info >> 12) & 3u) == kLeafConst) {
+        rw[0] = rw[1] = rw[2] = rw[3] = 0x01010101u * (m.info >> 24);
+        return;
+    }
+    const int i0 = y0 - (int)(m.rc & 0xFFFFu), j0 = x0 - (int)(m.rc >> 16);
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        rw[a] = 0u;
+#pragma unroll
+        for (int b = 0; b < 4; ++b) rw[a] |= affine_pixel(m, i0 + a, j0 + b) << (8 * b);
+    }
+}
+
+// The four output rows of a domain or residual cell from its window's sums.
+__device__ __forceinline__ void domain_rows(const DecodeMap& m, const uint32_t (&sums)[4][2],
+                                            const double* __restrict__ resid, int umin, int vmin,
+                                            uint32_t (&rw)[4]) {
+    if (m.info & kLeafInteger) {
+#pragma unroll
+        for (int p = 0; p < 4; ++p) rw[p] = integer_values(sums[p], (uint32_t)m.n1, (uint32_t)m.n0);
+    } else {
+        const bool residual = ((m.info >> 12) & 3u) == kLeafResidual;
+        const int S = (int)(m.info & 0xFFFu);
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+            rw[p] = 0u;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int sum = (int)((sums[p][q >> 1] >> (16 * (q & 1))) & 0xFFFFu);
+                double value = domain_value(sum, m);
+                if (residual)
+                    value = __dadd_rn(value, __ldg(resid + m.roff + (umin + p) * S + vmin + q));
+                rw[p] |= to_u8(value) << (8 * q);
+            }
+        }
+    }
+    to_output_order((int)((m.info >> 14) & 7u), rw);
+}
+
+__device__ __forceinline__ void store_rows(uint8_t* out, int w, int rows, const uint32_t (&rw)[4]) {
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+        if (a < rows) *reinterpret_cast<uint32_t*>(out + (size_t)a * w) = rw[a];
+}
+
+// Largest byte of |a - b| over the cell's rows in the plane, b(row) the previous words.
+template <class F>
+__device__ __forceinline__ uint32_t rows_delta(const uint32_t (&rw)[4], int rows, F b) {
+    uint32_t m = 0;
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+        if (a < rows) m = __vmaxu4(m, __vabsdiffu4(rw[a], b(a)));
+    return max(max(m & 255u, (m >> 8) & 255u), max((m >> 16) & 255u, m >> 24));
 }
 
 template <bool kStable>
@@ -240,91 +441,151 @@ __global__ void __launch_bounds__(128) decode_cell_kernel(
     }
     if (x0 >= w || y0 >= h) return;
     const int32_t li = owner[(size_t)(y0 >> lg) * mw + (x0 >> lg)];
-    uint64_t lo = 0, hi = 0;  // output rows 0-1 and 2-3, byte 4*a + b = pixel (y0 + a, x0 + b)
+    uint32_t rw[4] = {0, 0, 0, 0};  // output rows, byte b of word a = pixel (y0 + a, x0 + b)
     if (li >= 0) {
         const DecodeMap m = maps[li];
-        const uint32_t kind = (m.info >> 12) & 3u;
-        const int i0 = y0 - (int)(m.rc & 0xFFFFu), j0 = x0 - (int)(m.rc >> 16);
-        if (kind == kLeafConst) {
-            lo = hi = 0x0101010101010101ull * (uint64_t)(m.info >> 24);
-        } else if (kind == kLeafAffine) {
-#pragma unroll
-            for (int a = 0; a < 4; ++a)
-#pragma unroll
-                for (int b = 0; b < 4; ++b) {
-                    const uint64_t v = affine_pixel(m, i0 + a, j0 + b);
-                    if (a < 2) lo |= v << (8 * (4 * a + b));
-                    else hi |= v << (8 * (4 * (a - 2) + b));
-                }
+        if (((m.info >> 12) & 3u) < kLeafDomain) {
+            still_rows(m, x0, y0, rw);
         } else {
-            const int S = (int)(m.info & 0xFFFu);
-            const int k = (int)((m.info >> 14) & 7u);
-            const IsoInv t = iso_inverse(k, S - 1);
-            const int u00 = t.cu + t.ai * i0 + t.aj * j0, v00 = t.cv + t.bi * i0 + t.bj * j0;
-            const int umin = u00 - 3 * ((t.ai < 0) | (t.aj < 0));
-            const int vmin = v00 - 3 * ((t.bi < 0) | (t.bj < 0));
-            const size_t total = (size_t)w * h;
-            size_t off = ((size_t)(m.dom & 0xFFFFu) + 2 * umin) * w + (m.dom >> 16) + 2 * vmin;
-            // 2x2 sums of sample (umin + p, vmin + q) in 16-bit lanes; zero without a domain.
-            uint32_t sums[4][2] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}};
-            if (!(m.info & kLeafNoDomain)) {
-#pragma unroll
-                for (int r = 0; r < 8; ++r, off += w) {
-                    const uint64_t row = load8(src, off, total);
-                    const uint32_t s0 = pair_sums((uint32_t)row);
-                    const uint32_t s1 = pair_sums((uint32_t)(row >> 32));
-                    sums[r >> 1][0] += s0;
-                    sums[r >> 1][1] += s1;
-                }
-            }
-            // Values in sample order: byte q of word p is sample (umin + p, vmin + q).
-            uint32_t rw[4] = {0, 0, 0, 0};
-#pragma unroll
-            for (int p = 0; p < 4; ++p)
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int sum = (int)((sums[p][q >> 1] >> (16 * (q & 1))) & 0xFFFFu);
-                    double value = domain_value(sum, m);
-                    if (kind == kLeafResidual)
-                        value = __dadd_rn(value, __ldg(resid + m.roff + (umin + p) * S + vmin + q));
-                    rw[p] |= to_u8(value) << (8 * q);
-                }
-            // Sample (p, q) is output pixel (a, b) with a = p (or 3 - p when u counts down)
-            // and b = q (or 3 - q when v counts down), transposed for isometries 1, 2, 6, 7.
-            const bool tr = (0xC6u >> k) & 1u, uneg = (0xACu >> k) & 1u, vneg = (0x9Au >> k) & 1u;
-            if (vneg) {
-#pragma unroll
-                for (int p = 0; p < 4; ++p) rw[p] = __byte_perm(rw[p], 0, 0x0123);
-            }
-            if (uneg) {
-                const uint32_t t0 = rw[0], t1 = rw[1];
-                rw[0] = rw[3];
-                rw[1] = rw[2];
-                rw[2] = t1;
-                rw[3] = t0;
-            }
-            if (tr) transpose4x4(rw[0], rw[1], rw[2], rw[3]);
-            lo = (uint64_t)rw[0] | ((uint64_t)rw[1] << 32);
-            hi = (uint64_t)rw[2] | ((uint64_t)rw[3] << 32);
+            int umin, vmin;
+            cell_sample(m, x0, y0, &umin, &vmin);
+            uint32_t sums[4][2] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}};  // zero without a domain
+            if (!(m.info & kLeafNoDomain))
+                window_sums<false>(
+                    src, ((size_t)(m.dom & 0xFFFFu) + 2 * umin) * w + (m.dom >> 16) + 2 * vmin, w,
+                    (size_t)w * h, sums);
+            domain_rows(m, sums, resid, umin, vmin, rw);
         }
     }
-    uint8_t* out = dst + (size_t)y0 * w + x0;
-    const uint32_t rows_out[4] = {(uint32_t)lo, (uint32_t)(lo >> 32), (uint32_t)hi,
-                                  (uint32_t)(hi >> 32)};
-    *reinterpret_cast<uint32_t*>(out) = rows_out[0];
-    if (y0 + 1 < h) *reinterpret_cast<uint32_t*>(out + w) = rows_out[1];
-    if (y0 + 2 < h) *reinterpret_cast<uint32_t*>(out + 2 * (size_t)w) = rows_out[2];
-    if (y0 + 3 < h) *reinterpret_cast<uint32_t*>(out + 3 * (size_t)w) = rows_out[3];
-    if (kStable) {
-        uint32_t m = 0;  // per-byte max |next - prev| over the cell's rows in the plane
-        const uint8_t* prev = src + (size_t)y0 * w + x0;
+    const size_t at = (size_t)y0 * w + x0;
+    store_rows(dst + at, w, h - y0, rw);
+    if (kStable)
+        fold_delta(rows_delta(rw, h - y0, [&](int a) {
+            return *reinterpret_cast<const uint32_t*>(src + at + (size_t)a * w);
+        }), ss.delta);
+}
+
+// ---- every step of a small plane's decode in one launch ----
+//
+// A step of a 512 x 512 plane is 16,384 cells: three dependent loads and a few dozen
+// instructions a cell, less than the launch around them.  Here one cooperative launch runs all
+// steps: a thread keeps its cell's leaf in registers, cells that read no domain are written to
+// both buffers once, and the blocks meet at a counter between steps.  What is read was written by
+// other SMs during the launch, so reads pass L1 by.  Bound: the counter's and the windows' round
+// trips to L2.  One B200, ten steps of 512 x 512: 39 us, 46 us as launches; of 1024 x 1024: 48
+// and 66.  Cooperative launches of several streams run one after the other, where the steps as
+// launches overlap (three streams: 39 us a decode against 33), so a plan's run, which does not
+// wait, keeps those; the calls that wait for the result take this one.  (One cluster of 16 blocks
+// of 1,024 threads and its hardware barrier: 51 us, bound by the windows' bytes through 16 SMs.)
+
+constexpr int kResidentThreads = 128;
+constexpr long long kBarrierCycles = 4000000000ll;  // ~2 s
+
+// All blocks arrive, then leave: the counter only grows during a launch.  A wait that runs out
+// sets the error word and the counter's top bit, which lets everybody through.
+__device__ __forceinline__ void grid_meet(uint32_t* counter, uint32_t target, int* err) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(counter) : "memory");
+        const long long t0 = clock64();
+        for (;;) {
+            uint32_t v;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(counter) : "memory");
+            if (v >= target) break;
+            if (clock64() - t0 > kBarrierCycles) {
+                atomicOr(err, 256);
+                atomicOr(counter, 0x80000000u);
+                break;
+            }
+        }
+    }
+    __syncthreads();
+}
+
+struct ResidentArgs {
+    uint8_t *buf0, *buf1;
+    int w, h, lg, mw;
+    const int32_t* owner;
+    const DecodeMap* maps;
+    const double* resid;
+    uint32_t iters;
+    uint32_t* sync;  // arrivals, blocks through
+    int* delta;      // kStable: per step
+    int threshold;
+    int* state;
+    int* err;
+};
+
+template <bool kStable>
+__global__ void __launch_bounds__(kResidentThreads) decode_resident_kernel(const ResidentArgs g) {
+    __shared__ int largest;
+    const uint32_t cw = (uint32_t)g.w / 4, cells = cw * (((uint32_t)g.h + 3) / 4);
+    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+    const int x0 = 4 * (int)(c % cw), y0 = 4 * (int)(c / cw);
+    const bool in = c < cells;
+    const int rows = in ? g.h - y0 : 0;
+    const size_t at = (size_t)y0 * g.w + x0, total = (size_t)g.w * g.h;
+    const int32_t li = in ? g.owner[(size_t)(y0 >> g.lg) * g.mw + (x0 >> g.lg)] : -1;
+    DecodeMap m{};
+    uint32_t rw[4] = {0, 0, 0, 0};
+    bool moving = false;
+    int umin = 0, vmin = 0;
+    size_t off = 0;
+    if (li >= 0) {
+        m = g.maps[li];
+        moving = ((m.info >> 12) & 3u) >= kLeafDomain;
+        if (moving) {
+            cell_sample(m, x0, y0, &umin, &vmin);
+            off = ((size_t)(m.dom & 0xFFFFu) + 2 * umin) * g.w + (m.dom >> 16) + 2 * vmin;
+        } else {
+            still_rows(m, x0, y0, rw);
+        }
+    }
+    // Step 0 reads 128 everywhere.
+    uint32_t before[4] = {0x80808080u, 0x80808080u, 0x80808080u, 0x80808080u};
+    uint32_t target = 0;
+    uint32_t used = 0;
+    for (uint32_t it = 0; it < g.iters; ++it) {
+        if (moving) {
+            uint32_t sums[4][2];
 #pragma unroll
-        for (int a = 0; a < 4; ++a)
-            if (y0 + a < h)
-                m = __vmaxu4(m, __vabsdiffu4(rows_out[a],
-                                             *reinterpret_cast<const uint32_t*>(prev + (size_t)a * w)));
-        m = max(max(m & 255u, (m >> 8) & 255u), max((m >> 16) & 255u, m >> 24));
-        fold_delta(m, ss.delta);
+            for (int p = 0; p < 4; ++p)
+                sums[p][0] = sums[p][1] = m.info & kLeafNoDomain ? 0u : 0x02000200u;
+            if (it > 0 && !(m.info & kLeafNoDomain))
+                window_sums<true>(it & 1 ? g.buf1 : g.buf0, off, g.w, total, sums);
+            domain_rows(m, sums, g.resid, umin, vmin, rw);
+        }
+        if (moving || it < 2) store_rows((it & 1 ? g.buf0 : g.buf1) + at, g.w, rows, rw);
+        if (kStable) {
+            fold_delta(rows_delta(rw, rows, [&](int a) { return before[a]; }), g.delta + it);
+#pragma unroll
+            for (int a = 0; a < 4; ++a) before[a] = rw[a];
+        }
+        if (!kStable && it + 1 == g.iters) break;
+        target += gridDim.x;
+        grid_meet(g.sync, target, g.err);
+        if (kStable) {
+            if (threadIdx.x == 0) largest = *(volatile int*)(g.delta + it);
+            __syncthreads();
+            if (largest <= g.threshold) {
+                used = it + 1;
+                break;
+            }
+            __syncthreads();  // everybody has read it
+        }
+    }
+    if (kStable && blockIdx.x == 0 && threadIdx.x == 0 && used) {
+        g.state[0] = 1;
+        g.state[1] = (int)used;
+    }
+    // The last block through leaves the words as they were.
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(g.sync + 1, 1u) == gridDim.x - 1) {
+            g.sync[0] = 0u;
+            g.sync[1] = 0u;
+        }
     }
 }
 
@@ -356,13 +617,8 @@ __global__ void decode_converged_kernel(const int* __restrict__ delta, int thres
 // row it starts at.
 __device__ __forceinline__ void cell_window(const DecodeMap& m, int x0, int y0, int w,
                                             size_t* off, int* row) {
-    const int S = (int)(m.info & 0xFFFu);
-    const int k = (int)((m.info >> 14) & 7u);
-    const IsoInv t = iso_inverse(k, S - 1);
-    const int i0 = y0 - (int)(m.rc & 0xFFFFu), j0 = x0 - (int)(m.rc >> 16);
-    const int u00 = t.cu + t.ai * i0 + t.aj * j0, v00 = t.cv + t.bi * i0 + t.bj * j0;
-    const int umin = u00 - 3 * ((t.ai < 0) | (t.aj < 0));
-    const int vmin = v00 - 3 * ((t.bi < 0) | (t.bj < 0));
+    int umin, vmin;
+    cell_sample(m, x0, y0, &umin, &vmin);
     *row = (int)(m.dom & 0xFFFFu) + 2 * umin;
     *off = (size_t)(*row) * w + (m.dom >> 16) + 2 * vmin;
 }
@@ -375,7 +631,7 @@ __device__ __forceinline__ bool is_domain_cell(const DecodeMap& m) {
 // a domain window) and the rows' cell counts.
 __global__ void sorted_key_kernel(int w, int h, int lg, int mw, const int32_t* __restrict__ owner,
                                   const DecodeMap* __restrict__ maps, uint32_t* __restrict__ key,
-                                  uint32_t* __restrict__ row_count) {
+                                  uint32_t* __restrict__ row_count, uint32_t* __restrict__ wide) {
     const int cw = w / 4, chh = (h + 3) / 4;
     const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= (long long)cw * chh) return;
@@ -390,6 +646,7 @@ __global__ void sorted_key_kernel(int w, int h, int lg, int mw, const int32_t* _
             cell_window(m, x0, y0, w, &off, &row);
             k = (uint32_t)row;
             atomicAdd(&row_count[row], 1u);
+            if (!(m.info & kLeafInteger)) *wide = 1u;
         }
     }
     key[c] = k;
@@ -429,13 +686,15 @@ __global__ void sorted_scan_kernel(const uint32_t* __restrict__ row_count, int h
     if (threadIdx.x == 0) cursor[h] = carry;  // the number of domain cells
 }
 
-// Pass 2: each domain cell takes the next slot of its source row and writes its job
-// (window offset, qalfa | isometry << 24, beta) there and the slot into inv.
+// Pass 2: each domain cell takes the next slot of its source row and writes its job there and
+// the slot into inv.  A job is 8 bytes when every leaf has the integer form (window offset;
+// A | isometry << 8 | base << 16), else 16 (window offset; qalfa | isometry << 24; beta).
 __global__ void sorted_scatter_kernel(int w, int h, int lg, int mw,
                                       const int32_t* __restrict__ owner,
                                       const DecodeMap* __restrict__ maps,
                                       const DecodeLeaf* __restrict__ leaves,
                                       const uint32_t* __restrict__ key, uint32_t* __restrict__ cursor,
+                                      const uint32_t* __restrict__ wide,
                                       uint4* __restrict__ jobs, uint32_t* __restrict__ inv) {
     const int cw = w / 4, chh = (h + 3) / 4;
     const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -451,52 +710,45 @@ __global__ void sorted_scatter_kernel(int w, int h, int lg, int mw,
     const uint32_t pos = atomicAdd(&cursor[row], 1u);
     const uint32_t qalfa = leaves[li].w & 0x1FFFFu;
     const uint32_t k = (m.info >> 14) & 7u;
-    jobs[pos] = make_uint4((uint32_t)off, qalfa | (k << 24),
-                           (uint32_t)__double2loint(m.b), (uint32_t)__double2hiint(m.b));
+    if (*wide)
+        jobs[pos] = make_uint4((uint32_t)off, qalfa | (k << 24),
+                               (uint32_t)__double2loint(m.b), (uint32_t)__double2hiint(m.b));
+    else
+        reinterpret_cast<uint2*>(jobs)[pos] =
+            make_uint2((uint32_t)off, (uint32_t)m.n1 | k << 8 | (uint32_t)m.n0 << 16);
     inv[c] = pos;
 }
 
-// Gather pass: job -> the cell's 16 output bytes (row-major 4x4) in the cell buffer.
+// Gather pass: job -> the cell's 16 output bytes (row-major 4x4) in the cell buffer.  Bound by
+// L1: every row of a window is a line of its own.  8192 x 8192 on one B200: 74 us, with two
+// 8-byte loads a row, f64 values and 16-byte jobs 84 us.
+template <bool kWide>
 __global__ void __launch_bounds__(128) sorted_gather_kernel(
     const uint8_t* __restrict__ src, size_t total, int w, const uint4* __restrict__ jobs,
     uint32_t n, DecodeConsts cst, uint4* __restrict__ cellbuf) {
     const uint32_t pos = blockIdx.x * blockDim.x + threadIdx.x;
     if (pos >= n) return;
-    const uint4 jb = jobs[pos];
-    size_t off = jb.x;
-    const int k = (int)(jb.y >> 24);
-    DecodeMap m;
-    // decode_expand's a = alfa / 4, alfa = (qalfa / 2^bits_alfa) * max_alfa (ifs.rs:434-439).
-    m.a = __dmul_rn(__dmul_rn(__ddiv_rn((double)(jb.y & 0x1FFFFu), cst.alfa_den), cst.max_alfa), 0.25);
-    m.b = __hiloint2double((int)jb.w, (int)jb.z);
-    uint32_t sums[4][2] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}};
+    uint32_t sums[4][2], rw[4];
+    int k;
+    if (kWide) {
+        const uint4 jb = jobs[pos];
+        k = (int)(jb.y >> 24);
+        DecodeMap m{};
+        m.info = kLeafDomain << 12 | (uint32_t)k << 14;
+        // decode_expand's a = alfa / 4, alfa = (qalfa / 2^bits_alfa) * max_alfa (ifs.rs:434-439).
+        m.a = __dmul_rn(__dmul_rn(__ddiv_rn((double)(jb.y & 0x1FFFFu), cst.alfa_den), cst.max_alfa), 0.25);
+        m.b = __hiloint2double((int)jb.w, (int)jb.z);
+        window_sums<false>(src, jb.x, w, total, sums);
+        domain_rows(m, sums, nullptr, 0, 0, rw);
+    } else {
+        const uint2 jb = reinterpret_cast<const uint2*>(jobs)[pos];
+        k = (int)(jb.y >> 8 & 7u);
+        window_sums<false>(src, jb.x, w, total, sums);
 #pragma unroll
-    for (int r = 0; r < 8; ++r, off += w) {
-        const uint64_t row = load8(src, off, total);
-        sums[r >> 1][0] += pair_sums((uint32_t)row);
-        sums[r >> 1][1] += pair_sums((uint32_t)(row >> 32));
+        for (int p = 0; p < 4; ++p)
+            rw[p] = integer_values(sums[p], jb.y & 63u, __byte_perm(jb.y, 0, 0x3232));
+        to_output_order(k, rw);
     }
-    uint32_t rw[4] = {0, 0, 0, 0};
-#pragma unroll
-    for (int p = 0; p < 4; ++p)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int sum = (int)((sums[p][q >> 1] >> (16 * (q & 1))) & 0xFFFFu);
-            rw[p] |= to_u8(domain_value(sum, m)) << (8 * q);
-        }
-    const bool tr = (0xC6u >> k) & 1u, uneg = (0xACu >> k) & 1u, vneg = (0x9Au >> k) & 1u;
-    if (vneg) {
-#pragma unroll
-        for (int p = 0; p < 4; ++p) rw[p] = __byte_perm(rw[p], 0, 0x0123);
-    }
-    if (uneg) {
-        const uint32_t t0 = rw[0], t1 = rw[1];
-        rw[0] = rw[3];
-        rw[1] = rw[2];
-        rw[2] = t1;
-        rw[3] = t0;
-    }
-    if (tr) transpose4x4(rw[0], rw[1], rw[2], rw[3]);
     cellbuf[pos] = make_uint4(rw[0], rw[1], rw[2], rw[3]);
 }
 
@@ -519,23 +771,16 @@ __global__ void __launch_bounds__(128) sorted_place_kernel(
             rw[1] = v.y;
             rw[2] = v.z;
             rw[3] = v.w;
-        } else if (kind == kLeafConst) {
-            rw[0] = rw[1] = rw[2] = rw[3] = 0x01010101u * (m.info >> 24);
         } else {
-            const int i0 = y0 - (int)(m.rc & 0xFFFFu), j0 = x0 - (int)(m.rc >> 16);
-#pragma unroll
-            for (int a = 0; a < 4; ++a)
-#pragma unroll
-                for (int b = 0; b < 4; ++b) rw[a] |= affine_pixel(m, i0 + a, j0 + b) << (8 * b);
+            still_rows(m, x0, y0, rw);
         }
     }
-    uint8_t* out = dst + (size_t)y0 * w + x0;
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-        if (y0 + a < h) *reinterpret_cast<uint32_t*>(out + (size_t)a * w) = rw[a];
+    store_rows(dst + (size_t)y0 * w + x0, w, h - y0, rw);
 }
 
 }  // namespace
+
+size_t decode_sorted_cells(int w, int h) { return (size_t)(w / 4) * ((h + 3) / 4); }
 
 cudaError_t launch_decode_expand(const DecodeLeaf* leaves, const int32_t* resid_off, int n,
                                  DecodeConsts c, DecodeMap* maps, cudaStream_t st) {
@@ -563,6 +808,40 @@ cudaError_t launch_decode_step(const uint8_t* src, uint8_t* dst, int w, int h, i
     return cudaGetLastError();
 }
 
+cudaError_t launch_decode_resident(uint8_t* buf0, uint8_t* buf1, int w, int h, int lg,
+                                   const int32_t* owner, const DecodeMap* maps,
+                                   const double* resid, uint32_t iters, uint32_t* sync, int* delta,
+                                   int threshold, int* state, int* err, int num_sms,
+                                   cudaStream_t st, bool* taken) {
+    *taken = false;
+    const bool aligned =
+        ((reinterpret_cast<uintptr_t>(buf0) | reinterpret_cast<uintptr_t>(buf1)) & 7) == 0;
+    if (lg < 2 || w % 4 != 0 || !aligned || iters == 0) return cudaSuccess;
+    const size_t cells = decode_sorted_cells(w, h);
+    ResidentArgs g{buf0, buf1, w, h, lg, (w + (1 << lg) - 1) >> lg, owner, maps, resid, iters,
+                   sync, delta, threshold, state, err};
+    const size_t blocks = (cells + kResidentThreads - 1) / kResidentThreads;
+    // Every block must be resident at once, and the counter must not reach its top bit.  Up to
+    // four blocks an SM (1.2 Mpixel): ten steps of 1024 x 1024 take 48 us here and 66 as launches,
+    // but of 1280 x 1280, 800 blocks polling one counter, 150 against 99.
+    if (blocks > (size_t)num_sms * 4 || (uint64_t)blocks * iters >= (1ull << 31)) return cudaSuccess;
+    const void* kernel = delta ? (const void*)decode_resident_kernel<true>
+                               : (const void*)decode_resident_kernel<false>;
+    int per_sm = 0;
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kResidentThreads, 0);
+    if (e != cudaSuccess) return e;
+    if (blocks > (size_t)num_sms * per_sm) return cudaSuccess;
+    void* args[] = {&g};
+    e = cudaLaunchCooperativeKernel(kernel, dim3((unsigned)blocks), dim3(kResidentThreads), args, 0,
+                                    st);
+    if (e == cudaErrorCooperativeLaunchTooLarge) {  // fewer SMs than the device has
+        cudaGetLastError();
+        return cudaSuccess;
+    }
+    *taken = e == cudaSuccess;
+    return e;
+}
+
 cudaError_t launch_decode_step_stable(const uint8_t* src, uint8_t* dst, int w, int h, int lg,
                                       const int32_t* owner, const DecodeMap* maps,
                                       const double* resid, const int* done, int* delta,
@@ -586,8 +865,6 @@ cudaError_t launch_decode_step_stable(const uint8_t* src, uint8_t* dst, int w, i
 }
 
 
-size_t decode_sorted_cells(int w, int h) { return (size_t)(w / 4) * ((h + 3) / 4); }
-
 bool decode_sorted_eligible(int w, int h, int lg, bool residuals) {
     return lg >= 2 && (w % 4) == 0 && !residuals && w > 0 && h > 0;
 }
@@ -601,21 +878,26 @@ cudaError_t launch_decode_sorted_build(int w, int h, int lg, const int32_t* owne
     cudaError_t e = cudaMemsetAsync(row_count, 0, (size_t)h * 4, st);
     if (e != cudaSuccess) return e;
     const unsigned blocks = (unsigned)((cells + 255) / 256);
-    sorted_key_kernel<<<blocks, 256, 0, st>>>(w, h, lg, mw, owner, maps, key, row_count);
+    uint32_t* wide = cursor + h + 1;
+    e = cudaMemsetAsync(wide, 0, 4, st);
+    if (e != cudaSuccess) return e;
+    sorted_key_kernel<<<blocks, 256, 0, st>>>(w, h, lg, mw, owner, maps, key, row_count, wide);
     sorted_scan_kernel<<<1, 1024, 0, st>>>(row_count, h, cursor);
     sorted_scatter_kernel<<<blocks, 256, 0, st>>>(w, h, lg, mw, owner, maps, leaves, key, cursor,
-                                                   jobs, inv);
+                                                   wide, jobs, inv);
     return cudaGetLastError();
 }
 
 cudaError_t launch_decode_sorted_step(const uint8_t* src, uint8_t* dst, int w, int h, int lg,
                                       const int32_t* owner, const DecodeMap* maps,
-                                      const uint4* jobs, uint32_t njobs, const uint32_t* inv,
-                                      DecodeConsts c, uint4* cellbuf, cudaStream_t st) {
+                                      const uint4* jobs, uint32_t njobs, bool wide_jobs,
+                                      const uint32_t* inv, DecodeConsts c, uint4* cellbuf,
+                                      cudaStream_t st) {
     const int mw = (w + (1 << lg) - 1) >> lg;
-    if (njobs)
-        sorted_gather_kernel<<<(njobs + 127) / 128, 128, 0, st>>>(src, (size_t)w * h, w, jobs,
-                                                                 njobs, c, cellbuf);
+    if (njobs) {
+        const auto gather = wide_jobs ? sorted_gather_kernel<true> : sorted_gather_kernel<false>;
+        gather<<<(njobs + 127) / 128, 128, 0, st>>>(src, (size_t)w * h, w, jobs, njobs, c, cellbuf);
+    }
     dim3 grid((w / 4 + 127) / 128, (h + 3) / 4);
     sorted_place_kernel<<<grid, 128, 0, st>>>(dst, w, h, lg, mw, owner, maps, inv, cellbuf);
     return cudaGetLastError();

@@ -166,13 +166,19 @@ constexpr uint32_t kLeafNoDomain = 1u << 17;
 //   residual: mode 3: the domain value + res[roff + u*size + v], res the residual pool;
 //             with qalfa == 0 (kLeafNoDomain) the domain is not read and sum = 0, so the
 //             value is (0.5 + 0*a) + b + res as in the reference.
+// Where kLeafInteger is set the pixels are also n / 64 rounded down, clamped to a byte, for
+// integers n (decode_expand_kernel says when):
+//   affine: n = n0 + n1 * i + n2 * j;
+//   domain: n = base + n1 * sum, base the signed half word that n0 holds twice.
 struct __align__(16) DecodeMap {
-    double a, b, gx, gy;
     uint32_t rc;    // row | col << 16
-    uint32_t info;  // size (0-11) | kind (12-13) | isometry (14-16) | no-domain (17) | const byte (24-31)
+    uint32_t info;  // size (0-11) | kind (12-13) | isometry (14-16) | no-domain (17) | integer (18) | const byte (24-31)
     uint32_t dom;   // dom_row | dom_col << 16
     int32_t roff;   // residual pool offset (kind residual), else -1
+    int32_t n0, n1, n2, unused;
+    double a, b, gx, gy;
 };
+constexpr uint32_t kLeafInteger = 1u << 18;
 // resid_off: per leaf, the offset of its size*size residual values in the pool (or -1);
 // may be null when no leaf is mode 3.
 cudaError_t launch_decode_expand(const DecodeLeaf* leaves, const int32_t* resid_off, int n,
@@ -191,12 +197,25 @@ cudaError_t launch_decode_step(const uint8_t* src, uint8_t* dst, int w, int h, i
                                const int32_t* owner, const DecodeMap* maps, const double* resid,
                                cudaStream_t st);
 
+// The steps of a decode as one cooperative launch whose threads each keep one 4x4 cell
+// (decode_resident_kernel): *taken says whether the plane was small enough; nothing is launched
+// otherwise.  The first step reads 128 everywhere, whatever buf0 holds.  sync: two words, zero
+// before the launch and left zero.  With delta (iters words, zero), the steps end as
+// launch_decode_step_stable's do, state[0] and state[1] being done and used.
+cudaError_t launch_decode_resident(uint8_t* buf0, uint8_t* buf1, int w, int h, int lg,
+                                   const int32_t* owner, const DecodeMap* maps,
+                                   const double* resid, uint32_t iters, uint32_t* sync, int* delta,
+                                   int threshold, int* state, int* err, int num_sms,
+                                   cudaStream_t st, bool* taken);
+
 // Source-ordered decode of large planes (decode.cu): the domain cells' jobs sorted by the
 // source row of their windows (built once per leaf list), then per step a gather into a
 // 16-byte-per-cell buffer and a placement in output order.  Eligible: cells of 4 x 4 pixels
 // or more (lg >= 2), width % 4 == 0, no mode-3 residuals.  key / inv hold one word per 4x4
 // cell, jobs and the cell buffer 16 bytes per domain cell (at most one per cell), row_count
-// h words and cursor h + 1 (cursor[h]: the number of domain cells after the build).
+// h words and cursor h + 2 (after the build cursor[h] is the number of domain cells and
+// cursor[h + 1] nonzero when some cell's leaf has no integer form: jobs are then 16 bytes, else
+// 8).
 size_t decode_sorted_cells(int w, int h);
 bool decode_sorted_eligible(int w, int h, int lg, bool residuals);
 cudaError_t launch_decode_sorted_build(int w, int h, int lg, const int32_t* owner,
@@ -205,8 +224,8 @@ cudaError_t launch_decode_sorted_build(int w, int h, int lg, const int32_t* owne
                                        uint4* jobs, uint32_t* inv, cudaStream_t st);
 cudaError_t launch_decode_sorted_step(const uint8_t* src, uint8_t* dst, int w, int h, int lg,
                                       const int32_t* owner, const DecodeMap* maps,
-                                      const uint4* jobs, uint32_t njobs, const uint32_t* inv,
-                                      DecodeConsts c, uint4* cellbuf, cudaStream_t st);
+                                      const uint4* jobs, uint32_t njobs, bool wide_jobs,
+                                      const uint32_t* inv, DecodeConsts c, uint4* cellbuf, cudaStream_t st);
 
 // RD pricing of one node size (rdprice.cu): count nodes of size x size at (rows, cols), k
 // candidates each; out[i] the node's priced winner, levels[levels_at[i]..] its mode-3 levels.

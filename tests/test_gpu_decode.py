@@ -240,3 +240,35 @@ def test_source_ordered_plan_steps_match_the_oracle(ctx, monkeypatch, w, h, seed
         got = dev.cpu().numpy().reshape(h, w)
         assert np.array_equal(got, orc.decode(_ohdr(hdr), leaves, iters)), iters
     plan.close()
+
+
+@pytest.mark.parametrize("w,h,bits_alfa,bits_beta,int_max_alfa",
+                         [(64, 64, 4, 7, 32), (132, 92, 4, 7, 32), (96, 64, 5, 7, 64),
+                          (96, 64, 3, 1, 8), (96, 64, 5, 16, 32), (64, 64, 6, 7, 255),
+                          (1024, 1024, 4, 7, 32), (2048, 1536, 4, 7, 32)])
+def test_integer_values_and_one_launch_steps(ctx, w, h, bits_alfa, bits_beta, int_max_alfa):
+    # Every contrast and offset of the header's widths (those with an integer form and those
+    # without), affine leaves past both ends of a byte, planes on both sides of the largest one
+    # whose steps run in one launch; the plan into a buffer at an 8-byte address.
+    torch = pytest.importorskip("torch")
+    leaves = synthetic.quadtree_leaves(w, h, w + bits_alfa, bits_alfa=bits_alfa,
+                                       bits_beta=bits_beta)
+    rng = np.random.default_rng(w * bits_beta)
+    dom = (leaves["mode"] != 1) & (leaves["qalfa"] != 0)
+    leaves["qalfa"][dom] = rng.integers(1, (1 << bits_alfa) + 1, int(dom.sum()))
+    leaves["qbeta"] = rng.integers(0, 1 << bits_beta, len(leaves))
+    affine = np.flatnonzero(leaves["mode"] == 1)
+    leaves["qgx"][affine[::2]] = rng.integers(-5000, 5001, len(affine[::2]))
+    leaves["qgy"][affine[1::3]] = rng.integers(-1 << 30, 1 << 30, len(affine[1::3]))
+    hdr = _hdr(w, h, bits_alfa, bits_beta, int_max_alfa)
+    plan = ctx.decode_plan(hdr, leaves)
+    buf = torch.zeros(w * h + 16, dtype=torch.uint8, device="cuda:0")
+    torch.cuda.synchronize()
+    for iters in (1, 2, 5):
+        want = orc.decode(_ohdr(hdr), leaves, iters)
+        assert np.array_equal(ctx.decode(hdr, leaves, iters), want)
+        for _ in range(2):
+            plan.run(iters, buf.data_ptr() + 8)
+        ctx.decode(hdr, leaves[:0], 1)  # waits for the context's stream
+        assert np.array_equal(buf.cpu().numpy()[8: 8 + w * h].reshape(h, w), want)
+    plan.close()
