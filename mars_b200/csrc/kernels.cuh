@@ -83,6 +83,9 @@ cudaError_t launch_reduce(const Partial* partials, int ntiles, int nranges, cons
 constexpr int kMaxTopK = 8;
 constexpr int kMaxTopKSplits = 64;  // domain-tile splits a ranked search may use
 int search_topk_splits(const LevelGeom& g, int nranges, int num_sms);
+// The most splits any CUDA-core kernel of the level takes (the allocation-free entry point's
+// scratch is sized by it).
+int search_simt_splits_most(const LevelGeom& g, int nranges, int num_sms);
 cudaError_t launch_search_topk(const int32_t* D, const uint8_t* plane, int w,
                                const uint32_t* rows, const uint32_t* cols, int nranges,
                                const LevelGeom& g, RangeStats rs, DomainStats ds,

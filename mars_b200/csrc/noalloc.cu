@@ -84,7 +84,9 @@ extern "C" int mars_search_blocks_noalloc(const uint8_t* d_plane, uint32_t width
     size_t off[12], need = 0;
     const size_t sizes[12] = {(size_t)g.dw * g.dh * 4, n * 4, n * 4, n * 8, n * 8, n * 8,
                               ndom * 4, ndom * 8, ndom * 4, ndom * 4,
-                              (size_t)nsplit * n * sizeof(mars::Partial), 0};
+                              (size_t)mars::search_simt_splits_most(g, (int)n, num_sms) * n *
+                                  sizeof(mars::Partial),
+                              0};
     for (int i = 0; i < 11; ++i) {
         off[i] = need;
         need += align256(sizes[i]);

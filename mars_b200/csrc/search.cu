@@ -387,6 +387,169 @@ __global__ void __launch_bounds__(RPB) search_simt_kernel(
     if (exact_counter && exact) atomicAdd(exact_counter, exact);
 }
 
+// The search of a level of 2 x 2 blocks (min_size 2, or the border blocks that forced splits
+// reach): a CTA per (range, split), a thread per domain.  A fit is four multiply-adds here and
+// the exact fits of what the bound lets through are all the work, so a thread per range, as
+// search_simt_kernel has it, is a serial chain of f64 divisions in too few warps: three
+// candidates a range of a 250 x 190 plane's 220 took 1,530 us (one B200).  The best one of each
+// of 220 ranges there takes 224 us, before 1,644; of 220 of a 1000 x 750 plane 2.3 and 2.8 ms, of
+// 16,384 57 and 121 ms; no count from 16 to 16,384 was slower, so size 2 has this kernel only.  Every
+// thread keeps the K best of its domains in registers and prunes against its own K-th; the CTA
+// then takes K times the best of the threads' heads.
+constexpr int kSmallThreads = 256;
+
+template <int K>
+__global__ void __launch_bounds__(kSmallThreads) search_small_kernel(
+    const int32_t* __restrict__ D, LevelGeom g, const uint8_t* __restrict__ plane, int w,
+    const uint32_t* __restrict__ rows, const uint32_t* __restrict__ cols, int nranges,
+    RangeStats rs, DomainStats ds, FitParams fp, Partial* __restrict__ partials,
+    unsigned long long* __restrict__ exact_counter) {
+    constexpr int S = 2, N = 4;
+    __shared__ unsigned long long best_rms[2][kSmallThreads / 32];
+    __shared__ uint32_t best_idx[2][kSmallThreads / 32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int r = blockIdx.x;
+    const uint32_t row = rows[r], col = cols[r];
+    const bool inside = row + (uint32_t)S <= (uint32_t)g.h && col + (uint32_t)S <= (uint32_t)g.w;
+    const double inf = __longlong_as_double(0x7ff0000000000000ll);
+    struct Entry {
+        double rms, sum;
+        uint32_t idx, q;  // qalfa | qbeta << 16
+        int32_t t1;
+    };
+    Entry e[K];
+#pragma unroll
+    for (int j = 0; j < K; ++j) e[j] = Entry{inf, inf, UINT32_MAX, 0u, 0};
+    uint32_t exact = 0;
+    if (inside) {
+        int rr[N];
+#pragma unroll
+        for (int p = 0; p < N; ++p) rr[p] = plane[(size_t)(row + p / S) * w + col + p % S];
+        const int32_t t0 = rs.t0[r], t2 = rs.t2[r];
+        const int64_t nrr = rs.nrr[r];
+        const double rms0 = rs.rms0[r];
+        const float t0f = (float)t0;
+        Threshold th = make_threshold(inf, inf, UINT32_MAX, rms0, nrr, N, fp);
+        const int ndom = g.nrow_d * g.ncol_d;
+        const int stride = kSmallThreads * gridDim.y;
+        for (int dom = blockIdx.y * kSmallThreads + tid; dom < ndom; dom += stride) {
+            const int a = dom / g.ncol_d, b = dom - a * g.ncol_d;
+            const int32_t* at = D + (size_t)(a * g.step_c) * g.dw + b * g.step_c;
+            const int d[N] = {__ldg(at), __ldg(at + 1), __ldg(at + g.dw), __ldg(at + g.dw + 1)};
+            int acc[8], mx = 0;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                acc[k] = 0;
+#pragma unroll
+                for (int p = 0; p < N; ++p) acc[k] += rr[iso_src(k, p / S, p % S, S)] * d[p];
+                mx = max(mx, acc[k]);
+            }
+            const int32_t s1 = ds.s1x4[dom];
+            const float detf = ds.detf[dom], sdetf = ds.sdetf[dom];
+            int32_t lim = prune_below(th, (uint32_t)dom, (float)s1, t0f, detf, sdetf, 0.25f, fp);
+            if (mx < lim) continue;
+            const int64_t s2 = ds.s2x16[dom];
+            uint32_t left = 0xFFu;
+            for (;;) {
+                // The next isometry that the present bound lets through.
+                int32_t t1 = 0;
+                uint32_t iso = 8u;
+#pragma unroll
+                for (int k = 7; k >= 0; --k)
+                    if ((left >> k & 1u) && acc[k] >= lim) {
+                        iso = (uint32_t)k;
+                        t1 = acc[k];
+                    }
+                if (iso == 8u) break;
+                left &= ~((2u << iso) - 1u);
+                ++exact;
+                const FitResult f = fit_exact(N, s1, s2, t0, t1, t2, fp);
+                const uint32_t idx = (uint32_t)dom * 8u + iso;
+                if (!(f.rms < e[K - 1].rms || (f.rms == e[K - 1].rms && idx < e[K - 1].idx)))
+                    continue;
+                e[K - 1] = Entry{f.rms, f.sum, idx, f.qalfa | f.qbeta << 16, t1};
+#pragma unroll
+                for (int j = K - 1; j > 0; --j)
+                    if (e[j].rms < e[j - 1].rms ||
+                        (e[j].rms == e[j - 1].rms && e[j].idx < e[j - 1].idx)) {
+                        const Entry x = e[j];
+                        e[j] = e[j - 1];
+                        e[j - 1] = x;
+                    }
+                if (e[K - 1].idx != UINT32_MAX) {
+                    th = make_threshold(e[K - 1].sum, e[K - 1].rms, e[K - 1].idx >> 3, rms0, nrr, N, fp);
+                    lim = prune_below(th, (uint32_t)dom, (float)s1, t0f, detf, sdetf, 0.25f, fp);
+                }
+            }
+        }
+    }
+    // K times the smallest (rms, index) of the threads' heads: rms >= 0, so its bits order as
+    // integers, and +inf past every other.
+    Partial* out = partials + ((size_t)blockIdx.y * nranges + r) * K;
+    for (int j = 0; j < K; ++j) {
+        const unsigned long long bits = (unsigned long long)__double_as_longlong(e[0].rms);
+        const uint32_t hi = __reduce_min_sync(0xffffffffu, (uint32_t)(bits >> 32));
+        const uint32_t lo = __reduce_min_sync(
+            0xffffffffu, (uint32_t)(bits >> 32) == hi ? (uint32_t)bits : UINT32_MAX);
+        const unsigned long long top = (unsigned long long)hi << 32 | lo;
+        const uint32_t first = __reduce_min_sync(0xffffffffu, bits == top ? e[0].idx : UINT32_MAX);
+        if (lane == 0) {
+            best_rms[j & 1][warp] = top;
+            best_idx[j & 1][warp] = first;
+        }
+        __syncthreads();
+        unsigned long long win = best_rms[j & 1][0];
+        uint32_t wi = best_idx[j & 1][0];
+#pragma unroll
+        for (int v = 1; v < kSmallThreads / 32; ++v) {
+            const unsigned long long o = best_rms[j & 1][v];
+            const uint32_t oi = best_idx[j & 1][v];
+            if (o < win || (o == win && oi < wi)) {
+                win = o;
+                wi = oi;
+            }
+        }
+        if (wi == UINT32_MAX) {  // fewer than K candidates
+            if (tid == 0) out[j] = Partial{inf, inf, UINT32_MAX, 0, 0, 0, 0};
+        } else if (e[0].idx == wi) {
+            out[j] = Partial{e[0].rms, e[0].sum, wi, e[0].t1, (uint16_t)(e[0].q & 0xFFFFu),
+                             (uint16_t)(e[0].q >> 16), 0};
+#pragma unroll
+            for (int k = 0; k + 1 < K; ++k) e[k] = e[k + 1];
+            e[K - 1] = Entry{inf, inf, UINT32_MAX, 0u, 0};
+        }
+    }
+    if (exact_counter && exact) atomicAdd(exact_counter, (unsigned long long)exact);
+}
+
+// Splits of a level of 2 x 2 blocks: two CTAs an SM, 2,048 domains (eight a thread) at least.
+int small_splits(const LevelGeom& g, int nranges, int num_sms) {
+    const int want = (2 * num_sms + nranges - 1) / nranges;
+    return std::max(1, std::min({want, (g.nrow_d * g.ncol_d + 2047) / 2048, kMaxTopKSplits}));
+}
+
+cudaError_t launch_small(const int32_t* D, const uint8_t* plane, int w, const uint32_t* rows,
+                         const uint32_t* cols, int nranges, const LevelGeom& g, RangeStats rs,
+                         DomainStats ds, const FitParams& fp, int k, Partial* partials, int nsplit,
+                         unsigned long long* counter, cudaStream_t st) {
+    auto go = [&](auto kernel) {
+        kernel<<<dim3(nranges, nsplit), kSmallThreads, 0, st>>>(D, g, plane, w, rows, cols, nranges,
+                                                                rs, ds, fp, partials, counter);
+        return cudaGetLastError();
+    };
+    switch (k) {
+        case 1: return go(search_small_kernel<1>);
+        case 2: return go(search_small_kernel<2>);
+        case 3: return go(search_small_kernel<3>);
+        case 4: return go(search_small_kernel<4>);
+        case 5: return go(search_small_kernel<5>);
+        case 6: return go(search_small_kernel<6>);
+        case 7: return go(search_small_kernel<7>);
+        case 8: return go(search_small_kernel<8>);
+        default: return cudaErrorInvalidValue;
+    }
+}
+
 __global__ void reduce_kernel(const Partial* __restrict__ partials, int ntiles, int nranges,
                               LevelGeom g, RangeStats rs, DomainStats ds,
                               CandidateOut* __restrict__ out) {
@@ -523,7 +686,6 @@ cudaError_t launch_simt_k(const int32_t* D, const uint8_t* plane, int w, const u
                           DomainStats ds, const FitParams& fp, Partial* partials, int nsplit,
                           unsigned long long* counter, cudaStream_t st, int k) {
     switch (g.size) {
-        case 2: return launch_simt_t<2, 64, KMAX>(D, plane, w, rows, cols, nranges, g, rs, ds, fp, partials, nsplit, counter, st, k);
         case 4: return launch_simt_t<4, 64, KMAX>(D, plane, w, rows, cols, nranges, g, rs, ds, fp, partials, nsplit, counter, st, k);
         case 8: return launch_simt_t<8, 64, KMAX>(D, plane, w, rows, cols, nranges, g, rs, ds, fp, partials, nsplit, counter, st, k);
         case 16: return launch_simt_t<16, 64, KMAX>(D, plane, w, rows, cols, nranges, g, rs, ds, fp, partials, nsplit, counter, st, k);
@@ -584,6 +746,11 @@ int search_simt_tiles(const LevelGeom& g) {
 }
 
 int search_simt_splits(const LevelGeom& g, int nranges, int num_sms) {
+    if (g.size == 2) return small_splits(g, nranges, num_sms);
+    return search_simt_splits_most(g, nranges, num_sms);
+}
+
+int search_simt_splits_most(const LevelGeom& g, int nranges, int num_sms) {
     const int groups = (nranges + rpb_for(g.size) - 1) / rpb_for(g.size);
     const int want = (num_sms * 16 + groups - 1) / groups;
     return std::max(1, std::min(want, search_simt_tiles(g)));
@@ -595,6 +762,9 @@ cudaError_t launch_search_simt(const int32_t* D, const uint8_t* plane, int w,
                                const FitParams& fp, Partial* partials, int nsplit,
                                unsigned long long* counter, cudaStream_t st) {
     if (nranges == 0 || g.nrow_d <= 0 || g.ncol_d <= 0) return cudaSuccess;
+    if (g.size == 2)
+        return launch_small(D, plane, w, rows, cols, nranges, g, rs, ds, fp, 1, partials, nsplit,
+                            counter, st);
     return launch_simt_k<1>(D, plane, w, rows, cols, nranges, g, rs, ds, fp, partials, nsplit,
                             counter, st, 1);
 }
@@ -610,6 +780,9 @@ cudaError_t launch_search_topk(const int32_t* D, const uint8_t* plane, int w,
                                unsigned long long* counter, cudaStream_t st) {
     if (k < 1 || k > kMaxTopK || nsplit > kMaxTopKSplits) return cudaErrorInvalidValue;
     if (nranges == 0 || g.nrow_d <= 0 || g.ncol_d <= 0) return cudaSuccess;
+    if (g.size == 2)
+        return launch_small(D, plane, w, rows, cols, nranges, g, rs, ds, fp, k, partials, nsplit,
+                            counter, st);
     return launch_simt_k<kMaxTopK>(D, plane, w, rows, cols, nranges, g, rs, ds, fp, partials,
                                    nsplit, counter, st, k);
 }

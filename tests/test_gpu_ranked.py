@@ -124,3 +124,26 @@ def test_tensor_core_ranked_equals_oracle_at_stride_4():
         prov.close()
     finally:
         c.close()
+
+
+@pytest.mark.parametrize("w,h,shift", [(6, 4, 2), (4, 6, 2), (10, 6, 4), (130, 94, 2), (258, 70, 4),
+                                       (66, 66, 16)])
+@pytest.mark.parametrize("content", ["synthetic", "flat", "steps"])
+def test_two_by_two_blocks(ctx, w, h, shift, content):
+    # min_size 2: from one domain (eight candidates) to several splits of them, lists of every
+    # length, ties throughout (flat) and between domains (steps), and the single winner.
+    img = {"synthetic": lambda: synthetic.gray(w, h, w + h),
+           "flat": lambda: np.full((h, w), 77, np.uint8),
+           "steps": lambda: (np.add.outer(np.arange(h) // 4, np.arange(w) // 4) % 2 * 90
+                             ).astype(np.uint8)}[content]()
+    kw = dict(min_size=2, max_size=4, shift=shift)
+    p = orc.make_params(**kw)
+    nodes = [(0, 0), (h // 4 * 2, w // 4 * 2), ((h - 2) // 2 * 2, (w - 2) // 2 * 2)]
+    for k in (1, 2, 3, 4, 5, 6, 7, 8):
+        prov = ctx.search_provider(img, mb.make_params(**kw), k=k)
+        for r, c in nodes:
+            got, gev = prov.search_candidates(r, c, 2, shift, k)
+            want, oev = orc.search(img, r, c, 2, shift, p, k=k)
+            assert gev == oev
+            assert got.tobytes() == want.tobytes(), (k, r, c)
+        prov.close()
