@@ -2245,6 +2245,7 @@ int plan_encode_device(mars_search_plan* plan, const uint8_t* plane, const mars_
     mars::WalkScratch ws{};
     mars_leaf *d_warm, *d_leaves;
     MARS_CUDA(sc.get(&d_cands, nodes * sizeof(mars_candidate)));
+
     MARS_CUDA(sc.get(&d_px, (size_t)plan->w * plan->h));
     MARS_CUDA(sc.get(&ws.split, nodes));
     MARS_CUDA(sc.get(&ws.cnt, nodes));
@@ -2431,9 +2432,10 @@ namespace {
 // .ifs stream and every encoder output lie in.  The owner map's cell is the largest power
 // of two dividing every leaf's row, column and size (4 for the usual quadtree with
 // min_size 4), capped at 32; later leaves overwrite earlier ones, as in the reference.
-// Mode-3 residuals are rebuilt here on the host exactly as decode_leaf does
-// (ifs.rs:441-456) -- the inverse DCT uses the C library's cosine, as the reference's
-// does -- in domain-local (u, v) order, and their offsets are returned per leaf.
+// Mode-3 residuals are rebuilt exactly as decode_leaf does (ifs.rs:441-456) in domain-local
+// (u, v) order, their offsets returned per leaf: on the device over a basis made here
+// (upload_residuals; the basis is the C library's cosine, as the reference's is), or here for
+// lists with a mode-3 leaf wider than kResidualMost (resid_values is then not empty).
 int prepare_decode(const mars_header* hdr, const mars_leaf* leaves, size_t n,
                    const int32_t* residuals, size_t nresiduals, std::vector<mars::DecodeLeaf>* dl,
                    std::vector<int32_t>* owner, int* lg_out, mars::DecodeConsts* consts,
@@ -2482,13 +2484,21 @@ int prepare_decode(const mars_header* hdr, const mars_leaf* leaves, size_t n,
     if (nresiduals) {
         if (nresiduals > 0x7fffffffull) return fail(MARS_EINVAL, "residual pool too large");
         resid_off->assign(n, -1);
-        const double step = mars::codec::qstep_of(*hdr);
+        uint32_t most = 0;
         for (size_t k = 0; k < n; ++k) {
             if (offs[k] < 0) continue;
-            (*resid_off)[k] = (int32_t)resid_values->size();
-            const std::vector<double> v =
-                mars::residual::values(residuals + offs[k], leaves[k].size, step);
-            resid_values->insert(resid_values->end(), v.begin(), v.end());
+            (*resid_off)[k] = (int32_t)offs[k];
+            most = std::max(most, leaves[k].size);
+        }
+        if (most > mars::kResidualMost) {
+            const double step = mars::codec::qstep_of(*hdr);
+            resid_values->resize(nresiduals);
+            for (size_t k = 0; k < n; ++k) {
+                if (offs[k] < 0) continue;
+                const std::vector<double> v =
+                    mars::residual::values(residuals + offs[k], leaves[k].size, step);
+                std::copy(v.begin(), v.end(), resid_values->begin() + offs[k]);
+            }
         }
     }
     const int lg = __builtin_ctz(align_bits);
@@ -2502,6 +2512,44 @@ int prepare_decode(const mars_header* hdr, const mars_leaf* leaves, size_t n,
                         L.size >> lg, (int32_t)k);
     }
     *lg_out = lg;
+    return MARS_OK;
+}
+
+// The residual pool (nresiduals values, allocated by the caller) and the leaves' offsets of a
+// prepared list on the device; the staging buffers are the scratch's.
+int upload_residuals(mars_ctx* ctx, Scratch& sc, const mars_header* hdr, const mars_leaf* leaves,
+                     size_t n, const int32_t* residuals, size_t nresiduals,
+                     const mars::DecodeLeaf* d_leaves, const std::vector<int32_t>& roff,
+                     const std::vector<double>& rvals, int32_t* d_roff, double* d_rvals) {
+    const cudaStream_t st = ctx->stream;
+    MARS_CUDA(cudaMemcpyAsync(d_roff, roff.data(), n * 4, cudaMemcpyHostToDevice, st));
+    if (!rvals.empty()) {
+        MARS_CUDA(cudaMemcpyAsync(d_rvals, rvals.data(), rvals.size() * 8, cudaMemcpyHostToDevice, st));
+        return MARS_OK;
+    }
+    mars::ResidualBases bases{};
+    std::vector<double> all;
+    uint32_t most = 0;
+    bool have[mars::kResidualMost + 1] = {false};
+    for (size_t k = 0; k < n; ++k) {
+        const uint32_t size = leaves[k].size;
+        if (roff[k] < 0 || have[size]) continue;
+        have[size] = true;
+        most = std::max(most, size);
+        bases.at[size] = (uint32_t)all.size();
+        const std::vector<double>& b = mars::residual::basis(size);
+        all.insert(all.end(), b.begin(), b.end());
+    }
+    int32_t* d_levels = nullptr;
+    double* d_basis = nullptr;
+    MARS_CUDA(sc.get(&d_levels, nresiduals));
+    MARS_CUDA(sc.get(&d_basis, all.size()));
+    MARS_CUDA(cudaMemcpyAsync(d_levels, residuals, nresiduals * 4, cudaMemcpyHostToDevice, st));
+    MARS_CUDA(cudaMemcpyAsync(d_basis, all.data(), all.size() * 8, cudaMemcpyHostToDevice, st));
+    bases.basis = d_basis;
+    MARS_CUDA(mars::launch_residual_values(d_leaves, d_roff, (int)n, d_levels, bases, most,
+                                           mars::codec::qstep_of(*hdr), d_rvals, st));
+    ctx->launches += 1;
     return MARS_OK;
 }
 
@@ -2524,6 +2572,7 @@ struct mars_decode_plan {
     uint4* d_cellbuf = nullptr;
     uint32_t njobs = 0;
     bool wide_jobs = false;
+    bool pooled = false;  // buffers of the stream-ordered pool
 };
 
 namespace {
@@ -2568,16 +2617,16 @@ int mars_decode(mars_ctx* ctx, const mars_header* hdr, const mars_leaf* leaves, 
     MARS_CUDA(sc.get(&d_maps, n));
     MARS_CUDA(cudaMemcpyAsync(d_owner, owner.data(), owner.size() * 4, cudaMemcpyHostToDevice,
                               ctx->stream));
-    if (!rvals.empty()) {
-        MARS_CUDA(sc.get(&d_roff, n));
-        MARS_CUDA(sc.get(&d_rvals, rvals.size()));
-        MARS_CUDA(cudaMemcpyAsync(d_roff, roff.data(), n * 4, cudaMemcpyHostToDevice, ctx->stream));
-        MARS_CUDA(cudaMemcpyAsync(d_rvals, rvals.data(), rvals.size() * 8, cudaMemcpyHostToDevice,
-                                  ctx->stream));
-    }
     if (n) {
         MARS_CUDA(cudaMemcpyAsync(d_leaves, dl.data(), n * sizeof(mars::DecodeLeaf),
                                   cudaMemcpyHostToDevice, ctx->stream));
+        if (!roff.empty()) {
+            MARS_CUDA(sc.get(&d_roff, n));
+            MARS_CUDA(sc.get(&d_rvals, nresiduals));
+            if (int e = upload_residuals(ctx, sc, hdr, leaves, n, residuals, nresiduals, d_leaves,
+                                         roff, rvals, d_roff, d_rvals))
+                return e;
+        }
         MARS_CUDA(mars::launch_decode_expand(d_leaves, d_roff, (int)n, consts, d_maps,
                                              ctx->stream));
         ctx->launches += 1;
@@ -2606,10 +2655,25 @@ int mars_decode(mars_ctx* ctx, const mars_header* hdr, const mars_leaf* leaves, 
     return sync_bounded(ctx);
 }
 
-int mars_decode_plan_create(mars_ctx* ctx, const mars_header* hdr, const mars_leaf* leaves,
-                            size_t n, const int32_t* residuals, size_t nresiduals,
-                            mars_decode_plan** out) {
-    if (!ctx || !hdr || !out || (n && !leaves)) return fail(MARS_EINVAL, "NULL argument");
+}  // extern "C"
+
+namespace {
+
+void release_decode_plan(mars_decode_plan* p) {
+    cudaSetDevice(p->ctx->device);
+    cudaStreamSynchronize(p->ctx->stream);
+    for (void* q : {(void*)p->d_owner, (void*)p->d_maps, (void*)p->d_rvals, (void*)p->d_tmp,
+                    (void*)p->d_jobs, (void*)p->d_inv, (void*)p->d_cellbuf})
+        if (q) p->pooled ? cudaFreeAsync(q, p->ctx->stream) : cudaFree(q);
+    delete p;
+}
+
+// pooled: the plan lives for one call on the context's stream, so its buffers come from the
+// stream-ordered pool (eight cudaMalloc and cudaFree took half of a one-shot decode); a plan that
+// a program keeps may run on other streams and has its own.
+int create_decode_plan(mars_ctx* ctx, const mars_header* hdr, const mars_leaf* leaves, size_t n,
+                       const int32_t* residuals, size_t nresiduals, bool pooled,
+                       mars_decode_plan** out) {
     std::vector<mars::DecodeLeaf> dl;
     std::vector<int32_t> owner, roff;
     std::vector<double> rvals;
@@ -2620,78 +2684,74 @@ int mars_decode_plan_create(mars_ctx* ctx, const mars_header* hdr, const mars_le
         return e;
     std::lock_guard<std::mutex> lock(ctx->mu);
     MARS_CUDA(cudaSetDevice(ctx->device));
-    auto* p = new (std::nothrow) mars_decode_plan;
+    const cudaStream_t st = ctx->stream;
+    std::unique_ptr<mars_decode_plan, void (*)(mars_decode_plan*)> p(
+        new (std::nothrow) mars_decode_plan, release_decode_plan);
     if (!p) return fail(MARS_ENOMEM, "plan allocation failed");
     p->ctx = ctx;
     p->w = hdr->width;
     p->h = hdr->height;
     p->lg = lg;
     p->nleaves = n;
-    mars::DecodeLeaf* d_leaves = nullptr;
-    int32_t* d_roff = nullptr;
-    cudaError_t e = cudaMalloc(&p->d_owner, std::max<size_t>(1, owner.size()) * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&d_leaves, std::max<size_t>(1, n) * sizeof(mars::DecodeLeaf));
-    if (e == cudaSuccess) e = cudaMalloc(&p->d_maps, std::max<size_t>(1, n) * sizeof(mars::DecodeMap));
-    if (e == cudaSuccess) e = cudaMalloc(&p->d_tmp, (size_t)p->w * p->h);
-    if (e == cudaSuccess && !rvals.empty()) {
-        e = cudaMalloc(&d_roff, n * 4);
-        if (e == cudaSuccess) e = cudaMalloc(&p->d_rvals, rvals.size() * 8);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(d_roff, roff.data(), n * 4, cudaMemcpyHostToDevice, ctx->stream);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(p->d_rvals, rvals.data(), rvals.size() * 8, cudaMemcpyHostToDevice,
-                                ctx->stream);
-    }
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(p->d_owner, owner.data(), owner.size() * 4, cudaMemcpyHostToDevice,
-                            ctx->stream);
-    if (e == cudaSuccess && n)
-        e = cudaMemcpyAsync(d_leaves, dl.data(), n * sizeof(mars::DecodeLeaf),
-                            cudaMemcpyHostToDevice, ctx->stream);
-    if (e == cudaSuccess && n) {
-        e = mars::launch_decode_expand(d_leaves, d_roff, (int)n, consts, p->d_maps, ctx->stream);
-        ctx->launches += 1;
-    }
+    p->pooled = pooled;
     p->consts = consts;
-    uint32_t *d_key = nullptr, *d_rows = nullptr, *d_cursor = nullptr, counts[2] = {0, 0};
-    if (e == cudaSuccess && n && want_sorted_decode(p->w, p->h) &&
-        mars::decode_sorted_eligible((int)p->w, (int)p->h, lg, !rvals.empty())) {
-        const size_t cells = mars::decode_sorted_cells((int)p->w, (int)p->h);
-        e = cudaMalloc(&d_key, cells * 4);
-        if (e == cudaSuccess) e = cudaMalloc(&d_rows, (size_t)p->h * 4);
-        if (e == cudaSuccess) e = cudaMalloc(&d_cursor, ((size_t)p->h + 2) * 4);
-        if (e == cudaSuccess) e = cudaMalloc(&p->d_jobs, cells * sizeof(uint4));
-        if (e == cudaSuccess) e = cudaMalloc(&p->d_inv, cells * 4);
-        if (e == cudaSuccess) e = cudaMalloc(&p->d_cellbuf, cells * sizeof(uint4));
-        if (e == cudaSuccess)
-            e = mars::launch_decode_sorted_build((int)p->w, (int)p->h, lg, p->d_owner, p->d_maps,
-                                                 d_leaves, d_key, d_rows, d_cursor, p->d_jobs,
-                                                 p->d_inv, ctx->stream);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(counts, d_cursor + p->h, 8, cudaMemcpyDeviceToHost, ctx->stream);
-        ctx->launches += 3;
+    auto get = [&](auto** q, size_t count) {
+        const size_t bytes = std::max<size_t>(1, count) * sizeof(**q);
+        return pooled ? cudaMallocAsync((void**)q, bytes, st) : cudaMalloc((void**)q, bytes);
+    };
+    Scratch sc(st);
+    uint32_t counts[2] = {0, 0};
+    MARS_CUDA(get(&p->d_owner, owner.size()));
+    MARS_CUDA(get(&p->d_maps, n));
+    MARS_CUDA(get(&p->d_tmp, (size_t)p->w * p->h));
+    MARS_CUDA(cudaMemcpyAsync(p->d_owner, owner.data(), owner.size() * 4, cudaMemcpyHostToDevice, st));
+    if (n) {
+        mars::DecodeLeaf* d_leaves = nullptr;
+        int32_t* d_roff = nullptr;
+        MARS_CUDA(sc.get(&d_leaves, n));
+        MARS_CUDA(cudaMemcpyAsync(d_leaves, dl.data(), n * sizeof(mars::DecodeLeaf),
+                                  cudaMemcpyHostToDevice, st));
+        if (!roff.empty()) {
+            MARS_CUDA(sc.get(&d_roff, n));
+            MARS_CUDA(get(&p->d_rvals, nresiduals));
+            if (int e = upload_residuals(ctx, sc, hdr, leaves, n, residuals, nresiduals, d_leaves,
+                                         roff, rvals, d_roff, p->d_rvals))
+                return e;
+        }
+        MARS_CUDA(mars::launch_decode_expand(d_leaves, d_roff, (int)n, consts, p->d_maps, st));
+        ctx->launches += 1;
+        if (!pooled && want_sorted_decode(p->w, p->h) &&
+            mars::decode_sorted_eligible((int)p->w, (int)p->h, lg, !roff.empty())) {
+            const size_t cells = mars::decode_sorted_cells((int)p->w, (int)p->h);
+            uint32_t *d_rows = nullptr, *d_cursor = nullptr;
+            MARS_CUDA(sc.get(&d_rows, (size_t)p->h));
+            MARS_CUDA(sc.get(&d_cursor, (size_t)p->h + 2));
+            MARS_CUDA(get(&p->d_jobs, cells));
+            MARS_CUDA(get(&p->d_inv, cells));
+            MARS_CUDA(get(&p->d_cellbuf, cells));
+            MARS_CUDA(mars::launch_decode_sorted_build((int)p->w, (int)p->h, lg, p->d_owner,
+                                                       p->d_maps, d_leaves, (int)n, d_rows, d_cursor,
+                                                       p->d_jobs, p->d_inv, st));
+            MARS_CUDA(cudaMemcpyAsync(counts, d_cursor + p->h, 8, cudaMemcpyDeviceToHost, st));
+            ctx->launches += 3;
+        }
     }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    if (!pooled) MARS_CUDA(cudaStreamSynchronize(st));
     p->njobs = counts[0];
     p->wide_jobs = counts[1] != 0;
-    cudaFree(d_leaves);
-    cudaFree(d_roff);
-    cudaFree(d_key);
-    cudaFree(d_rows);
-    cudaFree(d_cursor);
-    if (e != cudaSuccess) {
-        cudaFree(p->d_owner);
-        cudaFree(p->d_maps);
-        cudaFree(p->d_rvals);
-        cudaFree(p->d_tmp);
-        cudaFree(p->d_jobs);
-        cudaFree(p->d_inv);
-        cudaFree(p->d_cellbuf);
-        delete p;
-        return fail(MARS_ECUDA, std::string("decode plan: ") + cudaGetErrorString(e));
-    }
-    *out = p;
+    *out = p.release();
     return MARS_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
+int mars_decode_plan_create(mars_ctx* ctx, const mars_header* hdr, const mars_leaf* leaves,
+                            size_t n, const int32_t* residuals, size_t nresiduals,
+                            mars_decode_plan** out) {
+    if (!ctx || !hdr || !out || (n && !leaves)) return fail(MARS_EINVAL, "NULL argument");
+    return create_decode_plan(ctx, hdr, leaves, n, residuals, nresiduals, false, out);
 }
 
 int mars_decode_plan_run(mars_decode_plan* p, uint32_t iterations, uint8_t* d_out) {
@@ -2770,18 +2830,21 @@ int mars_decode_until_stable(mars_ctx* ctx, const mars_header* hdr, const mars_l
                              uint8_t threshold, uint32_t max_iterations, uint8_t* out,
                              uint32_t* iterations_used) {
     if (!ctx || !hdr || !out || !iterations_used) return fail(MARS_EINVAL, "NULL argument");
+    if (n && !leaves) return fail(MARS_EINVAL, "NULL argument");
     mars_decode_plan* plan = nullptr;
-    if (int e = mars_decode_plan_create(ctx, hdr, leaves, n, residuals, nresiduals, &plan))
-        return e;
+    if (int e = create_decode_plan(ctx, hdr, leaves, n, residuals, nresiduals, true, &plan)) return e;
     std::unique_ptr<mars_decode_plan, void (*)(mars_decode_plan*)> guard(plan,
                                                                          mars_decode_plan_free);
     uint8_t* d_out = nullptr;
+    cudaStream_t st = nullptr;
     {
         std::lock_guard<std::mutex> lock(ctx->mu);
         MARS_CUDA(cudaSetDevice(ctx->device));
-        MARS_CUDA(cudaMalloc(&d_out, std::max<size_t>(1, (size_t)hdr->width * hdr->height)));
+        st = ctx->stream;
+        MARS_CUDA(cudaMallocAsync(&d_out, std::max<size_t>(1, (size_t)hdr->width * hdr->height), st));
     }
-    std::unique_ptr<uint8_t, cudaError_t (*)(void*)> dguard(d_out, cudaFree);
+    auto give_back = [st](uint8_t* q) { cudaFreeAsync(q, st); };
+    std::unique_ptr<uint8_t, decltype(give_back)> dguard(d_out, give_back);
     if (int e = mars_decode_plan_run_until_stable(plan, threshold, max_iterations, d_out,
                                                   iterations_used))
         return e;
@@ -2835,17 +2898,7 @@ int mars_zoom_leaves(const mars_header* hdr, const mars_leaf* leaves, size_t n, 
 }
 
 void mars_decode_plan_free(mars_decode_plan* p) {
-    if (!p) return;
-    cudaSetDevice(p->ctx->device);
-    cudaStreamSynchronize(p->ctx->stream);
-    cudaFree(p->d_owner);
-    cudaFree(p->d_maps);
-    cudaFree(p->d_rvals);
-    cudaFree(p->d_tmp);
-    cudaFree(p->d_jobs);
-    cudaFree(p->d_inv);
-    cudaFree(p->d_cellbuf);
-    delete p;
+    if (p) release_decode_plan(p);
 }
 
 int mars_ycbcr_device(mars_ctx* ctx, const uint8_t* d_r, const uint8_t* d_g, const uint8_t* d_b,

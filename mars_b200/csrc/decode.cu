@@ -20,6 +20,7 @@
 // values in sample order, moves them to output order with byte permutes (row reversal,
 // byte reversal, 4x4 transpose) and stores four 4-byte rows.  decode_pixel_kernel covers
 // any other geometry.
+#include "grid_meet.cuh"
 #include "kernels.cuh"
 
 namespace mars {
@@ -159,6 +160,52 @@ __global__ void decode_expand_kernel(const DecodeLeaf* __restrict__ leaves,
     }
     m.info = (uint32_t)L.size | (kind << 12) | ((uint32_t)L.iso << 14) | flags | (cbyte << 24);
     maps[k] = m;
+}
+
+// The values a residual leaf adds (residual.hpp values(), ifs.rs:441-456): dead-zone
+// dequantisation, then the inverse DCT, columns before rows.  Every output is one thread's
+// left-to-right f64 sum from -0.0, no product fused into it, over the host's basis: the host's
+// doubles.  A block a leaf.  Bound by the f64 sums' latency.  A one-shot decode until stable of
+// 1000 x 752 with a quarter of its domain leaves residual took 2.3 ms and more with the values made
+// on the host and sent, and 0.6 ms with this (0.44 ms without residuals).
+__global__ void __launch_bounds__(128) residual_values_kernel(
+    const DecodeLeaf* __restrict__ leaves, const int32_t* __restrict__ resid_off,
+    const int32_t* __restrict__ levels, const ResidualBases bases, double step,
+    double* __restrict__ values) {
+    extern __shared__ double coef[];
+    const int32_t at = resid_off[blockIdx.x];
+    if (at < 0) return;
+    const int n = (int)(leaves[blockIdx.x].y & 0xFFFu), nn = n * n;
+    const double* __restrict__ b = bases.basis + bases.at[n];
+    double* half = coef + nn;
+    const double threshold = __dmul_rn(0.5, step);  // the dead zone is half a step
+    for (int k = threadIdx.x; k < nn; k += blockDim.x) {
+        const int32_t level = levels[at + k];
+        double v = 0.0;
+        if (level != 0) {
+            const uint32_t size = level < 0 ? 0u - (uint32_t)level : (uint32_t)level;
+            const double mag = __dadd_rn(
+                threshold, __dmul_rn(__dadd_rn(__dsub_rn((double)size, 1.0), 0.5), step));
+            v = level < 0 ? -mag : mag;
+        }
+        coef[k] = v;
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < nn; t += blockDim.x) {
+        const int i = t / n, c = t - i * n;
+        double s = -0.0;
+#pragma unroll 4
+        for (int k = 0; k < n; ++k) s = __dadd_rn(s, __dmul_rn(coef[k * n + c], __ldg(b + k * n + i)));
+        half[t] = s;
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < nn; t += blockDim.x) {
+        const int r = t / n, i = t - r * n;
+        double s = -0.0;
+#pragma unroll 4
+        for (int k = 0; k < n; ++k) s = __dadd_rn(s, __dmul_rn(half[r * n + k], __ldg(b + k * n + i)));
+        values[at + t] = s;
+    }
 }
 
 __device__ __forceinline__ double domain_value(int sum, const DecodeMap& m) {
@@ -479,29 +526,6 @@ __global__ void __launch_bounds__(128) decode_cell_kernel(
 // of 1,024 threads and its hardware barrier: 51 us, bound by the windows' bytes through 16 SMs.)
 
 constexpr int kResidentThreads = 128;
-constexpr long long kBarrierCycles = 4000000000ll;  // ~2 s
-
-// All blocks arrive, then leave: the counter only grows during a launch.  A wait that runs out
-// sets the error word and the counter's top bit, which lets everybody through.
-__device__ __forceinline__ void grid_meet(uint32_t* counter, uint32_t target, int* err) {
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(counter) : "memory");
-        const long long t0 = clock64();
-        for (;;) {
-            uint32_t v;
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(counter) : "memory");
-            if (v >= target) break;
-            if (clock64() - t0 > kBarrierCycles) {
-                atomicOr(err, 256);
-                atomicOr(counter, 0x80000000u);
-                break;
-            }
-        }
-    }
-    __syncthreads();
-}
-
 struct ResidentArgs {
     uint8_t *buf0, *buf1;
     int w, h, lg, mw;
@@ -578,15 +602,7 @@ __global__ void __launch_bounds__(kResidentThreads) decode_resident_kernel(const
         g.state[0] = 1;
         g.state[1] = (int)used;
     }
-    // The last block through leaves the words as they were.
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        if (atomicAdd(g.sync + 1, 1u) == gridDim.x - 1) {
-            g.sync[0] = 0u;
-            g.sync[1] = 0u;
-        }
-    }
+    grid_leave(g.sync);
 }
 
 // After step `iter`: the first step whose delta met the threshold ends the decode.
@@ -613,43 +629,26 @@ __global__ void decode_converged_kernel(const int* __restrict__ delta, int thres
 // The values are the cell kernel's, operation for operation.  Maps with mode-3 residuals keep
 // the cell kernel.
 
-// The window of a domain cell: the byte offset of its top-left sample pixel and the source
-// row it starts at.
-__device__ __forceinline__ void cell_window(const DecodeMap& m, int x0, int y0, int w,
-                                            size_t* off, int* row) {
-    int umin, vmin;
-    cell_sample(m, x0, y0, &umin, &vmin);
-    *row = (int)(m.dom & 0xFFFFu) + 2 * umin;
-    *off = (size_t)(*row) * w + (m.dom >> 16) + 2 * vmin;
-}
-
 __device__ __forceinline__ bool is_domain_cell(const DecodeMap& m) {
     return ((m.info >> 12) & 3u) == kLeafDomain;
 }
 
-// Pass 1 of the list build: per 4x4 cell its window's source row (or ~0 for a cell without
-// a domain window) and the rows' cell counts.
-__global__ void sorted_key_kernel(int w, int h, int lg, int mw, const int32_t* __restrict__ owner,
-                                  const DecodeMap* __restrict__ maps, uint32_t* __restrict__ key,
-                                  uint32_t* __restrict__ row_count, uint32_t* __restrict__ wide) {
+// Pass 1 of the list build: the domain cells of each source row.
+__global__ void sorted_count_kernel(int w, int h, int lg, int mw, const int32_t* __restrict__ owner,
+                                    const DecodeMap* __restrict__ maps,
+                                    uint32_t* __restrict__ row_count, uint32_t* __restrict__ wide) {
     const int cw = w / 4, chh = (h + 3) / 4;
     const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= (long long)cw * chh) return;
     const int x0 = 4 * (int)(c % cw), y0 = 4 * (int)(c / cw);
     const int32_t li = owner[(size_t)(y0 >> lg) * mw + (x0 >> lg)];
-    uint32_t k = 0xFFFFFFFFu;
-    if (li >= 0) {
-        const DecodeMap m = maps[li];
-        if (is_domain_cell(m)) {
-            size_t off;
-            int row;
-            cell_window(m, x0, y0, w, &off, &row);
-            k = (uint32_t)row;
-            atomicAdd(&row_count[row], 1u);
-            if (!(m.info & kLeafInteger)) *wide = 1u;
-        }
-    }
-    key[c] = k;
+    if (li < 0) return;
+    const DecodeMap m = maps[li];
+    if (!is_domain_cell(m)) return;
+    int umin, vmin;
+    cell_sample(m, x0, y0, &umin, &vmin);
+    atomicAdd(&row_count[(m.dom & 0xFFFFu) + 2 * umin], 1u);
+    if (!(m.info & kLeafInteger)) *wide = 1u;
 }
 
 // Exclusive scan of the row counts (one block): the first list slot of each source row, and
@@ -686,37 +685,59 @@ __global__ void sorted_scan_kernel(const uint32_t* __restrict__ row_count, int h
     if (threadIdx.x == 0) cursor[h] = carry;  // the number of domain cells
 }
 
-// Pass 2: each domain cell takes the next slot of its source row and writes its job there and
-// the slot into inv.  A job is 8 bytes when every leaf has the integer form (window offset;
-// A | isometry << 8 | base << 16), else 16 (window offset; qalfa | isometry << 24; beta).
-__global__ void sorted_scatter_kernel(int w, int h, int lg, int mw,
-                                      const int32_t* __restrict__ owner,
+// Pass 2: the jobs, eight threads a leaf.  A thread takes a row of the leaf's windows and gives
+// its cells (those the leaf still owns) neighbouring slots, in the order of their windows: lanes
+// that run together then read one line of the plane where the leaf is wider than a cell, and the
+// place pass finds the leaf's cells side by side.  (With a slot for each cell as
+// it came, ten steps of 8192 x 8192 took 1,152 us, so 1,110.)
+// A job is 8 bytes when every leaf has the integer form (window offset; A | isometry << 8 |
+// base << 16), else 16 (window offset; qalfa | isometry << 24; beta).
+__global__ void sorted_scatter_kernel(int w, int lg, int mw, const int32_t* __restrict__ owner,
                                       const DecodeMap* __restrict__ maps,
-                                      const DecodeLeaf* __restrict__ leaves,
-                                      const uint32_t* __restrict__ key, uint32_t* __restrict__ cursor,
+                                      const DecodeLeaf* __restrict__ leaves, int nleaves,
+                                      uint32_t* __restrict__ cursor,
                                       const uint32_t* __restrict__ wide,
                                       uint4* __restrict__ jobs, uint32_t* __restrict__ inv) {
-    const int cw = w / 4, chh = (h + 3) / 4;
-    const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= (long long)cw * chh) return;
-    const uint32_t row = key[c];
-    if (row == 0xFFFFFFFFu) return;
-    const int x0 = 4 * (int)(c % cw), y0 = 4 * (int)(c / cw);
-    const int32_t li = owner[(size_t)(y0 >> lg) * mw + (x0 >> lg)];
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const int li = (int)(t / 8);
+    if (li >= nleaves) return;
     const DecodeMap m = maps[li];
-    size_t off;
-    int r;
-    cell_window(m, x0, y0, w, &off, &r);
-    const uint32_t pos = atomicAdd(&cursor[row], 1u);
-    const uint32_t qalfa = leaves[li].w & 0x1FFFFu;
-    const uint32_t k = (m.info >> 14) & 7u;
-    if (*wide)
-        jobs[pos] = make_uint4((uint32_t)off, qalfa | (k << 24),
-                               (uint32_t)__double2loint(m.b), (uint32_t)__double2hiint(m.b));
-    else
-        reinterpret_cast<uint2*>(jobs)[pos] =
-            make_uint2((uint32_t)off, (uint32_t)m.n1 | k << 8 | (uint32_t)m.n0 << 16);
-    inv[c] = pos;
+    if (!is_domain_cell(m)) return;
+    const int S = (int)(m.info & 0xFFFu), k = (int)((m.info >> 14) & 7u);
+    const int row = (int)(m.rc & 0xFFFFu), col = (int)(m.rc >> 16);
+    const bool tr = (0xC6u >> k) & 1u, uneg = (0xACu >> k) & 1u, vneg = (0x9Au >> k) & 1u;
+    const bool big = *wide;
+    for (int u = 4 * (int)(t % 8); u < S; u += 32) {
+        const int du = uneg ? S - 4 - u : u;
+        // The 4x4 of samples (u, v) is the output cell at this position in the leaf.
+        auto cell = [&](int v, int* x0, int* y0) {
+            const int dv = vneg ? S - 4 - v : v;
+            *y0 = row + (tr ? dv : du);
+            *x0 = col + (tr ? du : dv);
+        };
+        uint32_t held = 0;
+        for (int v = 0; v < S; v += 4) {
+            int x0, y0;
+            cell(v, &x0, &y0);
+            held += owner[(size_t)(y0 >> lg) * mw + (x0 >> lg)] == li;
+        }
+        if (!held) continue;
+        const uint32_t from = (m.dom & 0xFFFFu) + 2 * u;
+        uint32_t pos = atomicAdd(&cursor[from], held);
+        for (int v = 0; v < S; v += 4) {
+            int x0, y0;
+            cell(v, &x0, &y0);
+            if (owner[(size_t)(y0 >> lg) * mw + (x0 >> lg)] != li) continue;
+            const uint32_t off = (uint32_t)((size_t)from * w + (m.dom >> 16) + 2 * v);
+            if (big)
+                jobs[pos] = make_uint4(off, (leaves[li].w & 0x1FFFFu) | (uint32_t)k << 24,
+                                       (uint32_t)__double2loint(m.b), (uint32_t)__double2hiint(m.b));
+            else
+                reinterpret_cast<uint2*>(jobs)[pos] =
+                    make_uint2(off, (uint32_t)m.n1 | (uint32_t)k << 8 | (uint32_t)m.n0 << 16);
+            inv[(size_t)(y0 / 4) * (w / 4) + x0 / 4] = pos++;
+        }
+    }
 }
 
 // Gather pass: job -> the cell's 16 output bytes (row-major 4x4) in the cell buffer.  Bound by
@@ -786,6 +807,20 @@ cudaError_t launch_decode_expand(const DecodeLeaf* leaves, const int32_t* resid_
                                  DecodeConsts c, DecodeMap* maps, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
     decode_expand_kernel<<<(n + 255) / 256, 256, 0, st>>>(leaves, resid_off, n, c, maps);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_residual_values(const DecodeLeaf* leaves, const int32_t* resid_off, int n,
+                                   const int32_t* levels, const ResidualBases& bases, uint32_t most,
+                                   double step, double* values, cudaStream_t st) {
+    if (n <= 0) return cudaSuccess;
+    if (most > kResidualMost) return cudaErrorInvalidValue;
+    const size_t smem = 2 * (size_t)most * most * sizeof(double);
+    cudaError_t e = cudaFuncSetAttribute(residual_values_kernel,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)(2 * kResidualMost * kResidualMost * sizeof(double)));
+    if (e != cudaSuccess) return e;
+    residual_values_kernel<<<n, 128, smem, st>>>(leaves, resid_off, levels, bases, step, values);
     return cudaGetLastError();
 }
 
@@ -870,21 +905,20 @@ bool decode_sorted_eligible(int w, int h, int lg, bool residuals) {
 }
 
 cudaError_t launch_decode_sorted_build(int w, int h, int lg, const int32_t* owner,
-                                       const DecodeMap* maps, const DecodeLeaf* leaves,
-                                       uint32_t* key, uint32_t* row_count, uint32_t* cursor,
-                                       uint4* jobs, uint32_t* inv, cudaStream_t st) {
+                                       const DecodeMap* maps, const DecodeLeaf* leaves, int nleaves,
+                                       uint32_t* row_count, uint32_t* cursor, uint4* jobs,
+                                       uint32_t* inv, cudaStream_t st) {
     const int mw = (w + (1 << lg) - 1) >> lg;
     const size_t cells = decode_sorted_cells(w, h);
-    cudaError_t e = cudaMemsetAsync(row_count, 0, (size_t)h * 4, st);
-    if (e != cudaSuccess) return e;
-    const unsigned blocks = (unsigned)((cells + 255) / 256);
     uint32_t* wide = cursor + h + 1;
-    e = cudaMemsetAsync(wide, 0, 4, st);
+    cudaError_t e = cudaMemsetAsync(row_count, 0, (size_t)h * 4, st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(wide, 0, 4, st);
     if (e != cudaSuccess) return e;
-    sorted_key_kernel<<<blocks, 256, 0, st>>>(w, h, lg, mw, owner, maps, key, row_count, wide);
+    sorted_count_kernel<<<(unsigned)((cells + 255) / 256), 256, 0, st>>>(w, h, lg, mw, owner, maps,
+                                                                         row_count, wide);
     sorted_scan_kernel<<<1, 1024, 0, st>>>(row_count, h, cursor);
-    sorted_scatter_kernel<<<blocks, 256, 0, st>>>(w, h, lg, mw, owner, maps, leaves, key, cursor,
-                                                   wide, jobs, inv);
+    sorted_scatter_kernel<<<(unsigned)(((size_t)nleaves * 8 + 255) / 256), 256, 0, st>>>(
+        w, lg, mw, owner, maps, leaves, nleaves, cursor, wide, jobs, inv);
     return cudaGetLastError();
 }
 

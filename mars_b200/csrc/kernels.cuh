@@ -186,6 +186,18 @@ constexpr uint32_t kLeafInteger = 1u << 18;
 // may be null when no leaf is mode 3.
 cudaError_t launch_decode_expand(const DecodeLeaf* leaves, const int32_t* resid_off, int n,
                                  DecodeConsts c, DecodeMap* maps, cudaStream_t st);
+// The residual pool of a leaf list from its levels (residual_values_kernel): for each leaf k with
+// resid_off[k] >= 0, the size*size values at resid_off[k] from the levels there.  basis holds
+// basis(size, k, i) of every such leaf's size at [basis_at[size] + k * size + i]; sizes are at
+// most kResidualMost, the largest of them `most`.
+constexpr uint32_t kResidualMost = 64;
+struct ResidualBases {
+    const double* basis;
+    uint32_t at[kResidualMost + 1];
+};
+cudaError_t launch_residual_values(const DecodeLeaf* leaves, const int32_t* resid_off, int n,
+                                   const int32_t* levels, const ResidualBases& bases, uint32_t most,
+                                   double step, double* values, cudaStream_t st);
 // owner: leaf index (or -1) per cell of 2^lg x 2^lg pixels, row-major, ceil(w/2^lg) wide.
 // resid: the residual pool (f64), or null.
 // One step of decode_until_stable (ifs.rs:321-353): a no-op once *done is set; otherwise
@@ -214,7 +226,7 @@ cudaError_t launch_decode_resident(uint8_t* buf0, uint8_t* buf1, int w, int h, i
 // Source-ordered decode of large planes (decode.cu): the domain cells' jobs sorted by the
 // source row of their windows (built once per leaf list), then per step a gather into a
 // 16-byte-per-cell buffer and a placement in output order.  Eligible: cells of 4 x 4 pixels
-// or more (lg >= 2), width % 4 == 0, no mode-3 residuals.  key / inv hold one word per 4x4
+// or more (lg >= 2), width % 4 == 0, no mode-3 residuals.  inv holds one word per 4x4
 // cell, jobs and the cell buffer 16 bytes per domain cell (at most one per cell), row_count
 // h words and cursor h + 2 (after the build cursor[h] is the number of domain cells and
 // cursor[h + 1] nonzero when some cell's leaf has no integer form: jobs are then 16 bytes, else
@@ -222,9 +234,9 @@ cudaError_t launch_decode_resident(uint8_t* buf0, uint8_t* buf1, int w, int h, i
 size_t decode_sorted_cells(int w, int h);
 bool decode_sorted_eligible(int w, int h, int lg, bool residuals);
 cudaError_t launch_decode_sorted_build(int w, int h, int lg, const int32_t* owner,
-                                       const DecodeMap* maps, const DecodeLeaf* leaves,
-                                       uint32_t* key, uint32_t* row_count, uint32_t* cursor,
-                                       uint4* jobs, uint32_t* inv, cudaStream_t st);
+                                       const DecodeMap* maps, const DecodeLeaf* leaves, int nleaves,
+                                       uint32_t* row_count, uint32_t* cursor, uint4* jobs,
+                                       uint32_t* inv, cudaStream_t st);
 cudaError_t launch_decode_sorted_step(const uint8_t* src, uint8_t* dst, int w, int h, int lg,
                                       const int32_t* owner, const DecodeMap* maps,
                                       const uint4* jobs, uint32_t njobs, bool wide_jobs,

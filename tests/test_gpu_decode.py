@@ -272,3 +272,42 @@ def test_integer_values_and_one_launch_steps(ctx, w, h, bits_alfa, bits_beta, in
         ctx.decode(hdr, leaves[:0], 1)  # waits for the context's stream
         assert np.array_equal(buf.cpu().numpy()[8: 8 + w * h].reshape(h, w), want)
     plan.close()
+
+
+@pytest.mark.parametrize("w,h,min_size,max_size", [(64, 64, 2, 16), (96, 80, 4, 32),
+                                                   (256, 128, 4, 64), (512, 256, 8, 128)])
+def test_residuals_of_every_size(ctx, w, h, min_size, max_size):
+    # Mode-3 leaves of each size: rebuilt on the device up to 64, on the host beyond; levels of
+    # every magnitude and lists of zeros, against the oracle's inverse transform bit for bit.
+    leaves = synthetic.quadtree_leaves(w, h, w + max_size, min_size=min_size, max_size=max_size)
+    rng = np.random.default_rng(w)
+    pick = (leaves["mode"] == 2) & (rng.random(len(leaves)) < 0.7)
+    leaves["mode"][pick] = 3
+    assert pick.any()
+    n = int((leaves["size"][pick].astype(np.int64) ** 2).sum())
+    levels = np.where(rng.random(n) < 0.3, rng.integers(-63, 64, n), 0).astype(np.int32)
+    hdr = _hdr(w, h)
+    want = orc.decode(_ohdr(hdr), leaves, 3, levels)
+    assert np.array_equal(ctx.decode(hdr, leaves, 3, levels), want)
+    plane, used = ctx.decode_until_stable(hdr, leaves, 1, 6, levels)
+    oplane, oused = orc.decode_until_stable(_ohdr(hdr), leaves, 1, 6, levels)
+    assert used == oused and np.array_equal(plane, oplane)
+
+
+@pytest.mark.parametrize("w,h,bits_alfa", [(128, 96, 4), (516, 132, 4), (256, 258, 7)])
+def test_source_ordered_steps_with_overwritten_leaves(ctx, monkeypatch, w, h, bits_alfa):
+    # Leaves on top of others: a leaf's rows of windows keep holes, down to none of its cells.
+    monkeypatch.setenv("MARS_DECODE_SORTED", "1")
+    under = synthetic.quadtree_leaves(w, h, w, bits_alfa=bits_alfa)
+    over = synthetic.quadtree_leaves(w, h, w + 1, bits_alfa=bits_alfa)
+    leaves = np.concatenate([under, over[over["size"] <= 8][::2], under[under["size"] >= 16][::5]])
+    hdr = _hdr(w, h, bits_alfa)
+    plan = ctx.decode_plan(hdr, leaves)
+    torch = pytest.importorskip("torch")
+    out = torch.zeros(h, w, dtype=torch.uint8, device="cuda:0")
+    torch.cuda.synchronize()
+    for iters in (1, 4):
+        plan.run(iters, out.data_ptr())
+        ctx.decode(hdr, leaves[:0], 1)  # waits for the context's stream
+        assert np.array_equal(out.cpu().numpy(), orc.decode(_ohdr(hdr), leaves, iters))
+    plan.close()
