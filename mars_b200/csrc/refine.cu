@@ -32,6 +32,7 @@
 
 #include "codec.hpp"
 #include "context.hpp"
+#include "grid_meet.cuh"
 #include "residual.hpp"
 
 namespace {
@@ -141,6 +142,155 @@ __global__ void __launch_bounds__(kBlock) refine_forward_kernel(
     block_reduce<true>(change, part);
 }
 
+// ---- the forward solve in one launch ----
+//
+// A step of a 512 x 512 plane is a few loads a pixel, less than its launch, and the host looked
+// at the change every 8 steps.  One cooperative launch runs the whole solve: a thread keeps the
+// source position, contrast and offset of four pixels of a row (in one leaf), the blocks meet
+// between steps, and every 8th step's largest change goes through an atomic maximum.  Values,
+// step counts and the test are the launches'.  Reads pass L1 by: other SMs write the plane during
+// the launch.  Bound: the barrier's and the loads' round trips to L2.  One B200: 32 steps of
+// 512 x 512 with the linearisation and the host's part 197 us, 521 as launches with the seed sent
+// from the host; 152 steps of 640 x 600 686 us, 1,886.
+
+struct ForwardArgs {
+    float *x, *xn;
+    int w, h, lg, mw;
+    const int32_t* owner;
+    const RefineLeaf* leaves;
+    const float *s, *o, *resid;
+    uint32_t max_iters, chunk;
+    double tol;
+    int warm;
+    uint32_t* sync;                // arrivals, blocks through (zero)
+    unsigned long long* largest;   // three words in turn (zero): a check's largest change, as bits
+    uint32_t* iters;
+    int* err;
+};
+constexpr int kSolveThreads = 256;  // at most
+
+__device__ __forceinline__ float2 fresh_pair(const float* p) {
+    float2 v;
+    asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p) : "memory");
+    return v;
+}
+
+__global__ void __launch_bounds__(kSolveThreads) refine_solve_kernel(const ForwardArgs g) {
+    __shared__ unsigned long long seen;
+    const uint32_t quads = (uint32_t)g.w / 4 * (uint32_t)g.h;
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool in = t < quads;
+    const int y = (int)(t / (uint32_t)(g.w / 4)), x0 = 4 * (int)(t % (uint32_t)(g.w / 4));
+    const size_t p0 = (size_t)y * g.w + x0;
+    bool moving = false;
+    float s = 0.0f, o = 0.0f, r[4] = {0.0f, 0.0f, 0.0f, 0.0f}, v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    size_t q0 = 0;
+    int dq = 0;
+    bool residual = false;
+    if (in) {
+        const int32_t li = g.owner[(size_t)(y >> g.lg) * g.mw + (x0 >> g.lg)];
+        if (li >= 0) {
+            const RefineLeaf L = g.leaves[li];
+            const uint32_t kind = (L.info >> 12) & 3u;
+            const int i = y - (int)(L.rc & 0xFFFFu), j = x0 - (int)(L.rc >> 16);
+            if (kind == kRAffine) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const double a = round(__dadd_rn(__dadd_rn(L.b0, __dmul_rn(L.gx, (double)i)),
+                                                     __dmul_rn(L.gy, (double)(j + k))));
+                    v[k] = (float)fmin(fmax(a, 0.0), 255.0);
+                }
+            } else {
+                const int S = (int)(L.info & 0xFFFu), iso = (int)((L.info >> 14) & 7u);
+                int u0, v0, u1, v1;
+                inverse_iso(iso, S, i, j, &u0, &v0);
+                inverse_iso(iso, S, i, j + 1, &u1, &v1);
+                const int du = u1 - u0, dv = v1 - v0;
+                o = g.o[li];
+                moving = kind == kRDomain;
+                if (moving) {
+                    s = g.s[li];
+                    q0 = ((size_t)(L.dom & 0xFFFFu) + 2 * u0) * g.w + (L.dom >> 16) + 2 * v0;
+                    dq = 2 * (du * g.w + dv);
+                }
+                residual = L.roff >= 0;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    if (residual) r[k] = g.resid[L.roff + (u0 + k * du) * S + v0 + k * dv];
+                    const float a = residual ? o + r[k] : o;
+                    v[k] = fminf(fmaxf(a, 0.0f), 255.0f);  // without a domain
+                }
+            }
+        }
+    }
+    float before[4] = {128.0f, 128.0f, 128.0f, 128.0f};
+    if (g.warm && in) {
+        const float4 b = *reinterpret_cast<const float4*>(g.x + p0);
+        before[0] = b.x;
+        before[1] = b.y;
+        before[2] = b.z;
+        before[3] = b.w;
+    }
+    uint32_t it = 0, target = 0;
+    for (uint32_t check = 0; it < g.max_iters; ++check) {
+        const uint32_t end = min(g.max_iters, it + g.chunk);
+        for (; it < end; ++it) {
+            const float* from = it & 1 ? g.xn : g.x;
+            if (moving) {
+                float d[4] = {128.0f, 128.0f, 128.0f, 128.0f};
+                if (it > 0 || g.warm) {
+                    float2 a[4], b[4];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const float* q = from + ((ptrdiff_t)q0 + k * (ptrdiff_t)dq);
+                        a[k] = fresh_pair(q);
+                        b[k] = fresh_pair(q + g.w);
+                    }
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        d[k] = 0.25f * ((a[k].x + a[k].y) + (b[k].x + b[k].y));
+                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    float a = fmaf(s, d[k], o);
+                    if (residual) a += r[k];
+                    v[k] = fminf(fmaxf(a, 0.0f), 255.0f);
+                }
+            }
+            if (in && (moving || it < 2))
+                *reinterpret_cast<float4*>((it & 1 ? g.x : g.xn) + p0) =
+                    make_float4(v[0], v[1], v[2], v[3]);
+            if (it + 1 == end) {
+                // The difference of two floats in f64 is not rounded; of the largest one here,
+                // f32 would be.
+                double most = 0.0;
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (in) most = fmax(most, fabs((double)v[k] - (double)before[k]));
+                for (int s2 = 16; s2 > 0; s2 >>= 1)
+                    most = fmax(most, __shfl_xor_sync(0xffffffffu, most, s2));
+                if ((threadIdx.x & 31) == 0 && most > 0.0)
+                    atomicMax(g.largest + check % 3, (unsigned long long)__double_as_longlong(most));
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) before[k] = v[k];
+            target += gridDim.x;
+            mars::grid_meet(g.sync, target, g.err);
+        }
+        if (threadIdx.x == 0) {
+            seen = *(volatile unsigned long long*)(g.largest + check % 3);
+            // Read before this meeting by all, used again two checks on.
+            if (blockIdx.x == 0) g.largest[(check + 2) % 3] = 0ull;
+        }
+        __syncthreads();
+        const bool done = __longlong_as_double((long long)seen) < g.tol;
+        __syncthreads();
+        if (done) break;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) *g.iters = it;
+    mars::grid_leave(g.sync);
+}
+
 // The linearisation at x*: d_p, the clamp gate G_p, G_p s_L (domain pixels), g = 2 (x - t);
 // per-block sums of (x - t)^2.
 __global__ void __launch_bounds__(kBlock) refine_linearise_kernel(
@@ -164,6 +314,11 @@ __global__ void __launch_bounds__(kBlock) refine_linearise_kernel(
         e = (double)r * (double)r;
     }
     block_reduce<false>(e, part);
+}
+
+__global__ void refine_fill_kernel(float* __restrict__ x, size_t n, float v) {
+    const size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (p < n) x[p] = v;
 }
 
 // mu = spl * lam (the adjoint's warm start after the linearisation changed).
@@ -197,20 +352,210 @@ __global__ void __launch_bounds__(kBlock) refine_adjoint_kernel(
     block_reduce<false>(nn, part_norm);
 }
 
-// One block: the fixed-order sum (or max) of `n` partials into out[0].
+// ---- the adjoint solve in one launch ----
+//
+// Where every domain starts at an even row and column (as all that were searched at an even
+// stride do), a domain sample is one of the plane's aligned 2x2 quads: the quad's four pixels have
+// the same list.  So a thread takes a quad: one walk of the list serves four pixels, its first
+// entries, g, spl and lambda stay in registers from step to step, and only mu crosses L2.  lambda
+// is written once, at the end.  The values are refine_adjoint_kernel's but for the order of the
+// sums: lists are skewed (one of a smooth plane's domains may serve hundreds of leaves), so what
+// lists have past their first entries is cut into runs of 32, which the block's warps share (a
+// thread a list: 595 and 789 us where this takes 265 and 304).  Bound: the barrier's and the loads' round trips to L2.  One B200:
+// 24 steps of 512 x 512 with the gradients and the host's part 211 to 304 us, 374 to 1,087 as
+// launches of a thread a pixel.
+
+struct AdjointArgs {
+    float *lam, *mu, *mun;
+    const float *g, *spl;
+    int w, h;
+    const uint32_t *csr_off, *csr_pix;
+    uint32_t max_iters, chunk;
+    double tol;
+    int warm;  // lambda and mu hold the start; else it is zero
+    uint32_t* sync;
+    double *part_diff, *part_norm;  // a block's sums at a check, two checks in turn
+    uint32_t* iters;
+    double* sums;
+    int* err;
+};
+constexpr uint32_t kHeld = 8;       // list entries in registers
+constexpr uint32_t kPieces = 1024;  // runs of 32 entries that a block shares out
+
+__device__ __forceinline__ float fresh_if(const float* p, bool take) {
+    float v;
+    asm volatile("{.reg .pred q; setp.ne.u32 q, %2, 0; mov.f32 %0, 0f00000000;"
+                 " @q ld.global.cg.f32 %0, [%1];}"
+                 : "=f"(v)
+                 : "l"(p), "r"((uint32_t)take)
+                 : "memory");
+    return v;
+}
+__device__ __forceinline__ double fresh_double(const double* p) {
+    double v;
+    asm volatile("ld.global.cg.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
+    return v;
+}
+
+__global__ void __launch_bounds__(kSolveThreads) refine_adjoint_solve_kernel(const AdjointArgs g) {
+    __shared__ double total[2][kSolveThreads / 32];
+    __shared__ double both[2];
+    __shared__ uint2 piece[kPieces];
+    __shared__ float part[kPieces];
+    __shared__ uint32_t count[kSolveThreads / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const uint32_t qw = (uint32_t)g.w / 2, quads = qw * (((uint32_t)g.h + 1) / 2);
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool in = t < quads;
+    const int y = 2 * (int)(t / qw), x = 2 * (int)(t % qw);
+    const size_t p0 = (size_t)y * g.w + x;
+    const bool two = in && y + 1 < g.h;
+    float gg[4] = {0.0f, 0.0f, 0.0f, 0.0f}, sp[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    float lam[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    uint32_t e0 = 0, e1 = 0, held[kHeld];
+    if (in) {
+        e0 = g.csr_off[p0];
+        e1 = g.csr_off[p0 + 1];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (k >= 2 && !two) break;
+            const size_t p = p0 + (k >> 1) * (size_t)g.w + (k & 1);
+            gg[k] = g.g[p];
+            sp[k] = g.spl[p];
+            if (g.warm) lam[k] = g.lam[p];
+        }
+    }
+    const uint32_t len = e1 - e0;
+#pragma unroll
+    for (int j = 0; j < (int)kHeld; ++j) held[j] = (uint32_t)j < len ? g.csr_pix[e0 + j] : 0u;
+    // The block's pieces: thread t's are [first, last), and what found no room starts at rest.
+    const uint32_t wanted = len > kHeld ? (len - kHeld + 31) / 32 : 0u;
+    uint32_t first = wanted;
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, first, o);
+        if (lane >= o) first += v;
+    }
+    if (lane == 31) count[warp] = first;
+    __syncthreads();
+    uint32_t pieces = 0;
+    for (int k = 0; k < warps; ++k) {
+        if (k < warp) first += count[k];
+        pieces += count[k];
+    }
+    first = min(first - wanted, kPieces);
+    pieces = min(pieces, kPieces);
+    const uint32_t last = min(first + wanted, kPieces);
+    const uint32_t rest = min(e1, e0 + kHeld + 32 * (last - first));
+    for (uint32_t c = first; c < last; ++c) {
+        const uint32_t from = e0 + kHeld + 32 * (c - first);
+        piece[c] = make_uint2(from, min(from + 32, e1));
+    }
+    __syncthreads();
+    uint32_t it = 0, target = 0;
+    bool done = false;
+    for (uint32_t check = 0; it < g.max_iters && !done; ++check) {
+        // Blocks may still read the last check's sums when others reach the next one (a last
+        // stretch of one step): the two checks' places alternate.
+        const uint32_t place = (check & 1u) * gridDim.x;
+        const uint32_t end = min(g.max_iters, it + g.chunk);
+        for (; it < end; ++it) {
+            const float* mu = it & 1 ? g.mun : g.mu;
+            float acc = 0.0f;
+            if (it > 0 || g.warm) {  // mu is zero at first
+                float m[kHeld];
+#pragma unroll
+                for (int j = 0; j < (int)kHeld; ++j) m[j] = fresh_if(mu + held[j], (uint32_t)j < len);
+#pragma unroll
+                for (int j = 0; j < (int)kHeld; ++j) acc += m[j];
+                if (pieces) {
+                    for (uint32_t c0 = warp; c0 < pieces; c0 += 4 * warps) {
+                        float b[4];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            const uint32_t c = min(c0 + j * warps, pieces - 1);
+                            const uint32_t e = piece[c].x + lane, to = piece[c].y;
+                            b[j] = fresh_if(mu + __ldg(g.csr_pix + min(e, to - 1)), e < to);
+                        }
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            for (int o = 16; o > 0; o >>= 1)
+                                b[j] += __shfl_xor_sync(0xffffffffu, b[j], o);
+                            if (lane == 0 && c0 + j * warps < pieces) part[c0 + j * warps] = b[j];
+                        }
+                    }
+                    __syncthreads();
+                    for (uint32_t c = first; c < last; ++c) acc += part[c];
+                }
+                for (uint32_t e = rest; e < e1; ++e) acc += fresh_if(mu + __ldg(g.csr_pix + e), true);
+            }
+            float v[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) v[k] = fmaf(0.25f, acc, gg[k]);
+            float* to = (it & 1 ? g.mu : g.mun) + p0;
+            if (in) *reinterpret_cast<float2*>(to) = make_float2(sp[0] * v[0], sp[1] * v[1]);
+            if (two) *reinterpret_cast<float2*>(to + g.w) = make_float2(sp[2] * v[2], sp[3] * v[3]);
+            if (it + 1 == end) {
+                double dd = 0.0, nn = 0.0;
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (k < 2 ? in : two) {
+                        const double dv = (double)v[k] - (double)lam[k];
+                        dd += dv * dv;
+                        nn += (double)v[k] * (double)v[k];
+                    }
+                for (int o = 16; o > 0; o >>= 1) {
+                    dd += __shfl_xor_sync(0xffffffffu, dd, o);
+                    nn += __shfl_xor_sync(0xffffffffu, nn, o);
+                }
+                if (lane == 0) {
+                    total[0][warp] = dd;
+                    total[1][warp] = nn;
+                }
+                __syncthreads();
+                if (threadIdx.x < 2) {
+                    double a = 0.0;
+                    for (int k = 0; k < warps; ++k) a += total[threadIdx.x][k];
+                    (threadIdx.x ? g.part_norm : g.part_diff)[place + blockIdx.x] = a;
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) lam[k] = v[k];
+            target += gridDim.x;
+            mars::grid_meet(g.sync, target, g.err);
+        }
+        // Every block adds the blocks' sums in the same order.
+        if (warp < 2) {
+            const double* from = warp ? g.part_norm : g.part_diff;
+            double a = 0.0;
+            for (uint32_t k = lane; k < gridDim.x; k += 32) a += fresh_double(from + place + k);
+            for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+            if (lane == 0) both[warp] = a;
+        }
+        __syncthreads();
+        const double rel = both[1] > 0.0 ? sqrt(both[0] / both[1]) : 0.0;
+        done = rel < g.tol;
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            g.sums[0] = both[0];
+            g.sums[1] = both[1];
+            *g.iters = it;
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        if (k < 2 ? in : two) g.lam[p0 + (k >> 1) * (size_t)g.w + (k & 1)] = lam[k];
+    mars::grid_leave(g.sync);
+}
+
+// Block b: the fixed-order sum (or max) of the `n` partials of part (b = 0) or part2 into out[b].
 template <bool use_max>
 __global__ void __launch_bounds__(kBlock) reduce_parts_kernel(const double* __restrict__ part,
+                                                              const double* __restrict__ part2,
                                                               int n, double* __restrict__ out) {
-    __shared__ double sh[kBlock];
+    const double* from = blockIdx.x ? part2 : part;
     double a = 0.0;
-    for (int k = threadIdx.x; k < n; k += blockDim.x) a = use_max ? fmax(a, part[k]) : a + part[k];
-    sh[threadIdx.x] = a;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double r = sh[0];
-        for (int k = 1; k < kBlock; ++k) r = use_max ? fmax(r, sh[k]) : r + sh[k];
-        out[0] = r;
-    }
+    for (int k = threadIdx.x; k < n; k += blockDim.x) a = use_max ? fmax(a, from[k]) : a + from[k];
+    block_reduce<use_max>(a, out);
 }
 
 // One warp per leaf: the kGradStats sums over the pixels the leaf owns (a later leaf may
@@ -226,6 +571,7 @@ __global__ void refine_grad_kernel(const float* __restrict__ lam, const float* _
     const RefineLeaf L = leaves[li];
     const int S = (int)(L.info & 0xFFFu), r0 = (int)(L.rc & 0xFFFFu), c0 = (int)(L.rc >> 16);
     double acc[kGradStats] = {0.0, 0.0, 0.0, 0.0, 0.0};
+#pragma unroll 4
     for (int k = lane; k < S * S; k += 32) {
         const int y = r0 + k / S, x = c0 + k % S;
         if (owner[(size_t)(y >> lg) * mw + (x >> lg)] != li) continue;
@@ -283,6 +629,8 @@ struct mars_refine_plan {
     float *s = nullptr, *o = nullptr;
     double* stats = nullptr;
     double *part = nullptr, *part2 = nullptr, *red = nullptr;
+    unsigned long long* solve = nullptr;  // the one-launch solve's words
+    bool even_domains = true;             // every domain starts at an even row and column
 };
 
 namespace {
@@ -292,7 +640,7 @@ void free_plan(mars_refine_plan* p) {
                     (void*)p->csr_pix, (void*)p->t, (void*)p->x, (void*)p->xn, (void*)p->dm,
                     (void*)p->gate, (void*)p->spl, (void*)p->g, (void*)p->lam, (void*)p->lamn,
                     (void*)p->mu, (void*)p->mun, (void*)p->s, (void*)p->o, (void*)p->stats,
-                    (void*)p->part, (void*)p->part2, (void*)p->red})
+                    (void*)p->part, (void*)p->part2, (void*)p->red, (void*)p->solve})
         cudaFree(q);
     delete p;
 }
@@ -314,19 +662,65 @@ void dequantise(const mars_header& hdr, const mars_leaf& L, double* alfa, double
     if (*alfa > 0.0) *beta -= *alfa * 255.0;
 }
 
+// A solve as one cooperative launch of `threads` threads, each with a part of the plane: *taken
+// says whether all can be resident at once, in at most four blocks an SM (more blocks polling the
+// counter cost more than the launches they save).  The words: largest[3], sync[2], the step
+// count, then the adjoint's two sums.
+constexpr size_t kSolveWords = 3 * 8 + 4 * 4 + 2 * 8;
+
+template <class Args>
+int launch_solve(mars_refine_plan* p, void (*kernel)(Args), Args g, size_t threads,
+                 uint32_t max_iters, bool* taken) {
+    *taken = false;
+    const size_t sms = (size_t)p->ctx->num_sms;
+    const unsigned per = threads <= 2 * sms * 128 ? 128 : 256;
+    const size_t blocks = (threads + per - 1) / per;
+    if (max_iters == 0 || blocks > 4 * sms || (uint64_t)blocks * max_iters >= (1ull << 31))
+        return MARS_OK;
+    int per_sm = 0;
+    RF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, (int)per, 0));
+    if (blocks > sms * (size_t)per_sm) return MARS_OK;
+    const cudaStream_t st = p->ctx->stream;
+    RF_CUDA(cudaMemsetAsync(p->solve, 0, kSolveWords, st));
+    void* args[] = {&g};
+    const cudaError_t e = cudaLaunchCooperativeKernel((const void*)kernel, dim3((unsigned)blocks),
+                                                      dim3(per), args, 0, st);
+    if (e == cudaErrorCooperativeLaunchTooLarge) {  // fewer SMs than the device has
+        cudaGetLastError();
+        return MARS_OK;
+    }
+    RF_CUDA(e);
+    p->ctx->launches += 1;
+    *taken = true;
+    return MARS_OK;
+}
+
 // Iterates F until max |x' - x| < tol or max_iters, from the flat-128 seed (warm = false)
 // or from the current x; reduces every `chunk` steps.
 int run_forward(mars_refine_plan* p, uint32_t max_iters, double tol, bool warm, uint32_t* iters) {
     const cudaStream_t st = p->ctx->stream;
     const size_t n = (size_t)p->w * p->h;
-    if (!warm) {
-        std::vector<float> seed(n, 128.0f);
-        RF_CUDA(cudaMemcpyAsync(p->x, seed.data(), n * 4, cudaMemcpyHostToDevice, st));
-        if (int e = mars::ctx_sync(p->ctx)) return e;
-    }
     uint32_t it = 0;
     double change = 0.0;
     const uint32_t chunk = 8;
+    bool solved = false;
+    uint32_t* words = reinterpret_cast<uint32_t*>(p->solve + 3);
+    if (p->lg >= 2 && p->w % 4 == 0 && p->even_domains) {
+        const ForwardArgs g{p->x, p->xn, (int)p->w, (int)p->h, p->lg, p->mw, p->owner, p->dleaves,
+                            p->s, p->o, p->resid, max_iters, chunk, tol, warm, words, p->solve,
+                            words + 2, p->ctx->d_err};
+        if (int e = launch_solve(p, refine_solve_kernel, g, n / 4, max_iters, &solved)) return e;
+    }
+    if (solved) {
+        RF_CUDA(cudaMemcpyAsync(iters, words + 2, 4, cudaMemcpyDeviceToHost, st));
+        if (int e = mars::ctx_sync(p->ctx)) return e;
+        if (*iters & 1) std::swap(p->x, p->xn);
+        return MARS_OK;
+    }
+    if (!warm) {
+        refine_fill_kernel<<<p->nblocks, kBlock, 0, st>>>(p->x, n, 128.0f);
+        p->ctx->launches += 1;
+    }
     while (it < max_iters) {
         const uint32_t m = std::min(chunk, max_iters - it);
         for (uint32_t k = 0; k < m; ++k) {
@@ -335,7 +729,7 @@ int run_forward(mars_refine_plan* p, uint32_t max_iters, double tol, bool warm, 
                 p->resid, p->part);
             std::swap(p->x, p->xn);
         }
-        reduce_parts_kernel<true><<<1, kBlock, 0, st>>>(p->part, p->nblocks, p->red);
+        reduce_parts_kernel<true><<<1, kBlock, 0, st>>>(p->part, nullptr, p->nblocks, p->red);
         p->ctx->launches += m + 1;
         RF_CUDA(cudaGetLastError());
         RF_CUDA(cudaMemcpyAsync(&change, p->red, 8, cudaMemcpyDeviceToHost, st));
@@ -353,7 +747,7 @@ int run_linearise(mars_refine_plan* p, double* loss) {
     refine_linearise_kernel<<<p->nblocks, kBlock, 0, st>>>(
         p->x, p->t, (int)p->w, (int)p->h, p->lg, p->mw, p->owner, p->dleaves, p->s, p->o,
         p->resid, p->dm, p->gate, p->spl, p->g, p->part);
-    reduce_parts_kernel<false><<<1, kBlock, 0, st>>>(p->part, p->nblocks, p->red);
+    reduce_parts_kernel<false><<<1, kBlock, 0, st>>>(p->part, nullptr, p->nblocks, p->red);
     p->ctx->launches += 2;
     RF_CUDA(cudaGetLastError());
     RF_CUDA(cudaMemcpyAsync(loss, p->red, 8, cudaMemcpyDeviceToHost, st));
@@ -366,18 +760,37 @@ int run_backward(mars_refine_plan* p, uint32_t max_iters, double tol, bool warm,
                  double* residual) {
     const cudaStream_t st = p->ctx->stream;
     const size_t n = (size_t)p->w * p->h;
-    if (warm) {
-        refine_mu_kernel<<<p->nblocks, kBlock, 0, st>>>(p->lam, p->spl, n, p->mu);
-        p->ctx->launches += 1;
-    } else {
-        RF_CUDA(cudaMemsetAsync(p->lam, 0, n * 4, st));
-        RF_CUDA(cudaMemsetAsync(p->mu, 0, n * 4, st));
-    }
     uint32_t it = 0;
     double rel = 0.0;
     double sums[2] = {0.0, 0.0};
     const uint32_t chunk = 8;
-    while (it < max_iters) {
+    if (warm) {
+        refine_mu_kernel<<<p->nblocks, kBlock, 0, st>>>(p->lam, p->spl, n, p->mu);
+        p->ctx->launches += 1;
+    }
+    bool solved = false;
+    if (p->w % 2 == 0 && p->even_domains) {
+        uint32_t* words = reinterpret_cast<uint32_t*>(p->solve + 3);
+        double* dsums = reinterpret_cast<double*>(words + 4);
+        const AdjointArgs g{p->lam, p->mu, p->mun, p->g, p->spl, (int)p->w, (int)p->h, p->csr_off,
+                            p->csr_pix, max_iters, chunk, tol, warm, words, p->part, p->part2,
+                            words + 2, dsums, p->ctx->d_err};
+        if (int e = launch_solve(p, refine_adjoint_solve_kernel, g,
+                                 (size_t)(p->w / 2) * ((p->h + 1) / 2), max_iters, &solved))
+            return e;
+        if (solved) {
+            RF_CUDA(cudaMemcpyAsync(&it, words + 2, 4, cudaMemcpyDeviceToHost, st));
+            RF_CUDA(cudaMemcpyAsync(sums, dsums, 16, cudaMemcpyDeviceToHost, st));
+            if (int e = mars::ctx_sync(p->ctx)) return e;
+            rel = sums[1] > 0.0 ? std::sqrt(sums[0] / sums[1]) : 0.0;
+            if (it & 1) std::swap(p->mu, p->mun);
+        }
+    }
+    if (!solved && !warm) {
+        RF_CUDA(cudaMemsetAsync(p->lam, 0, n * 4, st));
+        RF_CUDA(cudaMemsetAsync(p->mu, 0, n * 4, st));
+    }
+    while (!solved && it < max_iters) {
         const uint32_t m = std::min(chunk, max_iters - it);
         for (uint32_t k = 0; k < m; ++k) {
             refine_adjoint_kernel<<<p->nblocks, kBlock, 0, st>>>(
@@ -386,9 +799,8 @@ int run_backward(mars_refine_plan* p, uint32_t max_iters, double tol, bool warm,
             std::swap(p->lam, p->lamn);
             std::swap(p->mu, p->mun);
         }
-        reduce_parts_kernel<false><<<1, kBlock, 0, st>>>(p->part, p->nblocks, p->red);
-        reduce_parts_kernel<false><<<1, kBlock, 0, st>>>(p->part2, p->nblocks, p->red + 1);
-        p->ctx->launches += m + 2;
+        reduce_parts_kernel<false><<<2, kBlock, 0, st>>>(p->part, p->part2, p->nblocks, p->red);
+        p->ctx->launches += m + 1;
         RF_CUDA(cudaGetLastError());
         RF_CUDA(cudaMemcpyAsync(sums, p->red, 16, cudaMemcpyDeviceToHost, st));
         if (int e = mars::ctx_sync(p->ctx)) return e;
@@ -516,6 +928,7 @@ int mars_refine_plan_create(mars_ctx* ctx, const mars_header* hdr, const mars_le
                     rvals.push_back((float)v);
             }
         }
+        if (domain && ((L.dom_row | L.dom_col) & 1u)) p->even_domains = false;
         p->kind[k] = (uint8_t)kind;
         r.info = L.size | (kind << 12) | (L.isometry << 14);
     }
@@ -572,9 +985,13 @@ int mars_refine_plan_create(mars_ctx* ctx, const mars_header* hdr, const mars_le
     for (float** b : {&p->s, &p->o})
         if (e == cudaSuccess) e = cudaMalloc(b, std::max<size_t>(1, n) * 4);
     if (e == cudaSuccess) e = cudaMalloc(&p->stats, std::max<size_t>(1, n) * kGradStats * 8);
-    if (e == cudaSuccess) e = cudaMalloc(&p->part, (size_t)p->nblocks * 8);
-    if (e == cudaSuccess) e = cudaMalloc(&p->part2, (size_t)p->nblocks * 8);
+    // A partial a block of the step launches, or two of the one-launch adjoint's.
+    const size_t solve_blocks = ((size_t)(w / 2) * ((h + 1) / 2) + 127) / 128;
+    const size_t parts = std::max<size_t>((size_t)p->nblocks, 2 * solve_blocks);
+    if (e == cudaSuccess) e = cudaMalloc(&p->part, parts * 8);
+    if (e == cudaSuccess) e = cudaMalloc(&p->part2, parts * 8);
     if (e == cudaSuccess) e = cudaMalloc(&p->red, 16);
+    if (e == cudaSuccess) e = cudaMalloc(&p->solve, kSolveWords);
     if (e != cudaSuccess) {
         free_plan(p.release());
         return fail(MARS_ECUDA, std::string("refine plan: ") + cudaGetErrorString(e));

@@ -71,6 +71,34 @@ def test_forward_and_gradients_match_fp64(ctx, kind, w, h, seed, modes):
     plan.close()
 
 
+@pytest.mark.parametrize("w,h,odd", [(32, 32, False), (100, 77, False), (102, 76, False),
+                                     (101, 64, False), (96, 64, True), (640, 520, False)])
+@pytest.mark.parametrize("steps", [1, 2, 9, 17])
+def test_given_step_counts_match_fp64(ctx, w, h, odd, steps):
+    # Solves in one launch and as launches (odd widths, odd domain columns), whose last stretch
+    # before a check is one step: the iterates after exactly `steps` of them.
+    img, oh, leaves, _ = _case("random", w, h, w + h, None)
+    if odd:
+        move = (leaves["mode"] == 2) & (leaves["dom_col"] + 2 * leaves["size"] < w)
+        leaves["dom_col"][move] += 1
+        assert move.any()
+    plan = ctx.refine_plan(_mb_hdr(oh), leaves, img)
+    s, o = plan.params()
+    for _ in range(2):
+        loss, used, x = plan.forward(s, o, max_iters=steps, tol=0.0, want_x=True)
+        gs, go, back, _ = plan.backward(max_iters=steps, tol=0.0)
+        assert (used, back) == (steps, steps)
+    ol, ox, ogs, ogo = orc.refine_eval(oh, leaves, img, s.astype(np.float64), o.astype(np.float64),
+                                       None, fwd_iters=steps, adj_iters=steps)
+    # A step rounds three times below 512 (2^-15 each) and the contraction keeps their sum
+    # within 16 steps' worth.
+    assert np.abs(x - ox).max() < 16 * 3 * 2.0 ** -15
+    assert loss == pytest.approx(ol, rel=1e-4)
+    g, og = np.concatenate([gs, go]).astype(np.float64), np.concatenate([ogs, ogo])
+    assert np.linalg.norm(g - og) <= 1e-3 * np.linalg.norm(og)
+    plan.close()
+
+
 def test_backward_needs_a_forward(ctx):
     img, oh, leaves, res = _case("random", 64, 64, 5, None)
     plan = ctx.refine_plan(_mb_hdr(oh), leaves, img, res)
