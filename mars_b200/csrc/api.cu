@@ -1653,6 +1653,12 @@ extern "C" {
 
 namespace {
 
+int plan_encode_device(mars_search_plan* plan, mars_search_plan* warm_plan, const uint8_t* plane,
+                       const mars_options* o, mars_header* header, mars_leaf** leaves,
+                       size_t* nleaves, int32_t** residuals, size_t* nresiduals,
+                       mars_counters* counters);
+int fisher_walk_on_device(mars_search_plan* fplan, mars_search_plan* wplan, bool* usable);
+
 // The plan mars_encode uses for a plane geometry it has encoded before: one search plan
 // per (width, height, params), made on the second encode of that geometry (the first takes
 // the one-shot path), for planes up to kPlanCachePixels and at most kPlanCacheSize
@@ -1731,6 +1737,11 @@ int mars_encode(mars_ctx* ctx, const uint8_t* plane, uint32_t width, uint32_t he
         mars_search_plan* wplan =
             params->has_lambda ? cached_encode_plan(ctx, width, height, &wp) : nullptr;
         if (fplan && (!params->has_lambda || wplan)) {
+            bool device_walk = false;
+            if (int e = fisher_walk_on_device(fplan, wplan, &device_walk)) return e;
+            if (device_walk)
+                return plan_encode_device(fplan, wplan, plane, options, header, leaves, nleaves,
+                                          residuals, nresiduals, counters);
             mars_table* ft = nullptr;
             mars_table* wt = nullptr;
             if (int e = mars_search_plan_run(fplan, plane, &ft)) return e;
@@ -2213,6 +2224,25 @@ bool plan_walk_on_host() {
     return on;
 }
 
+// Whether a Fisher encode's walks run on the device: both plans' trees can be walked there, over
+// the same nodes in the same order.
+int fisher_walk_on_device(mars_search_plan* fplan, mars_search_plan* wplan, bool* usable) {
+    *usable = false;
+    if (plan_walk_on_host()) return MARS_OK;
+    bool f = false, w = true;
+    if (int e = plan_walk_setup(fplan, &f)) return e;
+    if (wplan) {
+        if (int e = plan_walk_setup(wplan, &w)) return e;
+        w = w && fplan->jobs.size() == wplan->jobs.size();
+        for (size_t i = 0; w && i < fplan->jobs.size(); ++i)
+            w = fplan->jobs[i].size == wplan->jobs[i].size &&
+                fplan->jobs[i].rows == wplan->jobs[i].rows &&
+                fplan->jobs[i].cols == wplan->jobs[i].cols;
+    }
+    *usable = f && w;
+    return MARS_OK;
+}
+
 template <class T>
 int copy_out_array(const std::vector<T>& v, T** out, size_t* n) {
     *n = v.size();
@@ -2224,8 +2254,11 @@ int copy_out_array(const std::vector<T>& v, T** out, size_t* n) {
 
 // A planned encode with both walks on the device: the plan's search, then the warm-up walk
 // over its candidates, the rate snapshot on the host from the warm-up leaves, the pricing of
-// every node and the RD walk's decisions -- the host receives only leaves.
-int plan_encode_device(mars_search_plan* plan, const uint8_t* plane, const mars_options* o,
+// every node and the RD walk's decisions -- the host receives only leaves.  warm: the plan whose
+// candidates the warm-up walk of an RD encode reads, when not the same (a Fisher plan's
+// exhaustive partner, with the same nodes).
+int plan_encode_device(mars_search_plan* plan, mars_search_plan* warm_plan, const uint8_t* plane,
+                       const mars_options* o,
                        mars_header* header, mars_leaf** leaves, size_t* nleaves,
                        int32_t** residuals, size_t* nresiduals, mars_counters* counters) {
     mars_ctx* ctx = plan->ctx;
@@ -2242,10 +2275,13 @@ int plan_encode_device(mars_search_plan* plan, const uint8_t* plane, const mars_
     Scratch sc(st);
     unsigned char* d_cands;
     uint8_t* d_px;
+    unsigned char* d_wcands = nullptr;
+    uint64_t* d_evals = nullptr;  // a Fisher plan's, found by the run
     mars::WalkScratch ws{};
     mars_leaf *d_warm, *d_leaves;
     MARS_CUDA(sc.get(&d_cands, nodes * sizeof(mars_candidate)));
-
+    if (warm_plan) MARS_CUDA(sc.get(&d_wcands, nodes * sizeof(mars_candidate)));
+    if (plan->method == MARS_METHOD_FISHER) MARS_CUDA(sc.get(&d_evals, nodes));
     MARS_CUDA(sc.get(&d_px, (size_t)plan->w * plan->h));
     MARS_CUDA(sc.get(&ws.split, nodes));
     MARS_CUDA(sc.get(&ws.cnt, nodes));
@@ -2281,6 +2317,17 @@ int plan_encode_device(mars_search_plan* plan, const uint8_t* plane, const mars_
                                   cudaMemcpyDeviceToDevice, ctx->stream));
         MARS_CUDA(cudaMemcpyAsync(d_px, plan->d_plane, (size_t)plan->w * plan->h,
                                   cudaMemcpyDeviceToDevice, ctx->stream));
+        if (d_evals)
+            MARS_CUDA(cudaMemcpyAsync(d_evals, plan->d_evals, nodes * sizeof(uint64_t),
+                                      cudaMemcpyDeviceToDevice, ctx->stream));
+        if (warm_plan) {
+            MARS_CUDA(cudaMemcpyAsync(warm_plan->d_plane, plan->d_plane, (size_t)plan->w * plan->h,
+                                      cudaMemcpyDeviceToDevice, ctx->stream));
+            MARS_CUDA(cudaGraphLaunch(warm_plan->x_dev, ctx->stream));
+            ctx->launches += warm_plan->launches_per_run;
+            MARS_CUDA(cudaMemcpyAsync(d_wcands, warm_plan->d_out, nodes * sizeof(mars_candidate),
+                                      cudaMemcpyDeviceToDevice, ctx->stream));
+        }
         MARS_CUDA(cudaEventRecord(ev_search, ctx->stream));
     }
     MARS_CUDA(cudaStreamWaitEvent(st, ev_search, 0));
@@ -2288,7 +2335,9 @@ int plan_encode_device(mars_search_plan* plan, const uint8_t* plane, const mars_
     wp.px = d_px;
     // The warm-up walk (t_rms = 8 for the rate snapshot; the plain walk itself without RD).
     const double t_rms = prm.has_lambda ? 8.0 : prm.t_rms;
-    MARS_CUDA(mars::launch_warm_walk(wp, d_cands, sizeof(mars_candidate), t_rms, prm.min_size,
+    if (warm_plan) wp.evals = warm_plan->walk.evals;
+    else if (d_evals) wp.evals = d_evals;
+    MARS_CUDA(mars::launch_warm_walk(wp, warm_plan ? d_wcands : d_cands, sizeof(mars_candidate), t_rms, prm.min_size,
                                      prm.zero_threshold, hdr.bits_beta, ws, d_warm, st));
     ctx->launches += 2 * w.nlevels + 1;
     unsigned long long tot[2];
@@ -2366,6 +2415,10 @@ int plan_encode_device(mars_search_plan* plan, const uint8_t* plane, const mars_
     if (int e = sync_bounded(ctx, st)) return e;
     std::vector<mars_leaf> out(tot[0]);
     std::vector<int32_t> res(tot[1]);
+    std::vector<uint64_t> evals(d_evals ? nodes : 0);
+    if (d_evals)
+        MARS_CUDA(cudaMemcpyAsync(evals.data(), d_evals, nodes * sizeof(uint64_t),
+                                  cudaMemcpyDeviceToHost, st));
     MARS_CUDA(cudaMemcpyAsync(out.data(), d_leaves, out.size() * sizeof(mars_leaf),
                               cudaMemcpyDeviceToHost, st));
     if (!res.empty())
@@ -2373,6 +2426,10 @@ int plan_encode_device(mars_search_plan* plan, const uint8_t* plane, const mars_
                                   cudaMemcpyDeviceToHost, st));
     if (int e = sync_bounded(ctx, st)) return e;
     counters->search_evals = plan->total_evals;
+    if (d_evals) {
+        counters->search_evals = 0;
+        for (uint64_t e : evals) counters->search_evals += e;
+    }
     counters->warmup_evals = warm_evals;
     if (int e = copy_out_array(out, leaves, nleaves)) return e;
     if (int e = copy_out_array(res, residuals, nresiduals)) {
@@ -2407,7 +2464,7 @@ int mars_encode_planned(mars_search_plan* plan, const uint8_t* plane,
     if (!plan_walk_on_host())
         if (int e = plan_walk_setup(plan, &device_walk)) return e;
     if (device_walk)
-        return plan_encode_device(plan, plane, options, header, leaves, nleaves, residuals,
+        return plan_encode_device(plan, nullptr, plane, options, header, leaves, nleaves, residuals,
                                   nresiduals, counters);
     mars_table* table = nullptr;
     if (int e = mars_search_plan_run(plan, plane, &table)) return e;
