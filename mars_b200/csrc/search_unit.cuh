@@ -16,7 +16,8 @@
 // The filter stays exact.  Rounding to f16 moves a row by at most 2^-11 of its length (the
 // factor 64 keeps what a flushed subnormal could add below 2^-17), so rho is off by at most
 // 2^-10 + 2^-22 from the operands and, |products| summing to at most 1, by less than 2^-14 from
-// f32 accumulation; thresholds are lowered by 2^-9.  What passes is evaluated again from the
+// f32 accumulation, 0.00104 together; thresholds are lowered by 4.5 / 4096 = 0.0011.  (2^-9 let
+// twice as many pass where a step edge meets many like it.)  What passes is evaluated again from the
 // integers: the exact correlation, the full bound of fit.cuh with the largest contrast added,
 // then the f64 fit.  So the winners, their rms bits and the tie order are the integer path's.
 //
@@ -28,7 +29,11 @@
 // shared memory, and the fit warp of its column half evaluates them, up to 32 at a time, so the
 // scan does not wait for window loads and f64 divisions; at the end of an item the scan warps
 // evaluate what is left in theirs.  (Evaluated by the scan warps throughout, the registers kept
-// around it cost every tile more than the evaluation.)  A scan warp whose ring is full waits.
+// around it cost every tile more than the evaluation.)  A scan warp whose ring is full evaluates
+// some of it: the ranges of highest contrast are step edges that a thousand domains match nearly
+// alike, and two fit warps alone took 2.2 ms over such a tile of a 640 x 480 plane at stride 4,
+// ten times a usual tile and more than everything after it: every node of that plane alone
+// took 3.2 to 4.3 ms, 2.0 to 2.2 so.
 // Champions are guarded by a sequence lock per range, a ring's takers by a lock; every wait is
 // bounded.
 //
@@ -47,7 +52,9 @@
 //
 // Bound: the maxima and comparisons after the accumulator (5 ALU instructions per 8 fits, a half-
 // rate pipe) and the survivors.  Measured on one B200 at stride 2, sizes 32..4: the search of a
-// 512 x 512 plane 3.70 -> 2.35 ms, of a 1024 x 1024 plane 49.8 -> 27.3 ms; a 128 x 256 tile at
+// 512 x 512 plane 3.70 -> 2.35 ms, of a 1024 x 1024 plane 49.8 -> 27.3 ms (before the lower
+// allowance and the help with full rings: an encode of 512 x 512 by 14 % and of 1536 x 1024 by 9 %
+// faster with them); a 128 x 256 tile at
 // S = 4 takes 1,150 cycles with its survivors, the integer form's 2,900, the bare pipeline (MMA,
 // accumulator reads, maxima) 550.
 
@@ -65,7 +72,7 @@ constexpr int kSlots = 16;                                 // tiles announced ah
 constexpr int kGroup = 8;                                  // tiles that share their thresholds
 constexpr int kSets = 32;                                  // sets of thresholds in use
 constexpr float kUnitScale = 4096.0f;                      // 64 x 64
-constexpr float kUnitSlack = kUnitScale / 512.0f;          // 2^-9, the filter's allowance
+constexpr float kUnitSlack = 4.5f;                         // the filter's allowance
 constexpr float kUnitLeast = kUnitScale / 64.0f;           // thresholds below take the full form
 
 // A tile as the load warp announces it: what to do, which domains, and the set of thresholds its
@@ -443,11 +450,13 @@ __device__ __forceinline__ unsigned long long unit_take(USmem& sm, int first) {
     return e;
 }
 
-// Appends the warp's entries (lanes with `act`) to its own ring, waiting (bounded) for the fit
-// warp when they do not fit: false when the wait gave up.  head is the ring's next slot, tail
-// the last tail read.
-__device__ __forceinline__ bool unit_push(USmem& sm, int w, bool act, unsigned long long entry,
-                                          uint32_t& head, uint32_t& tail, int* err) {
+// Appends the warp's entries (lanes with `act`) to its own ring; while they do not fit, evaluates
+// some of it, or waits (bounded) for the fit warp that holds it: false when the wait gave up.  head
+// is the ring's next slot, tail the last tail read.
+template <int S>
+__device__ __forceinline__ bool unit_push(const ItemArgs& a, USmem& sm, const uint8_t* pix, int w,
+                                          bool act, unsigned long long entry, uint32_t& head,
+                                          uint32_t& tail, int* err) {
     volatile int* abort_flag = &sm.abort_flag;
     const uint32_t bal = __ballot_sync(0xffffffffu, act);
     const uint32_t count = __popc(bal);
@@ -456,12 +465,17 @@ __device__ __forceinline__ bool unit_push(USmem& sm, int w, bool act, unsigned l
         for (;;) {
             tail = __shfl_sync(0xffffffffu, *(volatile uint32_t*)&sm.utail[w], 0);
             if (head + count - tail <= (uint32_t)kRing) break;
+            const unsigned long long mine = unit_take<32>(sm, w);
+            if (__any_sync(0xffffffffu, mine != 0ull)) {
+                unit_fit<S>(a, sm, pix, mine, false, err);
+                continue;
+            }
             if (clock64() - t0 > kWaitCycles) {
                 *abort_flag = 1;
                 atomicOr(err, 128);
             }
             if (__any_sync(0xffffffffu, *abort_flag != 0)) return false;
-            __nanosleep(200);
+            __nanosleep(100);
         }
     }
     if (act)
@@ -869,8 +883,8 @@ __device__ __noinline__ void unit_scan_role(const ItemArgs& a, USmem& sm, const 
             for (int q = 0; q < 8; ++q) mask |= (top[q] >= __float_as_int(th[q]) ? 1u : 0u) << q;
             if (slow) mask |= unit_look_full(a, sm, slow, rb, tcol + 64u * hf, pos, ndom);
             while (__any_sync(0xffffffffu, mask != 0u)) {
-                if (!unit_push(sm, w, mask != 0u, unit_entry(pos, rb + __ffs(mask) - 1), head, tail,
-                               err))
+                if (!unit_push<S>(a, sm, pix, w, mask != 0u, unit_entry(pos, rb + __ffs(mask) - 1),
+                                  head, tail, err))
                     break;
                 mask &= mask - 1u;
             }
@@ -1337,8 +1351,11 @@ __global__ void __launch_bounds__(kUnitThreads, 1)
         const ItemArgs& a = L.args[j];
         // Split-major within a job: a range tile's later splits start after its earlier ones
         // have finished and begin from their champions (the shared records).
+        // The range tiles of either end of the contrast order are the slow ones (flat blocks in
+        // the full form, step edges with many survivors): both ends first.
         const int local = item - L.item_begin[j];
-        const int ntile = L.tile_begin[j] + local % L.tile_count[j];
+        const int turn = local % L.tile_count[j];
+        const int ntile = L.tile_begin[j] + (turn & 1 ? turn / 2 : L.tile_count[j] - 1 - turn / 2);
         const int split = local / L.tile_count[j];
         if (L.size[j] == 4)
             process_unit_item<4>(a, ntile, split, sm, stages, tmem, ps, err, exact);
