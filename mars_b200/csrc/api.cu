@@ -182,17 +182,18 @@ static_assert(sizeof(mars_candidate) == sizeof(mars::CandidateOut), "candidate l
 
 // Device waits are bounded: poll an event until it completes or the deadline passes.  The
 // work waited for is the context's stream's, or `stream`'s when one is given.
-int sync_bounded(mars_ctx* ctx, cudaStream_t stream = nullptr) {
+int sync_bounded(mars_ctx* ctx, cudaStream_t stream = nullptr, int* stream_err = nullptr) {
     static const double limit_s = [] {
         const char* e = std::getenv("MARS_SYNC_TIMEOUT_S");
         return e ? std::atof(e) : 300.0;
     }();
-    // On the context's stream (its callers hold ctx->mu) the kernel error word travels back
-    // with the work, ahead of the event; other streams read it after the wait.
-    const bool err_async = !stream && ctx->h_err;
+    // The kernel error word travels back with the work, ahead of the event, into the stream's
+    // pinned word (the context's own stream: its callers hold ctx->mu).
+    int* h_err = stream ? stream_err : ctx->h_err;
+    const bool err_async = h_err != nullptr;
     if (err_async)
-        MARS_CUDA(cudaMemcpyAsync(ctx->h_err, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost,
-                                  ctx->stream));
+        MARS_CUDA(cudaMemcpyAsync(h_err, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost,
+                                  stream ? stream : ctx->stream));
     cudaEvent_t ev;
     MARS_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
     MARS_CUDA(cudaEventRecord(ev, stream ? stream : ctx->stream));
@@ -220,7 +221,7 @@ int sync_bounded(mars_ctx* ctx, cudaStream_t stream = nullptr) {
     cudaEventDestroy(ev);
     int kerr = 0;
     if (err_async)
-        kerr = *reinterpret_cast<volatile int*>(ctx->h_err);
+        kerr = *reinterpret_cast<volatile int*>(h_err);
     else
         MARS_CUDA(cudaMemcpy(&kerr, ctx->d_err, sizeof kerr, cudaMemcpyDeviceToHost));
     if (kerr) {
@@ -809,6 +810,18 @@ bool all_levels_eligible(const mars_ctx* ctx, uint32_t w, uint32_t h, const std:
     return levels > 0 && levels + 1 <= mars::tc::kMaxLevelJobs;
 }
 
+// The context's branch streams and their events, on first use.  The caller holds ctx->mu.
+int make_branches(mars_ctx* ctx) {
+    if (!ctx->fork_ev) {
+        MARS_CUDA(cudaEventCreateWithFlags(&ctx->fork_ev, cudaEventDisableTiming));
+        for (int b = 0; b < mars_ctx::kBranches; ++b) {
+            MARS_CUDA(cudaStreamCreateWithFlags(&ctx->branch[b], cudaStreamNonBlocking));
+            MARS_CUDA(cudaEventCreateWithFlags(&ctx->join_ev[b], cudaEventDisableTiming));
+        }
+    }
+    return MARS_OK;
+}
+
 // run_jobs for the exhaustive single-candidate search with the correlation of every
 // tensor-core level in one persistent launch (launch_corr_all, which also writes the
 // levels' final candidates).  Every buffer is taken on the context's stream before the
@@ -820,13 +833,7 @@ int run_jobs_all_levels(mars_ctx* ctx, Scratch& sc, const uint8_t* d_plane, uint
                         mars::CandidateOut* d_out, const uint32_t* d_rc_in,
                         cudaEvent_t* timing = nullptr) {
     const cudaStream_t main = ctx->stream;
-    if (!ctx->fork_ev) {
-        MARS_CUDA(cudaEventCreateWithFlags(&ctx->fork_ev, cudaEventDisableTiming));
-        for (int b = 0; b < mars_ctx::kBranches; ++b) {
-            MARS_CUDA(cudaStreamCreateWithFlags(&ctx->branch[b], cudaStreamNonBlocking));
-            MARS_CUDA(cudaEventCreateWithFlags(&ctx->join_ev[b], cudaEventDisableTiming));
-        }
-    }
+    if (int e = make_branches(ctx)) return e;
     int32_t* d_D = nullptr;
     MARS_CUDA(sc.get(&d_D, std::max<size_t>(1, (size_t)(w / 2) * (h / 2))));
     MARS_CUDA(mars::launch_contract(d_plane, (int)w, (int)h, d_D, main));
@@ -1047,6 +1054,41 @@ int run_fisher_tc(mars_ctx* ctx, Scratch& sc, const uint8_t* d_plane, const int3
     return MARS_OK;
 }
 
+// One job of the classified search on the context's stream: its domain index, then its nodes'
+// searches.
+int run_fisher_level(mars_ctx* ctx, Scratch& sc, const uint8_t* d_plane, const int32_t* d_D,
+                     uint32_t w, uint32_t h, const mars::FitParams& fp, const Job& j,
+                     const uint32_t* d_rows, const uint32_t* d_cols, mars::CandidateOut* d_out,
+                     uint64_t* d_evals) {
+    const cudaStream_t st = ctx->stream;
+    const mars::LevelGeom g = level_geom(w, h, j.size, j.shift);
+    const int nrow = std::max(g.nrow_d, 0), ncol = std::max(g.ncol_d, 0);
+    const int n = (int)j.rows.size(), dw = (int)(w / 2);
+    const size_t npos = std::max<size_t>(1, (size_t)nrow * ncol);
+    mars::FisherIndex ix;
+    MARS_CUDA(sc.get(&ix.key, npos));
+    MARS_CUDA(sc.get(&ix.diso, npos));
+    MARS_CUDA(sc.get(&ix.list, npos));
+    MARS_CUDA(sc.get(&ix.counts, 72));
+    MARS_CUDA(sc.get(&ix.offsets, 72));
+    MARS_CUDA(sc.get(&ix.ref, 72));
+    MARS_CUDA(sc.get(&ix.work, mars::fisher_group_work_words(npos)));
+    MARS_CUDA(mars::launch_fisher_index(d_D, dw, (int)j.size, (int)j.shift, nrow, ncol, ix, st));
+    ctx->launches += nrow * ncol > 0 ? 4 : 2;
+    if (use_fisher_tc(ctx, j.size, j.shift) && nrow * ncol > 0 && n > 0)
+        return run_fisher_tc(ctx, sc, d_plane, d_D, w, h, g, fp, d_rows, d_cols, n, ix, d_out, d_evals);
+    const size_t parts = std::max<size_t>(1, (size_t)n * mars::fisher_warps_per_range((int)j.size));
+    mars::CandidateOut* part = nullptr;
+    uint32_t* part_e = nullptr;
+    MARS_CUDA(sc.get(&part, parts));
+    MARS_CUDA(sc.get(&part_e, parts));
+    MARS_CUDA(mars::launch_fisher_search(d_plane, (int)w, (int)h, d_D, dw, (int)j.size, (int)j.shift,
+                                         std::max(ncol, 1), d_rows, d_cols, n, ix, fp, d_out,
+                                         d_evals, part, part_e, st));
+    ctx->launches += 1 + (mars::fisher_warps_per_range((int)j.size) > 1);
+    return MARS_OK;
+}
+
 // Fisher's classified search for every job: per (size, shift) the domain index
 // (Fisher::index) and the searches of the job's nodes (Fisher::candidates +
 // search_block_fitted); per-node eval counts come back from the device.
@@ -1057,16 +1099,11 @@ int run_jobs_fisher(mars_ctx* ctx, Scratch& sc, const uint8_t* d_plane, uint32_t
                     const uint32_t* d_rc_in = nullptr) {
     const cudaStream_t st = ctx->stream;
     int32_t* d_D = nullptr;
-    const int dw = (int)(w / 2);
     MARS_CUDA(sc.get(&d_D, std::max<size_t>(1, (size_t)(w / 2) * (h / 2))));
     MARS_CUDA(mars::launch_contract(d_plane, (int)w, (int)h, d_D, st));
     ctx->launches += 1;
-    size_t total = 0, max_pos = 0;
-    for (const Job& j : jobs) {
-        total += j.rows.size();
-        const mars::LevelGeom g = level_geom(w, h, j.size, j.shift);
-        if (g.nrow_d > 0 && g.ncol_d > 0) max_pos = std::max(max_pos, (size_t)g.nrow_d * g.ncol_d);
-    }
+    size_t total = 0;
+    for (const Job& j : jobs) total += j.rows.size();
     const uint32_t* d_rc = d_rc_in;
     size_t off = 0;
     if (!d_rc) {
@@ -1082,42 +1119,35 @@ int run_jobs_fisher(mars_ctx* ctx, Scratch& sc, const uint8_t* d_plane, uint32_t
         MARS_CUDA(cudaMemcpyAsync(d, rc.data(), rc.size() * 4, cudaMemcpyHostToDevice, st));
         d_rc = d;
     }
-    mars::FisherIndex ix;
-    MARS_CUDA(sc.get(&ix.key, std::max<size_t>(1, max_pos)));
-    MARS_CUDA(sc.get(&ix.diso, std::max<size_t>(1, max_pos)));
-    MARS_CUDA(sc.get(&ix.list, std::max<size_t>(1, max_pos)));
-    MARS_CUDA(sc.get(&ix.counts, 72));
-    MARS_CUDA(sc.get(&ix.offsets, 72));
-    MARS_CUDA(sc.get(&ix.ref, 72));
-    MARS_CUDA(sc.get(&ix.work, mars::fisher_group_work_words(max_pos)));
-    size_t max_part = 1;
-    for (const Job& j : jobs)
-        max_part = std::max(max_part, j.rows.size() * (size_t)mars::fisher_warps_per_range((int)j.size));
-    mars::CandidateOut* part = nullptr;
-    uint32_t* part_e = nullptr;
-    MARS_CUDA(sc.get(&part, max_part));
-    MARS_CUDA(sc.get(&part_e, max_part));
+    // In a plan the levels are branches of its graph: each is a chain of some twenty kernels, most
+    // of them far from filling the device (an encode of 768 x 512, sizes 4..16: 2.1 ms on one stream, 1.95 so).  A one-shot
+    // table's launches reach the device one by one anyway and stay on one stream.
+    const bool fork = d_rc_in && jobs.size() > 1;
+    const int nb = fork ? (int)std::min<size_t>(jobs.size(), mars_ctx::kBranches) : 0;
+    if (fork) {
+        if (int e = make_branches(ctx)) return e;
+        MARS_CUDA(cudaEventRecord(ctx->fork_ev, st));
+        for (int b = 0; b < nb; ++b) MARS_CUDA(cudaStreamWaitEvent(ctx->branch[b], ctx->fork_ev, 0));
+    }
     off = 0;
-    for (const Job& j : jobs) {
-        const mars::LevelGeom g = level_geom(w, h, j.size, j.shift);
-        const int nrow = std::max(g.nrow_d, 0), ncol = std::max(g.ncol_d, 0);
-        const int n = (int)j.rows.size();
-        MARS_CUDA(mars::launch_fisher_index(d_D, dw, (int)j.size, (int)j.shift, nrow, ncol, ix, st));
-        ctx->launches += nrow * ncol > 0 ? 4 : 2;
-        if (use_fisher_tc(ctx, j.size, j.shift) && nrow * ncol > 0 && n > 0) {
-            if (int e = run_fisher_tc(ctx, sc, d_plane, d_D, w, h, g, fp, d_rc + off,
-                                      d_rc + total + off, n, ix, d_out + off, d_evals + off))
-                return e;
-        } else {
-            MARS_CUDA(mars::launch_fisher_search(d_plane, (int)w, (int)h, d_D, dw, (int)j.size,
-                                                 (int)j.shift, std::max(ncol, 1), d_rc + off,
-                                                 d_rc + total + off, n, ix, fp, d_out + off,
-                                                 d_evals + off, part, part_e, st));
-            ctx->launches += 1 + (mars::fisher_warps_per_range((int)j.size) > 1);
+    int err = MARS_OK;
+    for (size_t i = 0; i < jobs.size() && !err; ++i) {
+        const Job& j = jobs[i];
+        if (fork) ctx->stream = ctx->branch[i % mars_ctx::kBranches];
+        {
+            Scratch sb(ctx->stream);
+            err = run_fisher_level(ctx, sb, d_plane, d_D, w, h, fp, j, d_rc + off,
+                                   d_rc + total + off, d_out + off, d_evals + off);
         }
+        ctx->stream = st;
         off += j.rows.size();
     }
-    return MARS_OK;
+    // Join every branch that was forked, also after an error (a capture must end joined).
+    for (int b = 0; b < nb; ++b) {
+        MARS_CUDA(cudaEventRecord(ctx->join_ev[b], ctx->branch[b]));
+        MARS_CUDA(cudaStreamWaitEvent(st, ctx->join_ev[b], 0));
+    }
+    return err;
 }
 
 int run_jobs_branched(mars_ctx* ctx, Scratch& sc, const uint8_t* d_plane, uint32_t w, uint32_t h,
@@ -1253,7 +1283,7 @@ int mars_ctx_create(mars_ctx** out, int device) {
     if (e == cudaSuccess) e = cudaMalloc(&c->d_counter, sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaMalloc(&c->d_err, sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(c->d_err, 0, sizeof(int));
-    if (e == cudaSuccess) e = cudaMallocHost(&c->h_err, sizeof(int));
+    if (e == cudaSuccess) e = cudaMallocHost(&c->h_err, (1 + mars_ctx::kCallStreams) * sizeof(int));
     if (e == cudaSuccess) {
         void* fn = nullptr;
         cudaDriverEntryPointQueryResult q;
@@ -1276,6 +1306,7 @@ int mars_ctx_create(mars_ctx** out, int device) {
         return fail(MARS_ECUDA, std::string("context setup: ") + cudaGetErrorString(e));
     }
     c->stream = c->own_stream;
+    c->call_streams.reserve(mars_ctx::kCallStreams);
     *out = c;
     return MARS_OK;
 }
@@ -1288,6 +1319,10 @@ void mars_ctx_destroy(mars_ctx* ctx) {
     cudaStreamSynchronize(ctx->stream);
     if (ctx->d_counter) cudaFree(ctx->d_counter);
     if (ctx->d_err) cudaFree(ctx->d_err);
+    for (auto& cs : ctx->call_streams) {
+        cudaStreamSynchronize(cs.first);
+        cudaStreamDestroy(cs.first);
+    }
     if (ctx->h_err) cudaFreeHost(ctx->h_err);
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
     for (int b = 0; b < mars_ctx::kBranches; ++b) {
@@ -1506,18 +1541,44 @@ bool price_on_device_for(const mars_options& o) {
 }
 
 // A stream of its own for one call, so concurrent encodes on a context do not wait behind
-// each other's searches; destroyed (after its queued work) when the call returns.
-struct OwnStream {
+// each other's searches, and a pinned word for the wait.  It goes back to the context's idle ones
+// with whatever is still queued on it (the call's frees), which the next call's work follows.
+// Making and destroying a stream, and the first allocations on it, took 0.2 ms of a 0.4 ms encode.
+struct CallStream {
+    mars_ctx* ctx;
     cudaStream_t st = nullptr;
-    ~OwnStream() {
-        if (st) cudaStreamDestroy(st);
+    int* h_err = nullptr;  // null when every kept stream is in use: this one is not kept
+    explicit CallStream(mars_ctx* c) : ctx(c) {}
+    int open() {
+        {
+            std::lock_guard<std::mutex> lock(ctx->call_mu);
+            if (!ctx->call_streams.empty()) {
+                st = ctx->call_streams.back().first;
+                h_err = ctx->call_streams.back().second;
+                ctx->call_streams.pop_back();
+                return MARS_OK;
+            }
+        }
+        MARS_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+        std::lock_guard<std::mutex> lock(ctx->call_mu);
+        if (ctx->call_words < mars_ctx::kCallStreams) h_err = ctx->h_err + ++ctx->call_words;
+        return MARS_OK;
+    }
+    ~CallStream() {
+        if (!st) return;
+        if (!h_err) {
+            cudaStreamDestroy(st);
+            return;
+        }
+        std::lock_guard<std::mutex> lock(ctx->call_mu);
+        ctx->call_streams.emplace_back(st, h_err);
     }
 };
 
 int price_on_device(mars_ctx* ctx, mars::codec::PriceBatch& b) {
     MARS_CUDA(cudaSetDevice(ctx->device));
-    OwnStream own;
-    MARS_CUDA(cudaStreamCreateWithFlags(&own.st, cudaStreamNonBlocking));
+    CallStream own(ctx);
+    if (int e = own.open()) return e;
     const cudaStream_t st = own.st;
     Scratch sc(st);
     const size_t nodes = b.row.size();
@@ -1591,7 +1652,7 @@ int price_on_device(mars_ctx* ctx, mars::codec::PriceBatch& b) {
         b.levels.resize(b.nlevels);
         MARS_CUDA(cudaMemcpyAsync(b.levels.data(), d_lev, b.nlevels, cudaMemcpyDeviceToHost, st));
     }
-    return sync_bounded(ctx, st);
+    return sync_bounded(ctx, st, own.h_err);
 }
 
 // The walks of encode_image_with_search over filled tables (`table` for the final walk,
@@ -1858,13 +1919,7 @@ int run_jobs_branched(mars_ctx* ctx, Scratch& sc, const uint8_t* d_plane, uint32
                       const mars::FitParams& fp, const std::vector<Job>& jobs,
                       mars::CandidateOut* d_out, const uint32_t* d_rc, uint32_t k) {
     const cudaStream_t main = ctx->stream;
-    if (!ctx->fork_ev) {
-        MARS_CUDA(cudaEventCreateWithFlags(&ctx->fork_ev, cudaEventDisableTiming));
-        for (int b = 0; b < mars_ctx::kBranches; ++b) {
-            MARS_CUDA(cudaStreamCreateWithFlags(&ctx->branch[b], cudaStreamNonBlocking));
-            MARS_CUDA(cudaEventCreateWithFlags(&ctx->join_ev[b], cudaEventDisableTiming));
-        }
-    }
+    if (int e = make_branches(ctx)) return e;
     int32_t* d_D = nullptr;
     MARS_CUDA(sc.get(&d_D, std::max<size_t>(1, (size_t)(w / 2) * (h / 2))));
     MARS_CUDA(mars::launch_contract(d_plane, (int)w, (int)h, d_D, main));
@@ -2269,8 +2324,8 @@ int plan_encode_device(mars_search_plan* plan, mars_search_plan* warm_plan, cons
     const mars::WalkPlan& w = plan->walk;
     const size_t nodes = w.nodes;
     MARS_CUDA(cudaSetDevice(ctx->device));
-    OwnStream own;
-    MARS_CUDA(cudaStreamCreateWithFlags(&own.st, cudaStreamNonBlocking));
+    CallStream own(ctx);
+    if (int e = own.open()) return e;
     const cudaStream_t st = own.st;
     Scratch sc(st);
     unsigned char* d_cands;
@@ -2342,11 +2397,11 @@ int plan_encode_device(mars_search_plan* plan, mars_search_plan* warm_plan, cons
     ctx->launches += 2 * w.nlevels + 1;
     unsigned long long tot[2];
     MARS_CUDA(cudaMemcpyAsync(tot, ws.totals, sizeof tot, cudaMemcpyDeviceToHost, st));
-    if (int e = sync_bounded(ctx, st)) return e;
+    if (int e = sync_bounded(ctx, st, own.h_err)) return e;
     std::vector<mars_leaf> warm(tot[0]);
     MARS_CUDA(cudaMemcpyAsync(warm.data(), d_warm, warm.size() * sizeof(mars_leaf),
                               cudaMemcpyDeviceToHost, st));
-    if (int e = sync_bounded(ctx, st)) return e;
+    if (int e = sync_bounded(ctx, st, own.h_err)) return e;
     const uint64_t warm_evals = tot[1];
     *header = hdr;
     if (!prm.has_lambda) {
@@ -2412,7 +2467,7 @@ int plan_encode_device(mars_search_plan* plan, mars_search_plan* warm_plan, cons
                                    prm.min_size, ws, d_leaves, d_res, st));
     ctx->launches += 2 * w.nlevels + 1;
     MARS_CUDA(cudaMemcpyAsync(tot, ws.totals, sizeof tot, cudaMemcpyDeviceToHost, st));
-    if (int e = sync_bounded(ctx, st)) return e;
+    if (int e = sync_bounded(ctx, st, own.h_err)) return e;
     std::vector<mars_leaf> out(tot[0]);
     std::vector<int32_t> res(tot[1]);
     std::vector<uint64_t> evals(d_evals ? nodes : 0);
@@ -2424,7 +2479,7 @@ int plan_encode_device(mars_search_plan* plan, mars_search_plan* warm_plan, cons
     if (!res.empty())
         MARS_CUDA(cudaMemcpyAsync(res.data(), d_res, res.size() * sizeof(int32_t),
                                   cudaMemcpyDeviceToHost, st));
-    if (int e = sync_bounded(ctx, st)) return e;
+    if (int e = sync_bounded(ctx, st, own.h_err)) return e;
     counters->search_evals = plan->total_evals;
     if (d_evals) {
         counters->search_evals = 0;
