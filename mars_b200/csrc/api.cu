@@ -2685,6 +2685,10 @@ struct mars_decode_plan {
     uint32_t njobs = 0;
     bool wide_jobs = false;
     bool pooled = false;  // buffers of the stream-ordered pool
+    // The last run's iterations and output, and the steps as a graph once a run repeats them.
+    uint32_t run_iters = 0, graph_iters = 0;
+    uint8_t *run_out = nullptr, *graph_out = nullptr;
+    cudaGraphExec_t graph = nullptr;
 };
 
 namespace {
@@ -2774,6 +2778,7 @@ namespace {
 void release_decode_plan(mars_decode_plan* p) {
     cudaSetDevice(p->ctx->device);
     cudaStreamSynchronize(p->ctx->stream);
+    if (p->graph) cudaGraphExecDestroy(p->graph);
     for (void* q : {(void*)p->d_owner, (void*)p->d_maps, (void*)p->d_rvals, (void*)p->d_tmp,
                     (void*)p->d_jobs, (void*)p->d_inv, (void*)p->d_cellbuf})
         if (q) p->pooled ? cudaFreeAsync(q, p->ctx->stream) : cudaFree(q);
@@ -2866,29 +2871,81 @@ int mars_decode_plan_create(mars_ctx* ctx, const mars_header* hdr, const mars_le
     return create_decode_plan(ctx, hdr, leaves, n, residuals, nresiduals, false, out);
 }
 
+}  // extern "C"
+
+namespace {
+
+int enqueue_decode_steps(mars_decode_plan* p, uint32_t iterations, uint8_t* d_out, cudaStream_t st) {
+    // Ping-pong so that the last iteration lands in d_out.
+    uint8_t* a = (iterations & 1) ? p->d_tmp : d_out;
+    uint8_t* b = (iterations & 1) ? d_out : p->d_tmp;
+    MARS_CUDA(cudaMemsetAsync(a, 128, (size_t)p->w * p->h, st));
+    for (uint32_t it = 0; it < iterations; ++it) {
+        if (p->d_jobs)
+            MARS_CUDA(mars::launch_decode_sorted_step(a, b, (int)p->w, (int)p->h, p->lg, p->d_owner,
+                                                      p->d_maps, p->d_jobs, p->njobs, p->wide_jobs,
+                                                      p->d_inv, p->consts, p->d_cellbuf, st));
+        else
+            MARS_CUDA(mars::launch_decode_step(a, b, (int)p->w, (int)p->h, p->lg, p->d_owner,
+                                               p->d_maps, p->d_rvals, st));
+        std::swap(a, b);
+    }
+    return MARS_OK;
+}
+
+// The steps as a graph, made when a run repeats the last one's iterations and output: a launch a
+// step costs the host 3 us, which is what a small plane's run takes (ten steps of 512 x 512
+// on one B200: alone 46 us, 33 so; among others 32 and 23).  Captured on
+// a stream of its own; null when that fails, and the steps are launched.
+constexpr uint32_t kDecodeGraphSteps = 64;
+
+cudaGraphExec_t decode_graph(mars_decode_plan* p, uint32_t iterations, uint8_t* d_out) {
+    if (p->graph && p->graph_iters == iterations && p->graph_out == d_out) return p->graph;
+    const bool again = p->run_iters == iterations && p->run_out == d_out;
+    p->run_iters = iterations;
+    p->run_out = d_out;
+    if (!again || iterations < 2 || iterations > kDecodeGraphSteps) return nullptr;
+    CallStream own(p->ctx);
+    if (own.open() != MARS_OK) return nullptr;
+    cudaGraph_t g = nullptr;
+    cudaGraphExec_t x = nullptr;
+    if (cudaStreamBeginCapture(own.st, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
+        const int e = enqueue_decode_steps(p, iterations, d_out, own.st);
+        if (cudaStreamEndCapture(own.st, &g) != cudaSuccess || e ||
+            cudaGraphInstantiate(&x, g, 0) != cudaSuccess)
+            x = nullptr;
+        if (g) cudaGraphDestroy(g);
+    }
+    cudaGetLastError();
+    if (!x) return nullptr;
+    if (p->graph) cudaGraphExecDestroy(p->graph);
+    p->graph = x;
+    p->graph_iters = iterations;
+    p->graph_out = d_out;
+    return x;
+}
+
+}  // namespace
+
+extern "C" {
+
 int mars_decode_plan_run(mars_decode_plan* p, uint32_t iterations, uint8_t* d_out) {
     if (!p || !d_out) return fail(MARS_EINVAL, "NULL argument");
     mars_ctx* ctx = p->ctx;
     std::lock_guard<std::mutex> lock(ctx->mu);
     MARS_CUDA(cudaSetDevice(ctx->device));
-    // Ping-pong so that the last iteration lands in d_out.
-    uint8_t* a = (iterations & 1) ? p->d_tmp : d_out;
-    uint8_t* b = (iterations & 1) ? d_out : p->d_tmp;
-    MARS_CUDA(cudaMemsetAsync(a, 128, (size_t)p->w * p->h, ctx->stream));
-    for (uint32_t it = 0; it < iterations; ++it) {
-        if (p->d_jobs) {
-            MARS_CUDA(mars::launch_decode_sorted_step(a, b, (int)p->w, (int)p->h, p->lg, p->d_owner,
-                                                      p->d_maps, p->d_jobs, p->njobs, p->wide_jobs,
-                                                      p->d_inv, p->consts, p->d_cellbuf, ctx->stream));
-            ctx->launches += 2;
-        } else {
-            MARS_CUDA(mars::launch_decode_step(a, b, (int)p->w, (int)p->h, p->lg, p->d_owner,
-                                               p->d_maps, p->d_rvals, ctx->stream));
-            ctx->launches += 1;
-        }
-        std::swap(a, b);
+    ctx->launches += (uint64_t)iterations * (p->d_jobs ? 2 : 1);
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ctx->stream, &capturing) != cudaSuccess) {
+        cudaGetLastError();
+        capturing = cudaStreamCaptureStatusActive;  // launch the steps
     }
-    return MARS_OK;
+    if (capturing == cudaStreamCaptureStatusNone)
+        if (cudaGraphExec_t x = decode_graph(p, iterations, d_out)) {
+            MARS_CUDA(cudaGraphLaunch(x, ctx->stream));
+            return MARS_OK;
+        }
+    return enqueue_decode_steps(p, iterations, d_out, ctx->stream);
 }
 
 int mars_decode_plan_run_until_stable(mars_decode_plan* p, uint8_t threshold,

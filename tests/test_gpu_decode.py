@@ -311,3 +311,24 @@ def test_source_ordered_steps_with_overwritten_leaves(ctx, monkeypatch, w, h, bi
         ctx.decode(hdr, leaves[:0], 1)  # waits for the context's stream
         assert np.array_equal(out.cpu().numpy(), orc.decode(_ohdr(hdr), leaves, iters))
     plan.close()
+
+
+@pytest.mark.parametrize("w,h,min_size", [(64, 64, 4), (100, 77, 2), (516, 260, 4)])
+def test_repeated_plan_runs(ctx, w, h, min_size):
+    # A run that repeats the last one's steps and output replays them; others change either, or
+    # both, between replays.
+    torch = pytest.importorskip("torch")
+    leaves = synthetic.quadtree_leaves(w, h, w, min_size=min_size)
+    hdr = _hdr(w, h)
+    plan = ctx.decode_plan(hdr, leaves)
+    outs = [torch.zeros(h, w, dtype=torch.uint8, device="cuda:0") for _ in range(2)]
+    want = {n: orc.decode(_ohdr(hdr), leaves, n) for n in (1, 2, 3, 70)}
+    torch.cuda.synchronize()
+    for k, n in [(0, 3)] * 3 + [(1, 3), (0, 3), (1, 2), (1, 2), (1, 2), (0, 3), (0, 3), (0, 1),
+                                (0, 1), (1, 70), (1, 70), (1, 2)]:
+        outs[k].fill_(7)
+        torch.cuda.synchronize()
+        plan.run(n, outs[k].data_ptr())
+        torch.cuda.synchronize()
+        assert np.array_equal(outs[k].cpu().numpy(), want[n]), (k, n)
+    plan.close()
