@@ -113,7 +113,7 @@ __device__ __forceinline__ void convert4(uint32_t a, uint32_t b, uint32_t c, uin
 }
 
 // Three input planes -> three output planes; `inverse` picks the direction.  T: uint4 where all
-// six planes start on 16 bytes, uint32_t on 4, uint8_t otherwise: a thread takes kPerThread
+// six planes start on 16 bytes and are large, uint32_t where they start on 4, uint8_t otherwise: a thread takes kPerThread
 // pixels, the last ones byte by byte.
 template <bool inverse, class T>
 __global__ void __launch_bounds__(256)
@@ -185,6 +185,27 @@ __device__ __forceinline__ bool output_chunk(const uint8_t* dst, size_t n, uint3
     return true;
 }
 
+// Bytes taken one by one: all loaded before the first is stored, so that a chunk across a row's
+// end costs one round trip (as a loop of loads and stores these chunks, one a row at odd widths,
+// made a small frame slower than a byte a thread was).
+template <int K>
+__device__ __forceinline__ void store_chunk(uint8_t* dst, const Chunk& c, const uint32_t (&v)[K]) {
+    if (c.end - c.begin == K) {
+        uint32_t w[K / 4];
+#pragma unroll
+        for (int k = 0; k < K / 4; ++k)
+            w[k] = v[4 * k] | v[4 * k + 1] << 8 | v[4 * k + 2] << 16 | v[4 * k + 3] << 24;
+        if (K == 16)
+            *reinterpret_cast<uint4*>(dst + c.begin) = make_uint4(w[0], w[1], w[K / 4 - 2], w[K / 4 - 1]);
+        else
+            *reinterpret_cast<uint2*>(dst + c.begin) = make_uint2(w[0], w[1]);
+        return;
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+        if (c.begin + k < c.end) dst[c.begin + k] = (uint8_t)v[k];
+}
+
 // 9.2 us a 3840 x 2160 plane with a byte a thread.
 __global__ void __launch_bounds__(256)
     downsample_box_kernel(const uint8_t* __restrict__ src, int w, int h, uint8_t* __restrict__ dst,
@@ -210,17 +231,21 @@ __global__ void __launch_bounds__(256)
         *reinterpret_cast<uint2*>(dst + c.begin) = make_uint2(out[0], out[1]);
         return;
     }
-    for (size_t i = c.begin; i < c.end; ++i) {
+    uint32_t v[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        // Past the chunk's end the last byte again.
         const int x0 = 2 * (int)c.x, y0 = 2 * (int)c.y;
         const int x1 = min(x0 + 1, w - 1), y1 = min(y0 + 1, h - 1);
         const uint32_t sum = (uint32_t)src[(size_t)y0 * w + x0] + src[(size_t)y0 * w + x1] +
                              src[(size_t)y1 * w + x0] + src[(size_t)y1 * w + x1];
-        dst[i] = (uint8_t)((sum + 2) / 4);
-        if (++c.x == (uint32_t)ow) {
+        v[k] = (sum + 2) / 4;
+        if (c.begin + k + 1 < c.end && ++c.x == (uint32_t)ow) {
             c.x = 0;
             ++c.y;
         }
     }
+    store_chunk<8>(dst, c, v);
 }
 
 // 22.3 us for a 3840 x 2160 output with a byte a thread.
@@ -247,13 +272,16 @@ __global__ void __launch_bounds__(256)
         *reinterpret_cast<uint4*>(dst + c.begin) = make_uint4(o[0], o[1], o[2], o[3]);
         return;
     }
-    for (size_t i = c.begin; i < c.end; ++i) {
-        dst[i] = src[(size_t)min((int)(c.y / 2), sh - 1) * sw + min((int)(c.x / 2), sw - 1)];
-        if (++c.x == (uint32_t)w) {
+    uint32_t v[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+        v[k] = src[(size_t)min((int)(c.y / 2), sh - 1) * sw + min((int)(c.x / 2), sw - 1)];
+        if (c.begin + k + 1 < c.end && ++c.x == (uint32_t)w) {
             c.x = 0;
             ++c.y;
         }
     }
+    store_chunk<16>(dst, c, v);
 }
 
 // Sum of squared differences: per-thread partial sums over 16-byte chunks, a warp and block
@@ -317,7 +345,8 @@ cudaError_t launch_ycbcr(const uint8_t* r, const uint8_t* g, const uint8_t* b, s
         const size_t threads = (n + per_thread - 1) / per_thread;
         kernel<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(r, g, b, n, y, cb, cr);
     };
-    if (at % 16 == 0) inverse ? launch(convert_kernel<true, uint4>, 16) : launch(convert_kernel<false, uint4>, 16);
+    // Sixteen pixels a thread are a longer chain: worth it once they still fill the device.
+    if (at % 16 == 0 && n >= (1u << 21)) inverse ? launch(convert_kernel<true, uint4>, 16) : launch(convert_kernel<false, uint4>, 16);
     else if (at % 4 == 0) inverse ? launch(convert_kernel<true, uint32_t>, 4) : launch(convert_kernel<false, uint32_t>, 4);
     else inverse ? launch(convert_kernel<true, uint8_t>, 4) : launch(convert_kernel<false, uint8_t>, 4);
     return cudaGetLastError();
