@@ -1544,6 +1544,8 @@ bool price_on_device_for(const mars_options& o) {
 // each other's searches, and a pinned word for the wait.  It goes back to the context's idle ones
 // with whatever is still queued on it (the call's frees), which the next call's work follows.
 // Making and destroying a stream, and the first allocations on it, took 0.2 ms of a 0.4 ms encode.
+// (A context's very first encode is 0.15 ms slower while another context keeps such streams: 1.16
+// against 1.0 ms at 96 x 80.  Waiting for the frees before keeping a stream did not change that.)
 struct CallStream {
     mars_ctx* ctx;
     cudaStream_t st = nullptr;
