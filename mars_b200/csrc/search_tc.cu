@@ -50,6 +50,7 @@
 #include <memory>
 
 #include "kernels.cuh"
+#include "scan_state.cuh"
 #include "tc.cuh"
 #include "tc_ptx.cuh"
 

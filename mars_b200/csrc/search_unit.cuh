@@ -98,8 +98,7 @@ struct USmem {
     int last;  // this CTA finished the last split of its range tile
     ThrRec thr[kRangesPerTile];          // the full form's records (unit_publish)
     Champ ch[kRangesPerTile];
-    alignas(16) float uthr[kRangesPerTile];  // the scan's thresholds
-    uint32_t ufull[2];                   // ranges in the full form, a bit each, per half
+    float uscan[kRangesPerTile];         // the scan's state of each range (scan_state.cuh)
     int udone[2];                        // per half: scan warps through with the item
     uint32_t useq[kRangesPerTile];       // the champions' sequence locks
     uint32_t utail[kScanWarps];          // the rings' next slots to take, and
@@ -135,15 +134,21 @@ __device__ __forceinline__ unsigned long long unit_entry(int pos, int rl) {
     return 1ull << 63 | (unsigned long long)rl << 32 | (uint32_t)pos;
 }
 
+struct ScanWords {
+    float* at;
+    __device__ float load(int i) const { return *(volatile const float*)(at + i); }
+    __device__ void store(int i, float v) const { *(volatile float*)(at + i) = v; }
+};
+
 // The pruning records of range rl from its champion: the full form's (sqrt W, W / (2 a_min),
-// sqrt Nrr rounded up, tie domain) and the scan's threshold.  True: the range takes the full
-// form (its threshold is +inf).
-__device__ __forceinline__ bool unit_publish(USmem& sm, int rl, const FitParams& fp, int n) {
+// sqrt Nrr rounded up, tie domain), then the scan's state: its threshold, or the full form.
+__device__ __forceinline__ void unit_publish(USmem& sm, int rl, const FitParams& fp, int n) {
     const Champ& C = sm.ch[rl];
+    const ScanWords words{sm.uscan};
     if (!C.valid || C.nrr == 0) {
         sm.thr[rl] = ThrRec{INFINITY, INFINITY, 0.0f, -1};
-        sm.uthr[rl] = INFINITY;
-        return false;
+        scan_publish(words, rl, false, kScanNothing);
+        return;
     }
     const Threshold th = make_threshold(C.sum, C.rms, C.idx >> 3, C.rms0, C.nrr, n, fp);
     const float snrr = __fsqrt_ru(__ll2float_ru(C.nrr));
@@ -153,15 +158,8 @@ __device__ __forceinline__ bool unit_publish(USmem& sm, int rl, const FitParams&
     t.c = snrr;
     t.tie = th.mode == 2 ? -1 : (th.mode == 1 ? (int32_t)th.tie_dom : INT32_MAX);
     sm.thr[rl] = t;
-    if (th.wpos && th.mode == 2) {
-        const float u = __fdiv_rd(th.sqrt_w, snrr) * kUnitScale - kUnitSlack;
-        if (u >= kUnitLeast) {
-            sm.uthr[rl] = u;
-            return false;
-        }
-    }
-    sm.uthr[rl] = INFINITY;
-    return true;
+    const float u = __fdiv_rd(th.sqrt_w, snrr) * kUnitScale - kUnitSlack;
+    scan_publish(words, rl, !(th.wpos && th.mode == 2 && u >= kUnitLeast), u);
 }
 
 // fit.cuh's bound on Nrd for one (range record, domain), every step rounded toward -inf, with
@@ -207,10 +205,7 @@ __device__ bool unit_replace(USmem& sm, int rl, const FitParams& fp, int n, doub
             *(volatile uint32_t*)&C.idx = idx;
             *(volatile int32_t*)&C.t1x4 = t1;
             __threadfence_block();
-            if (!unit_publish(sm, rl, fp, n)) {
-                __threadfence_block();
-                atomicAnd(&sm.ufull[rl >> 4], ~(1u << (rl & 15)));
-            }
+            unit_publish(sm, rl, fp, n);
         }
         __threadfence_block();
         atomicExch(&sm.useq[rl], s + 2u);
@@ -652,14 +647,15 @@ __device__ __noinline__ void unit_load_role(const ItemArgs& a, USmem& sm, int nt
                     lo = fminf(lo, __shfl_sync(0xffffffffu, c.x, q));
                     hi = fmaxf(hi, __shfl_sync(0xffffffffu, c.y, q));
                 }
+                // The record may be of an earlier or a later champion than the state: any
+                // champion's bounds hold.
                 const float4 rr = lds_f4(&sm.thr[lane]);
-                const float u = *(volatile const float*)&sm.uthr[lane];
-                const bool full = *(volatile const uint32_t*)&sm.ufull[lane >> 4] >> (lane & 15) & 1u;
-                const uint32_t fulls = __ballot_sync(0xffffffffu, full);
+                const ScanState st = scan_read(ScanWords{sm.uscan}, lane);
+                const uint32_t fulls = __ballot_sync(0xffffffffu, st.full);
                 const float thr =
-                    full ? INFINITY
-                         : unit_tile_threshold(rr, u, inv, lo, hi, __fdividef(1.0f, lo),
-                                               __fdividef(1.0f, hi), a.fp);
+                    st.full ? INFINITY
+                            : unit_tile_threshold(rr, st.threshold, inv, lo, hi,
+                                                  __fdividef(1.0f, lo), __fdividef(1.0f, hi), a.fp);
                 if (!fulls && !__any_sync(0xffffffffu, thr <= kUnitScale * 1.002f)) continue;
                 const int set = sets++ % kSets;
                 sm.set[set][lane] = thr;
@@ -1025,10 +1021,9 @@ __device__ __forceinline__ void process_unit_item(const ItemArgs& a, int ntile, 
         sm.ukey[lane] = 0ull;
         sm.uinv[lane] = C.valid && C.nrr > 0 ? rsqrtf((float)C.nrr) : 0.0f;
         sm.useq[lane] = 0u;
-        const uint32_t full = __ballot_sync(0xffffffffu, unit_publish(sm, lane, a.fp, N));
+        unit_publish(sm, lane, a.fp, N);
         const uint32_t unseen = __ballot_sync(0xffffffffu, C.valid && C.nrr > 0 && fresh);
         if (lane < 2) {
-            sm.ufull[lane] = (full >> (16 * lane)) & 0xFFFFu;
             sm.udone[lane] = 0;
             sm.ukeyed[lane] = 0;
         }

@@ -92,3 +92,24 @@ def test_other_quantisers(both, size, alfa_bits, beta_bits, max_alfa):
     params = mb.make_params(shift=2, bits_alfa=alfa_bits, bits_beta=beta_bits, max_alfa=max_alfa)
     got, want = (c.search_grid(img, size, 2, params) for c in both)
     assert got[0].tobytes() == want[0].tobytes()
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("size,w,h,n", [
+    (4, 400, 300, 33),     # 227 tiles, the last group of three: 14 splits a range tile
+    (4, 400, 300, 2000),   # two splits
+    (8, 404, 300, 70),     # 218 tiles: the last group of two
+])
+def test_several_splits_a_range_tile(both, kind, size, w, h, n):
+    # Splits share champions as they find them, in whatever order they run: again and again.
+    img = _plane(kind, w, h)
+    params = mb.make_params(shift=2)
+    rows, cols = np.meshgrid(np.arange(h // size) * size, np.arange(w // size) * size,
+                             indexing="ij")
+    pick = np.random.default_rng(n).permutation(rows.size)[:n]
+    rows, cols = rows.ravel()[pick], cols.ravel()[pick]
+    want = both[1].search_blocks(img, size, 2, params, rows, cols)
+    for _ in range(5):
+        got = both[0].search_blocks(img, size, 2, params, rows, cols)
+        assert got[0].tobytes() == want[0].tobytes()
+        assert np.array_equal(got[1], want[1])
