@@ -671,8 +671,10 @@ cudaError_t launch_simt_t(const int32_t* D, const uint8_t* plane, int w, const u
     size_t smem = (size_t)strip_ld * strip_rows * 4 + 3 * (size_t)tr * tcn * 4;
     if (S > 8) smem += (size_t)S * S * RPB;
     auto kern = search_simt_kernel<S, RPB, KMAX>;
+    // The limit is the device's: the same for every stride, whatever another thread launches.
+    // (simt_tile stays within the budget.)
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+                                         (int)kSmemBudget);
     if (e != cudaSuccess) return e;
     dim3 grid((nranges + RPB - 1) / RPB, nsplit);
     kern<<<grid, RPB, smem, st>>>(D, g, plane, w, rows, cols, nranges, rs, ds, fp, partials,

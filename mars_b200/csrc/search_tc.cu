@@ -47,6 +47,7 @@
 #include <algorithm>
 #include <cstdint>
 #include <cstring>
+#include <iterator>
 #include <memory>
 
 #include "kernels.cuh"
@@ -1852,6 +1853,11 @@ bool all_levels_supported(int size, Path path) {
 }
 
 namespace {
+// The all-levels launch's shared memory by kind.
+constexpr size_t kAllLevelsSmem[5] = {smem_bytes<4, false>(), smem_bytes<8, false>(),
+                                      smem_bytes<16, true>(), smem_bytes<32, true>(),
+                                      smem_bytes<64, true>()};
+
 int all_levels_kind(int size) {
     if (size <= 8) return size == 4 ? 0 : 1;
     return size == 16 ? 2 : (size == 32 ? 3 : 4);
@@ -1953,7 +1959,9 @@ int ordered_jobs(const LevelJob* jobs, int njobs, bool unit, int* order) {
 }  // namespace
 
 // Two launches, the integer levels' on st_int and the unit levels' on st: each CTA fills an SM,
-// so the second launch's start on the SMs that the first one's leave.
+// so the second launch's start on the SMs that the first one's leave.  A kernel's limit of dynamic
+// shared memory is the device's, not the launch's: it is always set to what the largest level
+// takes, so that another thread's call between this one's two never lowers it.
 cudaError_t launch_corr_all(const LevelJob* jobs, int njobs, int* work, int* err,
                             unsigned long long* counter, int num_sms, cudaStream_t st,
                             cudaStream_t st_int) {
@@ -1977,14 +1985,12 @@ cudaError_t launch_corr_all(const LevelJob* jobs, int njobs, int* work, int* err
             L.tile_begin[k] = J.tile_begin;
             L.tile_count[k] = J.tile_count;
             L.item_begin[k + 1] = L.item_begin[k] + J.tile_count * J.msplit;
-            constexpr size_t sz[5] = {smem_bytes<4, false>(), smem_bytes<8, false>(),
-                                      smem_bytes<16, true>(), smem_bytes<32, true>(),
-                                      smem_bytes<64, true>()};
-            smem = std::max(smem, sz[L.kind[k]]);
+            smem = std::max(smem, kAllLevelsSmem[L.kind[k]]);
         }
         if (const int nitems = L.item_begin[n]) {
             cudaError_t e = cudaFuncSetAttribute(
-                corr_tc_all_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                corr_tc_all_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                (int)*std::max_element(std::begin(kAllLevelsSmem), std::end(kAllLevelsSmem)));
             if (e != cudaSuccess) return e;
             corr_tc_all_kernel<<<std::min(nitems, num_sms), kThreads, smem, st_int>>>(
                 L, work, err, counter);
@@ -2008,7 +2014,8 @@ cudaError_t launch_corr_all(const LevelJob* jobs, int njobs, int* work, int* err
         }
         if (const int nitems = L.item_begin[n]) {
             cudaError_t e = cudaFuncSetAttribute(
-                corr_unit_all_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                corr_unit_all_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                (int)std::max(unit_smem_bytes<4>(), unit_smem_bytes<8>()));
             if (e != cudaSuccess) return e;
             corr_unit_all_kernel<<<std::min(nitems, num_sms), kUnitThreads, smem, st>>>(
                 L, work + 1, err, counter);

@@ -1,0 +1,100 @@
+"""Contexts on several host threads at once: every call's records are those it gives alone."""
+import threading
+
+import pytest
+import torch
+
+import mars_b200 as mb
+from mars_b200 import synthetic
+
+pytestmark = pytest.mark.gpu
+
+
+def _side_by_side(calls, repeats):
+    """Runs each call `repeats` times on a thread of its own; the calls' results, by call."""
+    errors, start = [], threading.Barrier(len(calls))
+    results = [[] for _ in calls]
+
+    def work(call, out):
+        try:
+            start.wait(60)
+            for _ in range(repeats):
+                out.append(call())
+        except Exception as e:  # reported on the test's thread
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=a) for a in zip(calls, results)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join(120)
+    assert not errors, errors[0]
+    return results
+
+
+@pytest.mark.parametrize("path,first,second", [
+    ("auto", (4, 2), (8, 2)),      # the unit form's launch with and without size 8
+    ("simt", (16, 2), (16, 16)),   # the CUDA-core kernel's domain tiles, by stride
+])
+def test_contexts_of_different_levels(monkeypatch, path, first, second):
+    monkeypatch.setenv("MARS_UNIT_TILES", "0")
+    w = h = 192
+    plane = torch.from_numpy(synthetic.gray(w, h, 5)).cuda()
+    torch.cuda.synchronize()
+    ctxs = [mb.Context(0) for _ in range(4)]
+
+    def call(ctx, size, shift):
+        params = mb.make_params(min_size=size, max_size=size, shift=shift)
+        n = mb.C.c_size_t()
+        mb.check(mb.lib().mars_search_nodes_device(ctx.handle, plane.data_ptr(), w, h,
+                                                   mb.C.byref(params), None, 0, mb.C.byref(n),
+                                                   None))
+        out = torch.zeros(n.value, 80, dtype=torch.uint8, device="cuda")
+        torch.cuda.synchronize()
+
+        def run():
+            mb.check(mb.lib().mars_search_nodes_device(ctx.handle, plane.data_ptr(), w, h,
+                                                       mb.C.byref(params), out.data_ptr(), n.value,
+                                                       mb.C.byref(n), None))
+
+        def records():
+            torch.cuda.synchronize()
+            return out.cpu().numpy().tobytes()
+        return run, records
+
+    for ctx in ctxs:
+        ctx.set_search_path(path)
+    runs, records = zip(*[call(ctx, *level) for ctx, level in zip(ctxs, 2 * (first, second))])
+    for run in runs:
+        run()
+    alone = [r() for r in records]
+    # Calls that only launch: a collision on what they share is a matter of host time alone.
+    _side_by_side(runs, 3000)
+    assert [r() for r in records] == alone
+    for ctx in ctxs:
+        ctx.close()
+
+
+def test_two_contexts_tables_of_different_levels():
+    # The integer launch of a table's levels: size 16 alone beside 64.
+    img = synthetic.gray(192, 192, 5)
+    ctxs = [mb.Context(0) for _ in range(2)]
+
+    def call(ctx, size):
+        params = mb.make_params(min_size=size, max_size=size, shift=4)
+        grid = [i * size for i in range(192 // size)]
+        rows, cols = [r for r in grid for _ in grid], grid * len(grid)
+
+        def run():
+            table = ctx.search_provider(img, params)
+            records = table.search_many(rows, cols, size, 4)[0].tobytes()
+            table.close()
+            return records
+        return run
+
+    calls = [call(ctx, size) for ctx, size in zip(ctxs, (16, 64))]
+    alone = [c() for c in calls]
+    for want, got in zip(alone, _side_by_side(calls, 300)):
+        assert all(g == want for g in got)
+    for ctx in ctxs:
+        ctx.close()
