@@ -2170,7 +2170,7 @@ int mars_search_plan_kernel_ms(const mars_search_plan* p, float* ms) {
 void mars_search_plan_free(mars_search_plan* p) {
     if (!p) return;
     cudaSetDevice(p->ctx->device);
-    cudaStreamSynchronize(p->ctx->stream);
+    cudaStreamSynchronize(mars::ctx_stream(p->ctx));
     plan_release(p);
 }
 
@@ -2539,6 +2539,16 @@ void mars_bytes_free(uint8_t* bytes) { std::free(bytes); }
 
 namespace {
 
+// The host's part of a decode (prepare_decode): packed leaves, owner map and its cell, and the
+// residuals' offsets and values.
+struct DecodeLists {
+    std::vector<mars::DecodeLeaf> dl;
+    std::vector<int32_t> owner, roff;
+    std::vector<double> rvals;
+    int lg = 0;
+    mars::DecodeConsts consts;
+};
+
 // Leaf table and owner map of one leaf list, validated on the host so that every read and
 // write the gather kernel makes stays inside the plane.  Leaves are packed into 16 bytes
 // (the layout is documented beside DecodeLeaf), which bounds plane sides to 65535, leaf
@@ -2551,9 +2561,11 @@ namespace {
 // (upload_residuals; the basis is the C library's cosine, as the reference's is), or here for
 // lists with a mode-3 leaf wider than kResidualMost (resid_values is then not empty).
 int prepare_decode(const mars_header* hdr, const mars_leaf* leaves, size_t n,
-                   const int32_t* residuals, size_t nresiduals, std::vector<mars::DecodeLeaf>* dl,
-                   std::vector<int32_t>* owner, int* lg_out, mars::DecodeConsts* consts,
-                   std::vector<int32_t>* resid_off, std::vector<double>* resid_values) {
+                   const int32_t* residuals, size_t nresiduals, DecodeLists* lists) {
+    std::vector<mars::DecodeLeaf>* const dl = &lists->dl;
+    std::vector<int32_t>*const owner = &lists->owner, *const resid_off = &lists->roff;
+    std::vector<double>* const resid_values = &lists->rvals;
+    mars::DecodeConsts* const consts = &lists->consts;
     const uint32_t w = hdr->width, h = hdr->height;
     if (w == 0 || h == 0) return fail(MARS_EINVAL, "empty plane");
     if (w > 65535 || h > 65535) return fail(MARS_EINVAL, "plane sides must be at most 65535");
@@ -2625,7 +2637,7 @@ int prepare_decode(const mars_header* hdr, const mars_leaf* leaves, size_t n,
             std::fill_n(owner->begin() + (long)((size_t)((L.row >> lg) + i) * mw + (L.col >> lg)),
                         L.size >> lg, (int32_t)k);
     }
-    *lg_out = lg;
+    lists->lg = lg;
     return MARS_OK;
 }
 
@@ -2709,14 +2721,9 @@ extern "C" {
 int mars_decode(mars_ctx* ctx, const mars_header* hdr, const mars_leaf* leaves, size_t n,
                 const int32_t* residuals, size_t nresiduals, uint32_t iterations, uint8_t* out) {
     if (!ctx || !hdr || !out || (n && !leaves)) return fail(MARS_EINVAL, "NULL argument");
-    std::vector<mars::DecodeLeaf> dl;
-    std::vector<int32_t> owner, roff;
-    std::vector<double> rvals;
-    int lg = 0;
-    mars::DecodeConsts consts;
-    if (int e = prepare_decode(hdr, leaves, n, residuals, nresiduals, &dl, &owner, &lg, &consts,
-                               &roff, &rvals))
-        return e;
+    DecodeLists lists;
+    if (int e = prepare_decode(hdr, leaves, n, residuals, nresiduals, &lists)) return e;
+    const auto& [dl, owner, roff, rvals, lg, consts] = lists;
     const uint32_t w = hdr->width, h = hdr->height;
     std::lock_guard<std::mutex> lock(ctx->mu);
     MARS_CUDA(cudaSetDevice(ctx->device));
@@ -2777,35 +2784,34 @@ int mars_decode(mars_ctx* ctx, const mars_header* hdr, const mars_leaf* leaves, 
 
 namespace {
 
-void release_decode_plan(mars_decode_plan* p) {
+// After the work on st, the stream the plan was made or last run on.
+void release_decode_plan(mars_decode_plan* p, cudaStream_t st) {
     cudaSetDevice(p->ctx->device);
-    cudaStreamSynchronize(p->ctx->stream);
+    cudaStreamSynchronize(st);
     if (p->graph) cudaGraphExecDestroy(p->graph);
     for (void* q : {(void*)p->d_owner, (void*)p->d_maps, (void*)p->d_rvals, (void*)p->d_tmp,
                     (void*)p->d_jobs, (void*)p->d_inv, (void*)p->d_cellbuf})
-        if (q) p->pooled ? cudaFreeAsync(q, p->ctx->stream) : cudaFree(q);
+        if (q) p->pooled ? cudaFreeAsync(q, st) : cudaFree(q);
     delete p;
 }
 
-// pooled: the plan lives for one call on the context's stream, so its buffers come from the
-// stream-ordered pool (eight cudaMalloc and cudaFree took half of a one-shot decode); a plan that
-// a program keeps may run on other streams and has its own.
+struct ReleaseDecodePlan {
+    cudaStream_t st;
+    void operator()(mars_decode_plan* p) const { release_decode_plan(p, st); }
+};
+
+// The caller holds ctx->mu.  pooled: the plan lives for one call, which keeps the lock (the
+// context's stream may be another one without it), so its buffers come from that stream's pool
+// (eight cudaMalloc and cudaFree took half of a one-shot decode) and nothing is waited for; a plan
+// that a program keeps may run on other streams and has its own.
 int create_decode_plan(mars_ctx* ctx, const mars_header* hdr, const mars_leaf* leaves, size_t n,
-                       const int32_t* residuals, size_t nresiduals, bool pooled,
-                       mars_decode_plan** out) {
-    std::vector<mars::DecodeLeaf> dl;
-    std::vector<int32_t> owner, roff;
-    std::vector<double> rvals;
-    int lg = 0;
-    mars::DecodeConsts consts;
-    if (int e = prepare_decode(hdr, leaves, n, residuals, nresiduals, &dl, &owner, &lg, &consts,
-                               &roff, &rvals))
-        return e;
-    std::lock_guard<std::mutex> lock(ctx->mu);
+                       const int32_t* residuals, size_t nresiduals, const DecodeLists& lists,
+                       bool pooled, mars_decode_plan** out) {
+    const auto& [dl, owner, roff, rvals, lg, consts] = lists;
     MARS_CUDA(cudaSetDevice(ctx->device));
     const cudaStream_t st = ctx->stream;
-    std::unique_ptr<mars_decode_plan, void (*)(mars_decode_plan*)> p(
-        new (std::nothrow) mars_decode_plan, release_decode_plan);
+    std::unique_ptr<mars_decode_plan, ReleaseDecodePlan> p(new (std::nothrow) mars_decode_plan,
+                                                           ReleaseDecodePlan{st});
     if (!p) return fail(MARS_ENOMEM, "plan allocation failed");
     p->ctx = ctx;
     p->w = hdr->width;
@@ -2870,7 +2876,10 @@ int mars_decode_plan_create(mars_ctx* ctx, const mars_header* hdr, const mars_le
                             size_t n, const int32_t* residuals, size_t nresiduals,
                             mars_decode_plan** out) {
     if (!ctx || !hdr || !out || (n && !leaves)) return fail(MARS_EINVAL, "NULL argument");
-    return create_decode_plan(ctx, hdr, leaves, n, residuals, nresiduals, false, out);
+    DecodeLists lists;
+    if (int e = prepare_decode(hdr, leaves, n, residuals, nresiduals, &lists)) return e;
+    std::lock_guard<std::mutex> lock(ctx->mu);
+    return create_decode_plan(ctx, hdr, leaves, n, residuals, nresiduals, lists, false, out);
 }
 
 }  // extern "C"
@@ -2950,15 +2959,14 @@ int mars_decode_plan_run(mars_decode_plan* p, uint32_t iterations, uint8_t* d_ou
     return enqueue_decode_steps(p, iterations, d_out, ctx->stream);
 }
 
-int mars_decode_plan_run_until_stable(mars_decode_plan* p, uint8_t threshold,
-                                      uint32_t max_iterations, uint8_t* d_out,
-                                      uint32_t* iterations_used) {
-    if (!p || !d_out || !iterations_used) return fail(MARS_EINVAL, "NULL argument");
-    const uint32_t iters = std::max<uint32_t>(1, max_iterations);
-    if (iters > (1u << 20)) return fail(MARS_EINVAL, "max_iterations is above 2^20");
+}  // extern "C"
+
+namespace {
+
+// The caller holds p->ctx->mu.
+int run_until_stable(mars_decode_plan* p, uint8_t threshold, uint32_t iters, uint8_t* d_out,
+                     uint32_t* iterations_used) {
     mars_ctx* ctx = p->ctx;
-    std::lock_guard<std::mutex> lock(ctx->mu);
-    MARS_CUDA(cudaSetDevice(ctx->device));
     const size_t px = (size_t)p->w * p->h;
     Scratch sc(ctx->stream);
     // [0] done, [1] used, [2 + i] step i's max delta, then the one launch's two words
@@ -2996,32 +3004,44 @@ int mars_decode_plan_run_until_stable(mars_decode_plan* p, uint8_t threshold,
     return MARS_OK;
 }
 
+}  // namespace
+
+extern "C" {
+
+int mars_decode_plan_run_until_stable(mars_decode_plan* p, uint8_t threshold,
+                                      uint32_t max_iterations, uint8_t* d_out,
+                                      uint32_t* iterations_used) {
+    if (!p || !d_out || !iterations_used) return fail(MARS_EINVAL, "NULL argument");
+    const uint32_t iters = std::max<uint32_t>(1, max_iterations);
+    if (iters > (1u << 20)) return fail(MARS_EINVAL, "max_iterations is above 2^20");
+    std::lock_guard<std::mutex> lock(p->ctx->mu);
+    MARS_CUDA(cudaSetDevice(p->ctx->device));
+    return run_until_stable(p, threshold, iters, d_out, iterations_used);
+}
+
 int mars_decode_until_stable(mars_ctx* ctx, const mars_header* hdr, const mars_leaf* leaves,
                              size_t n, const int32_t* residuals, size_t nresiduals,
                              uint8_t threshold, uint32_t max_iterations, uint8_t* out,
                              uint32_t* iterations_used) {
     if (!ctx || !hdr || !out || !iterations_used) return fail(MARS_EINVAL, "NULL argument");
     if (n && !leaves) return fail(MARS_EINVAL, "NULL argument");
-    mars_decode_plan* plan = nullptr;
-    if (int e = create_decode_plan(ctx, hdr, leaves, n, residuals, nresiduals, true, &plan)) return e;
-    std::unique_ptr<mars_decode_plan, void (*)(mars_decode_plan*)> guard(plan,
-                                                                         mars_decode_plan_free);
-    uint8_t* d_out = nullptr;
-    cudaStream_t st = nullptr;
-    {
-        std::lock_guard<std::mutex> lock(ctx->mu);
-        MARS_CUDA(cudaSetDevice(ctx->device));
-        st = ctx->stream;
-        MARS_CUDA(cudaMallocAsync(&d_out, std::max<size_t>(1, (size_t)hdr->width * hdr->height), st));
-    }
-    auto give_back = [st](uint8_t* q) { cudaFreeAsync(q, st); };
-    std::unique_ptr<uint8_t, decltype(give_back)> dguard(d_out, give_back);
-    if (int e = mars_decode_plan_run_until_stable(plan, threshold, max_iterations, d_out,
-                                                  iterations_used))
-        return e;
+    DecodeLists lists;
+    if (int e = prepare_decode(hdr, leaves, n, residuals, nresiduals, &lists)) return e;
+    const uint32_t iters = std::max<uint32_t>(1, max_iterations);
+    if (iters > (1u << 20)) return fail(MARS_EINVAL, "max_iterations is above 2^20");
+    // One hold of the lock from the uploads to the plane: the context's stream stays the same.
     std::lock_guard<std::mutex> lock(ctx->mu);
-    MARS_CUDA(cudaMemcpyAsync(out, d_out, (size_t)hdr->width * hdr->height,
-                              cudaMemcpyDeviceToHost, ctx->stream));
+    mars_decode_plan* plan = nullptr;
+    if (int e = create_decode_plan(ctx, hdr, leaves, n, residuals, nresiduals, lists, true, &plan))
+        return e;
+    const cudaStream_t st = ctx->stream;
+    std::unique_ptr<mars_decode_plan, ReleaseDecodePlan> guard(plan, ReleaseDecodePlan{st});
+    const size_t px = (size_t)hdr->width * hdr->height;
+    Scratch sc(st);
+    uint8_t* d_out = nullptr;
+    MARS_CUDA(sc.get(&d_out, px));
+    if (int e = run_until_stable(plan, threshold, iters, d_out, iterations_used)) return e;
+    MARS_CUDA(cudaMemcpyAsync(out, d_out, px, cudaMemcpyDeviceToHost, st));
     return sync_bounded(ctx);
 }
 
@@ -3069,7 +3089,7 @@ int mars_zoom_leaves(const mars_header* hdr, const mars_leaf* leaves, size_t n, 
 }
 
 void mars_decode_plan_free(mars_decode_plan* p) {
-    if (p) release_decode_plan(p);
+    if (p) release_decode_plan(p, mars::ctx_stream(p->ctx));
 }
 
 int mars_ycbcr_device(mars_ctx* ctx, const uint8_t* d_r, const uint8_t* d_g, const uint8_t* d_b,
@@ -3168,6 +3188,10 @@ int mars_ifs_write(const mars_header* header, const mars_leaf* leaves, size_t n,
 
 namespace mars {
 int ctx_sync(mars_ctx* ctx) { return sync_bounded(ctx); }
+cudaStream_t ctx_stream(mars_ctx* ctx) {
+    std::lock_guard<std::mutex> lock(ctx->mu);
+    return ctx->stream;
+}
 }  // namespace mars
 
 extern "C" {

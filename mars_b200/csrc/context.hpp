@@ -54,6 +54,8 @@ int set_last_error(int code, const std::string& msg);
 // Waits for the context's stream with the library's deadline (MARS_SYNC_TIMEOUT_S) and
 // turns kernel-reported errors into a status.  The caller holds ctx->mu.
 int ctx_sync(mars_ctx* ctx);
+// The context's stream, read under its lock (a search may point it at a branch meanwhile).
+cudaStream_t ctx_stream(mars_ctx* ctx);
 // The bits_alfa / bits_beta / max_alfa checks every search entry point makes (MARS_EINVAL
 // with a message on failure).
 int check_fit_params(const mars_params& p);

@@ -1367,7 +1367,7 @@ int mars_refine_run(mars_refine_plan* p, uint32_t steps, float lr, uint32_t deco
 void mars_refine_plan_free(mars_refine_plan* p) {
     if (!p) return;
     cudaSetDevice(p->ctx->device);
-    cudaStreamSynchronize(p->ctx->stream);
+    cudaStreamSynchronize(mars::ctx_stream(p->ctx));
     free_plan(p);
 }
 

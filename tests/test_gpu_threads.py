@@ -1,6 +1,7 @@
 """Contexts on several host threads at once: every call's records are those it gives alone."""
 import threading
 
+import numpy as np
 import pytest
 import torch
 
@@ -98,3 +99,42 @@ def test_two_contexts_tables_of_different_levels():
         assert all(g == want for g in got)
     for ctx in ctxs:
         ctx.close()
+
+
+def test_one_shot_decodes_while_the_stream_changes():
+    w, h = 404, 300
+    leaves = synthetic.quadtree_leaves(w, h, 3, min_size=4)
+    hdr = mb.Header(bits_alfa=4, bits_beta=7, min_size=4, max_size=32, shift=2, width=w, height=h,
+                    int_max_alfa=32)
+    leaves["mode"][::3][leaves["mode"][::3] == 2] = 3
+    pick = leaves["mode"] == 3
+    levels = np.random.default_rng(1).integers(
+        -2, 3, int((leaves["size"][pick].astype(np.int64) ** 2).sum())).astype(np.int32)
+    ctx = mb.Context(0)
+    want = ctx.decode_until_stable(hdr, leaves, 1, 24, levels)
+    plan = ctx.decode_plan(hdr, leaves, levels)
+    other = torch.cuda.Stream()
+    done = threading.Event()
+
+    def switch():
+        while not done.is_set():
+            ctx.set_stream(other.cuda_stream)
+            ctx.set_stream(0)
+
+    def decode():
+        plane, used = ctx.decode_until_stable(hdr, leaves, 1, 24, levels)
+        made = ctx.decode_plan(hdr, leaves, levels)
+        made.close()  # released while the other thread changes the stream
+        return used, plane.tobytes()
+
+    turning = threading.Thread(target=switch)
+    turning.start()
+    try:
+        got = _side_by_side([decode, decode], 60)
+    finally:
+        done.set()
+        turning.join(60)
+    assert all(g == (want[1], want[0].tobytes()) for side in got for g in side)
+    torch.cuda.synchronize()
+    plan.close()
+    ctx.close()
