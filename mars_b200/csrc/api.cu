@@ -1319,10 +1319,7 @@ void mars_ctx_destroy(mars_ctx* ctx) {
     cudaStreamSynchronize(ctx->stream);
     if (ctx->d_counter) cudaFree(ctx->d_counter);
     if (ctx->d_err) cudaFree(ctx->d_err);
-    for (auto& cs : ctx->call_streams) {
-        cudaStreamSynchronize(cs.first);
-        cudaStreamDestroy(cs.first);
-    }
+    for (auto& cs : ctx->call_streams) cudaStreamDestroy(cs.first);  // frees may be queued there
     if (ctx->h_err) cudaFreeHost(ctx->h_err);
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
     for (int b = 0; b < mars_ctx::kBranches; ++b) {
@@ -1550,7 +1547,13 @@ struct CallStream {
     mars_ctx* ctx;
     cudaStream_t st = nullptr;
     int* h_err = nullptr;  // null when every kept stream is in use: this one is not kept
+    bool stuck = false;    // a wait failed: what is queued may stay, with the word's copy
     explicit CallStream(mars_ctx* c) : ctx(c) {}
+    int wait() {
+        const int e = sync_bounded(ctx, st, h_err);
+        stuck |= e != MARS_OK;
+        return e;
+    }
     int open() {
         {
             std::lock_guard<std::mutex> lock(ctx->call_mu);
@@ -1568,7 +1571,7 @@ struct CallStream {
     }
     ~CallStream() {
         if (!st) return;
-        if (!h_err) {
+        if (!h_err || stuck) {  // (a stuck stream's word is not given out again)
             cudaStreamDestroy(st);
             return;
         }
@@ -1654,7 +1657,7 @@ int price_on_device(mars_ctx* ctx, mars::codec::PriceBatch& b) {
         b.levels.resize(b.nlevels);
         MARS_CUDA(cudaMemcpyAsync(b.levels.data(), d_lev, b.nlevels, cudaMemcpyDeviceToHost, st));
     }
-    return sync_bounded(ctx, st, own.h_err);
+    return own.wait();
 }
 
 // The walks of encode_image_with_search over filled tables (`table` for the final walk,
@@ -2399,11 +2402,11 @@ int plan_encode_device(mars_search_plan* plan, mars_search_plan* warm_plan, cons
     ctx->launches += 2 * w.nlevels + 1;
     unsigned long long tot[2];
     MARS_CUDA(cudaMemcpyAsync(tot, ws.totals, sizeof tot, cudaMemcpyDeviceToHost, st));
-    if (int e = sync_bounded(ctx, st, own.h_err)) return e;
+    if (int e = own.wait()) return e;
     std::vector<mars_leaf> warm(tot[0]);
     MARS_CUDA(cudaMemcpyAsync(warm.data(), d_warm, warm.size() * sizeof(mars_leaf),
                               cudaMemcpyDeviceToHost, st));
-    if (int e = sync_bounded(ctx, st, own.h_err)) return e;
+    if (int e = own.wait()) return e;
     const uint64_t warm_evals = tot[1];
     *header = hdr;
     if (!prm.has_lambda) {
@@ -2469,7 +2472,7 @@ int plan_encode_device(mars_search_plan* plan, mars_search_plan* warm_plan, cons
                                    prm.min_size, ws, d_leaves, d_res, st));
     ctx->launches += 2 * w.nlevels + 1;
     MARS_CUDA(cudaMemcpyAsync(tot, ws.totals, sizeof tot, cudaMemcpyDeviceToHost, st));
-    if (int e = sync_bounded(ctx, st, own.h_err)) return e;
+    if (int e = own.wait()) return e;
     std::vector<mars_leaf> out(tot[0]);
     std::vector<int32_t> res(tot[1]);
     std::vector<uint64_t> evals(d_evals ? nodes : 0);
@@ -2481,7 +2484,7 @@ int plan_encode_device(mars_search_plan* plan, mars_search_plan* warm_plan, cons
     if (!res.empty())
         MARS_CUDA(cudaMemcpyAsync(res.data(), d_res, res.size() * sizeof(int32_t),
                                   cudaMemcpyDeviceToHost, st));
-    if (int e = sync_bounded(ctx, st, own.h_err)) return e;
+    if (int e = own.wait()) return e;
     counters->search_evals = plan->total_evals;
     if (d_evals) {
         counters->search_evals = 0;
