@@ -9,10 +9,12 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <map>
 #include <memory>
 #include <mutex>
 #include <string>
 #include <thread>
+#include <tuple>
 #include <unordered_map>
 #include <vector>
 
@@ -45,6 +47,71 @@ int fail(int code, const std::string& msg) {
 bool is_pow2(uint32_t x) { return x && !(x & (x - 1)); }
 
 }  // namespace
+
+// The streams that calls take for themselves (CallStream), kept between calls: at most kMost a
+// device, each with a pinned word, shared by the device's contexts and gone with the last of them.
+// Making and destroying a stream, and the first allocations on it, took 0.2 ms of a 0.4 ms encode.
+// Shared, because what the pool holds for a stream that stays alive slows the allocations on any
+// new one: with streams of their own, a context's first encode took 0.25 ms longer for each
+// context that lived beside it (96 x 80 on one B200: 0.97 ms alone, 2.46 ms beside six).
+struct CallStreams {
+    static constexpr size_t kMost = 8;
+    std::mutex mu;
+    int contexts = 0;
+    int* words = nullptr;
+    size_t given = 0;  // words given out
+    std::vector<std::pair<cudaStream_t, int*>> idle;
+
+    static cudaError_t join(int device, CallStreams** out) {
+        static std::mutex all_mu;
+        static auto* const all = new std::map<int, CallStreams>;  // not destroyed at exit
+        CallStreams* c;
+        {
+            std::lock_guard<std::mutex> lock(all_mu);
+            c = &(*all)[device];
+        }
+        std::lock_guard<std::mutex> lock(c->mu);
+        if (c->contexts == 0) {
+            c->idle.reserve(kMost);
+            if (cudaError_t e = cudaMallocHost(&c->words, kMost * sizeof(int))) return e;
+        }
+        ++c->contexts;
+        *out = c;
+        return cudaSuccess;
+    }
+    void leave() {
+        std::lock_guard<std::mutex> lock(mu);
+        if (--contexts > 0) return;
+        for (auto& i : idle) cudaStreamDestroy(i.first);  // frees may be queued there
+        idle.clear();
+        cudaFreeHost(words);
+        words = nullptr;
+        given = 0;
+    }
+    cudaError_t take(cudaStream_t* st, int** word) {
+        {
+            std::lock_guard<std::mutex> lock(mu);
+            if (!idle.empty()) {
+                std::tie(*st, *word) = idle.back();
+                idle.pop_back();
+                return cudaSuccess;
+            }
+        }
+        if (cudaError_t e = cudaStreamCreateWithFlags(st, cudaStreamNonBlocking)) return e;
+        std::lock_guard<std::mutex> lock(mu);
+        *word = given < kMost ? words + given++ : nullptr;
+        return cudaSuccess;
+    }
+    // keep: what was queued has been waited for.  (Otherwise the word is not given out again.)
+    void give(cudaStream_t st, int* word, bool keep) {
+        if (!word || !keep) {
+            cudaStreamDestroy(st);
+            return;
+        }
+        std::lock_guard<std::mutex> lock(mu);
+        idle.emplace_back(st, word);
+    }
+};
 
 namespace mars {
 // The message mars_last_error() reports, for entry points defined in other files.
@@ -1283,7 +1350,8 @@ int mars_ctx_create(mars_ctx** out, int device) {
     if (e == cudaSuccess) e = cudaMalloc(&c->d_counter, sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaMalloc(&c->d_err, sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(c->d_err, 0, sizeof(int));
-    if (e == cudaSuccess) e = cudaMallocHost(&c->h_err, (1 + mars_ctx::kCallStreams) * sizeof(int));
+    if (e == cudaSuccess) e = cudaMallocHost(&c->h_err, sizeof(int));
+    if (e == cudaSuccess) e = CallStreams::join(device, &c->calls);
     if (e == cudaSuccess) {
         void* fn = nullptr;
         cudaDriverEntryPointQueryResult q;
@@ -1302,11 +1370,11 @@ int mars_ctx_create(mars_ctx** out, int device) {
     if (e != cudaSuccess) {
         if (c->own_stream) cudaStreamDestroy(c->own_stream);
         if (c->h_err) cudaFreeHost(c->h_err);
+        if (c->calls) c->calls->leave();
         delete c;
         return fail(MARS_ECUDA, std::string("context setup: ") + cudaGetErrorString(e));
     }
     c->stream = c->own_stream;
-    c->call_streams.reserve(mars_ctx::kCallStreams);
     *out = c;
     return MARS_OK;
 }
@@ -1319,7 +1387,7 @@ void mars_ctx_destroy(mars_ctx* ctx) {
     cudaStreamSynchronize(ctx->stream);
     if (ctx->d_counter) cudaFree(ctx->d_counter);
     if (ctx->d_err) cudaFree(ctx->d_err);
-    for (auto& cs : ctx->call_streams) cudaStreamDestroy(cs.first);  // frees may be queued there
+    ctx->calls->leave();
     if (ctx->h_err) cudaFreeHost(ctx->h_err);
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
     for (int b = 0; b < mars_ctx::kBranches; ++b) {
@@ -1538,45 +1606,25 @@ bool price_on_device_for(const mars_options& o) {
 }
 
 // A stream of its own for one call, so concurrent encodes on a context do not wait behind
-// each other's searches, and a pinned word for the wait.  It goes back to the context's idle ones
-// with whatever is still queued on it (the call's frees), which the next call's work follows.
-// Making and destroying a stream, and the first allocations on it, took 0.2 ms of a 0.4 ms encode.
-// (A context's very first encode is 0.15 ms slower while another context keeps such streams: 1.16
-// against 1.0 ms at 96 x 80.  Waiting for the frees before keeping a stream did not change that.)
+// each other's searches, and a pinned word for the wait.  After its last wait it goes back to the
+// device's idle ones with only the call's frees queued on it, which the next call's work follows.
 struct CallStream {
     mars_ctx* ctx;
     cudaStream_t st = nullptr;
-    int* h_err = nullptr;  // null when every kept stream is in use: this one is not kept
-    bool stuck = false;    // a wait failed: what is queued may stay, with the word's copy
+    int* h_err = nullptr;   // null when every kept stream is in use: this one is not kept
+    bool waited = false;    // otherwise work may still be queued, with the word's copy
     explicit CallStream(mars_ctx* c) : ctx(c) {}
-    int wait() {
-        const int e = sync_bounded(ctx, st, h_err);
-        stuck |= e != MARS_OK;
-        return e;
-    }
     int open() {
-        {
-            std::lock_guard<std::mutex> lock(ctx->call_mu);
-            if (!ctx->call_streams.empty()) {
-                st = ctx->call_streams.back().first;
-                h_err = ctx->call_streams.back().second;
-                ctx->call_streams.pop_back();
-                return MARS_OK;
-            }
-        }
-        MARS_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-        std::lock_guard<std::mutex> lock(ctx->call_mu);
-        if (ctx->call_words < mars_ctx::kCallStreams) h_err = ctx->h_err + ++ctx->call_words;
+        MARS_CUDA(ctx->calls->take(&st, &h_err));
         return MARS_OK;
     }
+    int wait() {
+        const int e = sync_bounded(ctx, st, h_err);
+        waited = e == MARS_OK;
+        return e;
+    }
     ~CallStream() {
-        if (!st) return;
-        if (!h_err || stuck) {  // (a stuck stream's word is not given out again)
-            cudaStreamDestroy(st);
-            return;
-        }
-        std::lock_guard<std::mutex> lock(ctx->call_mu);
-        ctx->call_streams.emplace_back(st, h_err);
+        if (st) ctx->calls->give(st, h_err, waited);
     }
 };
 
@@ -2921,6 +2969,7 @@ cudaGraphExec_t decode_graph(mars_decode_plan* p, uint32_t iterations, uint8_t* 
     if (!again || iterations < 2 || iterations > kDecodeGraphSteps) return nullptr;
     CallStream own(p->ctx);
     if (own.open() != MARS_OK) return nullptr;
+    own.waited = true;  // captured, nothing queued
     cudaGraph_t g = nullptr;
     cudaGraphExec_t x = nullptr;
     if (cudaStreamBeginCapture(own.st, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {

@@ -15,6 +15,8 @@
 #include "../../include/mars_b200.h"
 #include "kernels.cuh"
 
+struct CallStreams;  // a device's idle call streams (api.cu)
+
 struct mars_ctx {
     int device = 0;
     int num_sms = 148;
@@ -24,7 +26,7 @@ struct mars_ctx {
     std::mutex mu;
     unsigned long long* d_counter = nullptr;  // survivors that took the exact f64 fit
     int* d_err = nullptr;                     // kernel-side error bits (bounded waits)
-    int* h_err = nullptr;                     // pinned copies of d_err, read by sync_bounded
+    int* h_err = nullptr;                     // pinned copy of d_err, read by sync_bounded
     int search_path = 0;                      // 0 auto, 1 CUDA cores only, 2 tensor cores
     bool tma_16_boxes = false;                // load A stages as 16 2-D boxes (A/B checks)
     bool fold_only = false;                   // no split-digit operand at sizes 16..64 (A/B)
@@ -36,12 +38,7 @@ struct mars_ctx {
     cudaStream_t branch[kBranches] = {};
     cudaEvent_t fork_ev = nullptr;
     cudaEvent_t join_ev[kBranches] = {};
-    // Streams for one call each (CallStream, api.cu), kept between calls: at most kCallStreams, each
-    // with one of the words after h_err.
-    static constexpr int kCallStreams = 8;
-    std::mutex call_mu;
-    std::vector<std::pair<cudaStream_t, int*>> call_streams;  // the idle ones
-    int call_words = 0;                                       // words given out
+    CallStreams* calls = nullptr;
     // Search plans mars_encode keeps for plane geometries it has met before (api.cu).
     std::mutex plan_cache_mu;
     std::vector<std::pair<std::string, mars_search_plan*>> plan_cache;

@@ -138,3 +138,23 @@ def test_one_shot_decodes_while_the_stream_changes():
     torch.cuda.synchronize()
     plan.close()
     ctx.close()
+
+
+def test_contexts_come_and_go_beside_each_other():
+    # Calls of every context take the device's call streams; the last context out gives them back.
+    params = mb.make_params(min_size=4, max_size=16, shift=4, lam=200.0)
+    images = [synthetic.gray(112, 80, seed) for seed in range(3)]
+
+    def encode(ctx, img):
+        _, leaves, levels, count = ctx.encode(img, params, allowed_modes=(1, 1, 1, 1))
+        return leaves.tobytes(), levels.tobytes(), count.search_evals
+
+    with mb.Context(0) as ctx:
+        want = [encode(ctx, img) for img in images]
+    for _ in range(3):
+        ctxs = [mb.Context(0) for _ in images]
+        got = _side_by_side([lambda c=c, i=i: encode(c, i) for c, i in zip(ctxs, images)], 8)
+        for w, g in zip(want, got):
+            assert all(x == w for x in g)
+        for ctx in ctxs:
+            ctx.close()
