@@ -1042,6 +1042,14 @@ bool use_fisher_tc(const mars_ctx* ctx, uint32_t size, uint32_t shift) {
     return mars::ftc::supported((int)size, (int)shift);
 }
 
+// Work on the context's stream, which may be a branch, after the allocations of a scratch on the
+// stream that it was forked from.
+cudaError_t after_scratch(mars_ctx* ctx, const Scratch& sc) {
+    if (sc.st == ctx->stream) return cudaSuccess;
+    const cudaError_t e = cudaEventRecord(ctx->fork_ev, sc.st);
+    return e == cudaSuccess ? cudaStreamWaitEvent(ctx->stream, ctx->fork_ev, 0) : e;
+}
+
 // One level of the classified search on tensor cores: statistics, each range's bucket,
 // the ranges grouped by bucket, then the batch (fisher_tc.cu).
 int run_fisher_tc(mars_ctx* ctx, Scratch& sc, const uint8_t* d_plane, const int32_t* d_D,
@@ -1061,9 +1069,6 @@ int run_fisher_tc(mars_ctx* ctx, Scratch& sc, const uint8_t* d_plane, const int3
     MARS_CUDA(sc.get(&ds.s2x16, npos));
     MARS_CUDA(sc.get(&ds.detf, npos));
     MARS_CUDA(sc.get(&ds.sdetf, npos));
-    MARS_CUDA(mars::launch_range_stats(d_plane, (int)w, (int)h, d_rows, d_cols, n, g.size, fp, rs,
-                                       st));
-    MARS_CUDA(mars::launch_domain_stats(d_D, g, ds, st));
     mars::ftc::FisherTcArgs a{};
     uint8_t *rbucket = nullptr, *riso = nullptr;
     uint32_t *rlist = nullptr, *plan = nullptr, *ref_scratch = nullptr;
@@ -1075,6 +1080,14 @@ int run_fisher_tc(mars_ctx* ctx, Scratch& sc, const uint8_t* d_plane, const int3
     MARS_CUDA(sc.get(&ref_scratch, 72));
     uint32_t* group_work = nullptr;
     MARS_CUDA(sc.get(&group_work, mars::fisher_group_work_words((size_t)n)));
+    MARS_CUDA(sc.get(&a.aglob, mars::ftc::a_bytes(g.size, npos)));
+    MARS_CUDA(sc.get(&a.bglob, mars::ftc::b_bytes(g.size, (size_t)n)));
+    MARS_CUDA(sc.get(&a.seeds, n));
+    MARS_CUDA(sc.get(&a.partials, mars::ftc::partials_max((size_t)n)));
+    MARS_CUDA(after_scratch(ctx, sc));
+    MARS_CUDA(mars::launch_range_stats(d_plane, (int)w, (int)h, d_rows, d_cols, n, g.size, fp, rs,
+                                       st));
+    MARS_CUDA(mars::launch_domain_stats(d_D, g, ds, st));
     a.plan.rcounts = plan;
     a.plan.roffsets = plan + 72;
     a.plan.p_base = plan + 144;
@@ -1090,10 +1103,6 @@ int run_fisher_tc(mars_ctx* ctx, Scratch& sc, const uint8_t* d_plane, const int3
     a.a_rows_max = mars::ftc::a_rows_max(npos);
     a.b_rows_max = mars::ftc::b_rows_max((size_t)n);
     a.items_max = mars::ftc::items_max((size_t)n);
-    MARS_CUDA(sc.get(&a.aglob, mars::ftc::a_bytes(g.size, npos)));
-    MARS_CUDA(sc.get(&a.bglob, mars::ftc::b_bytes(g.size, (size_t)n)));
-    MARS_CUDA(sc.get(&a.seeds, n));
-    MARS_CUDA(sc.get(&a.partials, mars::ftc::partials_max((size_t)n)));
     a.plane = d_plane;
     a.w = (int)w;
     a.h = (int)h;
@@ -1121,37 +1130,52 @@ int run_fisher_tc(mars_ctx* ctx, Scratch& sc, const uint8_t* d_plane, const int3
     return MARS_OK;
 }
 
+// The domain index and the partial results of the classified search's jobs: of one, or of the
+// largest of several that run one after the other.
+struct FisherBuffers {
+    mars::FisherIndex ix;
+    mars::CandidateOut* part = nullptr;
+    uint32_t* part_e = nullptr;
+};
+
+int fisher_buffers(Scratch& sc, uint32_t w, uint32_t h, const Job* jobs, size_t n, FisherBuffers* b) {
+    size_t npos = 1, parts = 1;
+    for (const Job* j = jobs; j != jobs + n; ++j) {
+        const mars::LevelGeom g = level_geom(w, h, j->size, j->shift);
+        if (g.nrow_d > 0 && g.ncol_d > 0) npos = std::max(npos, (size_t)g.nrow_d * g.ncol_d);
+        parts = std::max(parts, j->rows.size() * (size_t)mars::fisher_warps_per_range((int)j->size));
+    }
+    MARS_CUDA(sc.get(&b->ix.key, npos));
+    MARS_CUDA(sc.get(&b->ix.diso, npos));
+    MARS_CUDA(sc.get(&b->ix.list, npos));
+    MARS_CUDA(sc.get(&b->ix.counts, 72));
+    MARS_CUDA(sc.get(&b->ix.offsets, 72));
+    MARS_CUDA(sc.get(&b->ix.ref, 72));
+    MARS_CUDA(sc.get(&b->ix.work, mars::fisher_group_work_words(npos)));
+    MARS_CUDA(sc.get(&b->part, parts));
+    MARS_CUDA(sc.get(&b->part_e, parts));
+    return MARS_OK;
+}
+
 // One job of the classified search on the context's stream: its domain index, then its nodes'
-// searches.
+// searches.  sc: on this stream, or on the one that a branch was forked from.
 int run_fisher_level(mars_ctx* ctx, Scratch& sc, const uint8_t* d_plane, const int32_t* d_D,
                      uint32_t w, uint32_t h, const mars::FitParams& fp, const Job& j,
-                     const uint32_t* d_rows, const uint32_t* d_cols, mars::CandidateOut* d_out,
-                     uint64_t* d_evals) {
+                     const FisherBuffers& b, const uint32_t* d_rows, const uint32_t* d_cols,
+                     mars::CandidateOut* d_out, uint64_t* d_evals) {
     const cudaStream_t st = ctx->stream;
     const mars::LevelGeom g = level_geom(w, h, j.size, j.shift);
     const int nrow = std::max(g.nrow_d, 0), ncol = std::max(g.ncol_d, 0);
     const int n = (int)j.rows.size(), dw = (int)(w / 2);
-    const size_t npos = std::max<size_t>(1, (size_t)nrow * ncol);
-    mars::FisherIndex ix;
-    MARS_CUDA(sc.get(&ix.key, npos));
-    MARS_CUDA(sc.get(&ix.diso, npos));
-    MARS_CUDA(sc.get(&ix.list, npos));
-    MARS_CUDA(sc.get(&ix.counts, 72));
-    MARS_CUDA(sc.get(&ix.offsets, 72));
-    MARS_CUDA(sc.get(&ix.ref, 72));
-    MARS_CUDA(sc.get(&ix.work, mars::fisher_group_work_words(npos)));
+    const mars::FisherIndex& ix = b.ix;
+    MARS_CUDA(after_scratch(ctx, sc));
     MARS_CUDA(mars::launch_fisher_index(d_D, dw, (int)j.size, (int)j.shift, nrow, ncol, ix, st));
     ctx->launches += nrow * ncol > 0 ? 4 : 2;
     if (use_fisher_tc(ctx, j.size, j.shift) && nrow * ncol > 0 && n > 0)
         return run_fisher_tc(ctx, sc, d_plane, d_D, w, h, g, fp, d_rows, d_cols, n, ix, d_out, d_evals);
-    const size_t parts = std::max<size_t>(1, (size_t)n * mars::fisher_warps_per_range((int)j.size));
-    mars::CandidateOut* part = nullptr;
-    uint32_t* part_e = nullptr;
-    MARS_CUDA(sc.get(&part, parts));
-    MARS_CUDA(sc.get(&part_e, parts));
     MARS_CUDA(mars::launch_fisher_search(d_plane, (int)w, (int)h, d_D, dw, (int)j.size, (int)j.shift,
                                          std::max(ncol, 1), d_rows, d_cols, n, ix, fp, d_out,
-                                         d_evals, part, part_e, st));
+                                         d_evals, b.part, b.part_e, st));
     ctx->launches += 1 + (mars::fisher_warps_per_range((int)j.size) > 1);
     return MARS_OK;
 }
@@ -1187,8 +1211,9 @@ int run_jobs_fisher(mars_ctx* ctx, Scratch& sc, const uint8_t* d_plane, uint32_t
         d_rc = d;
     }
     // In a plan the levels are branches of its graph: each is a chain of some twenty kernels, most
-    // of them far from filling the device (an encode of 768 x 512, sizes 4..16: 2.1 ms on one stream, 1.95 so).  A one-shot
-    // table's launches reach the device one by one anyway and stay on one stream.
+    // of them far from filling the device (an encode of 768 x 512, sizes 4..16: 2.1 ms on one
+    // stream, 1.95 so).  A one-shot table's launches reach the device one by one anyway and stay on
+    // one stream, with one set of buffers.
     const bool fork = d_rc_in && jobs.size() > 1;
     const int nb = fork ? (int)std::min<size_t>(jobs.size(), mars_ctx::kBranches) : 0;
     if (fork) {
@@ -1197,15 +1222,18 @@ int run_jobs_fisher(mars_ctx* ctx, Scratch& sc, const uint8_t* d_plane, uint32_t
         for (int b = 0; b < nb; ++b) MARS_CUDA(cudaStreamWaitEvent(ctx->branch[b], ctx->fork_ev, 0));
     }
     off = 0;
-    int err = MARS_OK;
+    FisherBuffers buffers;
+    int err = fork ? MARS_OK : fisher_buffers(sc, w, h, jobs.data(), jobs.size(), &buffers);
     for (size_t i = 0; i < jobs.size() && !err; ++i) {
         const Job& j = jobs[i];
+        // Branches have buffers each, but of the main stream: what the pool holds for the branch
+        // streams, which stay, slows the first allocations on any new stream.  (Other contexts'
+        // first Fisher encodes, 96 x 80, each context used three times: 0.86 ms for the first,
+        // 3.2 ms for the seventh with buffers of the branches.)
+        if (fork && (err = fisher_buffers(sc, w, h, &j, 1, &buffers))) break;
         if (fork) ctx->stream = ctx->branch[i % mars_ctx::kBranches];
-        {
-            Scratch sb(ctx->stream);
-            err = run_fisher_level(ctx, sb, d_plane, d_D, w, h, fp, j, d_rc + off,
-                                   d_rc + total + off, d_out + off, d_evals + off);
-        }
+        err = run_fisher_level(ctx, sc, d_plane, d_D, w, h, fp, j, buffers, d_rc + off,
+                               d_rc + total + off, d_out + off, d_evals + off);
         ctx->stream = st;
         off += j.rows.size();
     }
