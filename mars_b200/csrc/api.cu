@@ -51,13 +51,17 @@ bool is_pow2(uint32_t x) { return x && !(x & (x - 1)); }
 // The streams that calls take for themselves (CallStream), kept between calls: at most kMost a
 // device, each with a pinned word, shared by the device's contexts and gone with the last of them.
 // Making and destroying a stream, and the first allocations on it, took 0.2 ms of a 0.4 ms encode.
-// Shared, because what the pool holds for a stream that stays alive slows the allocations on any
-// new one: with streams of their own, a context's first encode took 0.25 ms longer for each
-// context that lived beside it (96 x 80 on one B200: 0.97 ms alone, 2.46 ms beside six).
+// Shared, and with a pool of their own, because what a pool holds for a stream that stays alive
+// slows the allocations on any new stream, by 2.5 us each: with streams of its own a context's
+// first encode took 0.25 ms longer for each context that lived beside it (96 x 80 on one B200:
+// 0.97 ms alone, 2.46 ms beside six), and with the device's pool still 0.15 ms longer.
 struct CallStreams {
     static constexpr size_t kMost = 8;
+    static constexpr size_t kPoolKept = 32ull << 20;  // of the pool, without a context
     std::mutex mu;
     int contexts = 0;
+    cudaMemPool_t pool = nullptr;  // made with the first call stream; null: the device's
+    int device = 0;
     int* words = nullptr;
     size_t given = 0;  // words given out
     std::vector<std::pair<cudaStream_t, int*>> idle;
@@ -71,6 +75,7 @@ struct CallStreams {
             c = &(*all)[device];
         }
         std::lock_guard<std::mutex> lock(c->mu);
+        c->device = device;
         if (c->contexts == 0) {
             c->idle.reserve(kMost);
             if (cudaError_t e = cudaMallocHost(&c->words, kMost * sizeof(int))) return e;
@@ -84,6 +89,7 @@ struct CallStreams {
         if (--contexts > 0) return;
         for (auto& i : idle) cudaStreamDestroy(i.first);  // frees may be queued there
         idle.clear();
+        if (pool) cudaMemPoolTrimTo(pool, kPoolKept);
         cudaFreeHost(words);
         words = nullptr;
         given = 0;
@@ -99,8 +105,21 @@ struct CallStreams {
         }
         if (cudaError_t e = cudaStreamCreateWithFlags(st, cudaStreamNonBlocking)) return e;
         std::lock_guard<std::mutex> lock(mu);
+        if (!pool) make_pool();
         *word = given < kMost ? words + given++ : nullptr;
         return cudaSuccess;
+    }
+    void make_pool() {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location = {cudaMemLocationTypeDevice, device};
+        uint64_t keep = UINT64_MAX;
+        if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+            cudaGetLastError();
+            pool = nullptr;
+            return;
+        }
+        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
     }
     // keep: what was queued has been waited for.  (Otherwise the word is not given out again.)
     void give(cudaStream_t st, int* word, bool keep) {
@@ -322,12 +341,15 @@ using mars::make_fit_params;
 // to it at the end of the call (the pool keeps the memory cached between calls).
 struct Scratch {
     cudaStream_t st;
+    cudaMemPool_t pool;  // null: the device's
     std::vector<void*> ptrs;
-    explicit Scratch(cudaStream_t s) : st(s) {}
+    explicit Scratch(cudaStream_t s, cudaMemPool_t p = nullptr) : st(s), pool(p) {}
     template <class T>
     cudaError_t get(T** p, size_t count) {
         void* v = nullptr;
-        const cudaError_t e = cudaMallocAsync(&v, std::max<size_t>(count, 1) * sizeof(T), st);
+        const size_t bytes = std::max<size_t>(count, 1) * sizeof(T);
+        const cudaError_t e =
+            pool ? cudaMallocFromPoolAsync(&v, bytes, pool, st) : cudaMallocAsync(&v, bytes, st);
         if (e == cudaSuccess) ptrs.push_back(v);
         *p = (T*)v;
         return e;
@@ -1661,7 +1683,7 @@ int price_on_device(mars_ctx* ctx, mars::codec::PriceBatch& b) {
     CallStream own(ctx);
     if (int e = own.open()) return e;
     const cudaStream_t st = own.st;
-    Scratch sc(st);
+    Scratch sc(st, ctx->calls->pool);
     const size_t nodes = b.row.size();
     const bool residual = b.setup.allowed[3] != 0;
     size_t nbasis = 0;
@@ -2408,7 +2430,7 @@ int plan_encode_device(mars_search_plan* plan, mars_search_plan* warm_plan, cons
     CallStream own(ctx);
     if (int e = own.open()) return e;
     const cudaStream_t st = own.st;
-    Scratch sc(st);
+    Scratch sc(st, ctx->calls->pool);
     unsigned char* d_cands;
     uint8_t* d_px;
     unsigned char* d_wcands = nullptr;
