@@ -1821,7 +1821,8 @@ int plan_encode_device(mars_search_plan* plan, mars_search_plan* warm_plan, cons
                        const mars_options* o, mars_header* header, mars_leaf** leaves,
                        size_t* nleaves, int32_t** residuals, size_t* nresiduals,
                        mars_counters* counters);
-int fisher_walk_on_device(mars_search_plan* fplan, mars_search_plan* wplan, bool* usable);
+int fisher_walk_on_device(mars_search_plan* fplan, mars_search_plan* wplan, const mars_options* o,
+                          bool* usable);
 
 // The plan mars_encode uses for a plane geometry it has encoded before: one search plan
 // per (width, height, params), made on the second encode of that geometry (the first takes
@@ -1902,7 +1903,7 @@ int mars_encode(mars_ctx* ctx, const uint8_t* plane, uint32_t width, uint32_t he
             params->has_lambda ? cached_encode_plan(ctx, width, height, &wp) : nullptr;
         if (fplan && (!params->has_lambda || wplan)) {
             bool device_walk = false;
-            if (int e = fisher_walk_on_device(fplan, wplan, &device_walk)) return e;
+            if (int e = fisher_walk_on_device(fplan, wplan, options, &device_walk)) return e;
             if (device_walk)
                 return plan_encode_device(fplan, wplan, plane, options, header, leaves, nleaves,
                                           residuals, nresiduals, counters);
@@ -2383,10 +2384,18 @@ bool plan_walk_on_host() {
 }
 
 // Whether a Fisher encode's walks run on the device: both plans' trees can be walked there, over
-// the same nodes in the same order.
-int fisher_walk_on_device(mars_search_plan* fplan, mars_search_plan* wplan, bool* usable) {
+// the same nodes in the same order, and it pays.  Without residuals the walks are short, and the
+// host's over a downloaded table costs less than the device's launches and waits up to
+// kHostWalkNodes (device and host, threshold walk and RD, sizes 4..16 at stride 4 on one B200:
+// 630 nodes 304 and 271 us, 654 and 576; 1,575 nodes 340 and 333, 872 and 830; 4,032 nodes 394 and
+// 433, 1,159 and 1,282).  With residuals every node is priced there anyway (630 nodes: 702 and 824).
+constexpr size_t kHostWalkNodes = 2048;
+
+int fisher_walk_on_device(mars_search_plan* fplan, mars_search_plan* wplan, const mars_options* o,
+                          bool* usable) {
     *usable = false;
-    if (plan_walk_on_host()) return MARS_OK;
+    const bool residual = fplan->params.has_lambda && o->allowed_modes[3];
+    if (plan_walk_on_host() || (!residual && fplan->total < kHostWalkNodes)) return MARS_OK;
     bool f = false, w = true;
     if (int e = plan_walk_setup(fplan, &f)) return e;
     if (wplan) {

@@ -139,3 +139,26 @@ def test_device_walks_match_host_walks(case):
         assert res.returncode == 0, res.stderr.decode()[-2000:]
         out[where] = res.stdout
     assert out["device"] == out["host"]
+
+
+@pytest.mark.parametrize("w,h", [(160, 144), (176, 144)])  # 1,890 and 2,079 nodes
+@pytest.mark.parametrize("lam,modes", [(None, (1, 0, 1, 0)), (200.0, (1, 0, 1, 0)),
+                                       (200.0, (1, 1, 1, 1))])
+def test_repeated_fisher_encodes_walk_where_it_pays(w, h, lam, modes):
+    # A context's first encode of a geometry walks on the host; the later ones there or on the
+    # device, by the plan's nodes and the modes.
+    params = mb.make_params(min_size=4, max_size=16, shift=2, lam=lam)
+    imgs = [synthetic.gray(w, h, 40 + i) for i in range(3)]
+
+    def encode(c, img):
+        hd, leaves, levels, count = c.encode(img, params, allowed_modes=modes, method="fisher")
+        return (bytes(hd), leaves.tobytes(), levels.tobytes(), count.search_evals,
+                count.warmup_evals)
+
+    with mb.Context(0) as c:
+        encode(c, imgs[0])
+        encode(c, imgs[0])
+        again = [encode(c, img) for img in imgs]
+    for img, got in zip(imgs, again):
+        with mb.Context(0) as fresh:
+            assert got == encode(fresh, img)
