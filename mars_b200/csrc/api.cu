@@ -3001,8 +3001,11 @@ int enqueue_decode_steps(mars_decode_plan* p, uint32_t iterations, uint8_t* d_ou
     uint8_t* a = (iterations & 1) ? p->d_tmp : d_out;
     uint8_t* b = (iterations & 1) ? d_out : p->d_tmp;
     MARS_CUDA(cudaMemsetAsync(a, 128, (size_t)p->w * p->h, st));
+    // The source-ordered steps store words; into an output that starts between two, the plain
+    // steps go byte by byte.
+    const bool sorted = p->d_jobs && mars::decode_sorted_aligned(d_out);
     for (uint32_t it = 0; it < iterations; ++it) {
-        if (p->d_jobs)
+        if (sorted)
             MARS_CUDA(mars::launch_decode_sorted_step(a, b, (int)p->w, (int)p->h, p->lg, p->d_owner,
                                                       p->d_maps, p->d_jobs, p->njobs, p->wide_jobs,
                                                       p->d_inv, p->consts, p->d_cellbuf, st));

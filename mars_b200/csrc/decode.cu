@@ -922,11 +922,16 @@ cudaError_t launch_decode_sorted_build(int w, int h, int lg, const int32_t* owne
     return cudaGetLastError();
 }
 
+bool decode_sorted_aligned(const uint8_t* dst) {
+    return (reinterpret_cast<uintptr_t>(dst) & 3) == 0;
+}
+
 cudaError_t launch_decode_sorted_step(const uint8_t* src, uint8_t* dst, int w, int h, int lg,
                                       const int32_t* owner, const DecodeMap* maps,
                                       const uint4* jobs, uint32_t njobs, bool wide_jobs,
                                       const uint32_t* inv, DecodeConsts c, uint4* cellbuf,
                                       cudaStream_t st) {
+    if (!decode_sorted_aligned(dst)) return cudaErrorInvalidValue;
     const int mw = (w + (1 << lg) - 1) >> lg;
     if (njobs) {
         const auto gather = wide_jobs ? sorted_gather_kernel<true> : sorted_gather_kernel<false>;

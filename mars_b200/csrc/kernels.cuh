@@ -237,6 +237,7 @@ cudaError_t launch_decode_sorted_build(int w, int h, int lg, const int32_t* owne
                                        const DecodeMap* maps, const DecodeLeaf* leaves, int nleaves,
                                        uint32_t* row_count, uint32_t* cursor, uint4* jobs,
                                        uint32_t* inv, cudaStream_t st);
+bool decode_sorted_aligned(const uint8_t* dst);  // as a step's output has to be
 cudaError_t launch_decode_sorted_step(const uint8_t* src, uint8_t* dst, int w, int h, int lg,
                                       const int32_t* owner, const DecodeMap* maps,
                                       const uint4* jobs, uint32_t njobs, bool wide_jobs,

@@ -332,3 +332,22 @@ def test_repeated_plan_runs(ctx, w, h, min_size):
         torch.cuda.synchronize()
         assert np.array_equal(outs[k].cpu().numpy(), want[n]), (k, n)
     plan.close()
+
+
+@pytest.mark.parametrize("at", [0, 1, 4, 6])
+def test_source_ordered_runs_into_any_address(ctx, monkeypatch, at):
+    torch = pytest.importorskip("torch")
+    monkeypatch.setenv("MARS_DECODE_SORTED", "1")
+    w, h = 516, 260
+    leaves = synthetic.quadtree_leaves(w, h, 8, min_size=4)
+    hdr = _hdr(w, h)
+    plan = ctx.decode_plan(hdr, leaves)
+    whole = torch.full((w * h + 16,), 7, dtype=torch.uint8, device="cuda:0")
+    torch.cuda.synchronize()
+    for n in (1, 2, 7):
+        plan.run(n, whole.data_ptr() + at)
+        torch.cuda.synchronize()
+        got = whole.cpu().numpy()
+        assert np.array_equal(got[at: at + w * h].reshape(h, w), orc.decode(_ohdr(hdr), leaves, n))
+        assert (got[:at] == 7).all() and (got[at + w * h:] == 7).all()
+    plan.close()
