@@ -2809,10 +2809,19 @@ struct mars_decode_plan {
     uint32_t njobs = 0;
     bool wide_jobs = false;
     bool pooled = false;  // buffers of the stream-ordered pool
-    // The last run's iterations and output, and the steps as a graph once a run repeats them.
-    uint32_t run_iters = 0, graph_iters = 0;
-    uint8_t *run_out = nullptr, *graph_out = nullptr;
-    cudaGraphExec_t graph = nullptr;
+    // The steps of a run as a graph (decode_graph), for the first few step counts that the plan
+    // meets.  They run over d_tmp and d_tmp2; the last one alone knows the run's output.
+    uint8_t* d_tmp2 = nullptr;
+    struct StepGraph {
+        uint32_t steps = 0;  // 0: free
+        bool tried = false;
+        cudaGraphExec_t exec = nullptr;
+        cudaGraphNode_t last = nullptr;
+        uint8_t* out = nullptr;
+        cudaGraph_t graph = nullptr;
+    };
+    static constexpr int kStepGraphs = 4;
+    StepGraph graphs[kStepGraphs];
 };
 
 namespace {
@@ -2898,9 +2907,12 @@ namespace {
 void release_decode_plan(mars_decode_plan* p, cudaStream_t st) {
     cudaSetDevice(p->ctx->device);
     cudaStreamSynchronize(st);
-    if (p->graph) cudaGraphExecDestroy(p->graph);
+    for (auto& g : p->graphs) {
+        if (g.exec) cudaGraphExecDestroy(g.exec);
+        if (g.graph) cudaGraphDestroy(g.graph);
+    }
     for (void* q : {(void*)p->d_owner, (void*)p->d_maps, (void*)p->d_rvals, (void*)p->d_tmp,
-                    (void*)p->d_jobs, (void*)p->d_inv, (void*)p->d_cellbuf})
+                    (void*)p->d_tmp2, (void*)p->d_jobs, (void*)p->d_inv, (void*)p->d_cellbuf})
         if (q) p->pooled ? cudaFreeAsync(q, st) : cudaFree(q);
     delete p;
 }
@@ -2939,6 +2951,7 @@ int create_decode_plan(mars_ctx* ctx, const mars_header* hdr, const mars_leaf* l
     MARS_CUDA(get(&p->d_owner, owner.size()));
     MARS_CUDA(get(&p->d_maps, n));
     MARS_CUDA(get(&p->d_tmp, (size_t)p->w * p->h));
+    if (!pooled) MARS_CUDA(get(&p->d_tmp2, (size_t)p->w * p->h));  // (pooled plans run once)
     MARS_CUDA(cudaMemcpyAsync(p->d_owner, owner.data(), owner.size() * 4, cudaMemcpyHostToDevice, st));
     if (n) {
         mars::DecodeLeaf* d_leaves = nullptr;
@@ -2996,15 +3009,14 @@ int mars_decode_plan_create(mars_ctx* ctx, const mars_header* hdr, const mars_le
 
 namespace {
 
-int enqueue_decode_steps(mars_decode_plan* p, uint32_t iterations, uint8_t* d_out, cudaStream_t st) {
-    // Ping-pong so that the last iteration lands in d_out.
-    uint8_t* a = (iterations & 1) ? p->d_tmp : d_out;
-    uint8_t* b = (iterations & 1) ? d_out : p->d_tmp;
-    MARS_CUDA(cudaMemsetAsync(a, 128, (size_t)p->w * p->h, st));
+// `steps` steps, a and b in turn, the first from a and the last into d_out.
+int enqueue_decode_steps(mars_decode_plan* p, uint32_t steps, uint8_t* a, uint8_t* b,
+                         uint8_t* d_out, cudaStream_t st) {
     // The source-ordered steps store words; into an output that starts between two, the plain
     // steps go byte by byte.
     const bool sorted = p->d_jobs && mars::decode_sorted_aligned(d_out);
-    for (uint32_t it = 0; it < iterations; ++it) {
+    for (; steps > 0; --steps) {
+        if (steps == 1) b = d_out;
         if (sorted)
             MARS_CUDA(mars::launch_decode_sorted_step(a, b, (int)p->w, (int)p->h, p->lg, p->d_owner,
                                                       p->d_maps, p->d_jobs, p->njobs, p->wide_jobs,
@@ -3017,37 +3029,61 @@ int enqueue_decode_steps(mars_decode_plan* p, uint32_t iterations, uint8_t* d_ou
     return MARS_OK;
 }
 
-// The steps as a graph, made when a run repeats the last one's iterations and output: a launch a
-// step costs the host 3 us, which is what a small plane's run takes (ten steps of 512 x 512
-// on one B200: alone 46 us, 33 so; among others 32 and 23).  Captured on
-// a stream of its own; null when that fails, and the steps are launched.
-constexpr uint32_t kDecodeGraphSteps = 64;
+// A run's steps as a graph: a launch a step costs the host 3 us, which is what a small plane's
+// step takes, and kernels of a graph follow each other 1 us closer.  The graph knows a step count
+// and the plan's own planes; the output is a parameter of its last kernel, set when it is another
+// than the last run's.  A count's second run makes it (a plan that runs once does not pay for
+// that), the plan's first kStepGraphs counts have one, others are launched step by step: no order
+// of runs makes a graph twice.  512 x 512 on one B200, us a run, run after run: ten steps into one
+// output or two by turns 35 and 35, ten and twelve steps by turns 38; launched step by step 59.
+// Null where there is none.
+constexpr uint32_t kGraphSteps = 64;  // at most
 
-cudaGraphExec_t decode_graph(mars_decode_plan* p, uint32_t iterations, uint8_t* d_out) {
-    if (p->graph && p->graph_iters == iterations && p->graph_out == d_out) return p->graph;
-    const bool again = p->run_iters == iterations && p->run_out == d_out;
-    p->run_iters = iterations;
-    p->run_out = d_out;
-    if (!again || iterations < 2 || iterations > kDecodeGraphSteps) return nullptr;
-    CallStream own(p->ctx);
-    if (own.open() != MARS_OK) return nullptr;
-    own.waited = true;  // captured, nothing queued
-    cudaGraph_t g = nullptr;
-    cudaGraphExec_t x = nullptr;
-    if (cudaStreamBeginCapture(own.st, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
-        const int e = enqueue_decode_steps(p, iterations, d_out, own.st);
-        if (cudaStreamEndCapture(own.st, &g) != cudaSuccess || e ||
-            cudaGraphInstantiate(&x, g, 0) != cudaSuccess)
-            x = nullptr;
-        if (g) cudaGraphDestroy(g);
+cudaGraphExec_t decode_graph(mars_decode_plan* p, uint32_t steps, uint8_t* d_out) {
+    if (steps < 2 || steps > kGraphSteps || !mars::decode_output_aligned(d_out)) return nullptr;
+    mars_decode_plan::StepGraph* g = nullptr;
+    for (auto& have : p->graphs) {
+        g = &have;
+        if (have.steps == steps || have.steps == 0) break;
+        g = nullptr;
     }
-    cudaGetLastError();
-    if (!x) return nullptr;
-    if (p->graph) cudaGraphExecDestroy(p->graph);
-    p->graph = x;
-    p->graph_iters = iterations;
-    p->graph_out = d_out;
-    return x;
+    if (!g) return nullptr;
+    if (g->steps == 0) {
+        g->steps = steps;
+        return nullptr;
+    }
+    if (!g->tried) {
+        g->tried = true;
+        CallStream own(p->ctx);
+        if (own.open() != MARS_OK) return nullptr;
+        own.waited = true;  // captured, nothing queued
+        if (cudaStreamBeginCapture(own.st, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        bool ok = cudaMemsetAsync(p->d_tmp, 128, (size_t)p->w * p->h, own.st) == cudaSuccess &&
+                  enqueue_decode_steps(p, steps, p->d_tmp, p->d_tmp2, d_out, own.st) == MARS_OK;
+        cudaStreamCaptureStatus status;
+        const cudaGraphNode_t* last = nullptr;
+        size_t nlast = 0;
+        ok = ok && cudaStreamGetCaptureInfo_v2(own.st, &status, nullptr, nullptr, &last, &nlast) ==
+                       cudaSuccess && nlast == 1;
+        if (ok) g->last = *last;
+        ok = cudaStreamEndCapture(own.st, &g->graph) == cudaSuccess && ok &&
+             cudaGraphInstantiate(&g->exec, g->graph, 0) == cudaSuccess;
+        cudaGetLastError();
+        if (!ok) g->exec = nullptr;
+        g->out = d_out;
+    }
+    if (g->exec && g->out != d_out) {
+        // (What is queued of earlier runs keeps its output.)
+        if (mars::decode_set_output(g->exec, g->last, p->d_jobs != nullptr, d_out) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        g->out = d_out;
+    }
+    return g->exec;
 }
 
 }  // namespace
@@ -3059,18 +3095,24 @@ int mars_decode_plan_run(mars_decode_plan* p, uint32_t iterations, uint8_t* d_ou
     mars_ctx* ctx = p->ctx;
     std::lock_guard<std::mutex> lock(ctx->mu);
     MARS_CUDA(cudaSetDevice(ctx->device));
-    ctx->launches += (uint64_t)iterations * (p->d_jobs ? 2 : 1);
+    ctx->launches +=
+        (uint64_t)iterations * (p->d_jobs && mars::decode_sorted_aligned(d_out) ? 2 : 1);
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(ctx->stream, &capturing) != cudaSuccess) {
         cudaGetLastError();
         capturing = cudaStreamCaptureStatusActive;  // launch the steps
     }
+    const size_t px = (size_t)p->w * p->h;
     if (capturing == cudaStreamCaptureStatusNone)
         if (cudaGraphExec_t x = decode_graph(p, iterations, d_out)) {
             MARS_CUDA(cudaGraphLaunch(x, ctx->stream));
             return MARS_OK;
         }
-    return enqueue_decode_steps(p, iterations, d_out, ctx->stream);
+    // Ping-pong so that the last iteration lands in d_out.
+    uint8_t* a = (iterations & 1) ? p->d_tmp : d_out;
+    uint8_t* b = (iterations & 1) ? d_out : p->d_tmp;
+    MARS_CUDA(cudaMemsetAsync(a, 128, px, ctx->stream));
+    return enqueue_decode_steps(p, iterations, a, b, d_out, ctx->stream);
 }
 
 }  // extern "C"

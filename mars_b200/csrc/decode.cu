@@ -843,6 +843,22 @@ cudaError_t launch_decode_step(const uint8_t* src, uint8_t* dst, int w, int h, i
     return cudaGetLastError();
 }
 
+bool decode_output_aligned(const uint8_t* out) { return (reinterpret_cast<uintptr_t>(out) & 7) == 0; }
+
+cudaError_t decode_set_output(cudaGraphExec_t exec, cudaGraphNode_t last, bool sorted, uint8_t* out) {
+    cudaKernelNodeParams k;
+    cudaError_t e = cudaGraphKernelNodeGetParams(last, &k);
+    if (e != cudaSuccess) return e;
+    // sorted_place_kernel's nine parameters begin with the output; the step kernels' ten have it
+    // second.
+    void* params[10];
+    const int n = sorted ? 9 : 10;
+    for (int i = 0; i < n; ++i) params[i] = k.kernelParams[i];
+    params[sorted ? 0 : 1] = &out;
+    k.kernelParams = params;
+    return cudaGraphExecKernelNodeSetParams(exec, last, &k);
+}
+
 cudaError_t launch_decode_resident(uint8_t* buf0, uint8_t* buf1, int w, int h, int lg,
                                    const int32_t* owner, const DecodeMap* maps,
                                    const double* resid, uint32_t iters, uint32_t* sync, int* delta,

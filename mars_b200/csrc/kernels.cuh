@@ -212,6 +212,11 @@ cudaError_t launch_decode_step(const uint8_t* src, uint8_t* dst, int w, int h, i
                                const int32_t* owner, const DecodeMap* maps, const double* resid,
                                cudaStream_t st);
 
+// Another output (decode_output_aligned) for the last node of a captured run of
+// launch_decode_step, or of launch_decode_sorted_step, with an aligned one.
+bool decode_output_aligned(const uint8_t* out);
+cudaError_t decode_set_output(cudaGraphExec_t exec, cudaGraphNode_t last, bool sorted, uint8_t* out);
+
 // The steps of a decode as one cooperative launch whose threads each keep one 4x4 cell
 // (decode_resident_kernel): *taken says whether the plane was small enough; nothing is launched
 // otherwise.  The first step reads 128 everywhere, whatever buf0 holds.  sync: two words, zero

@@ -350,4 +350,33 @@ def test_source_ordered_runs_into_any_address(ctx, monkeypatch, at):
         got = whole.cpu().numpy()
         assert np.array_equal(got[at: at + w * h].reshape(h, w), orc.decode(_ohdr(hdr), leaves, n))
         assert (got[:at] == 7).all() and (got[at + w * h:] == 7).all()
+
+
+@pytest.mark.parametrize("w,h,min_size,wide", [(64, 64, 4, None), (100, 77, 2, None),
+                                               (516, 260, 4, None), (516, 260, 4, "1")])
+def test_plan_runs_of_every_count(ctx, monkeypatch, w, h, min_size, wide):
+    # More step counts than a plan keeps graphs for, into three buffers by turns, one of them at an
+    # odd address; wide: the source-ordered steps.
+    torch = pytest.importorskip("torch")
+    if wide:
+        monkeypatch.setenv("MARS_DECODE_SORTED", wide)
+    leaves = synthetic.quadtree_leaves(w, h, w + 1, min_size=min_size)
+    hdr = _hdr(w, h)
+    plan = ctx.decode_plan(hdr, leaves)
+    apart = (w * h + 256) // 256 * 256
+    whole = torch.zeros(3 * apart, dtype=torch.uint8, device="cuda:0")
+    starts = (0, apart, 2 * apart - 1)
+    torch.cuda.synchronize()
+    for n in (3, 2, 10, 1, 65, 7, 4, 10, 2):
+        want = orc.decode(_ohdr(hdr), leaves, n)
+        for k in (0, 0, 1, 2, 1, 0):
+            whole.fill_(7)
+            torch.cuda.synchronize()
+            plan.run(n, whole.data_ptr() + starts[k])
+            torch.cuda.synchronize()
+            got = whole.cpu().numpy()
+            out = got[starts[k]: starts[k] + w * h].copy()
+            assert np.array_equal(out.reshape(h, w), want), (n, k)
+            got[starts[k]: starts[k] + w * h] = 7
+            assert (got == 7).all()  # nothing beside the output
     plan.close()
