@@ -364,6 +364,7 @@ cudaError_t launch_fisher_search(const uint8_t* plane, int w, int h, const int32
                                  const FitParams& fp, CandidateOut* out, uint64_t* evals,
                                  CandidateOut* part, uint32_t* part_e, cudaStream_t st) {
     if (nranges <= 0) return cudaSuccess;
+    if (size < 1 || (size & (size - 1))) return cudaErrorInvalidValue;  // fit_exact
     const int wpr = fisher_warps_per_range(size);
     const size_t smem = (size_t)(kFisherWarps / wpr) * 8 * size * size;
     if (smem > 48 * 1024) {

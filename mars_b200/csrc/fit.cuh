@@ -61,9 +61,11 @@ __device__ __forceinline__ uint32_t quantise_exact(double x, uint32_t max) {
 }
 
 // fit_f64 with the reference's operation order (encode.rs:247-289).  The divisions by powers of
-// two -- s0 (a block's pixel count, a power of four), 2^bits_alfa and, where it is one,
-// max_alfa -- are multiplications by the exact reciprocal, the same doubles: three of the
-// seven dependent f64 divisions, some 300 cycles each, that make a fit's latency.
+// two -- s0 (twice), 2^bits_alfa and, where it is one, max_alfa -- are multiplications by the exact
+// reciprocal, the same doubles: three of the seven dependent f64 divisions, some 300 cycles each,
+// that make a fit's latency, and a fourth for such a max_alfa.  s0i, a block's pixel count, must
+// be a power of two: every search's sizes are (launch_range_stats and launch_fisher_search refuse
+// others).
 __device__ __forceinline__ FitResult fit_exact(int64_t s0i, int64_t s1_x4, int64_t s2_x16,
                                                int64_t t0i, int64_t t1_x4, int64_t t2i,
                                                const FitParams& fp) {

@@ -732,6 +732,7 @@ cudaError_t launch_range_stats(const uint8_t* plane, int w, int h, const uint32_
                                const uint32_t* cols, int nranges, int size, const FitParams& fp,
                                RangeStats rs, cudaStream_t st) {
     if (nranges == 0) return cudaSuccess;
+    if (size < 1 || (size & (size - 1))) return cudaErrorInvalidValue;  // fit_exact
     if (size >= 16)
         range_stats_warp_kernel<<<(unsigned)(((size_t)nranges * 32 + 255) / 256), 256, 0, st>>>(
             plane, w, h, rows, cols, nranges, size, fp, rs);
