@@ -390,13 +390,58 @@ __global__ void __launch_bounds__(RPB) search_simt_kernel(
 // The search of a level of 2 x 2 blocks (min_size 2, or the border blocks that forced splits
 // reach): a CTA per (range, split), a thread per domain.  A fit is four multiply-adds here and
 // the exact fits of what the bound lets through are all the work, so a thread per range, as
-// search_simt_kernel has it, is a serial chain of f64 divisions in too few warps: three
-// candidates a range of a 250 x 190 plane's 220 took 1,530 us (one B200).  The best one of each
-// of 220 ranges there takes 224 us, before 1,644; of 220 of a 1000 x 750 plane 2.3 and 2.8 ms, of
-// 16,384 57 and 121 ms; no count from 16 to 16,384 was slower, so size 2 has this kernel only.  Every
-// thread keeps the K best of its domains in registers and prunes against its own K-th; the CTA
-// then takes K times the best of the threads' heads.
+// search_simt_kernel has it, is a serial chain of f64 divisions in too few warps.  Every thread
+// keeps the K best of its domains in registers; the CTA takes K times the best of the threads'
+// heads.  What a thread prunes against is the better of its own K-th and the K-th of its warp's
+// heads, from the first domain on: each thread makes one fit there, its best correlation's, and
+// the CTA's bound of those comes before the others.  A flat range's candidates all fit alike, so
+// the first ones win without a search.  One B200, every block of a 250 x 190 plane at stride 8, us:
+// noise 299 (a thread per range 1,867; with bounds of their own and a counter addition a thread
+// 2,036), areas of one value 91 (504; 2,050); three candidates a range at stride 2 4,503 (11,889;
+// 6,342).  220 blocks of that plane at stride 2 take 113 us (1,644).  No plane from 32 x 32 to
+// 1000 x 750, stride 2 to 16, of noise, ramps, flat areas or the synthetic fields was slower than
+// with a thread per range, for all its blocks, a 4th or a 16th, so size 2 has this kernel only.
 constexpr int kSmallThreads = 256;
+
+struct SmallEntry {
+    double rms, sum;
+    uint32_t idx, q;  // qalfa | qbeta << 16
+    int32_t t1;
+};
+
+__device__ __forceinline__ bool small_less(double r0, uint32_t i0, double r1, uint32_t i1) {
+    return r0 < r1 || (r0 == r1 && i0 < i1);
+}
+
+// The warp's smallest (rms, idx), where its lanes' `mine` is (rms >= 0: its bits order as
+// integers); idx UINT32_MAX: none.
+__device__ __forceinline__ uint32_t warp_first(double rms, uint32_t idx) {
+    const unsigned long long bits = (unsigned long long)__double_as_longlong(rms);
+    const uint32_t hi = __reduce_min_sync(0xffffffffu, (uint32_t)(bits >> 32));
+    const uint32_t lo = __reduce_min_sync(
+        0xffffffffu, (uint32_t)(bits >> 32) == hi ? (uint32_t)bits : UINT32_MAX);
+    return __reduce_min_sync(
+        0xffffffffu, bits == ((unsigned long long)hi << 32 | lo) ? idx : UINT32_MAX);
+}
+
+// The K-th smallest (rms, idx) of the warp's heads as (rms, sum, idx); idx UINT32_MAX: fewer.
+template <int K>
+__device__ __forceinline__ void warp_kth(const SmallEntry& head, double& rms, double& sum,
+                                         uint32_t& idx) {
+    double r = head.rms;
+    uint32_t at = UINT32_MAX;
+#pragma unroll 1
+    for (int j = 0; j < K; ++j) {
+        at = warp_first(r, r == head.rms ? head.idx : UINT32_MAX);
+        if (at == UINT32_MAX) break;
+        if (j + 1 < K && head.idx == at) r = __longlong_as_double(0x7ff0000000000000ll);
+    }
+    const uint32_t who = __ballot_sync(0xffffffffu, at != UINT32_MAX && head.idx == at);
+    const int lane = who ? __ffs(who) - 1 : 0;
+    rms = __shfl_sync(0xffffffffu, head.rms, lane);
+    sum = __shfl_sync(0xffffffffu, head.sum, lane);
+    idx = at;
+}
 
 template <int K>
 __global__ void __launch_bounds__(kSmallThreads) search_small_kernel(
@@ -407,32 +452,55 @@ __global__ void __launch_bounds__(kSmallThreads) search_small_kernel(
     constexpr int S = 2, N = 4;
     __shared__ unsigned long long best_rms[2][kSmallThreads / 32];
     __shared__ uint32_t best_idx[2][kSmallThreads / 32];
+    __shared__ double bound_rms[kSmallThreads / 32], bound_sum[kSmallThreads / 32];
+    __shared__ uint32_t bound_idx[kSmallThreads / 32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int r = blockIdx.x;
     const uint32_t row = rows[r], col = cols[r];
     const bool inside = row + (uint32_t)S <= (uint32_t)g.h && col + (uint32_t)S <= (uint32_t)g.w;
     const double inf = __longlong_as_double(0x7ff0000000000000ll);
-    struct Entry {
-        double rms, sum;
-        uint32_t idx, q;  // qalfa | qbeta << 16
-        int32_t t1;
-    };
-    Entry e[K];
+    Partial* out = partials + ((size_t)blockIdx.y * nranges + r) * K;
+    SmallEntry e[K];
 #pragma unroll
-    for (int j = 0; j < K; ++j) e[j] = Entry{inf, inf, UINT32_MAX, 0u, 0};
+    for (int j = 0; j < K; ++j) e[j] = SmallEntry{inf, inf, UINT32_MAX, 0u, 0};
     uint32_t exact = 0;
     if (inside) {
+        const int32_t t0 = rs.t0[r], t2 = rs.t2[r];
+        const int64_t nrr = rs.nrr[r];
+        if (nrr == 0) {
+            if (tid < K) {
+                Partial p{inf, inf, UINT32_MAX, 0, 0, 0, 0};
+                if (blockIdx.y == 0) {
+                    const int32_t s1 = ds.s1x4[0], t1 = s1 * (t0 / N);
+                    const FitResult f = fit_exact(N, s1, ds.s2x16[0], t0, t1, t2, fp);
+                    p = Partial{f.rms, f.sum, (uint32_t)tid, t1, (uint16_t)f.qalfa,
+                                (uint16_t)f.qbeta, 0};
+                }
+                out[tid] = p;
+            }
+            return;
+        }
         int rr[N];
 #pragma unroll
         for (int p = 0; p < N; ++p) rr[p] = plane[(size_t)(row + p / S) * w + col + p % S];
-        const int32_t t0 = rs.t0[r], t2 = rs.t2[r];
-        const int64_t nrr = rs.nrr[r];
         const double rms0 = rs.rms0[r];
         const float t0f = (float)t0;
+        // The bound's candidate, and the bound.
+        double brms = inf;
+        uint32_t bidx = UINT32_MAX;
         Threshold th = make_threshold(inf, inf, UINT32_MAX, rms0, nrr, N, fp);
+        auto tighten = [&](double rms, double sum, uint32_t idx) {
+            if (idx == UINT32_MAX || !small_less(rms, idx, brms, bidx)) return;
+            brms = rms;
+            bidx = idx;
+            th = make_threshold(sum, rms, idx >> 3, rms0, nrr, N, fp);
+        };
         const int ndom = g.nrow_d * g.ncol_d;
         const int stride = kSmallThreads * gridDim.y;
-        for (int dom = blockIdx.y * kSmallThreads + tid; dom < ndom; dom += stride) {
+        const int begin = blockIdx.y * kSmallThreads;
+        for (int base = begin; base < ndom; base += stride) {
+            // (Lanes past the last domain look at it without taking part.)
+            const int dom = min(base + tid, ndom - 1);
             const int a = dom / g.ncol_d, b = dom - a * g.ncol_d;
             const int32_t* at = D + (size_t)(a * g.step_c) * g.dw + b * g.step_c;
             const int d[N] = {__ldg(at), __ldg(at + 1), __ldg(at + g.dw), __ldg(at + g.dw + 1)};
@@ -446,11 +514,55 @@ __global__ void __launch_bounds__(kSmallThreads) search_small_kernel(
             }
             const int32_t s1 = ds.s1x4[dom];
             const float detf = ds.detf[dom], sdetf = ds.sdetf[dom];
+            uint32_t left = base + tid < ndom ? 0xFFu : 0u;
+            bool improved = false;
+            auto take = [&](uint32_t iso, int32_t t1) {
+                ++exact;
+                const FitResult f = fit_exact(N, s1, ds.s2x16[dom], t0, t1, t2, fp);
+                const uint32_t idx = (uint32_t)dom * 8u + iso;
+                if (!small_less(f.rms, idx, e[K - 1].rms, e[K - 1].idx)) return;
+                e[K - 1] = SmallEntry{f.rms, f.sum, idx, f.qalfa | f.qbeta << 16, t1};
+#pragma unroll
+                for (int j = K - 1; j > 0; --j)
+                    if (small_less(e[j].rms, e[j].idx, e[j - 1].rms, e[j - 1].idx)) {
+                        const SmallEntry x = e[j];
+                        e[j] = e[j - 1];
+                        e[j - 1] = x;
+                    }
+                improved |= e[0].idx == idx;
+                if (e[K - 1].idx != UINT32_MAX) tighten(e[K - 1].rms, e[K - 1].sum, e[K - 1].idx);
+            };
+            auto share = [&] {
+                double rms, sum;
+                uint32_t idx;
+                warp_kth<K>(e[0], rms, sum, idx);
+                tighten(rms, sum, idx);
+            };
+            if (base == begin) {
+                if (left) {
+                    uint32_t iso = 0u;
+#pragma unroll
+                    for (int k = 7; k >= 0; --k)
+                        if (acc[k] == mx) iso = (uint32_t)k;
+                    left &= ~(1u << iso);
+                    take(iso, mx);
+                }
+                double rms, sum;
+                uint32_t idx;
+                warp_kth<K>(e[0], rms, sum, idx);
+                if (lane == 0) {
+                    bound_rms[warp] = rms;
+                    bound_sum[warp] = sum;
+                    bound_idx[warp] = idx;
+                }
+                __syncthreads();
+#pragma unroll 1
+                for (int v = 0; v < kSmallThreads / 32; ++v)
+                    tighten(bound_rms[v], bound_sum[v], bound_idx[v]);
+                improved = false;
+            }
             int32_t lim = prune_below(th, (uint32_t)dom, (float)s1, t0f, detf, sdetf, 0.25f, fp);
-            if (mx < lim) continue;
-            const int64_t s2 = ds.s2x16[dom];
-            uint32_t left = 0xFFu;
-            for (;;) {
+            while (left && mx >= lim) {
                 // The next isometry that the present bound lets through.
                 int32_t t1 = 0;
                 uint32_t iso = 8u;
@@ -462,30 +574,15 @@ __global__ void __launch_bounds__(kSmallThreads) search_small_kernel(
                     }
                 if (iso == 8u) break;
                 left &= ~((2u << iso) - 1u);
-                ++exact;
-                const FitResult f = fit_exact(N, s1, s2, t0, t1, t2, fp);
-                const uint32_t idx = (uint32_t)dom * 8u + iso;
-                if (!(f.rms < e[K - 1].rms || (f.rms == e[K - 1].rms && idx < e[K - 1].idx)))
-                    continue;
-                e[K - 1] = Entry{f.rms, f.sum, idx, f.qalfa | f.qbeta << 16, t1};
-#pragma unroll
-                for (int j = K - 1; j > 0; --j)
-                    if (e[j].rms < e[j - 1].rms ||
-                        (e[j].rms == e[j - 1].rms && e[j].idx < e[j - 1].idx)) {
-                        const Entry x = e[j];
-                        e[j] = e[j - 1];
-                        e[j - 1] = x;
-                    }
-                if (e[K - 1].idx != UINT32_MAX) {
-                    th = make_threshold(e[K - 1].sum, e[K - 1].rms, e[K - 1].idx >> 3, rms0, nrr, N, fp);
-                    lim = prune_below(th, (uint32_t)dom, (float)s1, t0f, detf, sdetf, 0.25f, fp);
-                }
+                take(iso, t1);
+                lim = prune_below(th, (uint32_t)dom, (float)s1, t0f, detf, sdetf, 0.25f, fp);
             }
+            __syncwarp();
+            if (__any_sync(0xffffffffu, improved)) share();
         }
     }
     // K times the smallest (rms, index) of the threads' heads: rms >= 0, so its bits order as
     // integers, and +inf past every other.
-    Partial* out = partials + ((size_t)blockIdx.y * nranges + r) * K;
     for (int j = 0; j < K; ++j) {
         const unsigned long long bits = (unsigned long long)__double_as_longlong(e[0].rms);
         const uint32_t hi = __reduce_min_sync(0xffffffffu, (uint32_t)(bits >> 32));
@@ -516,10 +613,18 @@ __global__ void __launch_bounds__(kSmallThreads) search_small_kernel(
                              (uint16_t)(e[0].q >> 16), 0};
 #pragma unroll
             for (int k = 0; k + 1 < K; ++k) e[k] = e[k + 1];
-            e[K - 1] = Entry{inf, inf, UINT32_MAX, 0u, 0};
+            e[K - 1] = SmallEntry{inf, inf, UINT32_MAX, 0u, 0};
         }
     }
-    if (exact_counter && exact) atomicAdd(exact_counter, (unsigned long long)exact);
+    // One addition a CTA: with one a thread, 0.7 ns each at the one address, the counter took 0.17 us
+    // a range, more than the rest.
+    exact = __reduce_add_sync(0xffffffffu, exact);
+    if (lane == 0) bound_idx[warp] = exact;
+    __syncthreads();
+    if (exact_counter && tid == 0) {
+        for (int v = 1; v < kSmallThreads / 32; ++v) exact += bound_idx[v];
+        atomicAdd(exact_counter, (unsigned long long)exact);
+    }
 }
 
 // Splits of a level of 2 x 2 blocks: two CTAs an SM, 2,048 domains (eight a thread) at least.

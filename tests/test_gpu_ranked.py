@@ -147,3 +147,35 @@ def test_two_by_two_blocks(ctx, w, h, shift, content):
             assert gev == oev
             assert got.tobytes() == want.tobytes(), (k, r, c)
         prov.close()
+
+
+@pytest.mark.parametrize("w,h,shift", [(34, 26, 2), (122, 90, 2), (122, 90, 8)])
+@pytest.mark.parametrize("content", ["noise", "soft", "areas"])
+def test_two_by_two_blocks_of_a_whole_plane(ctx, w, h, shift, content):
+    # Every block, so that a CTA's bound comes from any of its warps; alone (several splits of the
+    # domains) and together; flat areas whose first candidates win without a search.
+    rng = np.random.default_rng(w + shift)
+    img = rng.integers(0, 256, (h, w))
+    if content == "soft":
+        img = np.add.outer(np.arange(h), np.arange(w)) * 0.4 + rng.normal(0, 1, (h, w))
+    elif content == "areas":
+        img = (np.arange(w) // 9 * 40 % 256 + np.arange(h)[:, None] // 7 * 30) % 256
+        img[:6, :6] = rng.integers(0, 256, (6, 6))
+    img = np.clip(img, 0, 255).astype(np.uint8)
+    p = orc.make_params(min_size=2, max_size=2, shift=shift)
+    rows, cols = (a.ravel() for a in np.meshgrid(np.arange(h // 2) * 2, np.arange(w // 2) * 2,
+                                                 indexing="ij"))
+    want, wev = orc.search_blocks(img, 2, shift, p, rows, cols)
+    got, gev = ctx.search_blocks(img, 2, shift, mb.make_params(shift=shift), rows, cols)
+    assert got.tobytes() == want.tobytes() and np.array_equal(gev, wev)
+    for i in rng.integers(0, len(rows), 12):
+        one, _ = ctx.search_blocks(img, 2, shift, mb.make_params(shift=shift), rows[i: i + 1],
+                                   cols[i: i + 1])
+        assert one.tobytes() == want[i: i + 1].tobytes(), i
+    for k in (2, 5, 8):
+        prov = ctx.search_provider(img, mb.make_params(min_size=2, max_size=2, shift=shift), k=k)
+        for i in rng.integers(0, len(rows), 12):
+            a, _ = prov.search_candidates(rows[i], cols[i], 2, shift, k)
+            b, _ = orc.search(img, rows[i], cols[i], 2, shift, p, k=k)
+            assert a.tobytes() == b.tobytes(), (k, i)
+        prov.close()
