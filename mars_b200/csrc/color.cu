@@ -206,6 +206,27 @@ __device__ __forceinline__ void store_chunk(uint8_t* dst, const Chunk& c, const 
         if (c.begin + k < c.end) dst[c.begin + k] = (uint8_t)v[k];
 }
 
+// A byte a thread, for small planes whose rows are no whole chunks: a chunk across a row's end is
+// eight or sixteen bytes one by one in one thread, which such a plane waits for.
+__global__ void __launch_bounds__(256)
+    downsample_box_bytes_kernel(const uint8_t* __restrict__ src, int w, int h,
+                                uint8_t* __restrict__ dst, int ow) {
+    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
+    if (x >= ow) return;
+    const int x1 = min(2 * x + 1, w - 1), y1 = min(2 * y + 1, h - 1);
+    const uint8_t *top = src + (size_t)(2 * y) * w, *low = src + (size_t)y1 * w;
+    const uint32_t sum = (uint32_t)top[2 * x] + top[x1] + low[2 * x] + low[x1];
+    dst[(size_t)y * ow + x] = (uint8_t)((sum + 2) / 4);
+}
+
+__global__ void __launch_bounds__(256)
+    upsample_nearest_bytes_kernel(const uint8_t* __restrict__ src, int sw, int sh,
+                                  uint8_t* __restrict__ dst, int w) {
+    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
+    if (x < w)
+        dst[(size_t)y * w + x] = src[(size_t)min(y / 2, sh - 1) * sw + min(x / 2, sw - 1)];
+}
+
 // 9.2 us a 3840 x 2160 plane with a byte a thread.
 __global__ void __launch_bounds__(256)
     downsample_box_kernel(const uint8_t* __restrict__ src, int w, int h, uint8_t* __restrict__ dst,
@@ -335,6 +356,12 @@ static unsigned chunk_blocks(const uint8_t* dst, size_t n, size_t k) {
     return (unsigned)((chunks + 255) / 256);
 }
 
+// Whether an output of w x h bytes goes byte by byte: less than `most`, rows no whole chunks of k.
+static bool ragged_bytes(const uint8_t* dst, int w, int h, size_t k, size_t most) {
+    return (size_t)w * h < most &&
+           (w % k != 0 || (reinterpret_cast<uintptr_t>(dst) & (k - 1)) != 0);
+}
+
 cudaError_t launch_ycbcr(const uint8_t* r, const uint8_t* g, const uint8_t* b, size_t n,
                          uint8_t* y, uint8_t* cb, uint8_t* cr, bool inverse, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
@@ -356,14 +383,23 @@ cudaError_t launch_downsample_box(const uint8_t* src, int w, int h, uint8_t* dst
                                   cudaStream_t st) {
     const int ow = (w + 1) / 2, oh = (h + 1) / 2;
     if (ow == 0 || oh == 0) return cudaSuccess;
-    downsample_box_kernel<<<chunk_blocks(dst, (size_t)ow * oh, 8), 256, 0, st>>>(src, w, h, dst, ow, oh);
+    // us in chunks and in bytes, launch after launch: halving 340 x 260 4.1 and 3.2, 1000 x 750 4.1
+    // and 3.2, 1601 x 1201 4.1 and 4.2; whole chunks a row, 512 x 512, 3.1 and 3.1.
+    if (ragged_bytes(dst, ow, oh, 8, 1u << 19))
+        downsample_box_bytes_kernel<<<dim3((ow + 255) / 256, oh), 256, 0, st>>>(src, w, h, dst, ow);
+    else
+        downsample_box_kernel<<<chunk_blocks(dst, (size_t)ow * oh, 8), 256, 0, st>>>(src, w, h, dst, ow, oh);
     return cudaGetLastError();
 }
 
 cudaError_t launch_upsample_nearest(const uint8_t* src, int sw, int sh, uint8_t* dst, int w,
                                     int h, cudaStream_t st) {
     if (w == 0 || h == 0) return cudaSuccess;
-    upsample_nearest_kernel<<<chunk_blocks(dst, (size_t)w * h, 16), 256, 0, st>>>(src, sw, sh, dst, w, h);
+    // To 340 x 260 4.1 and 3.2, to 486 x 324 4.1 and 3.2, to 604 x 506 4.1 and 4.1.
+    if (ragged_bytes(dst, w, h, 16, 1u << 18))
+        upsample_nearest_bytes_kernel<<<dim3((w + 255) / 256, h), 256, 0, st>>>(src, sw, sh, dst, w);
+    else
+        upsample_nearest_kernel<<<chunk_blocks(dst, (size_t)w * h, 16), 256, 0, st>>>(src, sw, sh, dst, w, h);
     return cudaGetLastError();
 }
 

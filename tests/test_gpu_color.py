@@ -177,3 +177,29 @@ def test_zoomed_and_auto_colour_decodes(ctx):
     ref = np.stack(orc.rgb_from_ycbcr(oplanes[0], orc.upsample_nearest(oplanes[1], W, H),
                                       orc.upsample_nearest(oplanes[2], W, H)), axis=-1)
     assert used == max(uses) and np.array_equal(out, ref)
+
+
+@pytest.mark.parametrize("offset", [0, 1, 4, 13])
+@pytest.mark.parametrize("shape", [(1301, 1623), (523, 511), (511, 513), (65, 33)])
+def test_ragged_planes_by_chunks_and_by_bytes(ctx, shape, offset):
+    # Rows that are no whole chunks, on either side of the sizes that go by bytes.
+    torch = pytest.importorskip("torch")
+    h, w = shape
+    hw, hh = (w + 1) // 2, (h + 1) // 2
+    host = np.random.default_rng(w + offset).integers(0, 256, (h, w), dtype=np.uint8)
+    src = torch.from_numpy(np.pad(host.ravel(), (offset, 16))).cuda()
+    down, up = (torch.full((n + 32,), 77, dtype=torch.uint8, device="cuda:0")
+                for n in (hh * hw, h * w))
+    torch.cuda.synchronize()
+    L = mb.lib()
+    mb.check(L.mars_downsample_box_device(ctx.handle, src.data_ptr() + offset, w, h,
+                                          down.data_ptr() + offset))
+    mb.check(L.mars_upsample_nearest_device(ctx.handle, down.data_ptr() + offset, hw, hh,
+                                            up.data_ptr() + offset, w, h))
+    torch.cuda.synchronize()
+    half = orc.downsample_box(host)
+    for buf, want in ((down, half), (up, orc.upsample_nearest(half, w, h))):
+        got = buf.cpu().numpy()
+        end = offset + want.size
+        assert (got[:offset] == 77).all() and (got[end:] == 77).all()
+        assert np.array_equal(got[offset:end].reshape(want.shape), want)
