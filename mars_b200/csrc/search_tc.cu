@@ -1488,7 +1488,10 @@ constexpr int kSeedCands = 8 * kSeedSide * kSeedSide;  // x 8 isometries
 // block (8 per CTA).  Lane l correlates candidates l, l + 32, l + 64 whole (S^2 terms) from the
 // range staged in shared memory; isometry::map is affine in (u, v), so a candidate walks the
 // staged range with a base and two strides and lanes of different isometries do not
-// diverge.  One (rms, reference index) reduction picks the winner.
+// diverge.  One (rms, reference index) reduction picks the winner.  Where that is no better than
+// the flat fit, the first domain's candidates are looked at as well: those of contrast 0 all fit
+// like the flat fit and the first of them wins, so that no later domain has to be searched for an
+// earlier one (unit_publish).
 template <int S>
 __global__ void __launch_bounds__(256) seed_small_kernel(
     const int32_t* __restrict__ D, LevelGeom g, const uint8_t* __restrict__ plane, int w,
@@ -1511,10 +1514,7 @@ __global__ void __launch_bounds__(256) seed_small_kernel(
     double best = INFINITY, best_sum = 0.0;
     uint32_t best_idx = UINT32_MAX;
     int32_t best_t1 = 0;
-    for (int c = lane; c < kSeedCands; c += 32) {
-        const int nb = c >> 3, k = c & 7;
-        const int a = min(max(ac + nb / kSeedSide - kSeedSide / 2, 0), g.nrow_d - 1);
-        const int bb = min(max(bc + nb % kSeedSide - kSeedSide / 2, 0), g.ncol_d - 1);
+    auto look = [&](int a, int bb, int k) {
         const int32_t* db = D + (size_t)(a * g.step_c) * g.dw + bb * g.step_c;
         // iso_src_rt(k, u, v, S) = base + u * du + v * dv
         int base, du, dv;
@@ -1544,20 +1544,35 @@ __global__ void __launch_bounds__(256) seed_small_kernel(
             best_idx = idx;
             best_t1 = t1;
         }
-    }
-    double br = best;
-    uint32_t bi = best_idx;
-    int bl = lane;
+    };
+    double br;
+    uint32_t bi;
+    int bl;
+    auto reduce = [&] {
+        br = best;
+        bi = best_idx;
+        bl = lane;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const double r2 = __shfl_xor_sync(0xffffffffu, br, o);
-        const uint32_t i2 = __shfl_xor_sync(0xffffffffu, bi, o);
-        const int l2 = __shfl_xor_sync(0xffffffffu, bl, o);
-        if (r2 < br || (r2 == br && i2 < bi)) {
-            br = r2;
-            bi = i2;
-            bl = l2;
+        for (int o = 16; o > 0; o >>= 1) {
+            const double r2 = __shfl_xor_sync(0xffffffffu, br, o);
+            const uint32_t i2 = __shfl_xor_sync(0xffffffffu, bi, o);
+            const int l2 = __shfl_xor_sync(0xffffffffu, bl, o);
+            if (r2 < br || (r2 == br && i2 < bi)) {
+                br = r2;
+                bi = i2;
+                bl = l2;
+            }
         }
+    };
+    for (int c = lane; c < kSeedCands; c += 32) {
+        const int nb = c >> 3;
+        look(min(max(ac + nb / kSeedSide - kSeedSide / 2, 0), g.nrow_d - 1),
+             min(max(bc + nb % kSeedSide - kSeedSide / 2, 0), g.ncol_d - 1), c & 7);
+    }
+    reduce();
+    if (!(br < rs.rms0[r])) {
+        if (lane < 8) look(0, 0, lane);
+        reduce();
     }
     if (lane == bl) out[r] = SeedOut{best, best_sum, best_idx, best_t1};
 }

@@ -21,9 +21,13 @@
 // integers: the exact correlation, the full bound of fit.cuh with the largest contrast added,
 // then the f64 fit.  So the winners, their rms bits and the tie order are the integer path's.
 //
-// Ranges whose W is not positive (flat blocks, a champion no better than the flat fit) have no
-// such number: they take the per-lane bound of fit.cuh on Nrd = rho sqrt(Ndd Nrr), the full
-// form, until their champion improves.
+// Ranges whose champion is no better than the flat fit have no such number: a candidate of
+// contrast 0 ties with that fit, and wins if its domain comes first.  They take the per-lane bound
+// of fit.cuh on Nrd = rho sqrt(Ndd Nrr), the full form, until their champion improves or is of
+// the first domain, which the seeds see to (seed_small_kernel); from then on W <= 0 leaves the
+// tile's contrast alone to give a threshold (unit_tile_threshold).  A tile whose threshold is low
+// takes the full form too.  (A checkerboard of 4 x 4 squares, 1024 x 1024 at S = 8, stride 4, where
+// nothing beats the flat fit: 1.8 ms, 13.1 with every tile in the full form; the integer form 2.8.)
 //
 // Survivors leave the scan at once: a scan warp appends (domain, range) to its own ring in
 // shared memory, and the fit warp of its column half evaluates them, up to 32 at a time, so the
@@ -73,7 +77,9 @@ constexpr int kGroup = 8;                                  // tiles that share t
 constexpr int kSets = 32;                                  // sets of thresholds in use
 constexpr float kUnitScale = 4096.0f;                      // 64 x 64
 constexpr float kUnitSlack = 4.5f;                         // the filter's allowance
-constexpr float kUnitLeast = kUnitScale / 64.0f;           // thresholds below take the full form
+constexpr float kUnitLeast = kUnitScale / 64.0f;           // tiles' thresholds below take the full form
+constexpr float kUnitAlike = 1.1f;                         // the contrasts of tiles that are alike
+constexpr float kUnitNone = 1e-30f;                        // a champion's W gives no threshold
 
 // A tile as the load warp announces it: what to do, which domains, and the set of thresholds its
 // ranges take there.  The load warp is at most kMaxStages tiles ahead of the MMAs and those two
@@ -152,14 +158,17 @@ __device__ __forceinline__ void unit_publish(USmem& sm, int rl, const FitParams&
     }
     const Threshold th = make_threshold(C.sum, C.rms, C.idx >> 3, C.rms0, C.nrr, n, fp);
     const float snrr = __fsqrt_ru(__ll2float_ru(C.nrr));
+    // Whether no candidate of contrast 0 can win any more: the champion is better than the flat
+    // fit, or as good and of the first domain, whose candidates the seed was chosen among.
+    const bool settled = th.mode == 2 || (th.mode == 1 && th.tie_dom == 0);
     ThrRec t;
     t.sqrt_w = th.wpos ? th.sqrt_w : -INFINITY;
     t.w2a = th.w2a;
     t.c = snrr;
-    t.tie = th.mode == 2 ? -1 : (th.mode == 1 ? (int32_t)th.tie_dom : INT32_MAX);
+    t.tie = settled ? -1 : (th.mode == 1 ? (int32_t)th.tie_dom : INT32_MAX);
     sm.thr[rl] = t;
-    const float u = __fdiv_rd(th.sqrt_w, snrr) * kUnitScale - kUnitSlack;
-    scan_publish(words, rl, !(th.wpos && th.mode == 2 && u >= kUnitLeast), u);
+    const float u = th.wpos ? __fdiv_rd(th.sqrt_w, snrr) * kUnitScale - kUnitSlack : 0.0f;
+    scan_publish(words, rl, !settled, fmaxf(u, kUnitNone));
 }
 
 // fit.cuh's bound on Nrd for one (range record, domain), every step rounded toward -inf, with
@@ -557,14 +566,15 @@ __device__ __noinline__ uint32_t unit_look_full(const ItemArgs& a, USmem& sm, ui
 // ihi their reciprocals): the smallest rho that a fit with a contrast in a_min..a_max needs
 // there, in accumulator units.  It is u = sqrt(W / Nrr) where the best contrast
 // sqrt(W) / sqrt(Ndd) is allowed, and grows away from there, so the tile's end nearest to that
-// counts.  rr: the range's record (sqrt W, W / (2 a_min)), inv: 1 / sqrt(Nrr).  The steps'
+// counts; with W <= 0 it grows with the contrast.  rr: the range's record (sqrt W, W / (2 a_min)), inv: 1 / sqrt(Nrr).  The steps'
 // rounding, and reciprocals good to a few units in the last place, stay far below the 1e-5
 // taken off.
 __device__ __forceinline__ float unit_tile_threshold(const float4& rr, float u, float inv, float lo,
                                                      float hi, float ilo, float ihi,
                                                      const FitParams& fp) {
     const float weak = rr.y * fp.min_over_max * ihi + fp.max_half * hi;
-    const float strong = rr.y * ilo + fp.a_half * lo;
+    // (W <= 0: what the two terms' rounding could leave of their difference is taken off the first.)
+    const float strong = fminf(rr.y, rr.y * 1.00001f) * ilo + fp.a_half * lo;
     // Nrd needed over sqrt(Ndd)
     const float tau = rr.x > 1.0001f * fp.a_max * hi
                           ? weak
@@ -651,11 +661,13 @@ __device__ __noinline__ void unit_load_role(const ItemArgs& a, USmem& sm, int nt
                 // champion's bounds hold.
                 const float4 rr = lds_f4(&sm.thr[lane]);
                 const ScanState st = scan_read(ScanWords{sm.uscan}, lane);
-                const uint32_t fulls = __ballot_sync(0xffffffffu, st.full);
-                const float thr =
-                    st.full ? INFINITY
-                            : unit_tile_threshold(rr, st.threshold, inv, lo, hi,
-                                                  __fdividef(1.0f, lo), __fdividef(1.0f, hi), a.fp);
+                float thr = unit_tile_threshold(rr, st.threshold, inv, lo, hi, __fdividef(1.0f, lo),
+                                                __fdividef(1.0f, hi), a.fp);
+                // Where the contrast alone gives the threshold, only tiles of one contrast scan.
+                const bool full = st.full || thr < kUnitLeast ||
+                                  (st.threshold < kUnitLeast && hi > kUnitAlike * lo);
+                const uint32_t fulls = __ballot_sync(0xffffffffu, full);
+                if (full) thr = INFINITY;
                 if (!fulls && !__any_sync(0xffffffffu, thr <= kUnitScale * 1.002f)) continue;
                 const int set = sets++ % kSets;
                 sm.set[set][lane] = thr;

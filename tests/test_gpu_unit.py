@@ -1,8 +1,11 @@
 """The unit-vector correlation (block sizes 4 and 8) against the CUDA-core kernel: the same
 records, byte for byte, at the edges of its tiles (32 ranges, 128 domains) and on planes that
 leave its quick test: flat and nearly flat blocks, ties, saturated and high-contrast ones."""
+import time
+
 import numpy as np
 import pytest
+import torch
 
 import mars_b200 as mb
 
@@ -113,3 +116,45 @@ def test_several_splits_a_range_tile(both, kind, size, w, h, n):
         got = both[0].search_blocks(img, size, 2, params, rows, cols)
         assert got[0].tobytes() == want[0].tobytes()
         assert np.array_equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("alfa_bits,beta_bits,max_alfa", [(4, 7, 1.0), (1, 1, 3.0), (2, 3, 0.3),
+                                                          (8, 2, 2.0)])
+@pytest.mark.parametrize("kind", ["ties", "faint", "noise"])
+@pytest.mark.parametrize("size", [4, 8])
+def test_ranges_that_nothing_fits_better_than_flat(both, size, kind, alfa_bits, beta_bits, max_alfa):
+    # Champions of contrast 0, W far below zero where the offset's steps are coarse; the first
+    # domain's flat quarter at (0, 0) included.
+    img = _plane(kind, 180, 132, 7)
+    for plane in (img, np.where(np.add.outer(np.arange(132), np.arange(180)) < 40, 90, img)):
+        plane = np.ascontiguousarray(plane, dtype=np.uint8)
+        params = mb.make_params(shift=2, bits_alfa=alfa_bits, bits_beta=beta_bits, max_alfa=max_alfa)
+        got, want = (c.search_grid(plane, size, 2, params) for c in both)
+        assert got[0].tobytes() == want[0].tobytes()
+
+
+@pytest.mark.parametrize("side,shift", [(512, 2), (1024, 8)])
+def test_no_slower_than_the_integer_form_where_nothing_fits(monkeypatch, side, shift):
+    # A checkerboard of 4 x 4 squares in blocks of 8: no domain correlates with any block.
+    plane = torch.from_numpy(_plane("ties", side, side)).cuda()
+    params = mb.make_params(min_size=8, max_size=8, shift=shift)
+    n = mb.C.c_size_t()
+    times, records = [], []
+    for tiles in ("0", str(1 << 40)):  # the unit form, the fold
+        monkeypatch.setenv("MARS_UNIT_TILES", tiles)
+        with mb.Context(0) as ctx:
+            args = (ctx.handle, plane.data_ptr(), side, side, mb.C.byref(params))
+            mb.check(mb.lib().mars_search_nodes_device(*args, None, 0, mb.C.byref(n), None))
+            out = torch.zeros(n.value, 80, dtype=torch.uint8, device="cuda")
+            best = float("inf")
+            for _ in range(5):
+                torch.cuda.synchronize()
+                t = time.perf_counter()
+                mb.check(mb.lib().mars_search_nodes_device(*args, out.data_ptr(), n.value,
+                                                           mb.C.byref(n), None))
+                torch.cuda.synchronize()
+                best = min(best, time.perf_counter() - t)
+            times.append(best)
+            records.append(out.cpu().numpy().tobytes())
+    assert records[0] == records[1]
+    assert times[0] < 1.5 * times[1]
