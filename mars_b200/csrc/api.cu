@@ -456,6 +456,7 @@ struct TcLevel {
     mars::tc::UnitSource unit{};
     uint32_t *d_domains = nullptr, *d_ranges = nullptr, *d_bins = nullptr;  // unit form
     float2* d_contrasts = nullptr;
+    uint4* d_windows = nullptr;
     mars::Partial* partials = nullptr;
     unsigned long long* gch = nullptr;
     int* tickets = nullptr;  // all-levels launch only
@@ -468,7 +469,7 @@ struct TcLevel {
 constexpr size_t kDomainTmpWords = 64ull << 20;
 
 // The unit form's A operand holds every domain window (32 or 128 bytes a position at sizes 4 and
-// 8), up to this many bytes a level: planes to about 11,500 pixels a side at size 8, stride 2.
+// 8; the survivors' samples take as many again), up to this many bytes a level: planes to about 11,500 pixels a side at size 8, stride 2.
 // Beyond it the fold reads the windows from copies of the plane.
 constexpr size_t kUnitBytes = 4ull << 30;
 // Its work items cost 25,000 cycles to set up, preview and drain, the fold's about 6,000, and its
@@ -504,6 +505,7 @@ int tc_level_setup(mars_ctx* ctx, Scratch& sc, uint32_t w, uint32_t h, size_t n,
     L.path = path;
     if (L.path == mars::tc::kUnit) {
         MARS_CUDA(sc.get(&L.d_a, mars::tc::unit_a_bytes(g)));
+        MARS_CUDA(sc.get(&L.d_windows, mars::tc::unit_a_bytes(g) / sizeof(uint4)));
         MARS_CUDA(sc.get(&L.d_domains, (size_t)g.nrow_d * g.ncol_d));
         MARS_CUDA(sc.get(&L.d_ranges, n));
         MARS_CUDA(sc.get(&L.d_bins, 2 * mars::tc::unit_bins_words()));
@@ -555,9 +557,9 @@ int tc_level_prep(mars_ctx* ctx, TcLevel& L, const uint8_t* d_plane, const int32
     const int n = (int)L.n;
     if (L.path == mars::tc::kUnit) {
         L.unit = mars::tc::UnitSource{L.d_a, L.d_domains, L.d_ranges, L.d_contrasts,
-                                      d_D,   d_plane,     d_rows,     d_cols};
+                                      L.d_windows, d_plane, d_rows, d_cols};
         MARS_CUDA(mars::tc::launch_unit_a(d_D, g, L.ds, L.d_bins, L.d_domains, L.d_contrasts, L.d_a,
-                                          sp));
+                                          L.d_windows, sp));
         MARS_CUDA(mars::tc::launch_unit_b(g.size, d_plane, (int)w, (int)h, d_rows, d_cols, n, L.rs,
                                           L.d_bins + mars::tc::unit_bins_words(), L.d_ranges, L.d_b,
                                           st));

@@ -1631,10 +1631,11 @@ static_assert(unit_smem_bytes<4>() <= 232448 && unit_smem_bytes<8>() <= 232448,
 
 template <int S>
 cudaError_t build_unit_a_t(const int32_t* D, const LevelGeom& g, DomainStats ds,
-                           const uint32_t* domains, uint8_t* out, cudaStream_t st) {
+                           const uint32_t* domains, uint8_t* out, uint4* windows,
+                           cudaStream_t st) {
     const long long total = (long long)domain_tiles(g, kUnit) * kM * UCfg<S>::KG;
     unit_a_kernel<S><<<(unsigned)((total + 255) / 256), 256, 0, st>>>(
-        D, g, ds, domains, total, reinterpret_cast<uint4*>(out));
+        D, g, ds, domains, total, reinterpret_cast<uint4*>(out), windows);
     return cudaGetLastError();
 }
 
@@ -1711,14 +1712,15 @@ size_t b_bytes(int size, int nranges, Path path) {
 size_t unit_bins_words() { return 2 * kBins; }
 
 cudaError_t launch_unit_a(const int32_t* D, const LevelGeom& g, DomainStats ds, uint32_t* bins,
-                          uint32_t* domains, float2* contrasts, uint8_t* out, cudaStream_t st) {
+                          uint32_t* domains, float2* contrasts, uint8_t* out, uint4* windows,
+                          cudaStream_t st) {
     const int ndom = g.nrow_d * g.ncol_d, tiles = domain_tiles(g, kUnit);
     cudaError_t e = launch_order_t<false>(ds, RangeStats{}, ndom, bins, domains, st);
     if (e != cudaSuccess) return e;
     tile_contrast_kernel<<<(tiles + 7) / 8, 256, 0, st>>>(ds, domains, ndom, tiles, contrasts);
     switch (g.size) {
-        case 4: return build_unit_a_t<4>(D, g, ds, domains, out, st);
-        case 8: return build_unit_a_t<8>(D, g, ds, domains, out, st);
+        case 4: return build_unit_a_t<4>(D, g, ds, domains, out, windows, st);
+        case 8: return build_unit_a_t<8>(D, g, ds, domains, out, windows, st);
         default: return cudaErrorInvalidValue;
     }
 }

@@ -236,29 +236,27 @@ __device__ __forceinline__ float4 lds_f4(const void* p) {
     return v;
 }
 
-// The exact correlations t1_x4 of each lane's entry (window at D + at, range rl) under the eight
-// isometries: 16 samples of the window at a time, packed in pairs of 16 bits (they are at most
-// 1020), against the range's permuted bytes.  Compact on purpose: this code runs rarely, and
-// what a cold instruction costs to fetch exceeds what it computes.
+// The exact correlations t1_x4 of each lane's entry (domain position pos, range rl) under the eight
+// isometries: 16 samples of the window at a time, in pairs of 16 bits (they are at most 1020),
+// against the range's permuted bytes.  The windows lie beside the A operand in its order, so 16
+// bytes a load, and those of the neighbouring domains that survive together share lines.  (Sample
+// by sample from the contracted plane, 64 loads of as many lines at S = 8, a 1024 x 1024 ramp, whose
+// blocks all match, took 31.7 ms at stride 8; 26.1 so, the integer form 25.2.)  Compact on purpose:
+// this code runs rarely, and what a cold instruction costs to fetch exceeds what it computes.
 template <int S>
 __device__ __forceinline__ void unit_correlate(const ItemArgs& a, const uint8_t* pix, bool act,
-                                               uint32_t at, int rl, uint32_t (&t1)[8]) {
+                                               uint32_t pos, int rl, uint32_t (&t1)[8]) {
     constexpr int N = S * S;
-    const int dw = a.g.dw;
 #pragma unroll
     for (int k = 0; k < 8; ++k) t1[k] = 0u;
     if (!act) return;
-    const int32_t* db = a.unit.D + at;
+    const uint4* dw = a.unit.windows + (size_t)(pos / 8) * N + pos % 8;
     const uint4* rr = reinterpret_cast<const uint4*>(pix + rl * 8 * N);
 #pragma unroll 1
     for (int c = 0; c < N / 16; ++c) {
-        uint32_t d[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int32_t* p = db + (size_t)(2 * i / S) * dw + 2 * i % S;
-            d[i] = (uint32_t)__ldg(p) | (uint32_t)__ldg(p + 1) << 16;
-        }
-        db += (size_t)(16 / S) * dw;
+        const uint4 lo = __ldg(dw), hi = __ldg(dw + 8);
+        const uint32_t d[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+        dw += 16;
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             const uint4 r = rr[k * (N / 16) + c];
@@ -279,7 +277,6 @@ template <int S>
 __device__ __noinline__ void unit_fit(const ItemArgs& a, USmem& sm, const uint8_t* pix,
                                       unsigned long long entry, bool best_only, int* err) {
     constexpr int N = S * S;
-    const LevelGeom& g = a.g;
     const int lane = threadIdx.x & 31;
     const bool act = entry != 0ull;
     const uint32_t dom = act ? a.unit.domains[(uint32_t)entry] : 0u;
@@ -288,17 +285,14 @@ __device__ __noinline__ void unit_fit(const ItemArgs& a, USmem& sm, const uint8_
     int s1 = 0;
     int64_t s2 = 0;
     float detf = 0.0f, sdetf = 0.0f;
-    uint32_t at = 0u;
     if (act) {
         s1 = a.ds.s1x4[dom];
         s2 = a.ds.s2x16[dom];
         detf = a.ds.detf[dom];
         sdetf = a.ds.sdetf[dom];
-        at = (dom / (uint32_t)g.ncol_d) * (uint32_t)(g.step_c * g.dw) +
-             (dom % (uint32_t)g.ncol_d) * (uint32_t)g.step_c;
     }
     uint32_t t1s[8];
-    unit_correlate<S>(a, pix, act, at, rl, t1s);
+    unit_correlate<S>(a, pix, act, (uint32_t)entry, rl, t1s);
     const int32_t t0 = sm.ch[rl].t0, t2 = sm.ch[rl].t2;
     uint32_t isos = act ? 0xFFu : 0u;
     if (best_only && act) {
@@ -1109,11 +1103,13 @@ __device__ __forceinline__ uint32_t pack_f16(float lo, float hi) {
 // A operand of one level, in contrast order: groups of 8 domains, each KG k-groups x (8 rows x
 // 16 B); a tile is 16 groups.  One thread per (domain, k-group): 8 samples of the contracted
 // window, centred and scaled to length 64; zero rows for flat domains and past the last one.
+// windows: the samples themselves, 16 bits each, in the same order.
 template <int S>
 __global__ void __launch_bounds__(256) unit_a_kernel(const int32_t* __restrict__ D, LevelGeom g,
                                                      DomainStats ds,
                                                      const uint32_t* __restrict__ domains,
-                                                     long long total, uint4* __restrict__ out) {
+                                                     long long total, uint4* __restrict__ out,
+                                                     uint4* __restrict__ windows) {
     using C_ = UCfg<S>;
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= total) return;
@@ -1122,30 +1118,33 @@ __global__ void __launch_bounds__(256) unit_a_kernel(const int32_t* __restrict__
     const long long rest = t >> 3;
     const int kg = (int)(rest % C_::KG);
     const long long pos = rest / C_::KG * 8 + r8;
-    uint4 pk = make_uint4(0u, 0u, 0u, 0u);
+    uint4 pk = make_uint4(0u, 0u, 0u, 0u), win = pk;
     if (pos < (long long)g.nrow_d * g.ncol_d) {
         const uint32_t dom = domains[pos];
         const int s1 = ds.s1x4[dom];
         const int64_t det = (int64_t)C_::N * ds.s2x16[dom] - (int64_t)s1 * s1;
-        if (det > 0) {
-            // |N D - s1|^2 = N det
-            const float inv = 64.0f * rsqrtf((float)C_::N * (float)det);
-            const int32_t* db = D + (size_t)(dom / (uint32_t)g.ncol_d) * g.step_c * g.dw +
-                                (size_t)(dom % (uint32_t)g.ncol_d) * g.step_c;
-            uint32_t h[4];
+        // |N D - s1|^2 = N det
+        const float inv = det > 0 ? 64.0f * rsqrtf((float)C_::N * (float)det) : 0.0f;
+        const int32_t* db = D + (size_t)(dom / (uint32_t)g.ncol_d) * g.step_c * g.dw +
+                            (size_t)(dom % (uint32_t)g.ncol_d) * g.step_c;
+        uint32_t h[4], d[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                float x[2];
+        for (int i = 0; i < 4; ++i) {
+            float x[2];
+            d[i] = 0u;
 #pragma unroll
-                for (int c = 0; c < 2; ++c) {
-                    const int e = kg * 8 + 2 * i + c;
-                    x[c] = (float)(C_::N * __ldg(db + (size_t)(e / S) * g.dw + e % S) - s1) * inv;
-                }
-                h[i] = pack_f16(x[0], x[1]);
+            for (int c = 0; c < 2; ++c) {
+                const int e = kg * 8 + 2 * i + c;
+                const int v = __ldg(db + (size_t)(e / S) * g.dw + e % S);
+                d[i] |= (uint32_t)v << (16 * c);
+                x[c] = (float)(C_::N * v - s1) * inv;
             }
-            pk = make_uint4(h[0], h[1], h[2], h[3]);
+            h[i] = det > 0 ? pack_f16(x[0], x[1]) : 0u;
         }
+        pk = make_uint4(h[0], h[1], h[2], h[3]);
+        win = make_uint4(d[0], d[1], d[2], d[3]);
     }
+    windows[t] = win;
     out[t] = pk;
 }
 

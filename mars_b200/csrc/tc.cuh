@@ -32,13 +32,13 @@ struct alignas(64) TcMaps {
 enum Path : int { kFold = 0, kDigits = 1, kUnit = 2 };
 
 // What the unit form reads beside the B operand: the A operand, the domains and ranges in its and
-// B's row order (by contrast), each domain tile's smallest and largest contrast; and the
-// contracted plane, the range plane and the range origins its survivors are evaluated from.
+// B's row order (by contrast), each domain tile's smallest and largest contrast; and the domains'
+// windows in A's order, the range plane and the range origins its survivors are evaluated from.
 struct UnitSource {
     const uint8_t* aglob = nullptr;
     const uint32_t *domains = nullptr, *ranges = nullptr;
     const float2* contrasts = nullptr;
-    const int32_t* D = nullptr;
+    const uint4* windows = nullptr;
     const uint8_t* plane = nullptr;
     const uint32_t *rows = nullptr, *cols = nullptr;
 };
@@ -83,7 +83,8 @@ size_t phase_bytes(int w, int h, int shift);
 // of row_pitch(w / 2) bytes (plus slack).
 int digit_phase_count(int shift);
 size_t digit_plane_bytes(int w, int h, int shift);
-// Levels the unit form serves (block sizes 4 and 8), and its A operand's bytes.
+// Levels the unit form serves (block sizes 4 and 8), and the bytes of its A operand, and as many
+// of the domains' windows.
 bool unit_supported(int size, int shift);
 size_t unit_a_bytes(const LevelGeom& g);
 // Domain tiles of a level: 128 positions of one domain row each, or, in the unit form, any 128
@@ -120,7 +121,8 @@ cudaError_t launch_corr(const TcMaps& maps, const uint8_t* bglob, const LevelGeo
 // unit_bins_words() words of scratch for each call).  launch_corr_all correlates it.
 size_t unit_bins_words();
 cudaError_t launch_unit_a(const int32_t* D, const LevelGeom& g, DomainStats ds, uint32_t* bins,
-                          uint32_t* domains, float2* contrasts, uint8_t* out, cudaStream_t st);
+                          uint32_t* domains, float2* contrasts, uint8_t* out, uint4* windows,
+                          cudaStream_t st);
 cudaError_t launch_unit_b(int size, const uint8_t* plane, int w, int h, const uint32_t* rows,
                           const uint32_t* cols, int nranges, RangeStats rs, uint32_t* bins,
                           uint32_t* ranges, uint8_t* out, cudaStream_t st);
