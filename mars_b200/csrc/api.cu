@@ -916,14 +916,16 @@ bool all_levels_eligible(const mars_ctx* ctx, uint32_t w, uint32_t h, const std:
     return levels > 0 && levels + 1 <= mars::tc::kMaxLevelJobs;
 }
 
-// The context's branch streams and their events, on first use.  The caller holds ctx->mu.
-int make_branches(mars_ctx* ctx) {
-    if (!ctx->fork_ev) {
+// The context's first n branch streams and their events, on first use (50 us each).  The caller
+// holds ctx->mu.
+int make_branches(mars_ctx* ctx, int n) {
+    if (!ctx->fork_ev)
         MARS_CUDA(cudaEventCreateWithFlags(&ctx->fork_ev, cudaEventDisableTiming));
-        for (int b = 0; b < mars_ctx::kBranches; ++b) {
+    for (int b = 0; b < n; ++b) {
+        if (!ctx->branch[b])
             MARS_CUDA(cudaStreamCreateWithFlags(&ctx->branch[b], cudaStreamNonBlocking));
+        if (!ctx->join_ev[b])
             MARS_CUDA(cudaEventCreateWithFlags(&ctx->join_ev[b], cudaEventDisableTiming));
-        }
     }
     return MARS_OK;
 }
@@ -939,7 +941,9 @@ int run_jobs_all_levels(mars_ctx* ctx, Scratch& sc, const uint8_t* d_plane, uint
                         mars::CandidateOut* d_out, const uint32_t* d_rc_in,
                         cudaEvent_t* timing = nullptr) {
     const cudaStream_t main = ctx->stream;
-    if (int e = make_branches(ctx)) return e;
+    // A level's range side and seeds run on branch b, its domain side on branch b + half.
+    const int half = (int)std::min<size_t>(jobs.size(), mars_ctx::kBranches / 2), nb = 2 * half;
+    if (int e = make_branches(ctx, nb)) return e;
     int32_t* d_D = nullptr;
     MARS_CUDA(sc.get(&d_D, std::max<size_t>(1, (size_t)(w / 2) * (h / 2))));
     MARS_CUDA(mars::launch_contract(d_plane, (int)w, (int)h, d_D, main));
@@ -1013,25 +1017,21 @@ int run_jobs_all_levels(mars_ctx* ctx, Scratch& sc, const uint8_t* d_plane, uint
     int* d_work = nullptr;
     MARS_CUDA(sc.get(&d_work, 2));
     MARS_CUDA(cudaMemsetAsync(d_work, 0, 2 * sizeof(int), main));
-    // Every branch is forked: a level's range side and seeds run on branch b, its domain side on
-    // branch b + kBranches / 2.
     MARS_CUDA(cudaEventRecord(ctx->fork_ev, main));
-    const int nb = mars_ctx::kBranches;
-    constexpr int kHalf = mars_ctx::kBranches / 2;
     for (int b = 0; b < nb; ++b) MARS_CUDA(cudaStreamWaitEvent(ctx->branch[b], ctx->fork_ev, 0));
     int err = MARS_OK;
     size_t off = 0;
     for (size_t i = 0; i < jobs.size() && !err; ++i) {
         const Job& j = jobs[i];
-        const int b = (int)(i % kHalf);
+        const int b = (int)i % half;
         const cudaStream_t bs = ctx->branch[b];
         const uint32_t* rows = d_rc + off;
         const uint32_t* cols = d_rc + total + off;
         const int l = level_of[i];
         if (l >= 0) {
             TcLevel& L = lv[l];
-            const cudaStream_t bd = ctx->branch[b + kHalf];
-            const cudaEvent_t ev = ctx->join_ev[b + kHalf];
+            const cudaStream_t bd = ctx->branch[b + half];
+            const cudaEvent_t ev = ctx->join_ev[b + half];
             err = tc_level_stats(ctx, L, d_plane, d_D, w, h, fp, rows, cols, bs, bd, ev);
             if (!err)
                 err = tc_level_prep(ctx, L, d_plane, d_D, d_plane, w, h, fp, rows, cols, bs, bd, ev);
@@ -1187,15 +1187,28 @@ int fisher_buffers(Scratch& sc, uint32_t w, uint32_t h, const Job* jobs, size_t 
         if (g.nrow_d > 0 && g.ncol_d > 0) npos = std::max(npos, (size_t)g.nrow_d * g.ncol_d);
         parts = std::max(parts, j->rows.size() * (size_t)mars::fisher_warps_per_range((int)j->size));
     }
-    MARS_CUDA(sc.get(&b->ix.key, npos));
-    MARS_CUDA(sc.get(&b->ix.diso, npos));
-    MARS_CUDA(sc.get(&b->ix.list, npos));
-    MARS_CUDA(sc.get(&b->ix.counts, 72));
-    MARS_CUDA(sc.get(&b->ix.offsets, 72));
-    MARS_CUDA(sc.get(&b->ix.ref, 72));
-    MARS_CUDA(sc.get(&b->ix.work, mars::fisher_group_work_words(npos)));
-    MARS_CUDA(sc.get(&b->part, parts));
-    MARS_CUDA(sc.get(&b->part_e, parts));
+    // One allocation: in a plan's graphs each is a node to allocate and one to free.
+    size_t bytes = 0;
+    unsigned char* base = nullptr;
+    auto place = [&](auto** p, size_t count) {
+        if (base) *p = reinterpret_cast<std::remove_reference_t<decltype(*p)>>(base + bytes);
+        bytes += (count * sizeof(**p) + 255) / 256 * 256;
+    };
+    auto all = [&] {
+        place(&b->ix.key, npos);
+        place(&b->ix.diso, npos);
+        place(&b->ix.list, npos);
+        place(&b->ix.counts, 72);
+        place(&b->ix.offsets, 72);
+        place(&b->ix.ref, 72);
+        place(&b->ix.work, mars::fisher_group_work_words(npos));
+        place(&b->part, parts);
+        place(&b->part_e, parts);
+    };
+    all();
+    MARS_CUDA(sc.get(&base, bytes));
+    bytes = 0;
+    all();
     return MARS_OK;
 }
 
@@ -1259,7 +1272,7 @@ int run_jobs_fisher(mars_ctx* ctx, Scratch& sc, const uint8_t* d_plane, uint32_t
     const bool fork = d_rc_in && jobs.size() > 1;
     const int nb = fork ? (int)std::min<size_t>(jobs.size(), mars_ctx::kBranches) : 0;
     if (fork) {
-        if (int e = make_branches(ctx)) return e;
+        if (int e = make_branches(ctx, nb)) return e;
         MARS_CUDA(cudaEventRecord(ctx->fork_ev, st));
         for (int b = 0; b < nb; ++b) MARS_CUDA(cudaStreamWaitEvent(ctx->branch[b], ctx->fork_ev, 0));
     }
@@ -2043,7 +2056,8 @@ int run_jobs_branched(mars_ctx* ctx, Scratch& sc, const uint8_t* d_plane, uint32
                       const mars::FitParams& fp, const std::vector<Job>& jobs,
                       mars::CandidateOut* d_out, const uint32_t* d_rc, uint32_t k) {
     const cudaStream_t main = ctx->stream;
-    if (int e = make_branches(ctx)) return e;
+    const int nb = (int)std::min<size_t>(jobs.size(), mars_ctx::kBranches);
+    if (int e = make_branches(ctx, nb)) return e;
     int32_t* d_D = nullptr;
     MARS_CUDA(sc.get(&d_D, std::max<size_t>(1, (size_t)(w / 2) * (h / 2))));
     MARS_CUDA(mars::launch_contract(d_plane, (int)w, (int)h, d_D, main));
@@ -2051,7 +2065,6 @@ int run_jobs_branched(mars_ctx* ctx, Scratch& sc, const uint8_t* d_plane, uint32
     size_t total = 0;
     for (const Job& j : jobs) total += j.rows.size();
     MARS_CUDA(cudaEventRecord(ctx->fork_ev, main));
-    const int nb = (int)std::min<size_t>(jobs.size(), mars_ctx::kBranches);
     for (int b = 0; b < nb; ++b) MARS_CUDA(cudaStreamWaitEvent(ctx->branch[b], ctx->fork_ev, 0));
     size_t off = 0;
     int err = MARS_OK;
