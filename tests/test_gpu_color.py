@@ -1,5 +1,7 @@
 """The colour input and metric kernels (color.cu) against the oracle, bit-exact, and the
 colour encode/decode pipeline (color.rs:400-528 without regions) end to end."""
+import time
+
 import numpy as np
 import pytest
 
@@ -106,6 +108,34 @@ def test_planes_at_any_address(ctx, shape, offset):
     want = orc.upsample_nearest(want, w, h)
     assert np.array_equal(taken(up, shape), want)
     assert mse.value == orc.mse(host[0], want)
+
+
+@pytest.mark.parametrize("inverse", [False, True])
+def test_conversion_at_odd_addresses_in_time(ctx, inverse):
+    # A 4K frame whose planes start one byte off: 2.2 times as long as a byte a thread was, and
+    # 3.2 times the aligned time, before four bytes shared a conversion.
+    torch = pytest.importorskip("torch")
+    n = 3840 * 2160
+    bufs = [torch.randint(0, 256, (n + 16,), dtype=torch.uint8, device="cuda:0") for _ in range(6)]
+    call = mb.lib().mars_rgb_from_ycbcr_device if inverse else mb.lib().mars_ycbcr_device
+    times, outs = [], []
+    for off in (0, 1):
+        if off:
+            for b in bufs[:3]:
+                b[1:] = b[:-1].clone()
+        at = [b.data_ptr() + off for b in bufs]
+        best = float("inf")
+        for _ in range(5):
+            torch.cuda.synchronize()
+            t = time.perf_counter()
+            for _ in range(100):
+                mb.check(call(ctx.handle, *at[:3], n, *at[3:]))
+            torch.cuda.synchronize()
+            best = min(best, time.perf_counter() - t)
+        times.append(best)
+        outs.append([b[off: n + off].clone() for b in bufs[3:]])
+    assert all(torch.equal(x, y) for x, y in zip(*outs))
+    assert times[1] < 2.5 * times[0]
 
 
 @pytest.mark.parametrize("n", [1, 15, 16, 17, 4096, 1 << 20, (1 << 20) + 3])
