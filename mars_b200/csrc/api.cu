@@ -469,7 +469,8 @@ struct TcLevel {
 constexpr size_t kDomainTmpWords = 64ull << 20;
 
 // The unit form's A operand holds every domain window (32 or 128 bytes a position at sizes 4 and
-// 8; the survivors' samples take as many again), up to this many bytes a level: planes to about 11,500 pixels a side at size 8, stride 2.
+// 8; the survivors' samples take as many again), up to this many bytes a level: planes to about
+// 11,500 pixels a side at size 8, stride 2.
 // Beyond it the fold reads the windows from copies of the plane.
 constexpr size_t kUnitBytes = 4ull << 30;
 // Its work items cost 25,000 cycles to set up, preview and drain, the fold's about 6,000, and its
@@ -894,10 +895,10 @@ int run_jobs(mars_ctx* ctx, Scratch& sc, const uint8_t* d_plane, uint32_t w, uin
     return MARS_OK;
 }
 
-// Whether the exhaustive single-candidate search of `jobs` runs its tensor-core levels as
-// one all-levels persistent launch: not pinned off (mars_ctx_set_search_path 5 or the
+// Whether the exhaustive single-candidate search of `jobs` runs its tensor-core levels in the
+// all-levels persistent launches: not pinned off (mars_ctx_set_search_path 5 or the
 // MARS_LEVEL_LAUNCH=per_level environment variable), every tensor-core level a kind the
-// kernel holds, at most kMaxLevelJobs of them.
+// kernels hold, at most kMaxLevelJobs of them.
 bool all_levels_eligible(const mars_ctx* ctx, uint32_t w, uint32_t h, const std::vector<Job>& jobs) {
     static const bool env_per_level = [] {
         const char* e = std::getenv("MARS_LEVEL_LAUNCH");
@@ -931,10 +932,10 @@ int make_branches(mars_ctx* ctx, int n) {
 }
 
 // run_jobs for the exhaustive single-candidate search with the correlation of every
-// tensor-core level in one persistent launch (launch_corr_all, which also writes the
-// levels' final candidates).  Every buffer is taken on the context's stream before the
+// tensor-core level in two persistent launches, of the unit form's levels and of the others
+// (launch_corr_all; they also write the levels' final candidates).  Every buffer is taken on the context's stream before the
 // fork; each level's statistics, operands and seeds (and every other level, whole) then
-// run on one of the branch streams; the persistent launch follows the join.  The caller
+// run on one of the branch streams; the persistent launches follow the join.  The caller
 // holds ctx->mu and has checked all_levels_eligible.
 int run_jobs_all_levels(mars_ctx* ctx, Scratch& sc, const uint8_t* d_plane, uint32_t w,
                         uint32_t h, const mars::FitParams& fp, const std::vector<Job>& jobs,
@@ -2537,8 +2538,8 @@ int plan_encode_device(mars_search_plan* plan, mars_search_plan* warm_plan, cons
     const double t_rms = prm.has_lambda ? 8.0 : prm.t_rms;
     if (warm_plan) wp.evals = warm_plan->walk.evals;
     else if (d_evals) wp.evals = d_evals;
-    MARS_CUDA(mars::launch_warm_walk(wp, warm_plan ? d_wcands : d_cands, sizeof(mars_candidate), t_rms, prm.min_size,
-                                     prm.zero_threshold, hdr.bits_beta, ws, d_warm, st));
+    MARS_CUDA(mars::launch_warm_walk(wp, warm_plan ? d_wcands : d_cands, sizeof(mars_candidate),
+                                     t_rms, prm.min_size, prm.zero_threshold, hdr.bits_beta, ws, d_warm, st));
     ctx->launches += 2 * w.nlevels + 1;
     unsigned long long tot[2];
     MARS_CUDA(cudaMemcpyAsync(tot, ws.totals, sizeof tot, cudaMemcpyDeviceToHost, st));

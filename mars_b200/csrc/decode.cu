@@ -15,11 +15,13 @@
 //
 // decode_cell_kernel (lg >= 2, width % 4 == 0): one thread per 4x4 output cell.  A cell lies
 // in one leaf, and the inverse isometry maps it onto a 4x4 set of domain samples, i.e. one
-// 8x8 byte window of the previous iterate: the thread reads it as eight 8-byte rows, forms
+// 8x8 byte window of the previous iterate: the thread takes its eight rows from aligned 16-byte
+// loads (and 8 bytes more where a row reaches past them) that are in flight together, forms
 // the sixteen 2x2 sums with byte-pair SIMD adds in 16-bit lanes, evaluates the sixteen
-// values in sample order, moves them to output order with byte permutes (row reversal,
-// byte reversal, 4x4 transpose) and stores four 4-byte rows.  decode_pixel_kernel covers
-// any other geometry.
+// values in sample order (in integers where the leaf allows it, else in f64), moves them to
+// output order with byte permutes (row reversal, byte reversal, 4x4 transpose) and stores four
+// 4-byte rows.  decode_pixel_kernel covers any other geometry; decode_resident_kernel runs every
+// step of a small plane in one launch, the sorted_* kernels a step of a large one.
 #include "grid_meet.cuh"
 #include "kernels.cuh"
 

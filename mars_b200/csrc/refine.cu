@@ -361,9 +361,9 @@ __global__ void __launch_bounds__(kBlock) refine_adjoint_kernel(
 // is written once, at the end.  The values are refine_adjoint_kernel's but for the order of the
 // sums: lists are skewed (one of a smooth plane's domains may serve hundreds of leaves), so what
 // lists have past their first entries is cut into runs of 32, which the block's warps share (a
-// thread a list: 595 and 789 us where this takes 265 and 304).  Bound: the barrier's and the loads' round trips to L2.  One B200:
-// 24 steps of 512 x 512 with the gradients and the host's part 211 to 304 us, 374 to 1,087 as
-// launches of a thread a pixel.
+// thread a list: 595 and 789 us where this takes 265 and 304).  Bound: the barrier's and the loads'
+// round trips to L2.  One B200: 24 steps of 512 x 512 with the gradients and the host's part 211 to
+// 304 us, 374 to 1,087 as launches of a thread a pixel.
 
 struct AdjointArgs {
     float *lam, *mu, *mun;

@@ -38,8 +38,8 @@
 //
 // One body (process_item) serves three kernels: corr_tc_kernel<S, DIG, false>, one level
 // per launch (CTA = range tile x domain-tile split); corr_tc_kernel<S, DIG, true>, the
-// ranked search keeping each range's best k; and corr_tc_all_kernel, every tensor-core
-// level of a plane in one persistent launch over (level, range tile, split) work items.
+// ranked search keeping each range's best k; and corr_tc_all_kernel, every level of a
+// plane that is not in the unit form (search_unit.cuh) in one persistent launch over (level, range tile, split) work items.
 #include <cuda.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -1120,7 +1120,7 @@ __device__ __forceinline__ int iso_src_rt(int k, int u, int v, int S) {
 
 #include "search_unit.cuh"
 
-// All tensor-core levels of a plane in one persistent launch: one CTA per SM takes work
+// All of a plane's levels but the unit form's in one persistent launch: one CTA per SM takes work
 // items -- (level job, range tile, domain-tile split) -- from a global counter until none
 // are left.  TMEM, the mbarriers and the epilogue's queues are set up once per CTA; the
 // pipelines' phases carry over from item to item (PipeState).  Jobs are ordered by item

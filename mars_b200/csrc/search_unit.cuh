@@ -17,8 +17,8 @@
 // factor 64 keeps what a flushed subnormal could add below 2^-17), so rho is off by at most
 // 2^-10 + 2^-22 from the operands and, |products| summing to at most 1, by less than 2^-14 from
 // f32 accumulation, 0.00104 together; thresholds are lowered by 4.5 / 4096 = 0.0011.  (2^-9 let
-// twice as many pass where a step edge meets many like it.)  What passes is evaluated again from the
-// integers: the exact correlation, the full bound of fit.cuh with the largest contrast added,
+// twice as many pass where a step edge meets many like it.)  What passes is evaluated again from
+// the integers: the exact correlation, the full bound of fit.cuh with the largest contrast added,
 // then the f64 fit.  So the winners, their rms bits and the tie order are the integer path's.
 //
 // Ranges whose champion is no better than the flat fit have no such number: a candidate of
@@ -77,7 +77,7 @@ constexpr int kGroup = 8;                                  // tiles that share t
 constexpr int kSets = 32;                                  // sets of thresholds in use
 constexpr float kUnitScale = 4096.0f;                      // 64 x 64
 constexpr float kUnitSlack = 4.5f;                         // the filter's allowance
-constexpr float kUnitLeast = kUnitScale / 64.0f;           // tiles' thresholds below take the full form
+constexpr float kUnitLeast = kUnitScale / 64.0f;           // a tile's threshold below: full form
 constexpr float kUnitAlike = 1.1f;                         // the contrasts of tiles that are alike
 constexpr float kUnitNone = 1e-30f;                        // a champion's W gives no threshold
 
@@ -197,8 +197,8 @@ __device__ __forceinline__ bool unit_better(USmem& sm, int rl, double rms, uint3
     return s0 != s1 || (s0 & 1u) || rms < r || (rms == r && idx < i);
 }
 
-// One lane of a warp at a time: replaces range rl's champion by (rms, sum, idx, t1) if that is better, under the range's
-// lock (bounded: a holder only does arithmetic).  True when it was replaced.
+// One lane of a warp at a time: replaces range rl's champion by (rms, sum, idx, t1) if that is
+// better, under the range's lock (bounded: a holder only does arithmetic).  True when it was replaced.
 __device__ bool unit_replace(USmem& sm, int rl, const FitParams& fp, int n, double rms, double sum,
                              uint32_t idx, int32_t t1, int* err) {
     for (int spin = 0; spin < (1 << 22); ++spin) {
@@ -240,8 +240,8 @@ __device__ __forceinline__ float4 lds_f4(const void* p) {
 // isometries: 16 samples of the window at a time, in pairs of 16 bits (they are at most 1020),
 // against the range's permuted bytes.  The windows lie beside the A operand in its order, so 16
 // bytes a load, and those of the neighbouring domains that survive together share lines.  (Sample
-// by sample from the contracted plane, 64 loads of as many lines at S = 8, a 1024 x 1024 ramp, whose
-// blocks all match, took 31.7 ms at stride 8; 26.1 so, the integer form 25.2.)  Compact on purpose:
+// by sample from the contracted plane, 64 loads of as many lines at S = 8, a 1024 x 1024 ramp,
+// whose blocks all match, took 31.7 ms at stride 8; 26.1 so, the integer form 25.2.)  Compact on purpose:
 // this code runs rarely, and what a cold instruction costs to fetch exceeds what it computes.
 template <int S>
 __device__ __forceinline__ void unit_correlate(const ItemArgs& a, const uint8_t* pix, bool act,
@@ -560,9 +560,9 @@ __device__ __noinline__ uint32_t unit_look_full(const ItemArgs& a, USmem& sm, ui
 // ihi their reciprocals): the smallest rho that a fit with a contrast in a_min..a_max needs
 // there, in accumulator units.  It is u = sqrt(W / Nrr) where the best contrast
 // sqrt(W) / sqrt(Ndd) is allowed, and grows away from there, so the tile's end nearest to that
-// counts; with W <= 0 it grows with the contrast.  rr: the range's record (sqrt W, W / (2 a_min)), inv: 1 / sqrt(Nrr).  The steps'
-// rounding, and reciprocals good to a few units in the last place, stay far below the 1e-5
-// taken off.
+// counts; with W <= 0 it grows with the contrast.  rr: the range's record (sqrt W, W / (2 a_min)),
+// inv: 1 / sqrt(Nrr).  The steps' rounding, and reciprocals good to a few units in the last place,
+// stay far below the 1e-5 taken off.
 __device__ __forceinline__ float unit_tile_threshold(const float4& rr, float u, float inv, float lo,
                                                      float hi, float ilo, float ihi,
                                                      const FitParams& fp) {
@@ -1148,8 +1148,8 @@ __global__ void __launch_bounds__(256) unit_a_kernel(const int32_t* __restrict__
     out[t] = pk;
 }
 
-// B operand of one level, in contrast order: per range a row group of its 8 isometries, KG k-groups x (8 rows x
-// 16 B); a tile is 32 ranges.  One thread per (row, k-group); zero rows for flat blocks, blocks
+// B operand of one level, in contrast order: per range a row group of its 8 isometries, KG k-groups
+// x (8 rows x 16 B); a tile is 32 ranges.  One thread per (row, k-group); zero rows for flat blocks, blocks
 // outside the plane and padding.
 template <int S>
 __global__ void __launch_bounds__(256) unit_b_kernel(const uint8_t* __restrict__ plane, int w, int h,
@@ -1325,8 +1325,8 @@ __device__ __forceinline__ void unit_teardown(uint32_t tmem, unsigned long long 
     }
 }
 
-// Every unit level of a plane, or one level alone, in one persistent launch: the work items of corr_tc_all_kernel
-// (level job, range tile, split), taken from a counter by one CTA per SM.
+// Every unit level of a plane, or one level alone, in one persistent launch: the work items of
+// corr_tc_all_kernel (level job, range tile, split), taken from a counter by one CTA per SM.
 struct UnitLevels {
     ItemArgs args[kMaxLevelJobs];
     int size[kMaxLevelJobs];
