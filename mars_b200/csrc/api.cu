@@ -532,24 +532,33 @@ int tc_level_setup(mars_ctx* ctx, Scratch& sc, uint32_t w, uint32_t h, size_t n,
     return MARS_OK;
 }
 
+// Whether a level's domain statistics run on its second stream.  Not where the seeds' kernel, with
+// fewer blocks than SMs, would then run beside B's and be crowded on the SMs that this one leaves:
+// the 64 x 64 blocks of a 512 x 512 plane, stride 8, took 369 us so, 210 with the statistics on one
+// stream and the planes and B beside them.  (The unit form's A operand needs them there.)
+bool domains_apart(const mars_ctx* ctx, const TcLevel& L) {
+    return L.path == mars::tc::kUnit || L.n >= (size_t)ctx->num_sms;
+}
+
 // A level's statistics: the ranges' on stream st, the domains' on sp (the same stream, or a second
-// one: `stats_done` is then recorded).
+// one: `stats_done` is then recorded) where domains_apart.
 int tc_level_stats(mars_ctx* ctx, const TcLevel& L, const uint8_t* d_plane, const int32_t* d_D,
                    uint32_t w, uint32_t h, const mars::FitParams& fp, const uint32_t* d_rows,
                    const uint32_t* d_cols, cudaStream_t st, cudaStream_t sp,
                    cudaEvent_t stats_done) {
-    MARS_CUDA(mars::launch_domain_stats(d_D, L.g, L.ds, sp, L.dtmp));
-    if (sp != st) MARS_CUDA(cudaEventRecord(stats_done, sp));
+    const bool apart = sp != st && domains_apart(ctx, L);
     MARS_CUDA(mars::launch_range_stats(d_plane, (int)w, (int)h, d_rows, d_cols, (int)L.n, L.g.size,
                                        fp, L.rs, st));
+    MARS_CUDA(mars::launch_domain_stats(d_D, L.g, L.ds, apart ? sp : st, L.dtmp));
+    if (apart) MARS_CUDA(cudaEventRecord(stats_done, sp));
     ctx->launches += 2;
     return MARS_OK;
 }
 
 // The rest of a level before its correlation: the A operand (planes or unit vectors), the B
 // operand, seed champions, the shared champion records and tickets.  Range-side work and the
-// seeds run on stream st, domain-side work on sp, as the statistics (`stats_done` orders the seeds
-// after the domains').
+// seeds run on stream st, the operands' (the unit form's B aside) on sp (`stats_done` orders the
+// seeds after the domains' statistics).
 int tc_level_prep(mars_ctx* ctx, TcLevel& L, const uint8_t* d_plane, const int32_t* d_D,
                   const uint8_t* d_dplane, uint32_t w, uint32_t h, const mars::FitParams& fp,
                   const uint32_t* d_rows, const uint32_t* d_cols, cudaStream_t st, cudaStream_t sp,
@@ -579,7 +588,7 @@ int tc_level_prep(mars_ctx* ctx, TcLevel& L, const uint8_t* d_plane, const int32
         const int rt = mars::tc::ranges_per_tile(L.path);
         MARS_CUDA(cudaMemsetAsync(L.tickets, 0, (L.n + rt - 1) / rt * sizeof(int), st));
     }
-    if (sp != st) MARS_CUDA(cudaStreamWaitEvent(st, stats_done, 0));
+    if (sp != st && domains_apart(ctx, L)) MARS_CUDA(cudaStreamWaitEvent(st, stats_done, 0));
     MARS_CUDA(mars::tc::launch_seed(d_D, g, d_plane, (int)w, d_rows, d_cols, n, L.rs, L.ds, fp,
                                     L.d_seed, st));
     ctx->launches += 3;
