@@ -259,12 +259,24 @@ __global__ void decode_pixel_kernel(const uint8_t* __restrict__ src, uint8_t* __
     const int32_t li = owner[(size_t)(y >> lg) * mw + (x >> lg)];
     uint32_t out = 0;
     if (li >= 0) {
-        const DecodeMap m = maps[li];
+        // The f64 form throughout: a pixel has little arithmetic, and a map's integer form is 16
+        // bytes more to load (ten steps of 6002 x 6000: 2,258 us with it, 2,221 without).
+        DecodeMap m;
+        const uint4 head = *reinterpret_cast<const uint4*>(&maps[li].rc);
+        const double2 ab = *reinterpret_cast<const double2*>(&maps[li].a);
+        m.rc = head.x;
+        m.info = head.y & ~kLeafInteger;
+        m.dom = head.z;
+        m.roff = (int32_t)head.w;
+        m.a = ab.x;
+        m.b = ab.y;
         const uint32_t kind = (m.info >> 12) & 3u;
         const int i = y - (int)(m.rc & 0xFFFFu), j = x - (int)(m.rc >> 16);
         if (kind == kLeafConst) {
             out = m.info >> 24;
         } else if (kind == kLeafAffine) {
+            m.gx = maps[li].gx;
+            m.gy = maps[li].gy;
             out = affine_pixel(m, i, j);
         } else {
             const int S = (int)(m.info & 0xFFFu);
@@ -275,13 +287,9 @@ __global__ void decode_pixel_kernel(const uint8_t* __restrict__ src, uint8_t* __
                 const size_t p = ((size_t)(m.dom & 0xFFFFu) + 2 * u) * w + (m.dom >> 16) + 2 * v;
                 sum = (int)src[p] + (int)src[p + w] + (int)src[p + 1] + (int)src[p + w + 1];
             }
-            if (m.info & kLeafInteger) {
-                out = sixty_fourths((int)(int16_t)m.n0 + m.n1 * sum);
-            } else {
-                double value = domain_value(sum, m);
-                if (kind == kLeafResidual) value = __dadd_rn(value, resid[m.roff + u * S + v]);
-                out = to_u8(value);
-            }
+            double value = domain_value(sum, m);
+            if (kind == kLeafResidual) value = __dadd_rn(value, resid[m.roff + u * S + v]);
+            out = to_u8(value);
         }
     }
     dst[(size_t)y * w + x] = (uint8_t)out;
