@@ -3055,12 +3055,11 @@ namespace {
 // `steps` steps, a and b in turn, the first from a and the last into d_out.
 int enqueue_decode_steps(mars_decode_plan* p, uint32_t steps, uint8_t* a, uint8_t* b,
                          uint8_t* d_out, cudaStream_t st) {
-    // The source-ordered steps store words; into an output that starts between two, the plain
-    // steps go byte by byte.
-    const bool sorted = p->d_jobs && mars::decode_sorted_aligned(d_out);
     for (; steps > 0; --steps) {
         if (steps == 1) b = d_out;
-        if (sorted)
+        // The source-ordered steps store words; into an output that starts between two, the plain
+        // step goes byte by byte.
+        if (p->d_jobs && mars::decode_sorted_aligned(b))
             MARS_CUDA(mars::launch_decode_sorted_step(a, b, (int)p->w, (int)p->h, p->lg, p->d_owner,
                                                       p->d_maps, p->d_jobs, p->njobs, p->wide_jobs,
                                                       p->d_inv, p->consts, p->d_cellbuf, st));
@@ -3081,6 +3080,7 @@ int enqueue_decode_steps(mars_decode_plan* p, uint32_t steps, uint8_t* a, uint8_
 // output or two by turns 35 and 35, ten and twelve steps by turns 38; launched step by step 59.
 // Null where there is none.
 constexpr uint32_t kGraphSteps = 64;  // at most
+constexpr size_t kOwnPixels = 256 * 256;
 
 cudaGraphExec_t decode_graph(mars_decode_plan* p, uint32_t steps, uint8_t* d_out) {
     if (steps < 2 || steps > kGraphSteps || !mars::decode_output_aligned(d_out)) return nullptr;
@@ -3138,8 +3138,8 @@ int mars_decode_plan_run(mars_decode_plan* p, uint32_t iterations, uint8_t* d_ou
     mars_ctx* ctx = p->ctx;
     std::lock_guard<std::mutex> lock(ctx->mu);
     MARS_CUDA(cudaSetDevice(ctx->device));
-    ctx->launches +=
-        (uint64_t)iterations * (p->d_jobs && mars::decode_sorted_aligned(d_out) ? 2 : 1);
+    ctx->launches += (uint64_t)iterations * (p->d_jobs ? 2 : 1) -
+                     (iterations && p->d_jobs && !mars::decode_sorted_aligned(d_out) ? 1 : 0);
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(ctx->stream, &capturing) != cudaSuccess) {
         cudaGetLastError();
@@ -3151,9 +3151,12 @@ int mars_decode_plan_run(mars_decode_plan* p, uint32_t iterations, uint8_t* d_ou
             MARS_CUDA(cudaGraphLaunch(x, ctx->stream));
             return MARS_OK;
         }
-    // Ping-pong so that the last iteration lands in d_out.
-    uint8_t* a = (iterations & 1) ? p->d_tmp : d_out;
-    uint8_t* b = (iterations & 1) ? d_out : p->d_tmp;
+    // Ping-pong so that the last iteration lands in d_out; an output that the cell and the sorted
+    // steps do not take is the last step's alone (2048 x 2048 at an odd address, ten steps: 139 us,
+    // 330 with every other step there; of 64 x 64 the cell steps are the slower ones, 53 and 43).
+    const bool own = iterations > 1 && px >= kOwnPixels && !mars::decode_output_aligned(d_out);
+    uint8_t* a = own || (iterations & 1) ? p->d_tmp : d_out;
+    uint8_t* b = own ? p->d_tmp2 : ((iterations & 1) ? d_out : p->d_tmp);
     MARS_CUDA(cudaMemsetAsync(a, 128, px, ctx->stream));
     return enqueue_decode_steps(p, iterations, a, b, d_out, ctx->stream);
 }

@@ -1,5 +1,7 @@
 """Parity of the decode gather (mars_decode, mars_decode_plan_*) against the oracle's
 decode_iterative (crates/mars-codec/src/ifs.rs:281-309, 406-484), bit-exact."""
+import time
+
 import numpy as np
 import pytest
 
@@ -379,4 +381,26 @@ def test_plan_runs_of_every_count(ctx, monkeypatch, w, h, min_size, wide):
             assert np.array_equal(out.reshape(h, w), want), (n, k)
             got[starts[k]: starts[k] + w * h] = 7
             assert (got == 7).all()  # nothing beside the output
+    plan.close()
+
+
+def test_runs_into_odd_addresses_in_time(ctx):
+    # Only the last step stores there.  (With every other one, one pixel a thread, 2.9 times the
+    # aligned time.)
+    torch = pytest.importorskip("torch")
+    w = h = 1280
+    plan = ctx.decode_plan(_hdr(w, h), synthetic.quadtree_leaves(w, h, 5, min_size=4))
+    out = torch.zeros(w * h + 8, dtype=torch.uint8, device="cuda:0")
+    times = []
+    for at in (0, 1):
+        best = float("inf")
+        for _ in range(5):
+            torch.cuda.synchronize()
+            t = time.perf_counter()
+            for _ in range(50):
+                plan.run(10, out.data_ptr() + at)
+            torch.cuda.synchronize()
+            best = min(best, time.perf_counter() - t)
+        times.append(best)
+    assert times[1] < 2.3 * times[0]
     plan.close()
