@@ -2918,13 +2918,15 @@ int mars_decode(mars_ctx* ctx, const mars_header* hdr, const mars_leaf* leaves, 
                                              ctx->stream));
         ctx->launches += 1;
     }
-    uint32_t* d_sync = nullptr;
-    MARS_CUDA(sc.get(&d_sync, 2));
-    MARS_CUDA(cudaMemsetAsync(d_sync, 0, 2 * sizeof(uint32_t), ctx->stream));
     bool resident = false;
-    MARS_CUDA(mars::launch_decode_resident(a, b, (int)w, (int)h, lg, d_owner, d_maps, d_rvals,
-                                           iterations, d_sync, nullptr, 0, nullptr, ctx->d_err,
-                                           ctx->num_sms, ctx->stream, &resident));
+    if (mars::decode_resident_fits(a, b, (int)w, (int)h, lg, iterations, ctx->num_sms)) {
+        uint32_t* d_sync = nullptr;
+        MARS_CUDA(sc.get(&d_sync, 2));
+        MARS_CUDA(cudaMemsetAsync(d_sync, 0, 2 * sizeof(uint32_t), ctx->stream));
+        MARS_CUDA(mars::launch_decode_resident(a, b, (int)w, (int)h, lg, d_owner, d_maps, d_rvals,
+                                               iterations, d_sync, nullptr, 0, nullptr, ctx->d_err,
+                                               ctx->num_sms, ctx->stream, &resident));
+    }
     if (resident) {
         ctx->launches += 1;
         if (iterations & 1) std::swap(a, b);

@@ -260,7 +260,7 @@ __global__ void decode_pixel_kernel(const uint8_t* __restrict__ src, uint8_t* __
     uint32_t out = 0;
     if (li >= 0) {
         // The f64 form throughout: a pixel has little arithmetic, and a map's integer form is 16
-        // bytes more to load (ten steps of 6002 x 6000: 2,258 us with it, 2,221 without).
+        // bytes more to load (ten steps of 6002 x 6000: 2,258 us with it, 2,223 without).
         DecodeMap m;
         const uint4 head = *reinterpret_cast<const uint4*>(&maps[li].rc);
         const double2 ab = *reinterpret_cast<const double2*>(&maps[li].a);
@@ -871,23 +871,32 @@ cudaError_t decode_set_output(cudaGraphExec_t exec, cudaGraphNode_t last, bool s
     return cudaGraphExecKernelNodeSetParams(exec, last, &k);
 }
 
+static size_t resident_blocks(int w, int h) {
+    return (decode_sorted_cells(w, h) + kResidentThreads - 1) / kResidentThreads;
+}
+
+// Every block must be resident at once, and the counter must not reach its top bit.  Up to four
+// blocks an SM (1.2 Mpixel): ten steps of 1024 x 1024 take 48 us here and 66 as launches, but of
+// 1280 x 1280, 800 blocks polling one counter, 150 against 99.
+bool decode_resident_fits(const uint8_t* buf0, const uint8_t* buf1, int w, int h, int lg,
+                          uint32_t iters, int num_sms) {
+    const bool aligned =
+        ((reinterpret_cast<uintptr_t>(buf0) | reinterpret_cast<uintptr_t>(buf1)) & 7) == 0;
+    const size_t blocks = resident_blocks(w, h);
+    return lg >= 2 && w % 4 == 0 && aligned && iters > 0 && blocks <= (size_t)num_sms * 4 &&
+           (uint64_t)blocks * iters < (1ull << 31);
+}
+
 cudaError_t launch_decode_resident(uint8_t* buf0, uint8_t* buf1, int w, int h, int lg,
                                    const int32_t* owner, const DecodeMap* maps,
                                    const double* resid, uint32_t iters, uint32_t* sync, int* delta,
                                    int threshold, int* state, int* err, int num_sms,
                                    cudaStream_t st, bool* taken) {
     *taken = false;
-    const bool aligned =
-        ((reinterpret_cast<uintptr_t>(buf0) | reinterpret_cast<uintptr_t>(buf1)) & 7) == 0;
-    if (lg < 2 || w % 4 != 0 || !aligned || iters == 0) return cudaSuccess;
-    const size_t cells = decode_sorted_cells(w, h);
+    if (!decode_resident_fits(buf0, buf1, w, h, lg, iters, num_sms)) return cudaSuccess;
+    const size_t blocks = resident_blocks(w, h);
     ResidentArgs g{buf0, buf1, w, h, lg, (w + (1 << lg) - 1) >> lg, owner, maps, resid, iters,
                    sync, delta, threshold, state, err};
-    const size_t blocks = (cells + kResidentThreads - 1) / kResidentThreads;
-    // Every block must be resident at once, and the counter must not reach its top bit.  Up to
-    // four blocks an SM (1.2 Mpixel): ten steps of 1024 x 1024 take 48 us here and 66 as launches,
-    // but of 1280 x 1280, 800 blocks polling one counter, 150 against 99.
-    if (blocks > (size_t)num_sms * 4 || (uint64_t)blocks * iters >= (1ull << 31)) return cudaSuccess;
     const void* kernel = delta ? (const void*)decode_resident_kernel<true>
                                : (const void*)decode_resident_kernel<false>;
     int per_sm = 0;

@@ -218,10 +218,12 @@ bool decode_output_aligned(const uint8_t* out);
 cudaError_t decode_set_output(cudaGraphExec_t exec, cudaGraphNode_t last, bool sorted, uint8_t* out);
 
 // The steps of a decode as one cooperative launch whose threads each keep one 4x4 cell
-// (decode_resident_kernel): *taken says whether the plane was small enough; nothing is launched
-// otherwise.  The first step reads 128 everywhere, whatever buf0 holds.  sync: two words, zero
+// (decode_resident_kernel): *taken says whether all can be resident; nothing is launched
+// otherwise, nor where decode_resident_fits says no.  The first step reads 128 everywhere, whatever buf0 holds.  sync: two words, zero
 // before the launch and left zero.  With delta (iters words, zero), the steps end as
 // launch_decode_step_stable's do, state[0] and state[1] being done and used.
+bool decode_resident_fits(const uint8_t* buf0, const uint8_t* buf1, int w, int h, int lg,
+                          uint32_t iters, int num_sms);
 cudaError_t launch_decode_resident(uint8_t* buf0, uint8_t* buf1, int w, int h, int lg,
                                    const int32_t* owner, const DecodeMap* maps,
                                    const double* resid, uint32_t iters, uint32_t* sync, int* delta,
