@@ -2702,6 +2702,12 @@ struct DecodeLists {
     mars::DecodeConsts consts;
 };
 
+// Residual lists of fewer levels than this are made on the host: one of 1,488 (130 x 96) takes 113 us
+// a one-shot decode either way alone, but the device's values wait for other calls' (four threads, a
+// context each: 61 us with the host's, 80 with the device's); one of 6,320 (256 x 256) takes 243 and
+// 150.
+constexpr size_t kHostResiduals = 2048;
+
 // Leaf table and owner map of one leaf list, validated on the host so that every read and
 // write the gather kernel makes stays inside the plane.  Leaves are packed into 16 bytes
 // (the layout is documented beside DecodeLeaf), which bounds plane sides to 65535, leaf
@@ -2712,7 +2718,8 @@ struct DecodeLists {
 // Mode-3 residuals are rebuilt exactly as decode_leaf does (ifs.rs:441-456) in domain-local
 // (u, v) order, their offsets returned per leaf: on the device over a basis made here
 // (upload_residuals; the basis is the C library's cosine, as the reference's is), or here for
-// lists with a mode-3 leaf wider than kResidualMost (resid_values is then not empty).
+// lists with a mode-3 leaf wider than kResidualMost or of fewer levels than kHostResiduals
+// (resid_values is then not empty).
 int prepare_decode(const mars_header* hdr, const mars_leaf* leaves, size_t n,
                    const int32_t* residuals, size_t nresiduals, DecodeLists* lists) {
     std::vector<mars::DecodeLeaf>* const dl = &lists->dl;
@@ -2769,7 +2776,7 @@ int prepare_decode(const mars_header* hdr, const mars_leaf* leaves, size_t n,
             (*resid_off)[k] = (int32_t)offs[k];
             most = std::max(most, leaves[k].size);
         }
-        if (most > mars::kResidualMost) {
+        if (most > mars::kResidualMost || nresiduals < kHostResiduals) {
             const double step = mars::codec::qstep_of(*hdr);
             resid_values->resize(nresiduals);
             for (size_t k = 0; k < n; ++k) {
