@@ -65,6 +65,7 @@ struct CallStreams {
     int* words = nullptr;
     size_t given = 0;  // words given out
     std::vector<std::pair<cudaStream_t, int*>> idle;
+    std::atomic<int> fisher{0};  // planned Fisher encodes in flight
 
     static cudaError_t join(int device, CallStreams** out) {
         static std::mutex all_mu;
@@ -1864,8 +1865,15 @@ int plan_encode_device(mars_search_plan* plan, mars_search_plan* warm_plan, cons
                        const mars_options* o, mars_header* header, mars_leaf** leaves,
                        size_t* nleaves, int32_t** residuals, size_t* nresiduals,
                        mars_counters* counters);
+struct FisherInFlight {
+    std::atomic<int>& count;
+    const bool alone;
+    explicit FisherInFlight(std::atomic<int>& c) : count(c), alone(c.fetch_add(1) == 0) {}
+    ~FisherInFlight() { count.fetch_sub(1); }
+};
+
 int fisher_walk_on_device(mars_search_plan* fplan, mars_search_plan* wplan, const mars_options* o,
-                          bool* usable);
+                          bool alone, bool* usable);
 
 // The plan mars_encode uses for a plane geometry it has encoded before: one search plan
 // per (width, height, params), made on the second encode of that geometry (the first takes
@@ -1945,8 +1953,10 @@ int mars_encode(mars_ctx* ctx, const uint8_t* plane, uint32_t width, uint32_t he
         mars_search_plan* wplan =
             params->has_lambda ? cached_encode_plan(ctx, width, height, &wp) : nullptr;
         if (fplan && (!params->has_lambda || wplan)) {
+            const FisherInFlight in_flight(ctx->calls->fisher);
             bool device_walk = false;
-            if (int e = fisher_walk_on_device(fplan, wplan, options, &device_walk)) return e;
+            if (int e = fisher_walk_on_device(fplan, wplan, options, in_flight.alone, &device_walk))
+                return e;
             if (device_walk)
                 return plan_encode_device(fplan, wplan, plane, options, header, leaves, nleaves,
                                           residuals, nresiduals, counters);
@@ -2431,14 +2441,19 @@ bool plan_walk_on_host() {
 // host's over a downloaded table costs less than the device's launches and waits up to
 // kHostWalkNodes (device and host, threshold walk and RD, sizes 4..16 at stride 4 on one B200:
 // 630 nodes 304 and 271 us, 654 and 576; 1,575 nodes 340 and 333, 872 and 830; 4,032 nodes 394 and
-// 433, 1,159 and 1,282).  With residuals every node is priced there anyway (630 nodes: 702 and 824).
+// 433, 1,159 and 1,282).  Nor does it pay beside other such encodes, whose host walks run on cores
+// of their own where the device's wait for one another (four contexts on four threads, us an encode
+// with the device's walks and the host's: 256 x 192 270 and 136, 512 x 512 669 and 473; RD 774 and
+// 473, 3,128 and 2,708; alone 386 and 409, 803 and 1,042; 1,262 and 1,154, 3,812 and 4,591).  With
+// residuals every node is priced on the device anyway (630 nodes: 702 and 824).
 constexpr size_t kHostWalkNodes = 2048;
 
 int fisher_walk_on_device(mars_search_plan* fplan, mars_search_plan* wplan, const mars_options* o,
-                          bool* usable) {
+                          bool alone, bool* usable) {
     *usable = false;
     const bool residual = fplan->params.has_lambda && o->allowed_modes[3];
-    if (plan_walk_on_host() || (!residual && fplan->total < kHostWalkNodes)) return MARS_OK;
+    if (plan_walk_on_host() || (!residual && (!alone || fplan->total < kHostWalkNodes)))
+        return MARS_OK;
     bool f = false, w = true;
     if (int e = plan_walk_setup(fplan, &f)) return e;
     if (wplan) {
