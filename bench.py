@@ -51,15 +51,15 @@ WORKLOAD = ("exhaustive search of every RD quadtree node of a 512x512 synthetic 
 # Figures that only ncu measures (bench.py cannot run under a profiler), copied from the
 # committed captures named beside them; re-captured whenever the kernel changes.
 # DRAM bytes (read + write) per launch of the dominant search kernel, s=4 level.
-NCU_SOURCE = "profiles/corr_tc_s4_512x512_ncu.md"
-NCU_TRAFFIC = {4: 21_360_000}
-# DRAM bytes (read + write) of one all-levels correlation launch (corr_tc_all_kernel, every
-# level of one 512x512 plane): profiles/corr_tc_all_512x512_ncu.md.
-NCU_ALL_SOURCE = "profiles/corr_tc_all_512x512_ncu.md"
-NCU_ALL_TRAFFIC = 42_626_816 + 299_264
+NCU_SOURCE = "profiles/corr_unit_all_512x512_ncu.md"
+NCU_TRAFFIC = {4: 11_900_160 + 4_096}
+# DRAM bytes (read + write) of the two all-levels correlation launches (corr_tc_all_kernel and
+# corr_unit_all_kernel, every level of one 512x512 plane): the same capture.
+NCU_ALL_SOURCE = NCU_SOURCE
+NCU_ALL_TRAFFIC = 10_899_712 + 33_518_848 + 44_544
 # Thread instructions per candidate fit of the correlation kernel's level (warp
 # instructions x 32 / fits, same capture): the issue cost behind the epilogue roofline.
-NCU_INSTR_PER_FIT = {4: 0.8684e9 * 32 / 8.52e9, 8: 0.3886e9 * 32 / 2.0e9}
+NCU_INSTR_PER_FIT = {4: 0.5203e9 * 32 / 8.52e9, 8: 0.1445e9 * 32 / 2.0e9}
 # DRAM bytes of one decode iteration, by plane side (profiles/decode_cell_4096x4096_ncu.md;
 # profiles/decode_sorted_16384x16384_ncu.md: dram__bytes.sum.per_second x
 # gpu__time_duration.sum of the gather and the place launch of one iteration).
@@ -896,7 +896,8 @@ def run_gpu(args):
                       "traffic_source": f"ncu ({NCU_SOURCE})", "ops_per_launch": ops,
                       "launch_ms": 1e3 * t_launch}
     if kernel_timed and t_kernel > 0:
-        roof_kernel = "corr_tc_all_kernel: every tensor-core level of the step, one launch"
+        roof_kernel = ("corr_tc_all_kernel and corr_unit_all_kernel: every tensor-core level of "
+                       "the step, two launches side by side")
         roof_ops = 2.0 * sum(macs_of_level(s) for s in SIZES)
         roof_ms = 1e3 * t_kernel / args.steps
         roof_traffic, roof_src = NCU_ALL_TRAFFIC, NCU_ALL_SOURCE
