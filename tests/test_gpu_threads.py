@@ -158,3 +158,29 @@ def test_contexts_come_and_go_beside_each_other():
             assert all(x == w for x in g)
         for ctx in ctxs:
             ctx.close()
+
+
+@pytest.mark.parametrize("lam,modes", [(None, (1, 0, 1, 0)), (200.0, (1, 0, 1, 0)),
+                                       (200.0, (1, 1, 1, 1))])
+def test_fisher_encodes_beside_each_other(lam, modes):
+    # 4,032 nodes: alone the walks run on the device, beside others without residuals on the host.
+    params = mb.make_params(min_size=4, max_size=16, shift=4, lam=lam)
+    images = [synthetic.gray(256, 192, seed) for seed in range(3)]
+
+    def encode(ctx, img):
+        _, leaves, levels, count = ctx.encode(img, params, allowed_modes=modes, method="fisher")
+        return leaves.tobytes(), levels.tobytes(), count.search_evals, count.warmup_evals
+
+    with mb.Context(0) as ctx:
+        want = [encode(ctx, img) for img in images]
+        again = [encode(ctx, img) for img in images]
+        assert again == want
+        got = _side_by_side([lambda i=i: encode(ctx, i) for i in images], 8)
+        for w, g in zip(want, got):
+            assert all(x == w for x in g)
+    ctxs = [mb.Context(0) for _ in images]
+    got = _side_by_side([lambda c=c, i=i: encode(c, i) for c, i in zip(ctxs, images)], 8)
+    for w, g in zip(want, got):
+        assert all(x == w for x in g)
+    for ctx in ctxs:
+        ctx.close()
